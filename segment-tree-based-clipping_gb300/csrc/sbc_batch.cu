@@ -303,6 +303,7 @@ struct PairResult {
 // order keys (okey).
 __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, int nc,
                                     const Caps& cp, PairWork& w, int lane) {
+  WarpGroup g;
   const int E = nb + nc, n2 = 2 * E;
   // ---- A1 edges; the x range on order keys (ties: the earlier vertex)
   long long kmin = LLONG_MAX, kmax = LLONG_MIN;
@@ -398,7 +399,7 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
     if (w.kes[i] == w.kee[i]) w.vl[i] = 1;
   }
   __syncwarp();
-  warp_excl_scan(w.vl, E + 1);
+  group_scan(g, w.vl, E + 1);
   __syncwarp();
   for (int i = lane; i < E; i += 32)
     if (w.vl[i] != w.vl[i + 1]) w.vloc[w.vl[i]] = i;
@@ -424,7 +425,7 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
   }
   if (lane == 0) w.eflag[n2 - 1] = 0;
   __syncwarp();
-  const int count = warp_excl_scan(w.eflag, n2);
+  const int count = group_scan(g, w.eflag, n2);
   __syncwarp();
   if (count < 1) return PS_UNDEF;
   double* ea = w.ea;
@@ -1257,20 +1258,20 @@ struct PipSmall {
     const int v = runIds[lo - 1];
     return u + 1 <= P.rv0[v] + P.run[v];
   }
-  __device__ int operator()(SerialArgs& a, int root, double rx, double ry) const {
-    const Pool& P = a.P;
-    const int lane = threadIdx.x & 31;
+  template <class G>
+  __device__ int operator()(G& g, const Pool& P, double rx, double ry) const {
+    const int lane = g.rank();
     int part = 0;
-    for (int v = lane; v < P.n; v += 32) {
+    for (int v = lane; v < P.n; v += G::N) {
       const int nx = P.next[v];
       part += pip_step(last_x(P, v), last_y(P, v), P.x[nx], P.y[nx], rx, ry);
     }
-    for (int u = lane; u < nb; u += 32) {
+    for (int u = lane; u < nb; u += G::N) {
       const int u2 = u + 1 == nb ? 0 : u + 1;
       const int st = pip_step(b[2 * u], b[2 * u + 1], b[2 * u2], b[2 * u2 + 1], rx, ry);
       if (st && internal(P, u)) part += st;
     }
-    return (__reduce_add_sync(kFullMask, part) % 2) != 0;
+    return (g.sum(part) % 2) != 0;
   }
 };
 
@@ -1401,7 +1402,8 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw(ClipArgs A) {
   __syncwarp();
   PwWork pw = w.pw;
   PwMid mid;
-  const int st = pw_clip_head(A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.phit,
+  WarpGroup g;
+  const int st = pw_clip_head(g, A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.phit,
                               pw_caps(nb, nc, K, 1), pw, &mid);
   if (st == PS_UNDEF) {
     if (lane == 0) batch_fail(A, p, w, PS_UNDEF, 0);
@@ -1431,9 +1433,10 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw2(ClipArgs A) {
   PwWork pw = w.pw;
   PwMid mid = pw_mid_load(pw.mid);
   int nr = 0, nv = 0;
-  int st = pw_clip_lists(b, nb, c, nc, pc, pw, &mid);
+  WarpGroup g;
+  int st = pw_clip_lists(g, b, nb, c, nc, pc, pw, &mid);
   if (st == PS_OK)
-    st = pw_clip_trace(b, nb, c, nc, pc, pw, mid, PipSmall{b, nb, nullptr, 0}, A.unite, &nr, &nv);
+    st = pw_clip_trace(g, b, nb, c, nc, pc, pw, mid, PipSmall{b, nb, nullptr, 0}, A.unite, &nr, &nv);
   if (st != PS_OK && st != PS_UNDEF) {
     if (lane == 0) w.state[3] = 1;  // the thread back end takes the pair
     return;

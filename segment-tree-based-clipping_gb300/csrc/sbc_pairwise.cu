@@ -63,6 +63,14 @@ constexpr int kPwMaxCells = 1 << 14;  // an overlay edge box over more cells: pa
 constexpr int kPwLongCells = 64;      // base edges over more cells per axis skip the grid
 constexpr int kPwPrepThreads = 256;
 constexpr int kPwPairBlock = 64;
+// A pair of at least this cost (8 * records + overlay vertices) gets a block
+// of kPwWideBlock threads instead of a warp.  A warp's time is about 1.2 us
+// per 10 records, a block's about a sixth of that plus its barriers, so the
+// line is where the kernel's tail stops being a warp's: a job of 237 overlays
+// took 7.6 ms with the line at 2,048 records, 5.9 at 1,024 and below; 34
+// overlays 5.2, 4.0 (1,024) and 3.4 (512); 3,466 overlays 8.2, 6.3 and 5.5.
+constexpr int kPwWideBlock = 256;
+constexpr long long kPwWideCost = 8 * 512;
 
 enum { PW_FAST = 0, PW_FALLBACK = 1, PW_INPUT = 2 };
 
@@ -651,9 +659,9 @@ __global__ void k_pw_split(int n, const PwHit* __restrict__ h, int* __restrict__
 // pointInPoly against the base side of a pair whose list has run nodes: the
 // steps of the edges between nodes, plus those of the base edges inside run
 // nodes, which come from the grid row holding ry (each edge counted in the
-// first cell of its box in that row).  Called by all 32 lanes of a warp with
+// first cell of its box in that row).  Called by all threads of a group with
 // the same arguments: the row's cells and the long edges are split over the
-// lanes and the steps summed (the winding number is order-free).
+// threads and the steps summed (the winding number is order-free).
 struct PwPip {
   const double* b;
   int nb;
@@ -676,19 +684,19 @@ struct PwPip {
     const int v = runIds[lo - 1];
     return u + 1 <= P.rv0[v] + P.run[v];
   }
-  __device__ int operator()(SerialArgs& a, int root, double rx, double ry) const {
-    const Pool& P = a.P;
-    const int lane = threadIdx.x & 31;
+  template <class G>
+  __device__ int operator()(G& grp, const Pool& P, double rx, double ry) const {
+    const int lane = grp.rank();
     // the edges between list nodes: every pool node is on the list
     int part = 0;
-    for (int v = lane; v < P.n; v += 32) {
+    for (int v = lane; v < P.n; v += G::N) {
       const int nx = P.next[v];
       part += pip_step(last_x(P, v), last_y(P, v), P.x[nx], P.y[nx], rx, ry);
     }
     const int cy = pw_celly(g, __double2float_rd(ry));
     // the step first: most edges of the row do not cross the ray, and only
     // those that do need the cell and run-membership tests
-    for (int cx = lane; cx < g.gx; cx += 32) {
+    for (int cx = lane; cx < g.gx; cx += G::N) {
       const int cell = cy * g.gx + cx;
       for (int k = gstart[cell]; k < gstart[cell + 1]; ++k) {
         const int u = gent[k];
@@ -696,12 +704,12 @@ struct PwPip {
         if (st && pw_cellx(g, fbox[u].x) == cx && internal(P, u)) part += st;
       }
     }
-    for (int k = lane; k < nlong; k += 32) {
+    for (int k = lane; k < nlong; k += G::N) {
       const int u = lng[k];
       const int st = pip_step(b[2 * u], b[2 * u + 1], b[2 * u + 2], b[2 * u + 3], rx, ry);
       if (st && internal(P, u)) part += st;
     }
-    return (__reduce_add_sync(kFullMask, part) % 2) != 0;
+    return (grp.sum(part) % 2) != 0;
   }
 };
 
@@ -715,7 +723,7 @@ struct PwPairArgs {
   const int* hstart;
   const PwHit* hits;
   const int* pass_of;  // null: every fast pair, pass 0
-  const int* order;    // pairs by decreasing expected work (warp w takes order[w])
+  const int* order;    // pairs by decreasing expected work
   unsigned char* arena;
   const long long* aoff;
   int* status;  // per pair: PS_* code
@@ -724,14 +732,6 @@ struct PwPairArgs {
   int* nverts;
   PwPip pip;
 };
-
-__device__ int pw_clip_pair(const PwPairArgs& A, int p, const PwCaps& cp, PwWork& w, int* nrings_out,
-                            int* nverts_out) {
-  const long long o = A.coff[p];
-  const int nc = (int)(A.coff[p + 1] - o);
-  return pw_clip_core(A.b, A.nb, A.cxy + 2 * o, nc, A.hits + A.hstart[p], cp, w, A.pip, A.unite,
-                      nrings_out, nverts_out);
-}
 
 __global__ void k_pw_sizes(int nov, const long long* __restrict__ coff, int nb,
                            const PwPair* __restrict__ pp, const int* __restrict__ pairK,
@@ -747,6 +747,30 @@ __global__ void k_pw_sizes(int nov, const long long* __restrict__ coff, int nb,
   bytes[p] = run ? (long long)pw_arena_bytes(nb, (int)(coff[p + 1] - coff[p]), pairK[p], pass) : 0;
 }
 
+// entry wi of the queue by the calling group
+template <class G>
+__device__ void pw_queue_pair(G& g, const PwPairArgs& A, const int* pairK, int wi) {
+  const int p = A.order[wi];
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  if (pass < 0) return;
+  if (A.pp[p].mode != PW_FAST) {
+    A.status[p] = A.pp[p].mode == PW_INPUT ? PS_UNDEF + 100 : PS_FALLBACK;
+    A.nrings[p] = A.nverts[p] = 0;
+    return;
+  }
+  const long long o = A.coff[p];
+  const int nc = (int)(A.coff[p + 1] - o);
+  const PwCaps cp = pw_caps(A.nb, nc, pairK[p], pass);
+  Carver cv{A.arena + A.aoff[p], 0};
+  PwWork w = pw_carve(cv, cp);
+  int nr = 0, nv = 0;
+  const int st = pw_clip_core(g, A.b, A.nb, A.cxy + 2 * o, nc, A.hits + A.hstart[p], cp, w, A.pip,
+                              A.unite, &nr, &nv);
+  A.status[p] = st;
+  A.nrings[p] = st == PS_OK ? nr : 0;
+  A.nverts[p] = st == PS_OK ? nv : 0;
+}
+
 // Persistent work queue, one pair per warp at a time (32 pairs sharing a warp
 // would take turns through diverging paths; one warp shares a pair's
 // data-parallel steps among its lanes instead).  The queue hands out pairs by
@@ -754,28 +778,33 @@ __global__ void k_pw_sizes(int nov, const long long* __restrict__ coff, int nb,
 // empty.
 __global__ void __launch_bounds__(kPwPairBlock)
 k_pw_pairs(PwPairArgs A, const int* __restrict__ pairK, int* __restrict__ queue) {
+  WarpGroup g;
   for (;;) {
     int wi = 0;
     if ((threadIdx.x & 31) == 0) wi = atomicAdd(queue, 1);
     wi = __shfl_sync(kFullMask, wi, 0);
     if (wi >= A.nov) return;
-    const int p = A.order[wi];
-    const int pass = A.pass_of ? A.pass_of[p] : 0;
-    if (pass < 0) continue;
-    if (A.pp[p].mode != PW_FAST) {
-      A.status[p] = A.pp[p].mode == PW_INPUT ? PS_UNDEF + 100 : PS_FALLBACK;
-      A.nrings[p] = A.nverts[p] = 0;
-      continue;
-    }
-    const int nc = (int)(A.coff[p + 1] - A.coff[p]);
-    const PwCaps cp = pw_caps(A.nb, nc, pairK[p], pass);
-    Carver cv{A.arena + A.aoff[p], 0};
-    PwWork w = pw_carve(cv, cp);
-    int nr = 0, nv = 0;
-    const int st = pw_clip_pair(A, p, cp, w, &nr, &nv);
-    A.status[p] = st;
-    A.nrings[p] = st == PS_OK ? nr : 0;
-    A.nverts[p] = st == PS_OK ? nv : 0;
+    pw_queue_pair(g, A, pairK, wi);
+  }
+}
+
+// The same with a block per pair, for the head of the queue.  Bound by the
+// latency of its steps (dependent loads between barriers), not by bytes: the
+// largest pairs used to be the whole kernel's tail on one warp each (4,000
+// overlays of a 200,000-vertex base: 15.3 ms, and 40 pairs beside it on the
+// workers; here 5.2 ms with those 40 among them).
+__global__ void __launch_bounds__(kPwWideBlock)
+k_pw_pairs_wide(PwPairArgs A, const int* __restrict__ pairK, int* __restrict__ queue) {
+  using G = BlockGroup<kPwWideBlock>;
+  __shared__ G::Shared sh;
+  G g(&sh);
+  for (;;) {
+    int wi = 0;
+    if (threadIdx.x == 0) wi = atomicAdd(queue, 1);
+    wi = g.same(wi);
+    if (wi >= A.nov) return;
+    pw_queue_pair(g, A, pairK, wi);
+    g.sync();
   }
 }
 
@@ -840,6 +869,15 @@ unsigned PairwiseRunner::pair_grid(int nov, bool reserve) {
   pair_blocks_ = (unsigned)std::max(1, sms * slots);
   const unsigned need = grid_for(32LL * nov, kPwPairBlock);
   return need < pair_blocks_ ? need : pair_blocks_;
+}
+
+// a block per wide pair, up to every block slot of every SM
+unsigned PairwiseRunner::wide_grid(int n) {
+  int dev = 0, sms = 0, per_sm = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pw_pairs_wide, kPwWideBlock, 0);
+  return (unsigned)std::min(n, std::max(1, sms * per_sm));
 }
 
 // Time the job under a few settings and keep the fastest (results depend on
@@ -1206,7 +1244,8 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   }
   cudaMemcpyAsync(pass, hpass.data(), sizeof(int) * nov, cudaMemcpyHostToDevice, st);
   // longest first: the warps that start first take the pairs with the most
-  // records and vertices
+  // records and vertices, and the first `wide` of them get a block each
+  int wide = 0;
   {
     std::vector<long long> cost(nov);
     order_h.resize(nov);
@@ -1216,12 +1255,13 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     }
     std::stable_sort(order_h.begin(), order_h.end(),
                      [&](int a, int b) { return cost[a] > cost[b]; });
+    while (wide < nov && cost[order_h[wide]] >= kPwWideCost) ++wide;
   }
   int* order = (int*)pool.get("pw_order", sizeof(int) * (nov + 1));
   int* queue = (int*)pool.get("pw_queue", 256);
   if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise)");
   cudaMemcpyAsync(order, order_h.data(), sizeof(int) * nov, cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(queue, 0, 2 * sizeof(int), st);
+  cudaMemsetAsync(queue, 0, 4 * sizeof(int), st);
   PwPip pip{d_bxy, nb, g, gstart, gent, lng, (int)hlong, fbox, nullptr, 0};
   {
     ::sbc::KProbe kp_("k_pw_sizes", st);
@@ -1242,11 +1282,23 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
                 status, pl_.unite ? 1 : 0, nrings, nverts, pip};
   cudaEventRecord(ev_[0], st);
   cudaStreamWaitEvent(st2_, ev_[0], 0);
-  {
-    // coordinates and records in; rings out
-    ::sbc::KProbe kp_("k_pw_pairs", st2_, 16.0 * totalC + 40.0 * (double)nh);
-    k_pw_pairs<<<pair_grid(nov, big_pairs > 0), kPwPairBlock, 0, st2_>>>(pa, pairK, queue);
-  }
+  // the two queues side by side
+  auto clip_pairs = [&](cudaStream_t sw, cudaStream_t sn, int* q, bool reserve) {
+    PwPairArgs part = pa;
+    part.nov = wide;
+    if (wide > 0) {
+      ::sbc::KProbe kp_("k_pw_pairs_wide", sw);
+      k_pw_pairs_wide<<<wide_grid(wide), kPwWideBlock, 0, sw>>>(part, pairK, q);
+    }
+    part.nov = nov - wide;
+    part.order = order + wide;
+    if (nov > wide) {
+      // coordinates and records in; rings out
+      ::sbc::KProbe kp_("k_pw_pairs", sn, 16.0 * totalC + 40.0 * (double)nh);
+      k_pw_pairs<<<pair_grid(nov - wide, reserve), kPwPairBlock, 0, sn>>>(part, pairK, q + 1);
+    }
+  };
+  clip_pairs(st2_, st, queue, big_pairs > 0);
   cudaEventRecord(ev_[1], st2_);
   struct Stash {
     std::vector<int> off;
@@ -1400,10 +1452,7 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise arena)");
     pa.arena = arena1;
     pa.aoff = aoff1;
-    {
-      ::sbc::KProbe kp_("k_pw_pairs", st);
-      k_pw_pairs<<<pair_grid(nov, false), kPwPairBlock, 0, st>>>(pa, pairK, queue + 1);
-    }
+    clip_pairs(st, st, queue + 2, false);
     cudaMemcpyAsync(hst.data(), status, sizeof(int) * nov, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise clip");
   }

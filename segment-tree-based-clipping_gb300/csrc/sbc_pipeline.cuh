@@ -419,7 +419,13 @@ class PairwiseRunner {
   // diagnostics of the last run
   int fallback_pairs = 0;           // pairs clipped by the whole pair pipeline
   int big_pairs = 0;                // pairs whose records went to its rows A9-A18
-  int big_k = 8192;                 // records from which a pair counts as big
+  // Records from which a pair's rows A9-A18 run through the pair pipeline on
+  // a worker stream instead of one block of k_pw_pairs_wide.  A block takes
+  // about 2.5 ms for 30,000 records and a hundred blocks run at once, where
+  // the eight workers cleared a pair in about 0.35 ms: 10,000 overlays of a
+  // 200,000-vertex base (123 pairs of 8,192 to 30,000 records) took 57.0 ms
+  // split at 8,192, 37.6 at 16,384 and 31.9 at 32,768.
+  int big_k = 32768;
   int big_workers = 8;              // host threads, each with a pipeline and a stream, for big pairs
   int pair_reserve = 1;             // block slots per SM the per-pair kernel leaves to big pairs
   long long hits = 0, tested = 0, grid_cells = 0;
@@ -435,6 +441,7 @@ class PairwiseRunner {
   std::vector<int> order_h;
   unsigned pair_blocks_ = 0;
   unsigned pair_grid(int nov, bool reserve);
+  unsigned wide_grid(int n);
   // the last run, for area and backward
   int last_nb_ = 0;
   long long last_totalC_ = 0, last_nh_ = 0;

@@ -1,14 +1,16 @@
 // sbc_pwpair.cuh -- one pair's rows A9-A18 (src/clip.cpp:368-695,
-// foster/polyclip.h:337-787) by one warp, its lanes sharing the per-record,
-// per-run and per-slot steps: the overlay's merged arrays in full, the base's
-// only where intersections are (a stretch of plain base vertices is one run
-// node of the linked list, sbc_serial.cuh).  Used by the one-base-many-
+// foster/polyclip.h:337-787) by one group of threads (sbc_group.cuh: a warp,
+// or a block for a large pair), sharing the per-record, per-run and per-slot
+// steps: the overlay's merged arrays in full, the base's only where
+// intersections are (a stretch of plain base vertices is one run node of the
+// linked list, sbc_serial.cuh).  Used by the one-base-many-
 // overlays engine (sbc_pairwise.cu) and by the batched small-pair engine
 // (sbc_batch.cu); each supplies the pointInPoly functor of the base side.
 #pragma once
 
 #include <climits>
 
+#include "sbc_group.cuh"
 #include "sbc_pairops.cuh"
 #include "sbc_serial.cuh"
 
@@ -144,30 +146,18 @@ __host__ __device__ __forceinline__ size_t pw_arena_bytes(int nb, int nc, int K,
   return (cv.off + 255) & ~(size_t)255;
 }
 
-// ---------------------------------------------------------------- warp helpers
-// first i in [0, n) with pred(i), or -1; called by all 32 lanes
-template <class Pred>
-__device__ int warp_first(int n, Pred pred) {
-  const int lane = threadIdx.x & 31;
-  for (int i0 = 0; i0 < n; i0 += 32) {
-    const int i = i0 + lane;
-    const unsigned m = __ballot_sync(kFullMask, i < n && pred(i));
-    if (m) return i0 + __ffs(m) - 1;
-  }
-  return -1;
-}
-
+// ---------------------------------------------------------------- group helpers
 // pointInPoly against a pool every node of which is on its one list (the
 // pairwise back end never unlinks a list node): the winding steps of the
-// edges v -> next[v], summed over the lanes
-__device__ int warp_ppip(const Pool& p, double rx, double ry) {
-  const int lane = threadIdx.x & 31;
+// edges v -> next[v], summed over the group
+template <class G>
+__device__ int group_ppip(G& g, const Pool& p, double rx, double ry) {
   int part = 0;
-  for (int v = lane; v < p.n; v += 32) {
+  for (int v = g.rank(); v < p.n; v += G::N) {
     const int nx = p.next[v];
     part += pip_step(last_x(p, v), last_y(p, v), p.x[nx], p.y[nx], rx, ry);
   }
-  return __reduce_add_sync(kFullMask, part);
+  return g.sum(part);
 }
 
 // rcopy of a plain pool whose list is its nodes in index order: ring node
@@ -230,12 +220,13 @@ __device__ __forceinline__ unsigned walk_compose(unsigned g, unsigned f) {
 // never unlinked, so every pool node is on its list throughout.
 template <class Pip>
 __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
-  const int lane = threadIdx.x & 31;
+  WarpGroup g;
+  const int lane = g.rank();
   Pool& P = a.P;
   Pool& Q = a.Q;
   // (2) chains: rare (overlapping edges), so the serial pass runs only when
   // a chain start exists
-  if (warp_first(P.n, [&](int v) {
+  if (g.first(P.n, [&](int v) {
         return P.isect[v] && (P.label[v] == L_LEFT_ON || P.label[v] == L_RIGHT_ON);
       }) >= 0) {
     int V = 0;
@@ -264,8 +255,8 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
     __syncwarp();
   }
   auto pip_of = [&](int s, double rx, double ry) -> int {
-    if (s == 0) return pipP(a, 0, rx, ry);
-    return (warp_ppip(Q, rx, ry) % 2) != 0;
+    if (s == 0) return pipP(g, P, rx, ry);
+    return (group_ppip(g, Q, rx, ry) % 2) != 0;
   };
   // (3.5) sides without crossings
   int noIsect[2] = {0, 0}, ident[2] = {0, 0};
@@ -273,7 +264,7 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
     Pool& p = side(a, s);
     Pool& o = side(a, 1 - s);
     const int n = p.n;
-    const bool cross = warp_first(n, [&](int v) {
+    const bool cross = g.first(n, [&](int v) {
                          if (!p.isect[v]) return false;
                          const int l = p.label[v];
                          // noCrossingVertex(UNION), foster/polygon.h:465-475
@@ -282,17 +273,17 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
                        }) >= 0;
     if (cross) continue;
     noIsect[s] = 1;
-    if (warp_first(n, [&](int v) { return p.label[v] != L_ON_ON; }) < 0) {
+    if (g.first(n, [&](int v) { return p.label[v] != L_ON_ON; }) < 0) {
       ident[s] = 1;
       continue;
     }
     double px, py;
-    const int f = warp_first(n, [&](int v) { return !p.isect[v]; });
+    const int f = g.first(n, [&](int v) { return !p.isect[v]; });
     if (f >= 0) {
       px = p.x[f];
       py = p.y[f];
     } else {
-      const int V = warp_first(n, [&](int v) {
+      const int V = g.first(n, [&](int v) {
         const int nbV = p.nb[v], nbN = p.nb[p.next[v]];
         return nbV < 0 || (nbN != o.prev[nbV] && nbN != o.next[nbV]);
       });
@@ -307,7 +298,7 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
   }
   if (ident[0] && ident[1]) {
     const int target = P.nb[0];
-    if (warp_first(Q.n, [&](int v) { return v == target; }) >= 0 && rcopy(a, P, 0)) return 3;
+    if (g.first(Q.n, [&](int v) { return v == target; }) >= 0 && rcopy(a, P, 0)) return 3;
   }
   __syncwarp();
   // (4) entry/exit walk from a non-intersection vertex of each side
@@ -318,10 +309,10 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
     unsigned char* split = s == 0 ? a.splitP : a.splitQ;
     unsigned char* cross = s == 0 ? a.crossP : a.crossQ;
     const int n0 = p.n;  // this side's list is still its pool in index order
-    int V = warp_first(n0, [&](int v) { return !p.isect[v]; });
+    int V = g.first(n0, [&](int v) { return !p.isect[v]; });
     int start = V;
     if (V < 0) {
-      const int U = warp_first(n0, [&](int v) {
+      const int U = g.first(n0, [&](int v) {
         const int nbV = p.nb[v], nbN = p.nb[p.next[v]];
         return nbV < 0 || (nbN != o.prev[nbV] && nbN != o.next[nbV]);
       });
@@ -373,7 +364,7 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
   }
   // (5) split pairs: rare (bouncing vertices), serial when present
   const int nP0 = P.n;
-  if (warp_first(nP0, [&](int v) { return a.splitP[v] != 0; }) >= 0) {
+  if (g.first(nP0, [&](int v) { return a.splitP[v] != 0; }) >= 0) {
     for (int IP = 0; IP < nP0; ++IP) {
       if (!a.splitP[IP]) continue;
       int IQ = P.nb[IP];
@@ -507,6 +498,249 @@ __device__ int pw_label_trace(SerialArgs& a, const Pip& pipP) {
   return 0;
 }
 
+// The same for a block, where every intersection node of both lists is a
+// plain crossing (no overlaps, touches or delayed crossings) linked one to
+// one with the other list's: -1, with nothing changed, where it is not so.
+//
+// The entry/exit status then alternates along each list, so an intersection's
+// neighbour in the direction that its status gives is its partner, and it is
+// that one's: the legs along P pair the crossings up, and so do the legs along
+// Q.  A ring of the serial walk (createResult2, polyclip.h:717-759) is an
+// alternating cycle of the two pairings, started at its crossing that comes
+// first on P, along P.  From crossing k two legs lead to S(k) (along P, then
+// along Q); a cycle's crossings fall into two orbits of S, one for each sense.
+// Pointer doubling finds each orbit's least crossing and the vertices from
+// each crossing to it; the sense whose orbit holds the cycle's least crossing
+// is the ring's.  Ring order and offsets are a scan over the first crossings,
+// and every leg is written to its own place.  Serial on one warp this took a
+// dependent load per list node (a pair of 2,048-vertex stars has 17,000
+// crossings); here it is about log2(longest ring) rounds.
+template <class G, class Pip>
+__device__ int pw_label_trace_block(G& g, SerialArgs& a, const Pip& pipP, PwWork& w,
+                                    const PwCaps& cp) {
+  const int lane = g.rank();
+  constexpr int N = G::N;
+  Pool& P = a.P;
+  Pool& Q = a.Q;
+  const int nP = P.n, nQ = Q.n;
+  // ---- plain crossings only, linked one to one
+  bool odd = false;
+  int cntP = 0, cntQ = 0;
+  for (int v = lane; v < nP && !odd; v += N) {
+    if (!P.isect[v]) continue;
+    ++cntP;
+    const int q = P.nb[v];
+    if (P.label[v] != L_CROSSING || q < 0 || !Q.isect[q] || Q.nb[q] != v) odd = true;
+  }
+  for (int v = lane; v < nQ && !odd; v += N) {
+    if (!Q.isect[v]) continue;
+    ++cntQ;
+    const int p = Q.nb[v];
+    if (Q.label[v] != L_CROSSING || p < 0 || !P.isect[p] || P.nb[p] != v) odd = true;
+  }
+  if (g.any(odd)) return -1;
+  const int n = g.sum(cntP);
+  if (n != g.sum(cntQ) || n == 0 || (n & 1) || n > cp.K) return -1;
+  const int VP = g.first(nP, [&](int v) { return !P.isect[v]; });
+  const int VQ = g.first(nQ, [&](int v) { return !Q.isect[v]; });
+  if (VP < 0 || VQ < 0) return -1;
+  // ---- crossings in list order: node of crossing k on P, of crossing m on Q;
+  // each node's number goes into its entry/exit word
+  int* nodeP = w.re_e;
+  int* nodeQ = w.re_s;
+  auto number = [&](Pool& p, int* node, int from, int* c0) {
+    int carry = 0, below = 0;
+    for (int i0 = 0; i0 < p.n; i0 += N) {
+      const int v = i0 + lane;
+      const bool x = v < p.n && p.isect[v];
+      int tot;
+      const int k = carry + g.before(x, &tot);
+      if (x) {
+        node[k] = v;
+        p.enex[v] = k;
+        if (v < from) ++below;
+      }
+      carry += tot;
+    }
+    *c0 = g.sum(below);
+  };
+  int cP, cQ;  // crossings before the start node of the entry/exit walk
+  number(P, nodeP, VP, &cP);
+  number(Q, nodeQ, VQ, &cQ);
+  // ---- (4) status: entry first when the start lies outside the other polygon
+  const int sP = (group_ppip(g, Q, P.x[VP], P.y[VP]) % 2) != 0 ? 0 : 1;
+  const int sQ = pipP(g, P, Q.x[VQ], Q.y[VQ]) ? 0 : 1;
+  auto forward = [&](int k, int c0, int s0) {  // leaves along its list forwards
+    const int entry = s0 ^ ((k - c0) & 1);
+    return (entry != 0) != (a.unite != 0);
+  };
+  // ---- vertices before each P node (a run node holds several)
+  int* pre = P.label;
+  int TP = 0;
+  for (int i0 = 0; i0 < nP; i0 += N) {
+    const int v = i0 + lane;
+    int tot;
+    const int e = g.excl(v < nP ? (is_run(P, v) ? P.run[v] + 1 : 1) : 0, &tot);
+    if (v < nP) pre[v] = TP + e;
+    TP += tot;
+  }
+  g.sync();
+  auto partner = [&](int k, bool fwd) { return fwd ? (k + 1 == n ? 0 : k + 1) : (k == 0 ? n - 1 : k - 1); };
+  // the legs from crossing k: the vertices after it up to and with its partner
+  struct Legs {
+    int kp, m1, m2, lenP, lenQ;
+    bool fP, fQ;
+  };
+  auto legs = [&](int k) {
+    Legs l;
+    l.fP = forward(k, cP, sP);
+    l.kp = partner(k, l.fP);
+    const int u = nodeP[k], v = nodeP[l.kp];
+    l.lenP = l.fP ? pre[v] - pre[u] : pre[u] - pre[v];  // crossings are single vertices
+    if (l.lenP <= 0) l.lenP += TP;
+    const int q1 = P.nb[v];
+    l.m1 = Q.enex[q1];
+    l.fQ = forward(l.m1, cQ, sQ);
+    l.m2 = partner(l.m1, l.fQ);
+    const int q2 = nodeQ[l.m2];
+    l.lenQ = l.fQ ? q2 - q1 : q1 - q2;
+    if (l.lenQ <= 0) l.lenQ += nQ;
+    return l;
+  };
+  // ---- orbits of S: (next, least crossing of the window, vertices to it,
+  // vertices of the window); a round without a change has seen every orbit
+  int4* A = (int4*)w.sscr;
+  int4* B = (int4*)w.spx;
+  for (int k = lane; k < n; k += N) {
+    const Legs l = legs(k);
+    A[k] = make_int4(P.enex[Q.nb[nodeQ[l.m2]]], k, 0, l.lenP + l.lenQ);
+  }
+  g.sync();
+  for (;;) {
+    bool changed = false;
+    for (int k = lane; k < n; k += N) {
+      int4 x = A[k];
+      const int4 y = A[x.x];
+      if (y.y < x.y) {
+        x.y = y.y;
+        x.z = (int)((unsigned)x.w + (unsigned)y.z);
+        changed = true;
+      }
+      x.x = y.x;
+      x.w = (int)((unsigned)x.w + (unsigned)y.w);
+      B[k] = x;
+    }
+    int4* t = A;
+    A = B;
+    B = t;
+    if (!g.any(changed)) break;
+  }
+  // ---- rings in the order of their first crossings
+  int* off = w.re_nd;  // of a ring, at its first crossing
+  int* len = w.re_pre;
+  int rings = 0, verts = 0;
+  for (int i0 = 0; i0 < n; i0 += N) {
+    const int k = i0 + lane;
+    int m = 0;
+    if (k < n && A[k].y == k) {
+      const Legs l = legs(k);
+      if (k < A[l.kp].y) m = l.lenP + l.lenQ + A[P.enex[Q.nb[nodeQ[l.m2]]]].z;
+    }
+    int tr, tv;
+    const int r = rings + g.before(m > 0, &tr);
+    const int o = verts + g.excl(m, &tv);
+    if (m > 0 && r < a.rcap) {
+      off[k] = o;
+      len[k] = m;
+      a.rroot[r] = o;
+    }
+    rings += tr;
+    verts += tv;
+  }
+  if (rings > a.rcap) return 3;
+  if (verts > a.R.cap) {
+    a.rfull = 1;
+    return 3;
+  }
+  if (lane == 0) {
+    *a.nrings = rings;
+    g.s->count = 0;
+  }
+  g.sync();
+  // ---- the legs, each to its place; long stretches are listed and copied by
+  // whole warps (a block for the longest)
+  Pool& R = a.R;
+  int4* tasks = B;  // {kind, source, vertices, place}; kind: bit 0 backwards, bit 1 from Q
+  auto piece = [&](int kind, int src, int m, int at, int t0, int step) {
+    for (int t = t0; t < m; t += step) {
+      if (kind & 2) {
+        int v = (kind & 1) ? src - t : src + t;
+        if (v < 0) v += nQ;
+        if (v >= nQ) v -= nQ;
+        R.x[at + t] = Q.x[v];
+        R.y[at + t] = Q.y[v];
+      } else {
+        const int u = (kind & 1) ? src - t : src + t;
+        R.x[at + t] = P.rxy[2 * u];
+        R.y[at + t] = P.rxy[2 * u + 1];
+      }
+    }
+  };
+  constexpr int kShort = 16;
+  auto put = [&](int kind, int src, int m, int at) {
+    if (m > kShort) {
+      const int t = atomicAdd(&g.s->count, 1);
+      if (t < n) {
+        tasks[t] = make_int4(kind, src, m, at);
+        return;
+      }
+    }
+    piece(kind, src, m, at, 0, 1);
+  };
+  for (int k = lane; k < n; k += N) {
+    const Legs l = legs(k);
+    const int s = A[k].y;
+    if (s > A[l.kp].y) continue;  // the other sense
+    int at = off[s] + (s == k ? 0 : len[s] - A[k].z);
+    const int end = nodeP[l.kp];
+    for (int v = nodeP[k]; v != end;) {
+      v = l.fP ? (v + 1 == nP ? 0 : v + 1) : (v == 0 ? nP - 1 : v - 1);
+      if (is_run(P, v)) {
+        const int m = P.run[v] + 1;
+        put(l.fP ? 0 : 1, l.fP ? P.rv0[v] : P.rv0[v] + m - 1, m, at);
+        at += m;
+      } else {
+        R.x[at] = P.x[v];
+        R.y[at] = P.y[v];
+        ++at;
+      }
+    }
+    const int q1 = nodeQ[l.m1];
+    const int q0 = l.fQ ? (q1 + 1 == nQ ? 0 : q1 + 1) : (q1 == 0 ? nQ - 1 : q1 - 1);
+    put(l.fQ ? 2 : 3, q0, l.lenQ, at);
+  }
+  for (int v = lane; v < verts; v += N) {
+    R.next[v] = v + 1;
+    R.prev[v] = v - 1;
+  }
+  g.sync();
+  for (int r = lane; r < rings; r += N) {
+    const int o = a.rroot[r], e = r + 1 < rings ? a.rroot[r + 1] : verts;
+    R.next[e - 1] = o;
+    R.prev[o] = e - 1;
+  }
+  const int nt = min(g.s->count, n);
+  constexpr int kLong = 4096;
+  for (int t = g.warp(); t < nt; t += G::kWarps)
+    if (tasks[t].z <= kLong)
+      piece(tasks[t].x, tasks[t].y, tasks[t].z, tasks[t].w, threadIdx.x & 31, 32);
+  for (int t = 0; t < nt; ++t)
+    if (tasks[t].z > kLong) piece(tasks[t].x, tasks[t].y, tasks[t].z, tasks[t].w, lane, N);
+  R.n = verts;
+  g.sync();
+  return 0;
+}
+
 // global slot s of the base's merged list: its sparse index, or -1 for a
 // plain vertex slot (then *vtx is the vertex)
 // (hint: a run index near the answer; the search is narrowed to runs
@@ -537,76 +771,75 @@ __device__ __forceinline__ int pw_slot(const PwWork& w, int nr, int s, int* vtx,
   return -1;
 }
 
-// exclusive prefix sums of a[0..n) in place by the calling warp (all 32 lanes);
-// returns the total.  Element i is read and written by lane i % 32.
-__device__ int warp_excl_scan(int* a, int n) {
-  const int lane = threadIdx.x & 31;
-  int carry = 0;
-  for (int i0 = 0; i0 < n; i0 += 32) {
-    const int i = i0 + lane;
-    const int x = i < n ? a[i] : 0;
-    int s = x;
-    for (int d = 1; d < 32; d <<= 1) {
-      const int t = __shfl_up_sync(kFullMask, s, d);
-      if (lane >= d) s += t;
-    }
-    if (i < n) a[i] = carry + s - x;
-    carry += __shfl_sync(kFullMask, s, 31);
-  }
-  return carry;
-}
-
-// closes a lane-parallel step: orders its stores before the next step's
-// loads and tells every lane whether any lane failed
-__device__ __forceinline__ bool warp_fail(bool bad) {
-  __syncwarp();
-  return __any_sync(kFullMask, bad);
-}
-
-constexpr int kWarpSortMin = 32;  // runs longer than this are sorted by the whole warp
+constexpr int kWarpSortMin = 32;     // runs longer than this are sorted by a whole warp
+constexpr int kBlockSortMin = 1024;  // and, in a block, above this by the block
 
 // sorts scr[0..n) -- distinct 64-bit values, key(m) for m < n -- ascending,
-// by the whole warp: a bitonic network over the next power of two (padding
-// sorts last)
-template <class Key>
-__device__ void warp_bitonic(int n, unsigned long long* scr, Key key) {
-  const int lane = threadIdx.x & 31;
+// by the group: a bitonic network over the next power of two (padding sorts
+// last)
+template <class G, class Key>
+__device__ void group_sort(G& g, int n, unsigned long long* scr, Key key) {
   const int np = npow2_dev(n);
-  for (int m = lane; m < np; m += 32) scr[m] = m < n ? key(m) : ~0ull;
-  __syncwarp();
-  // each lane takes compare-exchange pairs (m, m + j): every lane works in
-  // every round
-  for (int k = 2; k <= np; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int q = lane; q < (np >> 1); q += 32) {
-        const int m = ((q & ~(j - 1)) << 1) | (q & (j - 1)), l = m | j;
-        const unsigned long long x = scr[m], y = scr[l];
-        if ((x > y) == ((m & k) == 0)) {
-          scr[m] = y;
-          scr[l] = x;
-        }
-      }
-      __syncwarp();
+  for (int m = g.rank(); m < np; m += G::N) scr[m] = m < n ? key(m) : ~0ull;
+  g.sync();
+  group_bitonic(g, np, [&](int m, int l, bool up) {
+    const unsigned long long x = scr[m], y = scr[l];
+    if ((x > y) == up) {
+      scr[m] = y;
+      scr[l] = x;
     }
+  });
 }
 
-// stable order of sorted[s..t) (holding s..t) by alpha mod 1e9, by the whole
-// warp: ties keep position order because the position is the key's low half.
-// False (on every lane) when an alpha is negative.
-__device__ bool warp_alpha_sort(int s, int t, const int* alpha, const int* order, int* sorted,
-                                unsigned long long* scr) {
-  const int lane = threadIdx.x & 31;
+// stable order of sorted[s..t) (holding s..t) by alpha mod 1e9, by the group:
+// ties keep position order because the position is the key's low half.
+// False (on every thread) when an alpha is negative.
+template <class G>
+__device__ bool group_alpha_sort(G& g, int s, int t, const int* alpha, const int* order,
+                                 int* sorted, unsigned long long* scr) {
   bool neg = false;
-  for (int x = s + lane; x < t; x += 32)
+  for (int x = s + g.rank(); x < t; x += G::N)
     if (alpha[order ? order[x] : x] < 0) neg = true;
-  if (warp_fail(neg)) return false;
-  warp_bitonic(t - s, scr, [&](int m) {
+  if (g.any(neg)) return false;
+  group_sort(g, t - s, scr, [&](int m) {
     const int x = s + m;
     return ((unsigned long long)(alpha[order ? order[x] : x] % 1000000000) << 32) | (unsigned)x;
   });
-  for (int m = lane; m < t - s; m += 32) sorted[s + m] = (int)(unsigned)scr[m];
-  __syncwarp();
+  for (int m = g.rank(); m < t - s; m += G::N) sorted[s + m] = (int)(unsigned)scr[m];
+  g.sync();
   return true;
+}
+
+// The items i < n: small(i) by one thread each; those with a length (len(i))
+// above kWarpSortMin by large(group, i): a warp each, or in a block the whole
+// block above kBlockSortMin.  list: room for the long items of a block.
+template <class G, class Len, class Small, class Large>
+__device__ void group_items(G& g, int n, int* list, Len len, Small small, Large large) {
+  if constexpr (!G::kBlock) {
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const int i = i0 + g.rank();
+      const int m = i < n ? len(i) : 0;
+      if (m > 0 && m <= kWarpSortMin) small(i);
+      for (unsigned b = __ballot_sync(kFullMask, m > kWarpSortMin); b; b &= b - 1)
+        large(g, i0 + __ffs(b) - 1);
+    }
+  } else {
+    if (g.rank() == 0) g.s->count = 0;
+    g.sync();
+    for (int i = g.rank(); i < n; i += G::N) {
+      const int m = len(i);
+      if (m > kWarpSortMin) list[atomicAdd(&g.s->count, 1)] = i;
+      else if (m > 0) small(i);
+    }
+    g.sync();
+    const int cnt = g.s->count;
+    for (int k = 0; k < cnt; ++k)
+      if (len(list[k]) > kBlockSortMin) large(g, list[k]);
+    WarpGroup wg;
+    for (int k = g.warp(); k < cnt; k += G::kWarps)
+      if (len(list[k]) <= kBlockSortMin) large(wg, list[k]);
+    g.sync();
+  }
 }
 
 // A13 for base run r (copyIntersectionsParallel for one edge): its slots,
@@ -678,16 +911,16 @@ __device__ __forceinline__ void pw_fill_edge(PwWork& w, const double* c, const i
   }
 }
 
-// Rows A9-A18 of one pair, run by all 32 lanes of a warp.  The serial steps
-// (the linked-list build of the base, labelling, tracing, clean-up) run on
-// every lane alike: the lanes read the same values, take the same branches
-// and store the same values, so the warp never diverges there.  The steps
-// that are independent per record, per run, per overlay edge or per slot
-// split their loops over the lanes and end with __syncwarp; where the serial
-// loop lets the last of several writes to one slot win, the lanes keep the
-// largest writer index with atomicMax and that writer stores.  Every return
-// is taken by all lanes together.
-// The scalars the two halves of the warp back end share.
+// Rows A9-A18 of one pair, run by all threads of a group.  The serial steps
+// (an odd linked-list build, rare labels, a warp's tracing) run on every lane
+// of a warp alike: the lanes read the same values, take the same branches and
+// store the same values, so the warp never diverges there; a block leaves
+// them to its first warp.  The steps that are independent per record, per
+// run, per overlay edge or per slot split their loops over the group and end
+// with a barrier; where the serial loop lets the last of several writes to
+// one slot win, the threads keep the largest writer index with atomicMax and
+// that writer stores.  Every return is taken by all threads together.
+// The scalars the halves of the back end share.
 struct PwMid {
   int nr, knd, nB, nQ;  // base runs, non-degenerate base records, slot counts
   int pn, qn, nruns;    // after the lists: node counts of P and Q, P's run nodes
@@ -708,34 +941,36 @@ __device__ __forceinline__ PwMid pw_mid_load(const int* d) {
 }
 
 // Rows A9-A14: records, counts, alpha order, merged arrays, initial labels.
-__device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, const PwHit* H,
+template <class G>
+__device__ int pw_clip_head(G& g, const double* b, int nb, const double* c, int nc, const PwHit* H,
                             const PwCaps& cp, PwWork& w, PwMid* mid) {
-  const int lane = threadIdx.x & 31;
+  const int lane = g.rank();
+  constexpr int N = G::N;
   const int K = cp.K;
   // ---- A9: records arrive in the reference's order (base id, then first
   // emission), sorted for all pairs at once
-  for (int i = lane; i < K; i += 32) {
+  for (int i = lane; i < K; i += N) {
     const PwHit& h = H[i];
     w.ub[i] = 2 * h.b;
     w.uc[i] = 2 * h.j;
     w.ut[i] = h.type;
   }
-  for (int r = lane; r <= K; r += 32) w.re_nd[r] = 0;
-  for (int i = lane; i <= nc; i += 32) w.cAll[i] = w.cND[i] = w.cfill[i] = 0;
-  __syncwarp();
+  for (int r = lane; r <= K; r += N) w.re_nd[r] = 0;
+  for (int i = lane; i <= nc; i += N) w.cAll[i] = w.cND[i] = w.cfill[i] = 0;
+  g.sync();
   const int* ub = w.ub;
   const int* uc = w.uc;
   const int* ut = w.ut;
   // ---- A10: base edges with records (runs), overlay counts
   int nr = 0, knd = 0;
-  for (int i0 = 0; i0 < K; i0 += 32) {
+  for (int i0 = 0; i0 < K; i0 += N) {
     const int i = i0 + lane;
     const bool ok = i < K;
     const int e = ok ? ub[i] >> 1 : 0;
     const bool start = ok && (i == 0 || e != (ub[i - 1] >> 1));
     const bool nd = ok && nd_b(ut[i]);
-    const unsigned sm = __ballot_sync(kFullMask, start);
-    const int ri = nr + __popc(sm & ((2u << lane) - 1u)) - 1;  // the run holding record i
+    int starts;
+    const int ri = nr + g.before(start, &starts) + (start ? 1 : 0) - 1;  // the run holding record i
     if (start) {
       w.re_e[ri] = e;
       w.re_s[ri] = i;
@@ -746,49 +981,53 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
       atomicAdd(&w.cAll[ec], 1);
       if (nd_c(ut[i])) atomicAdd(&w.cND[ec], 1);
     }
-    nr += __popc(sm);
-    knd += __popc(__ballot_sync(kFullMask, nd));
+    nr += starts;
+    knd += nd ? 1 : 0;
   }
+  knd = g.sum(knd);
   w.re_s[nr] = K;
-  __syncwarp();
-  for (int r = lane; r <= nr; r += 32) w.re_pre[r] = w.re_nd[r];  // re_nd[nr] is 0
-  warp_excl_scan(w.re_pre, nr + 1);
-  for (int r = lane; r <= nr; r += 32) w.re_si[r] = r + w.re_pre[r];
-  warp_excl_scan(w.cAll, nc + 1);
-  warp_excl_scan(w.cND, nc + 1);
-  __syncwarp();
+  g.sync();
+  for (int r = lane; r <= nr; r += N) w.re_pre[r] = w.re_nd[r];  // re_nd[nr] is 0
+  group_scan(g, w.re_pre, nr + 1);
+  for (int r = lane; r <= nr; r += N) w.re_si[r] = r + w.re_pre[r];
+  group_scan(g, w.cAll, nc + 1);
+  group_scan(g, w.cND, nc + 1);
+  g.sync();
   // records of each overlay edge, in record order
-  for (int i = lane; i < K; i += 32) {
+  for (int i = lane; i < K; i += N) {
     const int ec = uc[i] >> 1;
     w.csorted[w.cAll[ec] + atomicAdd(&w.cfill[ec], 1)] = i;
   }
-  __syncwarp();
-  for (int e0 = 0; e0 < nc; e0 += 32) {
-    const int e = e0 + lane;
-    const int s = e < nc ? w.cAll[e] : 0, t = e < nc ? w.cAll[e + 1] : 0;
-    if (t - s > 1 && t - s <= kWarpSortMin) {
-      int* v = w.csorted + s;
-      for (int i = 1; i < t - s; ++i) {
-        const int x = v[i];
-        int j = i;
-        while (j > 0 && v[j - 1] > x) {
-          v[j] = v[j - 1];
-          --j;
+  g.sync();
+  group_items(
+      g, nc, w.htmp,
+      [&](int e) {
+        const int m = w.cAll[e + 1] - w.cAll[e];
+        return m > 1 ? m : 0;
+      },
+      [&](int e) {
+        int* v = w.csorted + w.cAll[e];
+        const int m = w.cAll[e + 1] - w.cAll[e];
+        for (int i = 1; i < m; ++i) {
+          const int x = v[i];
+          int j = i;
+          while (j > 0 && v[j - 1] > x) {
+            v[j] = v[j - 1];
+            --j;
+          }
+          v[j] = x;
         }
-        v[j] = x;
-      }
-    }
-    for (unsigned m = __ballot_sync(kFullMask, t - s > kWarpSortMin); m; m &= m - 1) {
-      const int ee = e0 + __ffs(m) - 1;
-      const int s2 = w.cAll[ee], t2 = w.cAll[ee + 1];
-      warp_bitonic(t2 - s2, w.sscr, [&](int k) { return (unsigned long long)w.csorted[s2 + k]; });
-      for (int k = lane; k < t2 - s2; k += 32) w.csorted[s2 + k] = (int)w.sscr[k];
-      __syncwarp();
-    }
-  }
+      },
+      [&](auto& gg, int e) {
+        const int s = w.cAll[e], m = w.cAll[e + 1] - s;
+        unsigned long long* scr = w.sscr + 2 * s;  // an edge's own part
+        group_sort(gg, m, scr, [&](int k) { return (unsigned long long)w.csorted[s + k]; });
+        for (int k = gg.rank(); k < m; k += gg.N) w.csorted[s + k] = (int)scr[k];
+        gg.sync();
+      });
   const int nB = nb + knd, nQ = nc + w.cND[nc];
   // ---- A11 records
-  for (int i = lane; i < K; i += 32) {
+  for (int i = lane; i < K; i += N) {
     const int bi = ub[i] >> 1, ci = uc[i] >> 1;
     const int bi2 = bi + 1 == nb ? 0 : bi + 1;
     const double p1x = b[2 * bi], p1y = b[2 * bi + 1], p2x = b[2 * bi2], p2y = b[2 * bi2 + 1];
@@ -813,7 +1052,7 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     w.aC[i] = ty ? alpha_to_int(bt) : 0;
     w.sB[i] = w.sC[i] = i;
   }
-  __syncwarp();
+  g.sync();
   // ---- A12 per-edge alpha order (stable by alpha mod 1e9), one run or one
   // overlay edge per lane
   // (stable insertion for short runs on one lane; a long run -- an overlay
@@ -845,57 +1084,53 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     return true;
   };
   bool bad = false;
-  for (int r0 = 0; r0 < nr; r0 += 32) {
-    const int r = r0 + lane;
-    bool lng = false;
-    if (r < nr && w.re_nd[r] > 1) {
-      if (w.re_s[r + 1] - w.re_s[r] > kWarpSortMin) lng = true;
-      else if (!isort(w.re_s[r], w.re_s[r + 1], w.aB, nullptr, w.sB)) bad = true;
-    }
-    for (unsigned m = __ballot_sync(kFullMask, lng); m; m &= m - 1) {
-      const int rr = r0 + __ffs(m) - 1;
-      if (!warp_alpha_sort(w.re_s[rr], w.re_s[rr + 1], w.aB, nullptr, w.sB, w.sscr)) bad = true;
-    }
-  }
-  for (int e0 = 0; e0 < nc; e0 += 32) {
-    const int e = e0 + lane;
-    bool lng = false;
-    if (e < nc && w.cND[e + 1] - w.cND[e] > 1) {
-      if (w.cAll[e + 1] - w.cAll[e] > kWarpSortMin) lng = true;
-      else if (!isort(w.cAll[e], w.cAll[e + 1], w.aC, w.csorted, w.sC)) bad = true;
-    }
-    for (unsigned m = __ballot_sync(kFullMask, lng); m; m &= m - 1) {
-      const int ee = e0 + __ffs(m) - 1;
-      if (!warp_alpha_sort(w.cAll[ee], w.cAll[ee + 1], w.aC, w.csorted, w.sC, w.sscr)) bad = true;
-    }
-  }
-  if (warp_fail(bad)) return PS_FALLBACK;
+  group_items(
+      g, nr, w.htmp, [&](int r) { return w.re_nd[r] > 1 ? w.re_s[r + 1] - w.re_s[r] : 0; },
+      [&](int r) {
+        if (!isort(w.re_s[r], w.re_s[r + 1], w.aB, nullptr, w.sB)) bad = true;
+      },
+      [&](auto& gg, int r) {
+        const int s = w.re_s[r];
+        if (!group_alpha_sort(gg, s, w.re_s[r + 1], w.aB, nullptr, w.sB, w.sscr + 2 * s)) bad = true;
+      });
+  group_items(
+      g, nc, w.htmp,
+      [&](int e) { return w.cND[e + 1] - w.cND[e] > 1 ? w.cAll[e + 1] - w.cAll[e] : 0; },
+      [&](int e) {
+        if (!isort(w.cAll[e], w.cAll[e + 1], w.aC, w.csorted, w.sC)) bad = true;
+      },
+      [&](auto& gg, int e) {
+        const int s = w.cAll[e];
+        if (!group_alpha_sort(gg, s, w.cAll[e + 1], w.aC, w.csorted, w.sC, w.sscr + 2 * s)) bad = true;
+      });
+  if (g.any(bad)) return PS_FALLBACK;
   // ---- A13 merged arrays: the base's where it has records, the overlay's in
   // full.  A run (overlay edge) writes only its own slots and the neighbour
   // indices of its own records, so runs (edges) go one per lane.
-  for (int i = lane; i < nQ; i += 32) {
+  for (int i = lane; i < nQ; i += N) {
     w.ixC[2 * i] = w.ixC[2 * i + 1] = 0.0;
     w.alC[i] = w.nbC[i] = 0;
     w.nbCsi[i] = -1;
     w.cWin[i] = -1;
   }
-  for (int i = lane; i < K; i += 32) {
+  for (int i = lane; i < K; i += N) {
     w.bNI[i] = w.cNI[i] = 0;
     w.bSI[i] = -1;  // the sparse index of bNI[i] once a slot is written
   }
-  __syncwarp();
+  g.sync();
   // base runs (copyIntersectionsParallel per edge), in chunks of 32 runs
-  for (int r0 = 0; r0 < nr; r0 += 32) {
+  for (int r0 = 0; r0 < nr; r0 += N) {
     const int r = r0 + lane;
     if (r < nr) pw_fill_run(w, b, ub, ut, K, r);
     __syncwarp();
   }
   // overlay edges: the vertex slot, then the edge's intersection slots
-  for (int e0 = 0; e0 < nc; e0 += 32) {
+  for (int e0 = 0; e0 < nc; e0 += N) {
     const int e = e0 + lane;
     if (e < nc) pw_fill_edge(w, c, uc, ut, K, e);
     __syncwarp();
   }
+  g.sync();
   // neighbours: the last record written to a slot wins (spnode and cWin hold
   // the winning record until the winners have stored)
   int si0;  // sparse index of slot 0, where records never written point
@@ -903,7 +1138,7 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     int vtx;
     si0 = pw_slot(w, nr, 0, &vtx);
   }
-  for (int i = lane; i < K; i += 32) {
+  for (int i = lane; i < K; i += N) {
     const int si = w.bSI[i] < 0 ? si0 : w.bSI[i];
     if (si < 0) {
       bad = true;  // a plain slot would change
@@ -912,8 +1147,8 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     atomicMax(&w.spnode[si], i);
     atomicMax(&w.cWin[w.cNI[i]], i);
   }
-  if (warp_fail(bad)) return PS_FALLBACK;
-  for (int i = lane; i < K; i += 32) {
+  if (g.any(bad)) return PS_FALLBACK;
+  for (int i = lane; i < K; i += N) {
     const int si = w.bSI[i] < 0 ? si0 : w.bSI[i];
     const int cq = w.cNI[i];
     if (w.spnode[si] == i) w.spnb[si] = cq + 1;
@@ -922,16 +1157,16 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
       w.nbCsi[cq] = si;
     }
   }
-  __syncwarp();
+  g.sync();
   const int nsp = w.re_si[nr];
-  for (int s = lane; s < nsp; s += 32) w.spnode[s] = -1;
-  for (int q = lane; q < nQ; q += 32) w.cWin[q] = -1;
-  __syncwarp();
+  for (int s = lane; s < nsp; s += N) w.spnode[s] = -1;
+  for (int q = lane; q < nQ; q += N) w.cWin[q] = -1;
+  g.sync();
   // ---- A14 initial labels, one sparse slot per lane (spnode holds each
   // slot's run meanwhile); the overlay slot takes the label of the last base
   // slot naming it.  Loops over lanes run in chunks closed by __syncwarp, so
   // that lanes that branch apart join again every chunk.
-  for (int r0 = 0; r0 < nr; r0 += 32) {
+  for (int r0 = 0; r0 < nr; r0 += N) {
     const int r = r0 + lane;
     if (r < nr) {
       const int si0 = w.re_si[r], nd = w.re_nd[r];
@@ -939,7 +1174,8 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     }
     __syncwarp();
   }
-  for (int s0 = 0; s0 < nsp; s0 += 32) {
+  g.sync();
+  for (int s0 = 0; s0 < nsp; s0 += N) {
     const int si = s0 + lane;
     if (si < nsp && !bad && w.spal[si] != -100) {
       const int r = w.spnode[si];
@@ -1011,8 +1247,8 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     }
     __syncwarp();
   }
-  if (warp_fail(bad)) return PS_FALLBACK;
-  for (int s0 = 0; s0 < nsp; s0 += 32) {
+  if (g.any(bad)) return PS_FALLBACK;
+  for (int s0 = 0; s0 < nsp; s0 += N) {
     const int si = s0 + lane;
     if (si < nsp && w.spal[si] != -100) {
       const int r = w.spnode[si];
@@ -1021,18 +1257,21 @@ __device__ int pw_clip_head(const double* b, int nb, const double* c, int nc, co
     }
     __syncwarp();
   }
-  for (int s = lane; s < nsp; s += 32) w.spnode[s] = -1;
-  for (int q = lane; q < nQ; q += 32) w.labC[q] = w.cWin[q] >= 0 ? w.splab[w.cWinSI[q]] : 0;
-  __syncwarp();
+  g.sync();
+  for (int s = lane; s < nsp; s += N) w.spnode[s] = -1;
+  for (int q = lane; q < nQ; q += N) w.labC[q] = w.cWin[q] >= 0 ? w.splab[w.cWinSI[q]] : 0;
+  g.sync();
   *mid = PwMid{nr, knd, nB, nQ, 0, 0, 0};
   return PS_OK;
 }
 
 // Row A15 from the head's arrays: the linked lists (mid receives their node
 // counts and P's run nodes).
-__device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, const PwCaps& cp,
+template <class G>
+__device__ int pw_clip_lists(G& g, const double* b, int nb, const double* c, int nc, const PwCaps& cp,
                              PwWork& w, PwMid* mid) {
-  const int lane = threadIdx.x & 31;
+  const int lane = g.rank();
+  constexpr int N = G::N;
   const int nr = mid->nr, knd = mid->knd, nB = mid->nB, nQ = mid->nQ;
   // slot contents of the base's merged list
   auto info = [&](int s, int hint, double* x, double* y, int* al, int* nbv) {
@@ -1061,26 +1300,62 @@ __device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, c
   P.n = Q.n = w.R.n = 0;
   P.rxy = b;
   int nruns = 0, lastPlain = -1;
-  bool oddP = false;
-  for (int r = lane; r < nr && !oddP; r += 32) {
-    const int e = w.re_e[r], si = w.re_si[r], nd = w.re_nd[r];
-    if (!(w.spx[si] == b[2 * e] && w.spy[si] == b[2 * e + 1])) oddP = true;
-    if (nd == 0) continue;
-    const int nx = e + 1 == nb ? 0 : e + 1;
-    const double vx = b[2 * nx], vy = b[2 * nx + 1];
-    if (!(vx == vx && vy == vy)) oddP = true;
-    for (int q = 1; q <= nd; ++q)
-      if (w.spx[si + q] == vx && w.spy[si + q] == vy) oddP = true;
+  auto odd_base = [&]() {
+    bool odd = false;
+    for (int r = lane; r < nr && !odd; r += N) {
+      const int e = w.re_e[r], si = w.re_si[r], nd = w.re_nd[r];
+      if (!(w.spx[si] == b[2 * e] && w.spy[si] == b[2 * e + 1])) odd = true;
+      if (nd == 0) continue;
+      const int nx = e + 1 == nb ? 0 : e + 1;
+      const double vx = b[2 * nx], vy = b[2 * nx + 1];
+      if (!(vx == vx && vy == vy)) odd = true;
+      for (int q = 1; q <= nd; ++q)
+        if (w.spx[si + q] == vx && w.spy[si + q] == vy) odd = true;
+    }
+    return g.any(odd);
+  };
+  // The overlay's list is its merged array in order (node i is slot i) unless
+  // a slot's coordinates stop the reference's walk early: an overlay vertex
+  // whose slot does not hold its own coordinates (NaN), or an intersection
+  // slot of edge e that repeats vertex e + 1.  The walk then takes the serial
+  // path below, which follows the reference in every case.
+  auto odd_overlay = [&]() {
+    bool odd = false;
+    for (int e = lane; e < nc && !odd; e += N) {
+      const int vs = e + w.cND[e], ne = w.cND[e + 1] - w.cND[e];
+      const int nx = e + 1 == nc ? 0 : e + 1;
+      const double vx = c[2 * nx], vy = c[2 * nx + 1];
+      if (!(w.ixC[2 * vs] == c[2 * e] && w.ixC[2 * vs + 1] == c[2 * e + 1])) odd = true;
+      for (int q = 1; q <= ne; ++q)
+        if (w.ixC[2 * (vs + q)] == vx && w.ixC[2 * (vs + q) + 1] == vy) odd = true;
+    }
+    return g.any(odd);
+  };
+  bool oddP = odd_base();
+  if constexpr (G::kBlock) {
+    // a serial walk is one warp's work
+    if (oddP || odd_overlay()) {
+      int st = PS_OK;
+      if (g.warp() == 0) {
+        WarpGroup wg;
+        st = pw_clip_lists(wg, b, nb, c, nc, cp, w, mid);
+      }
+      st = g.same(st);
+      mid->pn = g.same(mid->pn);
+      mid->qn = g.same(mid->qn);
+      mid->nruns = g.same(mid->nruns);
+      return st;
+    }
   }
-  if (!__any_sync(kFullMask, oddP)) {
+  if (!oddP) {
     // nodes per run (stretch, vertex, intersections), offsets by a scan in re_s
-    for (int r = lane; r < nr; r += 32) {
+    for (int r = lane; r < nr; r += N) {
       const int e = w.re_e[r], pe = r == 0 ? 0 : w.re_e[r - 1] + 1;
       w.re_s[r] = (e > pe ? 1 : 0) + 1 + w.re_nd[r];
     }
-    if (lane == (nr & 31)) w.re_s[nr] = 0;
-    __syncwarp();
-    const int tot0 = warp_excl_scan(w.re_s, nr + 1);
+    if (lane == 0) w.re_s[nr] = 0;
+    g.sync();
+    const int tot0 = group_scan(g, w.re_s, nr + 1);
     const int pe_last = nr == 0 ? 0 : w.re_e[nr - 1] + 1;
     const int tail = pe_last < nb ? 1 : 0;
     if (tot0 + tail > P.cap) return PS_CAP;
@@ -1095,8 +1370,8 @@ __device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, c
       P.run[v] = 0;
       P.rv0[v] = 0;
     };
-    __syncwarp();
-    for (int r0 = 0; r0 < nr; r0 += 32) {
+    g.sync();
+    for (int r0 = 0; r0 < nr; r0 += N) {
       const int r = r0 + lane;
       if (r < nr) {
         const int e = w.re_e[r], pe = r == 0 ? 0 : w.re_e[r - 1] + 1, si = w.re_si[r];
@@ -1203,29 +1478,15 @@ __device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, c
     if (vn != nB) return PS_UNDEF;
   }
   }
-  __syncwarp();
-  for (int v = lane; v < P.n; v += 32) {
+  g.sync();
+  for (int v = lane; v < P.n; v += N) {
     P.next[v] = v + 1 == P.n ? 0 : v + 1;
     P.prev[v] = v == 0 ? P.n - 1 : v - 1;
   }
-  // The overlay's list is its merged array in order (node i is slot i) unless
-  // a slot's coordinates stop the reference's walk early: an overlay vertex
-  // whose slot does not hold its own coordinates (NaN), or an intersection
-  // slot of edge e that repeats vertex e + 1.  The walk then takes the serial
-  // path below, which follows the reference in every case.
-  bool odd = false;
-  for (int e = lane; e < nc && !odd; e += 32) {
-    const int vs = e + w.cND[e], ne = w.cND[e + 1] - w.cND[e];
-    const int nx = e + 1 == nc ? 0 : e + 1;
-    const double vx = c[2 * nx], vy = c[2 * nx + 1];
-    if (!(w.ixC[2 * vs] == c[2 * e] && w.ixC[2 * vs + 1] == c[2 * e + 1])) odd = true;
-    for (int q = 1; q <= ne; ++q)
-      if (w.ixC[2 * (vs + q)] == vx && w.ixC[2 * (vs + q) + 1] == vy) odd = true;
-  }
-  if (!__any_sync(kFullMask, odd)) {
+  if (G::kBlock || !odd_overlay()) {
     // node v = slot v; the first failing slot decides the status
     int first = INT_MAX;  // 4 * slot + 1 (undefined) or + 2 (pair pipeline)
-    for (int e0 = 0; e0 < nc; e0 += 32) {
+    for (int e0 = 0; e0 < nc; e0 += N) {
       const int e = e0 + lane;
       const int vs = e < nc ? e + w.cND[e] : 0, ne = e < nc ? w.cND[e + 1] - w.cND[e] : -1;
       for (int q = 0; q <= ne; ++q) {
@@ -1256,8 +1517,8 @@ __device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, c
       }
       __syncwarp();
     }
-    first = __reduce_min_sync(kFullMask, first);
-    __syncwarp();
+    first = g.min_of(first);
+    g.sync();
     if (first != INT_MAX) return (first & 3) == 1 ? PS_UNDEF : PS_FALLBACK;
     Q.n = nQ;
   } else {
@@ -1302,9 +1563,9 @@ __device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, c
       Q.prev[v] = (v + nQ - 1) % nQ;
     }
   }
-  for (int i = lane; i < cp.capP; i += 32) w.splitP[i] = w.crossP[i] = 0;
-  for (int i = lane; i < cp.capQ; i += 32) w.splitQ[i] = w.crossQ[i] = 0;
-  __syncwarp();
+  for (int i = lane; i < cp.capP; i += N) w.splitP[i] = w.crossP[i] = 0;
+  for (int i = lane; i < cp.capQ; i += N) w.splitQ[i] = w.crossQ[i] = 0;
+  g.sync();
   mid->pn = P.n;
   mid->qn = Q.n;
   mid->nruns = nruns;
@@ -1312,11 +1573,12 @@ __device__ int pw_clip_lists(const double* b, int nb, const double* c, int nc, c
 }
 
 // Rows A16-A18 from the lists: labelling, tracing, clean-up and the rings out.
-template <class Pip>
-__device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, const PwCaps& cp,
+template <class G, class Pip>
+__device__ int pw_clip_trace(G& g, const double* b, int nb, const double* c, int nc, const PwCaps& cp,
                              PwWork& w, const PwMid& mid, Pip pip, int unite, int* nrings_out,
                              int* nverts_out) {
-  const int lane = threadIdx.x & 31;
+  const int lane = g.rank();
+  constexpr int N = G::N;
   const int nB = mid.nB, nQ = mid.nQ;
   Pool& P = w.P;
   Pool& Q = w.Q;
@@ -1325,8 +1587,7 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
   P.rxy = b;
   w.R.n = 0;
   const int nruns = mid.nruns;
-  // ---- A16-A18 (serial, on every lane; pointInPoly against the base splits
-  // its grid row over the lanes)
+  // ---- A16-A18
   SerialArgs a;
   a.P = P;
   a.Q = Q;
@@ -1356,7 +1617,18 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
   *a.nrings = 0;
   pip.runIds = w.runIds;
   pip.nruns = nruns;
-  int st = pw_label_trace(a, pip);
+  int st = -1;
+  if constexpr (G::kBlock) {
+    st = pw_label_trace_block(g, a, pip, w, cp);
+    if (st < 0) {  // labels beyond plain crossings: the first warp's serial steps
+      if (g.warp() == 0) st = pw_label_trace(a, pip);
+      st = g.same(st);
+      a.R.n = g.same(a.R.n);
+      a.rfull = g.same(a.rfull);
+    }
+  } else {
+    st = pw_label_trace(a, pip);
+  }
   if (a.rfull) return PS_CAP;
   if (st) return st == 2 ? PS_UNDEF : PS_CAP;
   // cleanUpResult2 (ser_cleanup).  Rings are built one after another and
@@ -1364,11 +1636,11 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
   // in order.  A vertex with |area3| < eps marks its ring; with no ring
   // marked nothing is removed and the output is the pool itself.
   const int nring = *a.nrings;
-  for (int r = lane; r < nring; r += 32) w.sscr[r] = 0;
-  __syncwarp();
+  for (int r = lane; r < nring; r += N) w.sscr[r] = 0;
+  g.sync();
   {
     const Pool& R = a.R;
-    for (int v = lane; v < R.n; v += 32) {
+    for (int v = lane; v < R.n; v += N) {
       const double ar = fabs(area3(R.x[R.prev[v]], R.y[R.prev[v]], R.x[v], R.y[v],
                                    R.x[R.next[v]], R.y[R.next[v]]));
       if (!(ar < kEps)) continue;
@@ -1381,19 +1653,19 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
       if (lo > 0) w.sscr[lo - 1] = 1;
     }
   }
-  __syncwarp();
-  if (warp_first(nring, [&](int r) {
+  g.sync();
+  if (g.first(nring, [&](int r) {
         return w.sscr[r] != 0 || (r > 0 && a.rroot[r] <= a.rroot[r - 1]);
       }) < 0 &&
       (nring == 0 || a.rroot[0] == 0)) {
     const Pool& R = a.R;
-    for (int v = lane; v < R.n; v += 32) {
+    for (int v = lane; v < R.n; v += N) {
       w.rxy[2 * v] = R.x[v];
       w.rxy[2 * v + 1] = R.y[v];
     }
-    for (int r = lane; r < nring; r += 32) w.roff[r] = a.rroot[r];
+    for (int r = lane; r < nring; r += N) w.roff[r] = a.rroot[r];
     if (lane == 0) w.roff[nring] = R.n;
-    __syncwarp();
+    g.sync();
     *nrings_out = nring;
     *nverts_out = R.n;
     return PS_OK;
@@ -1403,7 +1675,7 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
   // sscr[r], 1 << 32 in the high half when it is not empty
   {
     Pool& R = a.R;
-    for (int r = lane; r < nring; r += 32) {
+    for (int r = lane; r < nring; r += N) {
       auto A3 = [&](int v) {
         return fabs(area3(R.x[R.prev[v]], R.y[R.prev[v]], R.x[v], R.y[v], R.x[R.next[v]],
                           R.y[R.next[v]]));
@@ -1440,24 +1712,23 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
       w.sscr[r] = len;
     }
   }
-  __syncwarp();
+  g.sync();
   // output offsets (one scan of both halves), then the rings' coordinates
   {
-    unsigned long long carry = 0;
-    for (int r0 = 0; r0 < nring; r0 += 32) {
+    int rings = 0, verts = 0;
+    for (int r0 = 0; r0 < nring; r0 += N) {
       const int r = r0 + lane;
       const unsigned long long x = r < nring ? w.sscr[r] : 0;
-      unsigned long long sc = x;
-      for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long t = __shfl_up_sync(kFullMask, sc, d);
-        if (lane >= d) sc += t;
-      }
-      if (r < nring) w.sscr[r] = carry + sc - x;
-      carry += __shfl_sync(kFullMask, sc, 31);
+      int n1, n0;
+      const int e1 = g.excl((int)(x >> 32), &n1), e0 = g.excl((int)(unsigned)x, &n0);
+      if (r < nring)
+        w.sscr[r] = ((unsigned long long)(unsigned)(rings + e1) << 32) | (unsigned)(verts + e0);
+      rings += n1;
+      verts += n0;
     }
-    __syncwarp();
+    g.sync();
     w.roff[0] = 0;
-    for (int r = lane; r < nring; r += 32) {
+    for (int r = lane; r < nring; r += N) {
       const int root = a.rroot[r];
       if (root < 0) continue;
       const unsigned long long off = w.sscr[r];
@@ -1472,14 +1743,14 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
       } while (v != root);
       w.roff[k + 1] = nv;
     }
-    __syncwarp();
-    *nrings_out = (int)(carry >> 32);
-    *nverts_out = (int)(unsigned)carry;
+    g.sync();
+    *nrings_out = rings;
+    *nverts_out = verts;
   }
   return PS_OK;
 }
 
-// One pair, rows A9-A18, by the calling warp (all 32 lanes): base b (nb
+// One pair, rows A9-A18, by the calling group: base b (nb
 // vertices), overlay c (nc), its K unique hits H in the reference's order
 // (base id, then first emission), a pointInPoly functor for the base side
 // (pip: its runIds / nruns are set by the tail), union or intersection.
@@ -1487,15 +1758,15 @@ __device__ int pw_clip_trace(const double* b, int nb, const double* c, int nc, c
 // sparse back end does not follow the arrays (the caller clips the pair
 // another way), PS_UNDEF or PS_CAP.  The head, the lists and the trace may
 // also run as separate kernels, PwMid carried between them.
-template <class Pip>
-__device__ int pw_clip_core(const double* b, int nb, const double* c, int nc, const PwHit* H,
+template <class G, class Pip>
+__device__ int pw_clip_core(G& g, const double* b, int nb, const double* c, int nc, const PwHit* H,
                             const PwCaps& cp, PwWork& w, Pip pip, int unite, int* nrings_out,
                             int* nverts_out) {
   PwMid mid;
-  int st = pw_clip_head(b, nb, c, nc, H, cp, w, &mid);
-  if (st == PS_OK) st = pw_clip_lists(b, nb, c, nc, cp, w, &mid);
+  int st = pw_clip_head(g, b, nb, c, nc, H, cp, w, &mid);
+  if (st == PS_OK) st = pw_clip_lists(g, b, nb, c, nc, cp, w, &mid);
   if (st != PS_OK) return st;
-  return pw_clip_trace(b, nb, c, nc, cp, w, mid, pip, unite, nrings_out, nverts_out);
+  return pw_clip_trace(g, b, nb, c, nc, cp, w, mid, pip, unite, nrings_out, nverts_out);
 }
 
 }  // namespace
