@@ -35,6 +35,27 @@ namespace {
 
 constexpr int kBatchBlock = 128;
 
+// A wide pair: a block of kWideBlock threads runs its front, its rows A9-A18
+// and its backward pass, and its candidate tests are shared by as many warps
+// as it has groups of kEdgeGroup base edges.  A warp per pair made the largest
+// pairs of a batch the tail of every kernel (12,000 pairs of 3 to 2,048
+// vertices: 221 ms forward and backward, 47 with blocks).  A pair is wide
+// above 256 edges or `min` edge pairs (kWideMin[0] while at most kWideFew pairs
+// of the batch are above that, else kWideMin[1]): a batch of many pairs of one
+// size fills the GPU with warps and does the least work so (pairs of 64 to
+// 127 vertices, forward and backward: 4,000 take 1.32 ms on warps and 2.1 on
+// blocks, 1,000 take 0.79 and 0.67, 128 take 0.64 and 0.34).  At 1,024 edge
+// pairs blocks gained nothing (512 pairs of 4 to 64 vertices: 0.37 ms on
+// warps, 0.47 on blocks).  Blocks of 64 and 128 threads were slower
+// on the largest pairs (the 12,000 pairs: 69.6 and 50.8 ms).
+constexpr int kWideBlock = 256, kWideEdges = 256;
+constexpr int kEdgeGroup = 32;
+constexpr int kWideMin[2] = {4096, 16384}, kWideFew = 1024;
+__host__ __device__ __forceinline__ bool wide_pair(int nb, int nc, int min) {
+  return (long long)nb * nc > min || nb + nc > kWideEdges;
+}
+__host__ __device__ __forceinline__ int edge_groups(int n) { return (n + kEdgeGroup - 1) / kEdgeGroup; }
+
 // ------------------------------------------------------------------ arena
 // capacities of one pair
 struct Caps {
@@ -105,9 +126,8 @@ struct PairWork {
   long long* fkey;
   int* fval;
   int* eflag;  // per sorted endpoint: entries it adds to the elementary array
-  unsigned long long* csort;  // the candidate sweep's overlay edges by box min x
-  float4* sbox;               // their boxes in that order
-  int* hsort;                 // the warp back end's hit order (a power-of-two network)
+  float4* gbox;  // the boxes of the overlay's edge groups (wide pairs)
+  int* hsort;    // the hits by base edge and first emission
   // components: the merged slot of each component's first vertex, ending
   // with the slot count (filled by the thread back end)
   int *rootB, *rootC;
@@ -211,9 +231,8 @@ __host__ __device__ __forceinline__ PairWork carve(Carver& cv, const Caps& c) {
   w.fkey = cv.take<long long>(npow2_dev(n2));
   w.fval = cv.take<int>(npow2_dev(n2));
   w.eflag = cv.take<int>(n2 + 1);
-  w.csort = cv.take<unsigned long long>(npow2_dev(c.nc));
-  w.sbox = cv.take<float4>(c.nc);
-  w.hsort = cv.take<int>(npow2_dev(K));
+  w.gbox = cv.take<float4>(edge_groups(c.nc));
+  w.hsort = cv.take<int>(K);
   w.rootB = cv.take<int>(c.nb + 1);
   w.rootC = cv.take<int>(c.nc + 1);
   return w;
@@ -290,25 +309,43 @@ struct PairResult {
 };
 
 // ------------------------------------------------------------------ one pair
-// Kernels per pair: the front (rows A1-A7, one warp), the candidate pairs
-// (A8, one warp), the warp back end (A9-A18) with the thread back end for the
+// Kernels per pair: the front (rows A1-A7, one group of threads: a warp, or a
+// block for a wide pair), the candidate pairs (A8), the group back end (A9-A18) with the thread back end for the
 // pairs it hands over, and the area; w.state carries the front's status,
 // logL, the hit count and the back end's route between them.
-// Rows A1-A7 of one pair by one warp, in the reference's order
+// Rows A1-A7 of one pair by one group, in the reference's order
 // (edge.h:190-202 edges; oacc_segment_tree.cpp:4513-4692 elementary
 // intervals; :203-206 and :616-689 realToInt borders; findBoarder; leaf
-// ranges), every loop shared among the lanes: the endpoint sort is a bitonic
-// network over (key, endpoint) pairs (the stable order), the elementary
-// array comes from a scan of per-endpoint entry counts.  Compares run on
-// order keys (okey).
-__device__ int clip_pair_front_warp(const double* b, int nb, const double* c, int nc,
-                                    const Caps& cp, PairWork& w, int lane) {
-  WarpGroup g;
+// ranges), every loop shared among the threads: the endpoint sort is a
+// bitonic network over (key, endpoint) pairs (the stable order) in the n_sort
+// slots skey / sval (shared memory) when it fits them, the elementary array
+// comes from a scan of per-endpoint entry counts.  Compares run on order keys
+// (okey).
+struct FrontRange {
+  long long kmin, kmax;
+  int imin, imax;
+  __device__ void join(long long km, long long kx, int im, int ix) {
+    if (km < kmin || (km == kmin && im < imin)) {
+      kmin = km;
+      imin = im;
+    }
+    if (kx > kmax || (kx == kmax && ix < imax)) {
+      kmax = kx;
+      imax = ix;
+    }
+  }
+};
+
+template <class G>
+__device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, int nc,
+                               const Caps& cp, PairWork& w, long long* skey, int* sval, int n_sort,
+                               FrontRange* s_range) {
+  const int lane = g.rank();
+  constexpr int N = G::N;
   const int E = nb + nc, n2 = 2 * E;
   // ---- A1 edges; the x range on order keys (ties: the earlier vertex)
-  long long kmin = LLONG_MAX, kmax = LLONG_MIN;
-  int imin = INT_MAX, imax = INT_MAX;
-  for (int e = lane; e < E; e += 32) {
+  FrontRange fr{LLONG_MAX, LLONG_MIN, INT_MAX, INT_MAX};
+  for (int e = lane; e < E; e += N) {
     double a0, a1, y0, y1;
     if (e < nb) {
       const int t = vsucc(w.bnx, nb, e);
@@ -335,77 +372,62 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
       w.kee[e] = k0;
       w.kes[e] = k1;
     }
-    if (k0 < kmin) {
-      kmin = k0;
-      imin = e;
-    }
-    if (k0 > kmax) {
-      kmax = k0;
-      imax = e;
-    }
+    fr.join(k0, k0, e, e);
     const bool xs = k0 < k1, ys = ky0 < ky1;
     w.fbox[e] = make_float4(__double2float_rd(xs ? a0 : a1), __double2float_rd(ys ? y0 : y1),
                             __double2float_ru(xs ? a1 : a0), __double2float_ru(ys ? y1 : y0));
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const long long km = __shfl_xor_sync(kFullMask, kmin, o), kx = __shfl_xor_sync(kFullMask, kmax, o);
-    const int im = __shfl_xor_sync(kFullMask, imin, o), ix = __shfl_xor_sync(kFullMask, imax, o);
-    if (km < kmin || (km == kmin && im < imin)) {
-      kmin = km;
-      imin = im;
-    }
-    if (kx > kmax || (kx == kmax && ix < imax)) {
-      kmax = kx;
-      imax = ix;
-    }
+  for (int o = 16; o > 0; o >>= 1)
+    fr.join(__shfl_xor_sync(kFullMask, fr.kmin, o), __shfl_xor_sync(kFullMask, fr.kmax, o),
+            __shfl_xor_sync(kFullMask, fr.imin, o), __shfl_xor_sync(kFullMask, fr.imax, o));
+  if constexpr (G::kBlock) {
+    if ((threadIdx.x & 31) == 0) s_range[g.warp()] = fr;
+    g.sync();
+    for (int k = 0; k < G::kWarps; ++k)
+      fr.join(s_range[k].kmin, s_range[k].kmax, s_range[k].imin, s_range[k].imax);
   }
   // the vertex values behind the extreme keys (edge e's first vertex)
   auto vx0 = [&](int e) { return e < nb ? bvx(b, nb, e) : bvx(c, nc, e - nb); };
-  const double minI = vx0(imin), maxI = vx0(imax);
-  __syncwarp();
+  const double minI = vx0(fr.imin), maxI = vx0(fr.imax);
+  g.sync();
   // ---- A4 elementary intervals: stable sort of the endpoints by key, the
   // endpoint index breaking ties
   auto kval = [&](int idx) { return (idx & 1) ? w.kee[idx >> 1] : w.kes[idx >> 1]; };
   auto val = [&](int idx) { return (idx & 1) ? w.ee[idx >> 1] : w.es[idx >> 1]; };
   const int np2 = npow2_dev(n2);
-  for (int m = lane; m < np2; m += 32) {
-    w.fkey[m] = m < n2 ? kval(m) : LLONG_MAX;
-    w.fval[m] = m < n2 ? m : INT_MAX;
+  long long* fkey = np2 <= n_sort ? skey : w.fkey;
+  int* fval = np2 <= n_sort ? sval : w.fval;
+  for (int m = lane; m < np2; m += N) {
+    fkey[m] = m < n2 ? kval(m) : LLONG_MAX;
+    fval[m] = m < n2 ? m : INT_MAX;
   }
-  __syncwarp();
-  // each lane takes compare-exchange pairs (m, m + j), not elements: every
-  // lane works in every round
-  for (int k = 2; k <= np2; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int q = lane; q < (np2 >> 1); q += 32) {
-        const int m = ((q & ~(j - 1)) << 1) | (q & (j - 1)), l = m | j;
-        const long long xk = w.fkey[m], yk = w.fkey[l];
-        const int xv = w.fval[m], yv = w.fval[l];
-        const bool gt = xk > yk || (xk == yk && xv > yv);
-        if (gt == ((m & k) == 0)) {
-          w.fkey[m] = yk;
-          w.fkey[l] = xk;
-          w.fval[m] = yv;
-          w.fval[l] = xv;
-        }
-      }
-      __syncwarp();
+  g.sync();
+  group_bitonic(g, np2, [&](int m, int l, bool up) {
+    const long long xk = fkey[m], yk = fkey[l];
+    const int xv = fval[m], yv = fval[l];
+    const bool gt = xk > yk || (xk == yk && xv > yv);
+    if (gt == up) {
+      fkey[m] = yk;
+      fkey[l] = xk;
+      fval[m] = yv;
+      fval[l] = xv;
     }
-  for (int i = lane; i < n2; i += 32) w.sidx[i] = w.fval[i];
-  for (int i = lane; i <= E; i += 32) w.vl[i] = 0;
-  __syncwarp();
-  for (int j = lane; j < E; j += 32) {
+  });
+  for (int i = lane; i < n2; i += N) w.sidx[i] = fval[i];
+  for (int i = lane; i <= E; i += N) w.vl[i] = 0;
+  g.sync();
+  for (int j = lane; j < E; j += N) {
     const int i = w.sidx[j] >> 1;
     if (w.kes[i] == w.kee[i]) w.vl[i] = 1;
   }
-  __syncwarp();
+  g.sync();
   group_scan(g, w.vl, E + 1);
-  __syncwarp();
-  for (int i = lane; i < E; i += 32)
+  g.sync();
+  for (int i = lane; i < E; i += N)
     if (w.vl[i] != w.vl[i + 1]) w.vloc[w.vl[i]] = i;
-  __syncwarp();
+  g.sync();
   // entries per sorted endpoint i (0, 1, or 2 for the last pair), then their places
-  for (int i = lane; i < n2 - 1; i += 32) {
+  for (int i = lane; i < n2 - 1; i += N) {
     const long long k0 = kval(w.sidx[i]), k1 = kval(w.sidx[i + 1]);
     const int intvi = w.sidx[i] >> 1;
     const int comid = w.vl[i / 2];
@@ -424,13 +446,13 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
     w.eflag[i] = n;
   }
   if (lane == 0) w.eflag[n2 - 1] = 0;
-  __syncwarp();
+  g.sync();
   const int count = group_scan(g, w.eflag, n2);
-  __syncwarp();
+  g.sync();
   if (count < 1) return PS_UNDEF;
   double* ea = w.ea;
   long long* kea = w.kea;
-  for (int i = lane; i < n2 - 1; i += 32) {
+  for (int i = lane; i < n2 - 1; i += N) {
     const int at = w.eflag[i], n = (i + 1 < n2 ? w.eflag[i + 1] : count) - at;
     if (n == 0) continue;
     const int si = w.sidx[i];
@@ -445,9 +467,9 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
       ea[at] = w.es[si >> 1];
     }
   }
-  __syncwarp();
+  g.sync();
   const int epc = npow2_dev(count) + 1;
-  for (int i = count + lane; i < epc; i += 32) {
+  for (int i = count + lane; i < epc; i += N) {
     ea[i] = ea[count - 1];
     kea[i] = kea[count - 1];
   }
@@ -463,7 +485,7 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
   double scale = 1.0;
   for (int t = 0; t < 11 - digits; ++t) scale = dmul(scale, 10.0);
   const bool shift = minI < 0;
-  __syncwarp();
+  g.sync();
   int zl = 0;
   bool bad = false;
   {
@@ -471,16 +493,16 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
       const double v = shift ? dmul(scale, dadd(ea[t], absMin)) : dmul(scale, ea[t]);
       return (long long)v;
     };
-    for (int i = 1 + lane; i < epc; i += 32) {
+    for (int i = 1 + lane; i < epc; i += N) {
       const long long ki = key(i);
       if (ki < 0 || ki >= 100000000000LL || (i + 1 < epc && key(i + 1) < ki)) bad = true;
       if (ki == 0) ++zl;
     }
   }
-  if (__any_sync(kFullMask, bad)) return PS_UNDEF;
-  const int z = __reduce_add_sync(kFullMask, zl);
+  if (g.any(bad)) return PS_UNDEF;
+  const int z = g.sum(zl);
   const BordersS B{kea, epc, z};
-  for (int e = lane; e < E; e += 32) {
+  for (int e = lane; e < E; e += N) {
     int a = -1, bb = -1;
     const long long kee = w.kee[e], kes = w.kes[e];
     const int en = find_border_s(B, kee);
@@ -520,62 +542,94 @@ __device__ int clip_pair_front_warp(const double* b, int nb, const double* c, in
     }
     w.lr[e] = make_int2(l, lo > l ? lo : l);
   }
-  __syncwarp();
+  g.sync();
   if (lane == 0) {
     w.state[1] = logL;
     w.state[2] = 0;
   }
-  __syncwarp();
+  if constexpr (G::kBlock) {
+    // the box of each group of overlay edges, a lane per edge
+    for (int q = g.warp(); q < edge_groups(nc); q += G::kWarps) {
+      const int j = q * kEdgeGroup + (threadIdx.x & 31);
+      const float inf = __int_as_float(0x7f800000);
+      float4 x = j < nc ? w.fbox[nb + j] : make_float4(inf, inf, -inf, -inf);
+      for (int o = 16; o > 0; o >>= 1) {
+        x.x = fminf(x.x, __shfl_xor_sync(kFullMask, x.x, o));
+        x.y = fminf(x.y, __shfl_xor_sync(kFullMask, x.y, o));
+        x.z = fmaxf(x.z, __shfl_xor_sync(kFullMask, x.z, o));
+        x.w = fmaxf(x.w, __shfl_xor_sync(kFullMask, x.w, o));
+      }
+      if ((threadIdx.x & 31) == 0) w.gbox[q] = x;
+    }
+  }
+  g.sync();
   return PS_OK;
 }
 
-// A8 for one pair by one warp: every base x overlay edge pair, float boxes
-// first; lanes take the pairs in strides of 32 (coalesced overlay boxes)
-// The edge pairs past the float box test and LSMF are queued per warp
-// (kCandQ entries of shared memory) and classified 32 at a time, so that
-// lineSegmentIntersection's FP64 work runs in full warps: only a few pairs in
-// a hundred pass the filters, and FP64 run by a few lanes costs the issue
-// slots of all 32.
+// A8 for one pair: the edge pairs whose float boxes meet and that pass LSMF
+// are queued per warp (kCandQ entries of shared memory) and classified 32 at
+// a time, so that lineSegmentIntersection's FP64 work runs in full warps: only
+// a few pairs in a hundred pass the filters, and FP64 run by a few lanes costs
+// the issue slots of all 32.
 constexpr int kCandQ = 64;
-constexpr long long kSweepMin = 16384;  // pairs with more edge pairs sweep in x
-template <bool kSweep, bool kComp>
-__device__ void clip_pair_cand(const double* b, int nb, const double* c, int nc, const Caps& cp,
-                               PairWork& w, int lane, int2* q) {
-  const unsigned full = 0xffffffffu;
-  // component successors only in the instantiation for batches with them
-  const int* bn = kComp ? w.bnx : nullptr;
-  const int* cn = kComp ? w.cnx : nullptr;
-  const int logL = w.state[1];
+
+__device__ __forceinline__ bool boxes_meet(const float4& fb, const float4& fc) {
+  return !(fb.x > fc.z || fb.z < fc.x || fb.y > fc.w || fb.w < fc.y);
+}
+
+// component successors only in the instantiation for batches with them
+template <bool kComp>
+struct CandQueue {
+  const double* b;
+  int nb;
+  const double* c;
+  int nc;
+  int cap;  // room for hits
+  PairWork& w;
+  int lane;
+  int2* q;
   int nq = 0;  // queued pairs (the same in every lane)
-  auto classify = [&](int count) {
+
+  __device__ int bsucc(int i) const { return vsucc(kComp ? w.bnx : nullptr, nb, i); }
+  __device__ int csucc(int i) const { return vsucc(kComp ? w.cnx : nullptr, nc, i); }
+  __device__ bool lsmf(int be, int j) const {
+    const int bt2 = bsucc(be), ct2 = csucc(j);
+    return lsmf_d(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
+                  bvx(c, nc, j), bvy(c, nc, j), bvx(c, nc, ct2), bvy(c, nc, ct2));
+  }
+  __device__ void classify(int count) {
+    bool hit = false;
+    int be = 0, j = 0, ty = 0;
+    double al = 0.0, bt = 0.0;
+    unsigned long long key = 0;
     if (lane < count) {
       const int2 e = q[lane];
-      const int be = e.x, j = e.y;
-      const int bt2 = vsucc(bn, nb, be), ct2 = vsucc(cn, nc, j);
-      const double p1x = bvx(b, nb, be), p1y = bvy(b, nb, be);
-      const double p2x = bvx(b, nb, bt2), p2y = bvy(b, nb, bt2);
-      const double q1x = bvx(c, nc, j), q1y = bvy(c, nc, j);
-      const double q2x = bvx(c, nc, ct2), q2y = bvy(c, nc, ct2);
-      double al, bt;
-      const int ty = seg_isect(p1x, p1y, p2x, p2y, q1x, q1y, q2x, q2y, &al, &bt);
-      unsigned long long key;
-      if (ty && emission_s(be, nb + j, 2 * j, w, logL, &key) > 0) {
-        // out of room: only counted, for the retry's capacity
-        const int k = atomicAdd(&w.state[2], 1);
-        if (k < cp.K) {
-          w.hb[k] = 2 * be;
-          w.hc[k] = 2 * j;
-          w.ht[k] = ty;
-          w.hkey[k] = key;
-          w.hal[k] = al;
-          w.hbt[k] = bt;
-        }
-      }
+      be = e.x;
+      j = e.y;
+      const int bt2 = bsucc(be), ct2 = csucc(j);
+      ty = seg_isect(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
+                     bvx(c, nc, j), bvy(c, nc, j), bvx(c, nc, ct2), bvy(c, nc, ct2), &al, &bt);
+      hit = ty && emission_s(be, nb + j, 2 * j, w, w.state[1], &key) > 0;
+    }
+    // one counter step per warp; out of room: only counted, for the retry's
+    // capacity
+    const unsigned m = __ballot_sync(kFullMask, hit);
+    int k0 = 0;
+    if (lane == 0 && m) k0 = atomicAdd(&w.state[2], __popc(m));
+    k0 = __shfl_sync(kFullMask, k0, 0);
+    const int k = k0 + __popc(m & ((1u << lane) - 1u));
+    if (hit && k < cap) {
+      w.hb[k] = 2 * be;
+      w.hc[k] = 2 * j;
+      w.ht[k] = ty;
+      w.hkey[k] = key;
+      w.hal[k] = al;
+      w.hbt[k] = bt;
     }
     __syncwarp();
-  };
-  auto enqueue = [&](bool pass, int be, int j) {
-    const unsigned m = __ballot_sync(full, pass);
+  }
+  __device__ void add(bool pass, int be, int j) {
+    const unsigned m = __ballot_sync(kFullMask, pass);
     if (m == 0u) return;  // nothing to queue (the same on every lane)
     if (pass) q[nq + __popc(m & ((1u << lane) - 1u))] = make_int2(be, j);
     nq += __popc(m);
@@ -589,102 +643,66 @@ __device__ void clip_pair_cand(const double* b, int nb, const double* c, int nc,
       nq = rest;
       __syncwarp();
     }
-  };
-  auto boxes_meet = [](const float4& fb, const float4& fc) {
-    return !(fb.x > fc.z || fb.z < fc.x || fb.y > fc.w || fb.w < fc.y);
-  };
-  if constexpr (kSweep) {
-    // Sweep in x: the overlay edges ordered by box min x (float order key,
-    // -0 as +0); a base edge's candidates are the overlay edges with min x
-    // in [its min x - the largest overlay x extent, its max x], every
-    // box-overlapping pair among them.  The order comes from the front's
-    // stable endpoint sort (w.sidx, by the exact x keys, so by the rounded-
-    // down float keys as well): the overlay edges' min-x endpoints, compacted
-    auto fk = [](float f) {
-      const unsigned u = __float_as_uint(f == 0.f ? 0.f : f);
-      return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-    };
-    {
-      const int n2 = 2 * (nb + nc);
-      int cnt = 0;
-      for (int i0 = 0; i0 < n2; i0 += 32) {
-        const int i = i0 + lane;
-        const int id = i < n2 ? w.sidx[i] : 1;
-        const bool take = !(id & 1) && (id >> 1) >= nb;
-        const unsigned m = __ballot_sync(full, take);
-        if (take) {
-          const int k = (id >> 1) - nb, at = cnt + __popc(m & ((1u << lane) - 1u));
-          const float4 bx = w.fbox[nb + k];
-          w.csort[at] = ((unsigned long long)fk(bx.x) << 32) | (unsigned)k;
-          w.sbox[at] = bx;
-        }
-        cnt += __popc(m);
-      }
-      __syncwarp();
-    }
-    float ext = 0.f;
-    for (int k = lane; k < nc; k += 32) ext = fmaxf(ext, __fsub_ru(w.fbox[nb + k].z, w.fbox[nb + k].x));
-    for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(full, ext, o));
-    // first sorted position whose min-x key exceeds kx (or reaches it: ge)
-    auto bound = [&](unsigned kx, bool ge) {
-      int lo = 0, hi = nc;
-      while (lo < hi) {
-        const int m = (lo + hi) >> 1;
-        const unsigned km = (unsigned)(w.csort[m] >> 32);
-        if (ge ? km < kx : km <= kx) lo = m + 1;
-        else hi = m;
-      }
-      return lo;
-    };
-    for (int be0 = 0; be0 < nb; be0 += 32) {
-      const int be = be0 + lane;
-      int k = 0, kend = 0;
-      float4 fb = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (be < nb) {
-        fb = w.fbox[be];
-        k = bound(fk(__fsub_rd(fb.x, ext)), true);
-        kend = bound(fk(fb.z), false);
-      }
-      while (__any_sync(full, k < kend)) {
-        bool pass = false;
-        int j = 0;
-        if (k < kend) {
-          const bool meet = boxes_meet(fb, w.sbox[k]);  // the boxes in sweep order
-          if (meet) j = (int)(unsigned)w.csort[k];
-          ++k;
-          if (meet) {
-            const int bt2 = vsucc(bn, nb, be), ct2 = vsucc(cn, nc, j);
-            pass = lsmf_d(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
-                          bvx(c, nc, j), bvy(c, nc, j), bvx(c, nc, ct2), bvy(c, nc, ct2));
-          }
-        }
-        enqueue(pass, be, j);
-      }
-    }
-    if (nq > 0) classify(nq);
-    return;
-  } else {
-    int be = 0, j = lane;
+  }
+};
+
+// every base x overlay edge pair of a small pair by one warp; lanes take the
+// pairs in strides of 32 (coalesced overlay boxes)
+template <bool kComp>
+__device__ void clip_pair_cand(CandQueue<kComp>& cq) {
+  const PairWork& w = cq.w;
+  const int nb = cq.nb, nc = cq.nc;
+  int be = 0, j = cq.lane;
+  while (j >= nc && be < nb) {
+    j -= nc;
+    ++be;
+  }
+  while (__any_sync(kFullMask, be < nb)) {
+    const bool pass = be < nb && boxes_meet(w.fbox[be], w.fbox[nb + j]) && cq.lsmf(be, j);
+    cq.add(pass, be, j);
+    j += 32;
     while (j >= nc && be < nb) {
       j -= nc;
       ++be;
     }
-    while (__any_sync(full, be < nb)) {
-      bool pass = false;
-      if (be < nb && boxes_meet(w.fbox[be], w.fbox[nb + j])) {
-        const int bt2 = vsucc(bn, nb, be), ct2 = vsucc(cn, nc, j);
-        pass = lsmf_d(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
-                      bvx(c, nc, j), bvy(c, nc, j), bvx(c, nc, ct2), bvy(c, nc, ct2));
-      }
-      enqueue(pass, be, j);
-      j += 32;
-      while (j >= nc && be < nb) {
-        j -= nc;
-        ++be;
+  }
+  if (cq.nq > 0) cq.classify(cq.nq);
+}
+
+// base edges [be0, be0 + 32) of a wide pair, a lane each, against the overlay
+// by one warp: consecutive edges lie near one another, so the box of the 32
+// base edges is tested against the boxes of the overlay's groups first (a
+// lane per group), and each group that meets it is walked edge by edge, its
+// boxes read by the whole warp at once (box: kEdgeGroup entries of shared
+// memory)
+template <bool kComp>
+__device__ void clip_pair_cand_group(CandQueue<kComp>& cq, int be0, float4* box) {
+  const PairWork& w = cq.w;
+  const int nb = cq.nb, nc = cq.nc, lane = cq.lane, ng = edge_groups(nc);
+  const int be = be0 + lane;
+  const float inf = __int_as_float(0x7f800000);
+  const float4 fb = be < nb ? w.fbox[be] : make_float4(inf, inf, -inf, -inf);
+  float4 all = fb;
+  for (int o = 16; o > 0; o >>= 1) {
+    all.x = fminf(all.x, __shfl_xor_sync(kFullMask, all.x, o));
+    all.y = fminf(all.y, __shfl_xor_sync(kFullMask, all.y, o));
+    all.z = fmaxf(all.z, __shfl_xor_sync(kFullMask, all.z, o));
+    all.w = fmaxf(all.w, __shfl_xor_sync(kFullMask, all.w, o));
+  }
+  for (int g0 = 0; g0 < ng; g0 += 32) {
+    const bool meet = g0 + lane < ng && boxes_meet(all, w.gbox[g0 + lane]);
+    for (unsigned m = __ballot_sync(kFullMask, meet); m; m &= m - 1) {
+      const int j0 = (g0 + __ffs(m) - 1) * kEdgeGroup, n = min(kEdgeGroup, nc - j0);
+      __syncwarp();
+      if (lane < n) box[lane] = w.fbox[nb + j0 + lane];
+      __syncwarp();
+      for (int t = 0; t < n; ++t) {
+        const bool pass = boxes_meet(fb, box[t]) && cq.lsmf(be, j0 + t);
+        cq.add(pass, be, j0 + t);
       }
     }
-    if (nq > 0) classify(nq);
   }
+  if (cq.nq > 0) cq.classify(cq.nq);
 }
 
 // A9-A13: records, counts, alpha order, merged arrays (one thread per pair)
@@ -1156,6 +1174,11 @@ struct ClipArgs {
   // component, indexed like bxy / cxy (null: every polygon one ring)
   const int* bnx = nullptr;
   const int* cnx = nullptr;
+  // the wide pairs among them, largest first, and the first of each one's
+  // base edge groups in the order of the candidate stage's warps (nwide + 1)
+  const int* wide = nullptr;
+  const int* wide_item = nullptr;
+  int nwide = 0, nitems = 0, wide_min = 0;
   __device__ bool small(int p, int* nb, int* nc) const {
     *nb = (int)(boff[p + 1] - boff[p]);
     *nc = (int)(coff[p + 1] - coff[p]);
@@ -1176,6 +1199,15 @@ struct ClipArgs {
   }
 };
 
+__device__ __forceinline__ void front_done(const ClipArgs& A, int p, PairWork& w, int st) {
+  w.state[0] = st;
+  if (st != PS_OK) {
+    A.status[p] = st == PS_UNDEF ? SBC_EUNDEF : SBC_ENOMEM;
+    A.nrings[p] = A.nverts[p] = 0;
+    A.area[p] = 0.0;
+  }
+}
+
 __global__ void __launch_bounds__(128) k_batch_front(ClipArgs A) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -1192,24 +1224,38 @@ __global__ void __launch_bounds__(128) k_batch_front(ClipArgs A) {
     }
     return;
   }
+  if (wide_pair(nb, nc, A.wide_min)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
-  const int st =
-      clip_pair_front_warp(A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp, w, lane);
-  if (lane == 0) {
-    w.state[0] = st;
-    if (st != PS_OK) {
-      A.status[p] = st == PS_UNDEF ? SBC_EUNDEF : SBC_ENOMEM;
-      A.nrings[p] = A.nverts[p] = 0;
-      A.area[p] = 0.0;
-    }
-  }
+  WarpGroup g;
+  const int st = clip_pair_front(g, A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp, w,
+                                 nullptr, nullptr, 0, nullptr);
+  if (lane == 0) front_done(A, p, w, st);
 }
 
-// instantiations with their own register budgets: the all-pairs test for
-// pairs up to kSweepMin edge pairs, the x sweep above; each with or without
-// component successors
-template <bool kSweep, bool kComp>
+// the front of the wide pairs, a block each; pairs of up to 1,024 edges (the
+// endpoints padded to a power of two) sort in shared memory
+constexpr int kFrontSort = 2048;
+__global__ void __launch_bounds__(kWideBlock) k_batch_front_wide(ClipArgs A) {
+  using G = BlockGroup<kWideBlock>;
+  __shared__ G::Shared sh;
+  __shared__ FrontRange s_range[G::kWarps];
+  __shared__ long long s_key[kFrontSort];
+  __shared__ int s_val[kFrontSort];
+  const int p = A.wide[blockIdx.x];
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  int nb, nc;
+  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  Caps cp;
+  PairWork w = A.work(p, nb, nc, pass, &cp);
+  G g(&sh);
+  const int st = clip_pair_front(g, A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp, w,
+                                 s_key, s_val, kFrontSort, s_range);
+  if (threadIdx.x == 0) front_done(A, p, w, st);
+}
+
+// the all-pairs test of the small pairs, with or without component successors
+template <bool kComp>
 __global__ void __launch_bounds__(128) k_batch_cand(ClipArgs A) {
   __shared__ int2 s_q[4][kCandQ];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1218,12 +1264,38 @@ __global__ void __launch_bounds__(128) k_batch_cand(ClipArgs A) {
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
+  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
+  Caps cp;
+  PairWork w = A.work(p, nb, nc, pass, &cp);
+  if (w.state[0] != PS_OK) return;
+  CandQueue<kComp> cq{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp.K, w, lane,
+                      s_q[threadIdx.x >> 5]};
+  clip_pair_cand(cq);
+}
+
+// the wide pairs, a warp per group of base edges
+template <bool kComp>
+__global__ void __launch_bounds__(128) k_batch_cand_wide(ClipArgs A) {
+  __shared__ int2 s_q[4][kCandQ];
+  __shared__ float4 s_box[4][kEdgeGroup];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int item = blockIdx.x * 4 + wi;
+  if (item >= A.nitems) return;
+  int lo = 0, hi = A.nwide - 1;  // the pair holding the item
+  while (lo < hi) {
+    const int m = (lo + hi + 1) >> 1;
+    if (A.wide_item[m] <= item) lo = m;
+    else hi = m - 1;
+  }
+  const int p = A.wide[lo];
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  int nb, nc;
   if (pass < 0 || !A.small(p, &nb, &nc)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
-  if (w.state[0] != PS_OK || ((long long)nb * nc > kSweepMin) != kSweep) return;
-  clip_pair_cand<kSweep, kComp>(A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp, w,
-                                lane, s_q[threadIdx.x >> 5]);
+  if (w.state[0] != PS_OK) return;
+  CandQueue<kComp> cq{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp.K, w, lane, s_q[wi]};
+  clip_pair_cand_group(cq, (item - A.wide_item[lo]) * kEdgeGroup, s_box[wi]);
 }
 
 // The back end in three kernels: A9-A13 on one thread per pair, the labels
@@ -1289,20 +1361,23 @@ __device__ __forceinline__ unsigned ptab_slot(long long kx, long long ky, int ma
   return (unsigned)(h >> 32) & (unsigned)mask;
 }
 
-__device__ void pair_tape_warp(const double* b, int nb, const double* c, int nc, const PwWork& pw,
-                               int K, PairWork& w, int nv, int lane) {
+template <class G>
+__device__ void pair_tape(G& g, const double* b, int nb, const double* c, int nc, const PwWork& pw,
+                          int K, PairWork& w, int nv) {
+  const int lane = g.rank();
+  constexpr int N = G::N;
   const int T = w.ptabn, mask = T - 1;
-  for (int i = lane; i < T; i += 32) {
+  for (int i = lane; i < T; i += N) {
     w.ptab[i] = -1;
     w.pbest[i] = INT_MAX;
   }
-  __syncwarp();
+  g.sync();
   auto cx = [&](int t) { return t < nb ? b[2 * t] : (t < nb + nc ? c[2 * (t - nb)] : pw.isxy[2 * (t - nb - nc)]); };
   auto cy = [&](int t) {
     return t < nb ? b[2 * t + 1] : (t < nb + nc ? c[2 * (t - nb) + 1] : pw.isxy[2 * (t - nb - nc) + 1]);
   };
   const int ncand = nb + nc + K;
-  for (int t = lane; t < ncand; t += 32) {
+  for (int t = lane; t < ncand; t += N) {
     if (t >= nb + nc && pw.ut[t - nb - nc] != 1) continue;  // crossings only
     const long long kx = okey(cx(t)), ky = okey(cy(t));
     unsigned h = ptab_slot(kx, ky, mask);
@@ -1315,8 +1390,8 @@ __device__ void pair_tape_warp(const double* b, int nb, const double* c, int nc,
       h = (h + 1) & (unsigned)mask;
     }
   }
-  __syncwarp();
-  for (int v = lane; v < nv; v += 32) {
+  g.sync();
+  for (int v = lane; v < nv; v += N) {
     const long long kx = okey(w.rxy[2 * v]), ky = okey(w.rxy[2 * v + 1]);
     unsigned h = ptab_slot(kx, ky, mask);
     int best = -1;
@@ -1335,7 +1410,74 @@ __device__ void pair_tape_warp(const double* b, int nb, const double* c, int nc,
     else if (best >= nb + nc) tp = make_int4(2, pw.ub[best - nb - nc] >> 1, pw.uc[best - nb - nc] >> 1, 0);
     w.tape[v] = tp;
   }
-  __syncwarp();
+  g.sync();
+}
+
+// A9: the hits in the reference's order (base edge, then first emission;
+// distinct keys) into w.phit: a counting sort by base edge, then each edge's
+// few hits by their keys.  (A bitonic network over all hits re-read two keys
+// per compare: 120 rounds for 20,000 hits.)
+template <class G>
+__device__ void order_hits(G& g, PairWork& w, int nb, int K) {
+  const int lane = g.rank();
+  constexpr int N = G::N;
+  int* start = w.bAll;
+  int* fill = w.bND;
+  for (int i = lane; i <= nb; i += N) start[i] = fill[i] = 0;
+  g.sync();
+  for (int h = lane; h < K; h += N) atomicAdd(&start[w.hb[h] >> 1], 1);
+  g.sync();
+  group_scan(g, start, nb + 1);
+  g.sync();
+  for (int h = lane; h < K; h += N) {
+    const int e = w.hb[h] >> 1;
+    w.hsort[start[e] + atomicAdd(&fill[e], 1)] = h;
+  }
+  g.sync();
+  group_items(
+      g, nb, w.pw.htmp,
+      [&](int e) {
+        const int m = start[e + 1] - start[e];
+        return m > 1 ? m : 0;
+      },
+      [&](int e) {
+        int* v = w.hsort + start[e];
+        const int m = start[e + 1] - start[e];
+        for (int i = 1; i < m; ++i) {
+          const int x = v[i];
+          const unsigned long long kx = w.hkey[x];
+          int j = i;
+          while (j > 0 && w.hkey[v[j - 1]] > kx) {
+            v[j] = v[j - 1];
+            --j;
+          }
+          v[j] = x;
+        }
+      },
+      [&](auto& gg, int e) {
+        // a network over hit indices, compared by their keys
+        const int s = start[e], m = start[e + 1] - s, np = npow2_dev(m);
+        unsigned long long* scr = w.pw.sscr + 2 * s;
+        for (int k = gg.rank(); k < np; k += gg.N) scr[k] = k < m ? w.hsort[s + k] : ~0ull;
+        gg.sync();
+        group_bitonic(gg, np, [&](int x, int y, bool up) {
+          const unsigned long long hx = scr[x], hy = scr[y];
+          const bool gt = hx == ~0ull ? hy != ~0ull : (hy != ~0ull && w.hkey[hx] > w.hkey[hy]);
+          const bool lt = hy == ~0ull ? hx != ~0ull : (hx != ~0ull && w.hkey[hx] < w.hkey[hy]);
+          if (up ? gt : lt) {
+            scr[x] = hy;
+            scr[y] = hx;
+          }
+        });
+        for (int k = gg.rank(); k < m; k += gg.N) w.hsort[s + k] = (int)scr[k];
+        gg.sync();
+      });
+  g.sync();
+  for (int i = lane; i < K; i += N) {
+    const int h = w.hsort[i];
+    w.phit[i] = PwHit{0, w.hb[h] >> 1, w.hc[h] >> 1, w.ht[h], w.hkey[h], w.hal[h], w.hbt[h]};
+  }
+  g.sync();
 }
 
 // One warp per pair, in two kernels: the records in the reference's order
@@ -1354,7 +1496,7 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw(ClipArgs A) {
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK) return;
@@ -1368,41 +1510,10 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw(ClipArgs A) {
     if (lane == 0) w.state[3] = 1;
     return;
   }
-  // A9 order (base id, then first emission; the hit index breaks ties, as a
-  // stable sort of the hits in index order would): a bitonic network over
-  // the hit indices, the lanes on compare-exchange pairs
-  {
-    const int np = npow2_dev(K);
-    for (int m = lane; m < np; m += 32) w.hsort[m] = m < K ? m : INT_MAX;
-    __syncwarp();
-    auto less = [&](int x, int y) {
-      if (y == INT_MAX) return x != INT_MAX;
-      if (x == INT_MAX) return false;
-      if (w.hb[x] != w.hb[y]) return w.hb[x] < w.hb[y];
-      if (w.hkey[x] != w.hkey[y]) return w.hkey[x] < w.hkey[y];
-      return x < y;
-    };
-    for (int k = 2; k <= np; k <<= 1)
-      for (int j = k >> 1; j > 0; j >>= 1) {
-        for (int q = lane; q < (np >> 1); q += 32) {
-          const int m = ((q & ~(j - 1)) << 1) | (q & (j - 1)), l = m | j;
-          const int x = w.hsort[m], y = w.hsort[l];
-          if (less(y, x) == ((m & k) == 0)) {
-            w.hsort[m] = y;
-            w.hsort[l] = x;
-          }
-        }
-        __syncwarp();
-      }
-  }
-  for (int i = lane; i < K; i += 32) {
-    const int h = w.hsort[i];
-    w.phit[i] = PwHit{0, w.hb[h] >> 1, w.hc[h] >> 1, w.ht[h], w.hkey[h], w.hal[h], w.hbt[h]};
-  }
-  __syncwarp();
+  WarpGroup g;
+  order_hits(g, w, nb, K);
   PwWork pw = w.pw;
   PwMid mid;
-  WarpGroup g;
   const int st = pw_clip_head(g, A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.phit,
                               pw_caps(nb, nc, K, 1), pw, &mid);
   if (st == PS_UNDEF) {
@@ -1422,7 +1533,7 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw2(ClipArgs A) {
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK || w.state[3] != 2) return;
@@ -1448,13 +1559,97 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw2(ClipArgs A) {
   for (int r = lane; r <= nr; r += 32) w.roff[r] = pw.roff[r];
   for (int i = lane; i < 2 * nv; i += 32) w.rxy[i] = pw.rxy[i];
   __syncwarp();
-  pair_tape_warp(b, nb, c, nc, pw, K, w, nv, lane);
+  pair_tape(g, b, nb, c, nc, pw, K, w, nv);
   if (lane == 0) {
     w.state[3] = 0;
     A.status[p] = SBC_OK;
     A.nrings[p] = nr;
     A.nverts[p] = nv;
     A.area[p] = 0.0;  // k_batch_area
+  }
+}
+
+// Each ring vertex's successor and predecessor on its ring (capR entries).
+template <class G>
+__device__ void ring_links(G& g, const int* roff, int nr, int nv, int* next, int* prev) {
+  for (int v = g.rank(); v < nv; v += G::N) {
+    next[v] = v + 1;
+    prev[v] = v - 1;
+  }
+  g.sync();
+  for (int r = g.rank(); r < nr; r += G::N) {
+    const int s = roff[r], e = roff[r + 1];
+    if (e > s) {
+      next[e - 1] = s;
+      prev[s] = e - 1;
+    }
+  }
+  g.sync();
+}
+
+// Rows A9-A18, provenance and area of the wide pairs, a block each, in one
+// kernel: a block's warps are at the same step, so its code size does not
+// cost instruction fetches as a warp per pair's does.
+__global__ void __launch_bounds__(kWideBlock, 2) k_batch_pw_wide(ClipArgs A) {
+  using G = BlockGroup<kWideBlock>;
+  __shared__ G::Shared sh;
+  __shared__ double s_sum[G::kWarps];
+  const int p = A.wide[blockIdx.x];
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  int nb, nc;
+  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  Caps cp;
+  PairWork w = A.work(p, nb, nc, pass, &cp);
+  if (w.state[0] != PS_OK) return;
+  const int K = w.state[2];
+  if (K > cp.K) {
+    __syncthreads();
+    if (threadIdx.x == 0) batch_fail(A, p, w, PS_CAP, K);
+    return;
+  }
+  if (A.multi(p, nb, nc)) {
+    if (threadIdx.x == 0) w.state[3] = 1;
+    return;
+  }
+  G g(&sh);
+  const int lane = g.rank();
+  order_hits(g, w, nb, K);
+  const double* b = A.bxy + 2 * A.boff[p];
+  const double* c = A.cxy + 2 * A.coff[p];
+  PwWork pw = w.pw;
+  int nr = 0, nv = 0;
+  const int st = pw_clip_core(g, b, nb, c, nc, w.phit, pw_caps(nb, nc, K, 1), pw,
+                              PipSmall{b, nb, nullptr, 0}, A.unite, &nr, &nv);
+  if (st == PS_UNDEF) {
+    if (lane == 0) batch_fail(A, p, w, PS_UNDEF, 0);
+    return;
+  }
+  if (st != PS_OK) {
+    if (lane == 0) w.state[3] = 1;  // the thread back end takes the pair
+    return;
+  }
+  for (int r = lane; r <= nr; r += G::N) w.roff[r] = pw.roff[r];
+  for (int i = lane; i < 2 * nv; i += G::N) w.rxy[i] = pw.rxy[i];
+  g.sync();
+  pair_tape(g, b, nb, c, nc, pw, K, w, nv);
+  // the area: every ring's shoelace terms in one sum, in an order fixed by
+  // the rings and the block size
+  ring_links(g, w.roff, nr, nv, pw.R.next, pw.R.prev);
+  double s2 = 0.0;
+  for (int v = lane; v < nv; v += G::N) {
+    const int u = pw.R.next[v];
+    s2 = dadd(s2, dsub(dmul(w.rxy[2 * v], w.rxy[2 * u + 1]), dmul(w.rxy[2 * u], w.rxy[2 * v + 1])));
+  }
+  for (int o = 16; o > 0; o >>= 1) s2 = dadd(s2, __shfl_xor_sync(kFullMask, s2, o));
+  if ((lane & 31) == 0) s_sum[g.warp()] = s2;
+  g.sync();
+  if (lane == 0) {
+    for (int k = 1; k < G::kWarps; ++k) s2 = dadd(s2, s_sum[k]);
+    w.state[3] = 0;
+    A.status[p] = SBC_OK;
+    A.nrings[p] = nr;
+    A.nverts[p] = nv;
+    A.area[p] = dmul(0.5, s2);
   }
 }
 
@@ -1516,6 +1711,7 @@ __global__ void __launch_bounds__(128) k_batch_area(ClipArgs A) {
   if (pass < 0 || !A.small(p, &nb, &nc) || A.status[p] != SBC_OK) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
+  if (wide_pair(nb, nc, A.wide_min) && w.state[3] == 0) return;  // k_batch_pw_wide's
   const double a = pair_area_warp(w.roff, w.rxy, A.nrings[p], lane);
   if (lane == 0) A.area[p] = a;
 }
@@ -1532,31 +1728,39 @@ __global__ void k_graph_passes(int n, const int* __restrict__ pass, const int* _
 
 // block sizes (threads) of the three kernels: tuning knobs, each at most
 // kBatchBlock (128) and a multiple of 32
-// the batch's component successors (null: one ring per polygon)
-ClipArgs with_components(ClipArgs a, const int* bnx, const int* cnx) {
+// the batch's component successors (null: one ring per polygon) and the
+// chunk's wide pairs
+ClipArgs with_extras(ClipArgs a, const int* bnx, const int* cnx, const int* wide,
+                     const int* wide_item, int nwide, int nitems, int wide_min) {
   a.bnx = bnx;
   a.cnx = cnx;
+  a.wide = wide;
+  a.wide_item = wide_item;
+  a.nwide = nwide;
+  a.nitems = nitems;
+  a.wide_min = wide_min;
   return a;
 }
 
 void launch_clip(const ClipArgs& A, const BatchShape& sh, double in_bytes, cudaStream_t st) {
+  const bool comps = A.bnx || A.cnx;
   {
     ::sbc::KProbe kp_("k_batch_front", st, in_bytes);
     k_batch_front<<<grid_for(32LL * A.np, sh.front), sh.front, 0, st>>>(A);
   }
-  {
-    ::sbc::KProbe kp_("k_batch_cand", st, in_bytes);
-    if (A.bnx || A.cnx)
-      k_batch_cand<false, true><<<grid_for(32LL * A.np, sh.cand), sh.cand, 0, st>>>(A);
-    else
-      k_batch_cand<false, false><<<grid_for(32LL * A.np, sh.cand), sh.cand, 0, st>>>(A);
+  if (A.nwide > 0) {
+    ::sbc::KProbe kp_("k_batch_front_wide", st);
+    k_batch_front_wide<<<A.nwide, kWideBlock, 0, st>>>(A);
   }
   {
-    ::sbc::KProbe kp_("k_batch_cand_sweep", st);
-    if (A.bnx || A.cnx)
-      k_batch_cand<true, true><<<grid_for(32LL * A.np, sh.cand), sh.cand, 0, st>>>(A);
-    else
-      k_batch_cand<true, false><<<grid_for(32LL * A.np, sh.cand), sh.cand, 0, st>>>(A);
+    ::sbc::KProbe kp_("k_batch_cand", st, in_bytes);
+    if (comps) k_batch_cand<true><<<grid_for(32LL * A.np, sh.cand), sh.cand, 0, st>>>(A);
+    else k_batch_cand<false><<<grid_for(32LL * A.np, sh.cand), sh.cand, 0, st>>>(A);
+  }
+  if (A.nwide > 0) {
+    ::sbc::KProbe kp_("k_batch_cand_wide", st);
+    if (comps) k_batch_cand_wide<true><<<grid_for(A.nitems, 4), 128, 0, st>>>(A);
+    else k_batch_cand_wide<false><<<grid_for(A.nitems, 4), 128, 0, st>>>(A);
   }
   {
     ::sbc::KProbe kp_("k_batch_pw", st, in_bytes + 20.0 * A.np);
@@ -1566,7 +1770,10 @@ void launch_clip(const ClipArgs& A, const BatchShape& sh, double in_bytes, cudaS
     ::sbc::KProbe kp_("k_batch_pw2", st, in_bytes);
     k_batch_pw2<<<grid_for(32LL * A.np, 128), 128, 0, st>>>(A);
   }
-
+  if (A.nwide > 0) {
+    ::sbc::KProbe kp_("k_batch_pw_wide", st);
+    k_batch_pw_wide<<<A.nwide, kWideBlock, 0, st>>>(A);
+  }
   {
     ::sbc::KProbe kp_("k_batch_back", st, in_bytes);
     k_batch_back<<<grid_for(A.np, sh.back), sh.back, 0, st>>>(A);
@@ -1634,6 +1841,45 @@ __global__ void k_batch_pack(int np, const long long* __restrict__ boff,
   for (int i = lane; i < 2 * nv; i += 32) xy[2 * v0 + i] = w.rxy[i];
 }
 
+// The gradient (gx, gy) of a crossing's coordinates chained to the ends of its
+// edges b1b2 and c1c2: I = (1 - alpha) b1 + alpha b2, alpha = A1 / (A1 - A2),
+// A1 = A(b1, c1, c2), A2 = A(b2, c1, c2); A(P, Q, R) partials: dP = (Qy - Ry,
+// Rx - Qx), dQ = (Ry - Py, Px - Rx), dR = (Py - Qy, Qx - Px)
+struct CrossGrad {
+  double gx, gy, b1x, b1y, b2x, b2y, c1x, c1y, c2x, c2y, al, k1, k2;
+  __device__ __forceinline__ CrossGrad(const double* b, int i1, int i2, const double* c, int j1,
+                                       int j2, double gx_, double gy_)
+      : gx(gx_), gy(gy_) {
+    b1x = b[2 * i1];
+    b1y = b[2 * i1 + 1];
+    b2x = b[2 * i2];
+    b2y = b[2 * i2 + 1];
+    c1x = c[2 * j1];
+    c1y = c[2 * j1 + 1];
+    c2x = c[2 * j2];
+    c2y = c[2 * j2 + 1];
+    const double A1 = (c1x - b1x) * (c2y - b1y) - (c1y - b1y) * (c2x - b1x);
+    const double A2 = (c1x - b2x) * (c2y - b2y) - (c1y - b2y) * (c2x - b2x);
+    const double d = A1 - A2;
+    al = A1 / d;
+    const double ga = gx * (b2x - b1x) + gy * (b2y - b1y);  // dA/dalpha
+    k1 = -A2 / (d * d) * ga;  // dalpha/dA1
+    k2 = A1 / (d * d) * ga;   // dalpha/dA2
+  }
+  __device__ __forceinline__ double2 b1() const {
+    return make_double2((1.0 - al) * gx + k1 * (c1y - c2y), (1.0 - al) * gy + k1 * (c2x - c1x));
+  }
+  __device__ __forceinline__ double2 b2() const {
+    return make_double2(al * gx + k2 * (c1y - c2y), al * gy + k2 * (c2x - c1x));
+  }
+  __device__ __forceinline__ double2 c1() const {
+    return make_double2(k1 * (c2y - b1y) + k2 * (c2y - b2y), k1 * (b1x - c2x) + k2 * (b2x - c2x));
+  }
+  __device__ __forceinline__ double2 c2() const {
+    return make_double2(k1 * (b1y - c1y) + k2 * (b2y - c1y), k1 * (c1x - b1x) + k2 * (c1x - b2x));
+  }
+};
+
 // d(area)/d(vertices), one warp per pair, from the forward pass's tape.  The
 // lanes take 32 ring vertices at a time and compute their contributions
 // (the crossings' FP64 chain rule in parallel, up to four target vertices
@@ -1646,12 +1892,14 @@ k_batch_backward(int np, const double* __restrict__ bxy, const long long* __rest
                  const double* __restrict__ cxy, const long long* __restrict__ coff, Arenas ar,
                  const int* __restrict__ status, const int* __restrict__ nrings,
                  const double* __restrict__ gA, const int* __restrict__ bnx,
-                 const int* __restrict__ cnx, double* __restrict__ gb, double* __restrict__ gc) {
+                 const int* __restrict__ cnx, int wide_min, double* __restrict__ gb,
+                 double* __restrict__ gc) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   if ((t >> 5) >= np) return;
   const int p = (int)(t >> 5);
   const int nb = (int)(boff[p + 1] - boff[p]), nc = (int)(coff[p + 1] - coff[p]);
+  if (ar.pass[p] >= 0 && wide_pair(nb, nc, wide_min)) return;  // k_batch_backward_wide
   double* gbp = gb + 2 * boff[p];
   double* gcp = gc + 2 * coff[p];
   for (int i = lane; i < 2 * nb; i += 32) gbp[i] = 0.0;
@@ -1683,30 +1931,16 @@ k_batch_backward(int np, const double* __restrict__ bxy, const long long* __rest
           tg[0] = (tp.x << 30) | tp.y;
           vv[0] = make_double2(gx, gy);
         } else if (tp.x == 2) {
-          // I = (1 - alpha) b1 + alpha b2, alpha = A1 / (A1 - A2),
-          // A1 = A(b1, c1, c2), A2 = A(b2, c1, c2)
           const int i1 = tp.y, i2 = vsucc(bn, nb, tp.y), j1 = tp.z, j2 = vsucc(cn, nc, tp.z);
-          const double b1x = b[2 * i1], b1y = b[2 * i1 + 1], b2x = b[2 * i2], b2y = b[2 * i2 + 1];
-          const double c1x = c[2 * j1], c1y = c[2 * j1 + 1], c2x = c[2 * j2], c2y = c[2 * j2 + 1];
-          const double A1 = (c1x - b1x) * (c2y - b1y) - (c1y - b1y) * (c2x - b1x);
-          const double A2 = (c1x - b2x) * (c2y - b2y) - (c1y - b2y) * (c2x - b2x);
-          const double d = A1 - A2;
-          const double al = A1 / d;
-          const double ga = gx * (b2x - b1x) + gy * (b2y - b1y);  // dA/dalpha
-          const double k1 = -A2 / (d * d) * ga, k2 = A1 / (d * d) * ga;  // dalpha/dA1, dalpha/dA2
-          // A(P, Q, R) partials: dP = (Qy - Ry, Rx - Qx), dQ = (Ry - Py, Px - Rx),
-          // dR = (Py - Qy, Qx - Px)
+          const CrossGrad k(b, i1, i2, c, j1, j2, gx, gy);
           tg[0] = i1;
-          vv[0] = make_double2((1.0 - al) * gx + k1 * (c1y - c2y),
-                               (1.0 - al) * gy + k1 * (c2x - c1x));
+          vv[0] = k.b1();
           tg[1] = i2;
-          vv[1] = make_double2(al * gx + k2 * (c1y - c2y), al * gy + k2 * (c2x - c1x));
+          vv[1] = k.b2();
           tg[2] = (1 << 30) | j1;
-          vv[2] = make_double2(k1 * (c2y - b1y) + k2 * (c2y - b2y),
-                               k1 * (b1x - c2x) + k2 * (b2x - c2x));
+          vv[2] = k.c1();
           tg[3] = (1 << 30) | j2;
-          vv[3] = make_double2(k1 * (b1y - c1y) + k2 * (b2y - c1y),
-                               k1 * (c1x - b1x) + k2 * (c1x - b2x));
+          vv[3] = k.c2();
         }
       }
 #pragma unroll
@@ -1730,6 +1964,145 @@ k_batch_backward(int np, const double* __restrict__ bxy, const long long* __rest
         __syncwarp();
       }
     }
+  }
+}
+
+// The wide pairs' gradients, a block each, gathered: a ring vertex that is
+// vertex e, and a crossing on edge e, go on edge e's list (a counting sort by
+// edge); a thread per edge adds up its list in ring order, the part of the
+// edge's far end kept aside and added to that vertex last.  A crossing is
+// computed for each of its two edges, and every sum has an order fixed by the
+// rings.  (One warp per pair added its groups to global memory 32 ring
+// vertices at a time: 14.1 ms for 12,000 pairs of 3 to 2,048 vertices.)
+__global__ void __launch_bounds__(kWideBlock)
+k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ bxy,
+                      const long long* __restrict__ boff, const double* __restrict__ cxy,
+                      const long long* __restrict__ coff, Arenas ar,
+                      const int* __restrict__ status, const int* __restrict__ nrings,
+                      const double* __restrict__ gA, const int* __restrict__ bnx,
+                      const int* __restrict__ cnx, double* __restrict__ gb,
+                      double* __restrict__ gc) {
+  using G = BlockGroup<kWideBlock>;
+  __shared__ G::Shared sh;
+  constexpr int N = G::N;
+  const int p = wide[blockIdx.x];
+  if (ar.pass[p] < 0) return;
+  const int nb = (int)(boff[p + 1] - boff[p]), nc = (int)(coff[p + 1] - coff[p]);
+  double* gbp = gb + 2 * boff[p];
+  double* gcp = gc + 2 * coff[p];
+  const int nr = nrings[p];
+  if (status[p] != SBC_OK || nr == 0) {
+    for (int i = threadIdx.x; i < 2 * nb; i += N) gbp[i] = 0.0;
+    for (int i = threadIdx.x; i < 2 * nc; i += N) gcp[i] = 0.0;
+    return;
+  }
+  G grp(&sh);
+  const int lane = grp.rank();
+  const double* b = bxy + 2 * boff[p];
+  const double* c = cxy + 2 * coff[p];
+  const int* bn = bnx ? bnx + boff[p] : nullptr;
+  const int* cn = cnx ? cnx + coff[p] : nullptr;
+  const Caps cp = caps_of(nb, nc, hit_cap(nb, nc, ar.pass[p], ar.need[p]));
+  Carver cv{const_cast<unsigned char*>(ar.at(p)), 0};
+  const PairWork w = carve(cv, cp);
+  const double g = gA[p];
+  const int nv = w.roff[nr];
+  int* next = w.R.next;
+  int* prev = w.R.prev;
+  ring_links(grp, w.roff, nr, nv, next, prev);
+  for (int side = 0; side < 2; ++side) {
+    const int n = side ? nc : nb;
+    int* start = side ? w.cAll : w.bAll;
+    int* fill = side ? w.cND : w.bND;
+    int* list = side ? w.R.label : w.R.enex;
+    double2* far = (double2*)(side ? w.ixC : w.ixB);  // the far ends' part
+    double* out = side ? gcp : gbp;
+    auto edge_of = [&](int4 tp) { return tp.x == 2 ? (side ? tp.z : tp.y) : (tp.x == side ? tp.y : -1); };
+    for (int i = lane; i <= n; i += N) start[i] = fill[i] = 0;
+    grp.sync();
+    for (int v = lane; v < nv; v += N) {
+      const int e = edge_of(w.tape[v]);
+      if (e >= 0) atomicAdd(&start[e], 1);
+    }
+    grp.sync();
+    group_scan(grp, start, n + 1);
+    grp.sync();
+    for (int v = lane; v < nv; v += N) {
+      const int e = edge_of(w.tape[v]);
+      if (e >= 0) list[start[e] + atomicAdd(&fill[e], 1)] = v;
+    }
+    grp.sync();
+    // ring vertex v's part for this side's edge e: its own vertex, its far end
+    auto part = [&](int v, int e, double2* own, double2* end) {
+      const int ip = next[v], im = prev[v];
+      // shoelace: dA/dx_i = (y_{i+1} - y_{i-1}) / 2, dA/dy_i = (x_{i-1} - x_{i+1}) / 2
+      const double gx = 0.5 * g * (w.rxy[2 * ip + 1] - w.rxy[2 * im + 1]);
+      const double gy = 0.5 * g * (w.rxy[2 * im] - w.rxy[2 * ip]);
+      const int4 tp = w.tape[v];
+      if (tp.x != 2) {
+        own->x += gx;
+        own->y += gy;
+        return;
+      }
+      const CrossGrad k(b, tp.y, vsucc(bn, nb, tp.y), c, tp.z, vsucc(cn, nc, tp.z), gx, gy);
+      const double2 d = side ? k.c1() : k.b1(), f = side ? k.c2() : k.b2();
+      own->x += d.x;
+      own->y += d.y;
+      end->x += f.x;
+      end->y += f.y;
+    };
+    auto store = [&](int e, double2 own, double2 end) {
+      out[2 * e] = own.x;
+      out[2 * e + 1] = own.y;
+      far[e] = end;
+    };
+    group_items(
+        grp, n, w.R.nb, [&](int e) { return max(1, start[e + 1] - start[e]); },
+        [&](int e) {
+          int* l = list + start[e];
+          const int m = start[e + 1] - start[e];
+          for (int i = 1; i < m; ++i) {
+            const int x = l[i];
+            int j = i;
+            while (j > 0 && l[j - 1] > x) {
+              l[j] = l[j - 1];
+              --j;
+            }
+            l[j] = x;
+          }
+          double2 own = make_double2(0.0, 0.0), end = own;
+          for (int i = 0; i < m; ++i) part(l[i], e, &own, &end);
+          store(e, own, end);
+        },
+        [&](auto& gg, int e) {
+          // lane by lane over the ordered list, the lanes' sums in a fixed order
+          // (scratch: R.x and R.y, adjacent in the arena)
+          int* l = list + start[e];
+          const int m = start[e + 1] - start[e];
+          unsigned long long* scr = (unsigned long long*)w.R.x + 2 * start[e];
+          group_sort(gg, m, scr, [&](int k) { return (unsigned long long)l[k]; });
+          const int lane32 = threadIdx.x & 31;
+          if (gg.warp() == 0) {
+            double2 own = make_double2(0.0, 0.0), end = own;
+            for (int i = lane32; i < m; i += 32) part((int)scr[i], e, &own, &end);
+            for (int o = 16; o > 0; o >>= 1) {
+              own.x += __shfl_xor_sync(kFullMask, own.x, o);
+              own.y += __shfl_xor_sync(kFullMask, own.y, o);
+              end.x += __shfl_xor_sync(kFullMask, end.x, o);
+              end.y += __shfl_xor_sync(kFullMask, end.y, o);
+            }
+            if (lane32 == 0) store(e, own, end);
+          }
+          gg.sync();
+        });
+    grp.sync();
+    const int* nx = side ? cn : bn;
+    for (int e = lane; e < n; e += N) {
+      const int t = vsucc(nx, n, e);  // every vertex follows one edge
+      out[2 * t] += far[e].x;
+      out[2 * t + 1] += far[e].y;
+    }
+    grp.sync();
   }
 }
 
@@ -1922,14 +2295,19 @@ int BatchRunner::plan(int np_, const long long* d_boff, const long long* d_coff,
   if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "batch sizes");
   in_verts = (double)(h_boff_[np] + h_coff_[np]);
   big_.clear();
+  // the wide line: the lower one while the blocks are few
+  int over = 0;
   for (int p = 0; p < np; ++p) {
     const long long nb = h_boff_[p + 1] - h_boff_[p], nc = h_coff_[p + 1] - h_coff_[p];
     if (nb >= 3 && nc >= 3 && (nb > split_now() || nc > split_now())) {
       BigOut b;
       b.p = p;
       big_.push_back(b);
+    } else {
+      over += nb * nc > kWideMin[0];
     }
   }
+  wide_min_ = over <= kWideFew ? kWideMin[0] : kWideMin[1];
   long long budget = arena_budget;
   if (budget <= 0) {
     size_t fr = 0, tot = 0;
@@ -1953,6 +2331,43 @@ int BatchRunner::plan(int np_, const long long* d_boff, const long long* d_coff,
   return kOk;
 }
 
+// The wide pairs of the chunk's n pairs from p0, the largest first (by the
+// power of two of their edge pairs: a block that starts late on a large pair
+// is the kernel's tail), and the base edge groups before each one.
+int BatchRunner::plan_wide(int p0, int n, cudaStream_t st) {
+  nwide_ = nitems_ = 0;
+  std::vector<std::vector<int>> by(48);
+  for (int i = 0; i < n; ++i) {
+    const long long nb = h_boff_[p0 + i + 1] - h_boff_[p0 + i];
+    const long long nc = h_coff_[p0 + i + 1] - h_coff_[p0 + i];
+    if (nb < 3 || nc < 3 || nb > split_now() || nc > split_now() ||
+        !wide_pair((int)nb, (int)nc, wide_min_))
+      continue;
+    int k = 0;
+    for (long long m = nb * nc; m > 1 && k < 47; m >>= 1) ++k;
+    by[k].push_back(i);
+  }
+  std::vector<int> wide, item(1, 0);
+  long long total = 0;
+  for (int k = 47; k >= 0; --k)
+    for (const int i : by[k]) {
+      wide.push_back(i);
+      total += edge_groups((int)(h_boff_[p0 + i + 1] - h_boff_[p0 + i]));
+      if (total > INT_MAX) return pl_.fail(kEInput, "too many vertices in one arena chunk");
+      item.push_back((int)total);
+    }
+  if (wide.empty()) return kOk;
+  BufferPool& pool = pl_.pool();
+  wide_ = (int*)pool.get("bt_wide", sizeof(int) * wide.size());
+  wide_item_ = (int*)pool.get("bt_wide_item", sizeof(int) * item.size());
+  if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (wide pairs)");
+  cudaMemcpyAsync(wide_, wide.data(), sizeof(int) * wide.size(), cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(wide_item_, item.data(), sizeof(int) * item.size(), cudaMemcpyHostToDevice, st);
+  nwide_ = (int)wide.size();
+  nitems_ = (int)total;
+  return kOk;
+}
+
 // The small pairs of chunk c: pass 0, then the pairs that ran out of hit
 // room again with the full product.  The chunk's arenas stay resident.
 int BatchRunner::run_chunk(int c, const double* d_bxy, const long long* d_boff,
@@ -1972,14 +2387,16 @@ int BatchRunner::run_chunk(int c, const double* d_bxy, const long long* d_boff,
     hp[i] = (nb >= 3 && nc >= 3 && !is_small[i]) ? -1 : 0;
   }
   cudaMemcpyAsync(pass + p0, hp.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
+  const int wrc = plan_wide(p0, n, st);
+  if (wrc) return wrc;
   // coordinates in; area, status, ring and vertex counts out
   const double in_bytes =
       16.0 * (double)(h_boff_[p1] - h_boff_[p0] + h_coff_[p1] - h_coff_[p0]);
-  launch_clip(with_components(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
+  launch_clip(with_extras(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
                                        arena[0], aoff[0] + p0, abase_[0], need_ + p0, need_ + p0,
                                        status + p0, nrings + p0, nverts + p0, area + p0,
                                        unite ? 1 : 0, split_now()},
-                              bnx, cnx),
+                              bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
               shape, in_bytes, st);
   std::vector<int> hs(n);
   cudaMemcpyAsync(hs.data(), status + p0, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
@@ -2007,11 +2424,11 @@ int BatchRunner::run_chunk(int c, const double* d_bxy, const long long* d_boff,
     if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "batch sizes");
     arena[1] = (unsigned char*)pool.get("bt_arena1", (size_t)total + 256);
     if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (batch arena)");
-    launch_clip(with_components(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
+    launch_clip(with_extras(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
                                          arena[1], aoff[1] + p0, 0, need_ + p0, need_ + p0,
                                          status + p0, nrings + p0, nverts + p0, area + p0,
                                          unite ? 1 : 0, split_now()},
-                                bnx, cnx),
+                                bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
                 shape, in_bytes, st);
   }
   // where each pair's data lives now: pass 0 arena, retry arena, or none
@@ -2256,7 +2673,14 @@ int BatchRunner::backward(const double* d_bxy, const long long* d_boff, const do
                           8.0 * n);
     k_batch_backward<<<grid_for(32LL * n, shape.bwd), shape.bwd, 0, st>>>(
         n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, ar, status + p0, nrings + p0, d_gA + p0, bnx,
-        cnx, d_gb, d_gc);
+        cnx, wide_min_, d_gb, d_gc);
+    if (nwide_ > 0) {
+      ::sbc::KProbe kw_("k_batch_backward_wide", st);
+      k_batch_backward_wide<<<nwide_, kWideBlock, 0, st>>>(wide_, d_bxy, d_boff + p0, d_cxy,
+                                                           d_coff + p0, ar, status + p0,
+                                                           nrings + p0, d_gA + p0, bnx, cnx, d_gb,
+                                                           d_gc);
+    }
   }
   for (const BigOut& bo : big_) {
     if (!bo.ok || bo.nverts == 0) continue;
@@ -2386,22 +2810,28 @@ int BatchRunner::graph_record(int np_, const double* d_bxy, const long long* d_b
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    launch_clip(with_components(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass0, arena[0],
+    launch_clip(with_extras(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass0, arena[0],
                                          aoff[0], abase_[0], need_scr, need_rec, status, nrings,
                                          nverts, area, unite ? 1 : 0, split_now()},
-                                bnx, cnx),
+                                bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
                 shape, in_bytes, st);
     if (retry)
-      launch_clip(with_components(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass1, arena[1],
+      launch_clip(with_extras(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass1, arena[1],
                                            aoff[1], 0, need_scr, need_rec, status, nrings, nverts,
                                            area, unite ? 1 : 0, split_now()},
-                                  bnx, cnx),
+                                  bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
                   shape, in_bytes, st);
     const Arenas ar{arena[0], aoff[0], abase_[0], arena[1], aoff[1], 0, pass, need_rec};
     {
       ::sbc::KProbe kp_("k_batch_backward", st);
       k_batch_backward<<<grid_for(32LL * np, shape.bwd), shape.bwd, 0, st>>>(
-          np, d_bxy, d_boff, d_cxy, d_coff, ar, status, nrings, d_gA, bnx, cnx, d_gb, d_gc);
+          np, d_bxy, d_boff, d_cxy, d_coff, ar, status, nrings, d_gA, bnx, cnx, wide_min_, d_gb,
+          d_gc);
+    }
+    if (nwide_ > 0) {
+      ::sbc::KProbe kp_("k_batch_backward_wide", st);
+      k_batch_backward_wide<<<nwide_, kWideBlock, 0, st>>>(
+          wide_, d_bxy, d_boff, d_cxy, d_coff, ar, status, nrings, d_gA, bnx, cnx, d_gb, d_gc);
     }
     if (out_area) cudaMemcpyAsync(out_area, area, sizeof(double) * np, cudaMemcpyDeviceToDevice, st);
     if (out_status)

@@ -376,7 +376,12 @@ class BatchRunner {
   int run_chunk(int c, const double* d_bxy, const long long* d_boff, const double* d_cxy,
                 const long long* d_coff, cudaStream_t st);
   int run_big(const double* d_bxy, const double* d_cxy, cudaStream_t st);
+  int plan_wide(int p0, int n, cudaStream_t st);
   Pipeline& pl_;
+  // the resident chunk's wide pairs (device lists, see ClipArgs)
+  int* wide_ = nullptr;
+  int* wide_item_ = nullptr;
+  int nwide_ = 0, nitems_ = 0, wide_min_ = 0;
   unsigned char* arena[2] = {nullptr, nullptr};
   long long* aoff[2] = {nullptr, nullptr};
   long long abase_[2] = {0, 0};

@@ -71,3 +71,92 @@ def test_overlaps_and_touches(mode):
             assert st != 0
             continue
         assert st == 0 and rings_equal(got, ref)
+
+
+# ------------------------------------------------------------------ batches
+def batch_pairs():
+    """Either side of the wide rule (16,384 edge pairs) and of the front's
+    shared-memory sort (1,024 edges), edge groups of 32 with a remainder, more
+    crossings than the first pass has room for, coordinates on a grid (shared
+    x values, vertical edges), overlapping edges, either orientation, one
+    polygon inside the other, disjoint ones."""
+    rng = np.random.default_rng(11)
+    out = []
+    for i, (nb, nc) in enumerate(((128, 128), (128, 129), (4, 4096), (4096, 5), (160, 161), (511, 513),
+                                  (512, 513), (1023, 33), (1000, 1100), (2048, 64), (2048, 2047))):
+        off = rng.uniform(-40.0, 40.0, 2)
+        out.append((gen.star(nb, 500 + i, R=100.0), gen.star(nc, 600 + i, centre=off, R=100.0)))
+    out.append((out[5][0], out[5][1][::-1].copy()))
+    out.append((gen.star(300, 41, R=100.0), gen.star(200, 42, R=10.0)))
+    out.append((gen.star(300, 43, R=10.0), gen.star(200, 44, centre=(1.0, 0.0), R=900.0)))
+    out.append((gen.star(300, 45, R=10.0), gen.star(200, 46, centre=(500.0, 0.0), R=9.0)))
+    for i in range(3):
+        b, c = gen.star(240, 51 + i, R=60.0), gen.star(180, 61 + i, centre=(9.0, -4.0), R=60.0)
+        out.append((np.round(b * 4) / 4, np.round(c * 4) / 4))
+    out.append((comb(90, 0.0, 1.0, 0.0, True, [1.0, 0.7, 1.0]), comb(80, 2.0, 1.0, 0.2937, False, [1.0, 1.4])))
+    out.append((comb(90, 0.0, 1.0, 0.0, True, [1.0, 0.7, 1.0]), comb(80, 2.0, 1.0, 3.1441, False, [1.5, 1.3])))
+    out.append((gen.star(3, 71), gen.star(4, 72)))
+    return out
+
+
+def test_batch_rings(mode):
+    cl, union = mode
+    pairs = batch_pairs()
+    rings, status = cl.clip_batch([b for b, _ in pairs], [c for _, c in pairs])
+    seen = 0
+    for (b, c), got, st in zip(pairs, rings, status):
+        try:
+            ref = want(b, c, union)
+        except oracle_py.OracleError:
+            assert st != 0
+            continue
+        assert st == 0 and rings_equal(got, ref), (len(b), len(c))
+        seen += 1
+    assert seen >= len(pairs) - 4
+
+
+def test_batch_area_and_gradient(clipper):
+    """Areas to 1e-12 of the sum of the rings' absolute terms and gradients to
+    1e-11 of their largest entry (both sides sum FP64 terms, here in another
+    order), the same bits twice."""
+    import area_grad
+    pairs = []
+    for b, c in batch_pairs():
+        try:
+            pairs.append((b, c, oracle_py.clip(b, [c])["overlays"][0]))
+        except oracle_py.OracleError:
+            pass
+    bases, ovs = [p[0] for p in pairs], [p[1] for p in pairs]
+    ga = np.random.default_rng(7).uniform(0.5, 2.0, len(pairs))
+    area, status = clipper.area_forward(bases, ovs)
+    gb, gc = clipper.area_backward(bases, ovs, ga)
+    gb2, gc2 = clipper.area_backward(bases, ovs, ga)
+    assert (status == 0).all()
+    for p, (b, c, o) in enumerate(pairs):
+        rings = oracle_py.rings_of(o)
+        ref = area_grad.shoelace(rings)
+        scale = sum(float(np.abs(r).max() ** 2) * len(r) for r in rings) + 1e-300
+        assert abs(area[p] - ref) <= 1e-12 * scale
+        _, rb, rc = area_grad.gradient_of_rings(b, c, rings, o["uniq_b"], o["uniq_c"], o["uniq_t"], o["isect_xy"])
+        top = ga[p] * max(np.abs(rb).max(), np.abs(rc).max(), 1e-300)
+        assert np.abs(gb[p] - ga[p] * rb).max() <= 1e-11 * top, (len(b), len(c))
+        assert np.abs(gc[p] - ga[p] * rc).max() <= 1e-11 * top, (len(b), len(c))
+        assert np.array_equal(gb[p], gb2[p]) and np.array_equal(gc[p], gc2[p])
+
+
+def test_batch_rule_on_either_side(clipper):
+    """More than 1,024 pairs above 4,096 edge pairs stay on warps, fewer run on
+    blocks: the same rings, and areas to the rounding of a sum in another
+    order."""
+    pairs = gen.small_pairs(1030, seed=4700, lo=70, hi=75)
+    bases, ovs = [b for b, _ in pairs], [c for _, c in pairs]
+    many, st = clipper.clip_batch(bases, ovs)
+    a_many, _ = clipper.area_forward(bases, ovs)
+    assert (st == 0).all()
+    few = [clipper.clip_batch(bases[i:i + 103], ovs[i:i + 103])[0] for i in range(0, 1030, 103)]
+    few = [r for part in few for r in part]
+    a_few = np.concatenate([clipper.area_forward(bases[i:i + 103], ovs[i:i + 103])[0] for i in range(0, 1030, 103)])
+    assert all(rings_equal(x, y) for x, y in zip(many, few))
+    assert np.abs(a_many - a_few).max() <= 1e-13
+    for i in (0, 511, 1029):
+        assert rings_equal(many[i], want(bases[i], ovs[i], False))
