@@ -25,6 +25,7 @@
 
 #include "../../include/sbclip.h"
 #include "sbc_pipeline.cuh"
+#include "sbc_clean.cuh"
 #include "sbc_pairops.cuh"
 #include "sbc_pwpair.cuh"
 #include "sbc_serial.cuh"
@@ -108,7 +109,9 @@ struct PairWork {
   // back end
   Pool P, Q, R;
   int *rroot, *counts;
-  // between the three kernels of a pair: [0] front status, [1] logL, [2] hits
+  // between the kernels of a pair: [0] front status, [1] logL, [2] hits, [3]
+  // route (0: done with its area, 1: the thread back end's, 2: head done, 3:
+  // rings done, no area yet), [4] vertices share an x value
   int* state;
   unsigned char *splitP, *splitQ, *crossP, *crossQ;
   // output: ring offsets, ring xy, provenance
@@ -215,7 +218,7 @@ __host__ __device__ __forceinline__ PairWork carve(Carver& cv, const Caps& c) {
   carve_pool(cv, c.capR, w.R);
   w.rroot = cv.take<int>(c.rcap);
   w.counts = cv.take<int>(4);
-  w.state = cv.take<int>(4);
+  w.state = cv.take<int>(8);
   w.splitP = cv.take<unsigned char>(c.capP);
   w.crossP = cv.take<unsigned char>(c.capP);
   w.splitQ = cv.take<unsigned char>(c.capQ);
@@ -413,7 +416,13 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
       fval[l] = xv;
     }
   });
-  for (int i = lane; i < n2; i += N) w.sidx[i] = fval[i];
+  // an x value of two vertices: more than the two endpoints of one
+  bool shared_x = false;
+  for (int i = lane; i < n2; i += N) {
+    w.sidx[i] = fval[i];
+    if (i + 2 < n2 && fkey[i] == fkey[i + 2]) shared_x = true;
+  }
+  shared_x = g.any(shared_x);
   for (int i = lane; i <= E; i += N) w.vl[i] = 0;
   g.sync();
   for (int j = lane; j < E; j += N) {
@@ -545,7 +554,8 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
   g.sync();
   if (lane == 0) {
     w.state[1] = logL;
-    w.state[2] = 0;
+    w.state[2] = w.state[3] = 0;
+    w.state[4] = shared_x;
   }
   if constexpr (G::kBlock) {
     // the box of each group of overlay edges, a lane per edge
@@ -1298,6 +1308,9 @@ __global__ void __launch_bounds__(128) k_batch_cand_wide(ClipArgs A) {
   clip_pair_cand_group(cq, (item - A.wide_item[lo]) * kEdgeGroup, s_box[wi]);
 }
 
+// status of a pair that the general-position kernels left to the others
+constexpr int kPending = -1;
+
 // The back end in three kernels: A9-A13 on one thread per pair, the labels
 // on one warp per pair, A15-A18 on one thread per pair.  w.state[0] carries
 // a pair's failure from one to the next.
@@ -1480,6 +1493,74 @@ __device__ void order_hits(G& g, PairWork& w, int nb, int K) {
   g.sync();
 }
 
+// ---- rows A9-A18, provenance and area of the pairs in general position
+// (sbc_clean.cuh); the others get status kPending.  Bound by the latency of
+// short dependent steps; shared memory holds a warp's working arrays up to
+// about 64 crossings, so those are chains of shared-memory loads where the
+// list-walking kernels chain L1 and L2 loads.  65,536 pairs of 4 to 64
+// vertices, forward and backward: 3.95 -> 2.79 ms a step; 1,500 pairs with
+// holes and islands, which used to walk their lists on one thread each:
+// 16.4 -> 1.1 ms.
+constexpr int kCleanSmem = 6144;
+
+template <class G>
+__device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, int nc,
+                            unsigned char* smem, size_t smem_bytes, double* s_sum) {
+  Caps cp;
+  PairWork w = A.work(p, nb, nc, pass, &cp);
+  if (w.state[0] != PS_OK) return;
+  const int K = w.state[2];
+  if (K > cp.K) {
+    g.sync();
+    if (g.rank() == 0) batch_fail(A, p, w, PS_CAP, K);
+    return;
+  }
+  bool done = false;
+  int nr = 0, nv = 0;
+  double area = 0.0;
+  if (!w.state[4]) {
+    // in the arena, over the thread back end's arrays: csorted and the many
+    // larger ones after it
+    Carver cv{clean_bytes(nb, nc, K) <= smem_bytes ? smem : (unsigned char*)w.csorted, 0};
+    const CleanMem m = clean_carve(cv, nb, nc, K);
+    const CleanIn in{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.bnx, w.cnx, K,
+                     w.hb, w.hc, w.ht, w.hkey, w.hal, w.hbt, A.unite, cp.rcap, w.rootB, w.rootC,
+                     w.vl, w.vloc, w.roff, w.rxy, w.tape};
+    done = clean_clip(g, in, m, s_sum, &nr, &nv, &area);
+  }
+  if (g.rank() == 0) {
+    A.status[p] = done ? SBC_OK : kPending;
+    A.nrings[p] = nr;
+    A.nverts[p] = nv;
+    A.area[p] = area;
+  }
+}
+
+__global__ void __launch_bounds__(128) k_batch_clean(ClipArgs A) {
+  __shared__ __align__(16) unsigned char s_mem[4][kCleanSmem];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((t >> 5) >= A.np) return;
+  const int p = (int)(t >> 5);
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  int nb, nc;
+  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
+  WarpGroup g;
+  batch_clean(g, A, p, pass, nb, nc, s_mem[threadIdx.x >> 5], kCleanSmem, nullptr);
+}
+
+__global__ void __launch_bounds__(kWideBlock, 3) k_batch_clean_wide(ClipArgs A) {
+  using G = BlockGroup<kWideBlock>;
+  __shared__ G::Shared sh;
+  __shared__ double s_sum[G::kWarps];
+  const int p = A.wide[blockIdx.x];
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  int nb, nc;
+  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  G g(&sh);
+  batch_clean(g, A, p, pass, nb, nc, nullptr, 0, s_sum);
+}
+
+// ---- the pairs left pending
 // One warp per pair, in two kernels: the records in the reference's order
 // and rows A9-A14 (k_batch_pw, w.state[3] = 2 when done), then rows A15-A18
 // (k_batch_pw2).  Two kernels keep each one's code small enough for the
@@ -1496,15 +1577,11 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw(ClipArgs A) {
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
+  if (pass < 0 || A.status[p] != kPending || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK) return;
   const int K = w.state[2];
-  if (K > cp.K) {
-    if (lane == 0) batch_fail(A, p, w, PS_CAP, K);
-    return;
-  }
   // several components: the thread back end follows them
   if (A.multi(p, nb, nc)) {
     if (lane == 0) w.state[3] = 1;
@@ -1533,7 +1610,7 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw2(ClipArgs A) {
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
+  if (pass < 0 || A.status[p] != kPending || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK || w.state[3] != 2) return;
@@ -1561,7 +1638,7 @@ __global__ void __launch_bounds__(128, 6) k_batch_pw2(ClipArgs A) {
   __syncwarp();
   pair_tape(g, b, nb, c, nc, pw, K, w, nv);
   if (lane == 0) {
-    w.state[3] = 0;
+    w.state[3] = 3;
     A.status[p] = SBC_OK;
     A.nrings[p] = nr;
     A.nverts[p] = nv;
@@ -1597,16 +1674,11 @@ __global__ void __launch_bounds__(kWideBlock, 2) k_batch_pw_wide(ClipArgs A) {
   const int p = A.wide[blockIdx.x];
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  if (pass < 0 || A.status[p] != kPending || !A.small(p, &nb, &nc)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK) return;
   const int K = w.state[2];
-  if (K > cp.K) {
-    __syncthreads();
-    if (threadIdx.x == 0) batch_fail(A, p, w, PS_CAP, K);
-    return;
-  }
   if (A.multi(p, nb, nc)) {
     if (threadIdx.x == 0) w.state[3] = 1;
     return;
@@ -1659,7 +1731,7 @@ __global__ void __launch_bounds__(kBatchBlock) k_batch_back(ClipArgs A) {
   const int p = t;
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  if (pass < 0 || A.status[p] != kPending || !A.small(p, &nb, &nc)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK || w.state[3] != 1) return;
@@ -1674,7 +1746,7 @@ __global__ void __launch_bounds__(128) k_batch_labels(ClipArgs A) {
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  if (pass < 0 || A.status[p] != kPending || !A.small(p, &nb, &nc)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK || w.state[3] != 1) return;
@@ -1688,7 +1760,7 @@ __global__ void __launch_bounds__(kBatchBlock) k_batch_back2(ClipArgs A) {
   const int p = t;
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc)) return;
+  if (pass < 0 || A.status[p] != kPending || !A.small(p, &nb, &nc)) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK || w.state[3] != 1) return;
@@ -1711,7 +1783,7 @@ __global__ void __launch_bounds__(128) k_batch_area(ClipArgs A) {
   if (pass < 0 || !A.small(p, &nb, &nc) || A.status[p] != SBC_OK) return;
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
-  if (wide_pair(nb, nc, A.wide_min) && w.state[3] == 0) return;  // k_batch_pw_wide's
+  if (w.state[3] == 0) return;  // done where the rings were
   const double a = pair_area_warp(w.roff, w.rxy, A.nrings[p], lane);
   if (lane == 0) A.area[p] = a;
 }
@@ -1762,6 +1834,18 @@ void launch_clip(const ClipArgs& A, const BatchShape& sh, double in_bytes, cudaS
     if (comps) k_batch_cand_wide<true><<<grid_for(A.nitems, 4), 128, 0, st>>>(A);
     else k_batch_cand_wide<false><<<grid_for(A.nitems, 4), 128, 0, st>>>(A);
   }
+  {
+    ::sbc::KProbe kp_("k_batch_clean", st, in_bytes + 20.0 * A.np);
+    k_batch_clean<<<grid_for(32LL * A.np, 128), 128, 0, st>>>(A);
+  }
+  if (A.nwide > 0) {
+    ::sbc::KProbe kp_("k_batch_clean_wide", st);
+    k_batch_clean_wide<<<A.nwide, kWideBlock, 0, st>>>(A);
+  }
+}
+
+// the kernels that follow the lists, for the pairs left pending
+void launch_general(const ClipArgs& A, const BatchShape& sh, double in_bytes, cudaStream_t st) {
   {
     ::sbc::KProbe kp_("k_batch_pw", st, in_bytes + 20.0 * A.np);
     k_batch_pw<<<grid_for(32LL * A.np, 128), 128, 0, st>>>(A);
@@ -2392,15 +2476,22 @@ int BatchRunner::run_chunk(int c, const double* d_bxy, const long long* d_boff,
   // coordinates in; area, status, ring and vertex counts out
   const double in_bytes =
       16.0 * (double)(h_boff_[p1] - h_boff_[p0] + h_coff_[p1] - h_coff_[p0]);
-  launch_clip(with_extras(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
+  std::vector<int> hs(n);
+  auto run_pass = [&](const ClipArgs& A) -> int {
+    launch_clip(A, shape, in_bytes, st);
+    for (int round = 0;; ++round) {
+      cudaMemcpyAsync(hs.data(), status + p0, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
+      if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "batch clip");
+      if (round || std::find(hs.begin(), hs.end(), kPending) == hs.end()) return kOk;
+      launch_general(A, shape, in_bytes, st);
+    }
+  };
+  const int rc0 = run_pass(with_extras(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
                                        arena[0], aoff[0] + p0, abase_[0], need_ + p0, need_ + p0,
                                        status + p0, nrings + p0, nverts + p0, area + p0,
                                        unite ? 1 : 0, split_now()},
-                              bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
-              shape, in_bytes, st);
-  std::vector<int> hs(n);
-  cudaMemcpyAsync(hs.data(), status + p0, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
-  if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "batch clip");
+                              bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_));
+  if (rc0) return rc0;
   int retry = 0;
   for (int i = 0; i < n; ++i) {
     hp[i] = -1;
@@ -2424,12 +2515,12 @@ int BatchRunner::run_chunk(int c, const double* d_bxy, const long long* d_boff,
     if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "batch sizes");
     arena[1] = (unsigned char*)pool.get("bt_arena1", (size_t)total + 256);
     if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (batch arena)");
-    launch_clip(with_extras(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
+    const int rc1 = run_pass(with_extras(ClipArgs{n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, pass + p0,
                                          arena[1], aoff[1] + p0, 0, need_ + p0, need_ + p0,
                                          status + p0, nrings + p0, nverts + p0, area + p0,
                                          unite ? 1 : 0, split_now()},
-                                bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
-                shape, in_bytes, st);
+                                bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_));
+    if (rc1) return rc1;
   }
   // where each pair's data lives now: pass 0 arena, retry arena, or none
   for (int i = 0; i < n; ++i) {
@@ -2810,17 +2901,19 @@ int BatchRunner::graph_record(int np_, const double* d_bxy, const long long* d_b
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    launch_clip(with_extras(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass0, arena[0],
-                                         aoff[0], abase_[0], need_scr, need_rec, status, nrings,
-                                         nverts, area, unite ? 1 : 0, split_now()},
-                                bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
-                shape, in_bytes, st);
+    auto record_pass = [&](const ClipArgs& A) {
+      launch_clip(A, shape, in_bytes, st);
+      launch_general(A, shape, in_bytes, st);
+    };
+    record_pass(with_extras(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass0, arena[0],
+                                     aoff[0], abase_[0], need_scr, need_rec, status, nrings,
+                                     nverts, area, unite ? 1 : 0, split_now()},
+                            bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_));
     if (retry)
-      launch_clip(with_extras(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass1, arena[1],
-                                           aoff[1], 0, need_scr, need_rec, status, nrings, nverts,
-                                           area, unite ? 1 : 0, split_now()},
-                                  bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_),
-                  shape, in_bytes, st);
+      record_pass(with_extras(ClipArgs{np, d_bxy, d_boff, d_cxy, d_coff, pass1, arena[1],
+                                       aoff[1], 0, need_scr, need_rec, status, nrings, nverts,
+                                       area, unite ? 1 : 0, split_now()},
+                              bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_));
     const Arenas ar{arena[0], aoff[0], abase_[0], arena[1], aoff[1], 0, pass, need_rec};
     {
       ::sbc::KProbe kp_("k_batch_backward", st);

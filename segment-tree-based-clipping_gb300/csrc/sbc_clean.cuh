@@ -1,0 +1,483 @@
+// sbc_clean.cuh -- rows A9-A18 of one pair in general position: every hit a
+// proper crossing inside both edges, labelled a crossing, and no ring vertex
+// in line with its neighbours.  That is nearly every pair of real-valued
+// polygons, with any number of components.
+//
+// In general position the reference's linked lists (copyToLinkedList,
+// src/clip.cpp:606-695; labelIntersections2 and createResult2,
+// foster/polyclip.h:337-759; Foster's component loops, lib/
+// optimizedFostersAlgorithm/polyclip.cpp:335-780) hold nothing that the order
+// of the crossings along each polygon does not say: a list is the vertices
+// with each edge's crossings after them, entry and exit alternate along a
+// component, and a ring is an alternating cycle of two pairings of the
+// crossings (each with its neighbour along the base, and along the overlay,
+// in the direction of its status).  So nothing of the merged arrays, labels,
+// lists or pools is built: a counting sort by edge, a sort of each edge's few
+// crossings, pointer doubling over the crossings, and each leg of a ring is
+// written to its place.  Every test that decides whether a pair is in general
+// position repeats the reference's own arithmetic; a pair that fails one is
+// left untouched for the engine that follows the lists.
+#pragma once
+
+#include "sbc_group.cuh"
+#include "sbc_pairops.cuh"
+#include "sbc_serial.cuh"
+
+namespace sbc {
+namespace {
+
+struct CleanIn {
+  const double* b;
+  int nb;
+  const double* c;
+  int nc;
+  const int* bnx;  // successor of each vertex within its component (null: one ring)
+  const int* cnx;
+  int K;  // hits: 2 * base edge, 2 * overlay edge, type, first emission, alpha, beta
+  const int *hb, *hc, *ht;
+  const unsigned long long* hkey;
+  const double *hal, *hbt;
+  int unite;
+  int rcap;            // room for rings
+  int *rootB, *rootC;  // scratch: first vertices of the components (n + 1)
+  int *inB, *inC;      // scratch: per component, first vertex inside the other polygon
+  int* roff;           // out: rings, their vertices, and where each vertex comes from
+  double* rxy;
+  int4* tape;  // {0, base vertex} {1, overlay vertex} {2, base edge, overlay edge}, ring in .w
+};
+
+// Working arrays, in shared memory or the pair's arena.  A hit h has rank
+// rP[h] along the base and rQ[h] along the overlay; hP and hQ are the
+// inverses, and ends[e] is one past edge e's last rank.
+struct CleanMem {
+  int *endB, *endC;
+  int *hP, *hQ, *rP, *rQ, *eP, *eQ, *aB, *aC;
+  double *x, *y;
+  int4 *A, *B;
+};
+
+__host__ __device__ __forceinline__ CleanMem clean_carve(Carver& cv, int nb, int nc, int K) {
+  CleanMem m;
+  m.endB = cv.take<int>(nb + 1);
+  m.endC = cv.take<int>(nc + 1);
+  m.hP = cv.take<int>(K);
+  m.hQ = cv.take<int>(K);
+  m.rP = cv.take<int>(K);
+  m.rQ = cv.take<int>(K);
+  m.eP = cv.take<int>(K);
+  m.eQ = cv.take<int>(K);
+  m.aB = cv.take<int>(K);
+  m.aC = cv.take<int>(K);
+  m.x = cv.take<double>(K);
+  m.y = cv.take<double>(K);
+  m.A = cv.take<int4>(K + 4);
+  m.B = cv.take<int4>(K + 4);
+  return m;
+}
+
+__host__ __device__ __forceinline__ size_t clean_bytes(int nb, int nc, int K) {
+  Carver cv{nullptr, 0};
+  clean_carve(cv, nb, nc, K);
+  return (cv.off + 15) & ~(size_t)15;
+}
+
+// the components of an n-vertex polygon: their first vertices, then n
+template <class G>
+__device__ int clean_components(G& g, int n, const int* nx, int* root) {
+  int count = 0;
+  for (int i0 = 0; i0 < n; i0 += G::N) {
+    const int v = i0 + g.rank();
+    const bool first = v < n && (v == 0 || nx[v - 1] != v);
+    int tot;
+    const int k = count + g.before(first, &tot);
+    if (first) root[k] = v;
+    count += tot;
+  }
+  if (g.rank() == 0) root[count] = n;
+  g.sync();
+  return count;
+}
+
+// Done (true: rings, their count and vertices, and the area), or not in
+// general position (false, the same on every thread; the outputs' contents
+// are then unspecified).  s_sum: a shared double per warp of a block.
+template <class G>
+__device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s_sum,
+                           int* nrings_out, int* nverts_out, double* area_out) {
+  const int lane = g.rank();
+  constexpr int N = G::N;
+  const int K = in.K, nb = in.nb, nc = in.nc;
+  const double *b = in.b, *c = in.c;
+  auto bsucc = [&](int i) { return in.bnx ? in.bnx[i] : (i + 1 == nb ? 0 : i + 1); };
+  auto csucc = [&](int i) { return in.cnx ? in.cnx[i] : (i + 1 == nc ? 0 : i + 1); };
+  // ---- A10-A12: ranks along both polygons
+  for (int i = lane; i <= nb; i += N) m.endB[i] = 0;
+  for (int i = lane; i <= nc; i += N) m.endC[i] = 0;
+  g.sync();
+  bool bad = false;
+  for (int h = lane; h < K; h += N) {
+    const int e = in.hb[h] >> 1, f = in.hc[h] >> 1;
+    if (in.ht[h] != 1) bad = true;
+    atomicAdd(&m.endB[e], 1);
+    atomicAdd(&m.endC[f], 1);
+    // the crossing (saveIntersectionsParallel, oacc_segment_tree.cpp:7257-7341)
+    const double al = in.hal[h], oma = dsub(1.0, al);
+    const int e2 = bsucc(e), f2 = csucc(f);
+    const double p1x = b[2 * e], p1y = b[2 * e + 1], p2x = b[2 * e2], p2y = b[2 * e2 + 1];
+    const double x = dadd(dmul(oma, p1x), dmul(al, p2x)), y = dadd(dmul(oma, p1y), dmul(al, p2y));
+    m.x[h] = x;
+    m.y[h] = y;
+    const int a = alpha_to_int(al), t = alpha_to_int(in.hbt[h]);
+    if (a < 0 || t < 0) bad = true;
+    m.aB[h] = a % 1000000000;
+    m.aC[h] = t % 1000000000;
+    // apart from the four ends (an equal slot stops the list walk early, and
+    // provenance goes by coordinates)
+    auto meets = [&](double px, double py) { return px == x && py == y; };
+    if (meets(p1x, p1y) || meets(p2x, p2y) || meets(c[2 * f], c[2 * f + 1]) ||
+        meets(c[2 * f2], c[2 * f2 + 1]))
+      bad = true;
+  }
+  if (g.any(bad)) return false;
+  if (K > 0) {
+    group_scan(g, m.endB, nb + 1);
+    group_scan(g, m.endC, nc + 1);
+    g.sync();
+    for (int h = lane; h < K; h += N) {  // a start moves up to its end
+      m.hP[atomicAdd(&m.endB[in.hb[h] >> 1], 1)] = h;
+      m.hQ[atomicAdd(&m.endC[in.hc[h] >> 1], 1)] = h;
+    }
+    g.sync();
+  }
+  auto startB = [&](int e) { return e == 0 ? 0 : m.endB[e - 1]; };
+  auto startC = [&](int e) { return e == 0 ? 0 : m.endC[e - 1]; };
+  // per edge: alpha order, ties in record order (base edge, then emission)
+  auto order = [&](int n, auto start, const int* end, int* list, auto less) {
+    group_items(
+        g, n, m.eP, [&](int e) { const int k = end[e] - start(e); return k > 1 ? k : 0; },
+        [&](int e) {
+          int* v = list + start(e);
+          const int k = end[e] - start(e);
+          for (int i = 1; i < k; ++i) {
+            const int x = v[i];
+            int j = i;
+            while (j > 0 && less(x, v[j - 1])) {
+              v[j] = v[j - 1];
+              --j;
+            }
+            v[j] = x;
+          }
+        },
+        [&](auto& gg, int e) {
+          const int s = start(e), k = end[e] - s, np = npow2_dev(k);
+          unsigned* scr = (unsigned*)m.A + 4 * s;
+          for (int i = gg.rank(); i < np; i += gg.N) scr[i] = i < k ? (unsigned)list[s + i] : ~0u;
+          gg.sync();
+          group_bitonic(gg, np, [&](int i, int j, bool up) {
+            const unsigned x = scr[i], y = scr[j];
+            const bool lt = x != ~0u && (y == ~0u || (x != y && less((int)x, (int)y)));
+            const bool gt = y != ~0u && (x == ~0u || (x != y && less((int)y, (int)x)));
+            if (up ? gt : lt) {
+              scr[i] = y;
+              scr[j] = x;
+            }
+          });
+          for (int i = gg.rank(); i < k; i += gg.N) list[s + i] = (int)scr[i];
+          gg.sync();
+        });
+    g.sync();
+  };
+  if (K > 0) {
+    order(nb, startB, m.endB, m.hP, [&](int u, int v) {
+      return m.aB[u] != m.aB[v] ? m.aB[u] < m.aB[v] : in.hkey[u] < in.hkey[v];
+    });
+    order(nc, startC, m.endC, m.hQ, [&](int u, int v) {
+      if (m.aC[u] != m.aC[v]) return m.aC[u] < m.aC[v];
+      return in.hb[u] != in.hb[v] ? in.hb[u] < in.hb[v] : in.hkey[u] < in.hkey[v];
+    });
+    for (int k = lane; k < K; k += N) {
+      const int h = m.hP[k], q = m.hQ[k];
+      m.rP[h] = k;
+      m.eP[k] = in.hb[h] >> 1;
+      m.rQ[q] = k;
+      m.eQ[k] = in.hc[q] >> 1;
+    }
+    g.sync();
+    // ---- A14: every initial label a crossing (calculateInitLabelParallel,
+    // oacc_segment_tree.cpp:7925-7988): the overlay's neighbours of the
+    // crossing lie on different sides of the base there
+    for (int k = lane; k < K && !bad; k += N) {
+      const int h = m.hP[k], e = m.eP[k], q = m.rQ[h], f = m.eQ[q];
+      const double cx = m.x[h], cy = m.y[h];
+      const int hm = k > startB(e) ? m.hP[k - 1] : -1, hp = k + 1 < m.endB[e] ? m.hP[k + 1] : -1;
+      const int gm = q > startC(f) ? m.hQ[q - 1] : -1, gp = q + 1 < m.endC[f] ? m.hQ[q + 1] : -1;
+      // a crossing next to this one on both polygons: another label
+      if ((hm >= 0 && (hm == gm || hm == gp)) || (hp >= 0 && (hp == gm || hp == gp))) {
+        bad = true;
+        break;
+      }
+      // nor two crossings of an edge at one point (provenance by coordinates)
+      auto at = [&](int o) { return o >= 0 && m.x[o] == cx && m.y[o] == cy; };
+      if (at(hm) || at(hp) || at(gm) || at(gp)) {
+        bad = true;
+        break;
+      }
+      const int e2 = bsucc(e), f2 = csucc(f);
+      const double pmx = hm >= 0 ? m.x[hm] : b[2 * e], pmy = hm >= 0 ? m.y[hm] : b[2 * e + 1];
+      const double ppx = hp >= 0 ? m.x[hp] : b[2 * e2], ppy = hp >= 0 ? m.y[hp] : b[2 * e2 + 1];
+      const double s3 = area3(pmx, pmy, cx, cy, ppx, ppy);
+      auto right = [&](double qx, double qy) {
+        const double s1 = area3(qx, qy, pmx, pmy, cx, cy), s2 = area3(qx, qy, cx, cy, ppx, ppy);
+        if (s3 > 0) return !(s1 > 0 && s2 > 0);
+        return s1 < 0 && s2 < 0;
+      };
+      const bool rm = gm >= 0 ? right(m.x[gm], m.y[gm]) : right(c[2 * f], c[2 * f + 1]);
+      const bool rp = gp >= 0 ? right(m.x[gp], m.y[gp]) : right(c[2 * f2], c[2 * f2 + 1]);
+      if (rm == rp) bad = true;
+    }
+    if (g.any(bad)) return false;
+  }
+  // ---- components, and whether each one's first vertex lies in the other
+  // polygon (pointInPoly over the list's edges, a thread per polygon edge)
+  const int ncb = in.bnx ? clean_components(g, nb, in.bnx, in.rootB) : 1;
+  const int ncc = in.cnx ? clean_components(g, nc, in.cnx, in.rootC) : 1;
+  auto inside = [&](bool overlay, double rx, double ry) {
+    const double* p = overlay ? c : b;
+    const int n = overlay ? nc : nb;
+    int part = 0;
+    for (int e = lane; e < n; e += N) {
+      double x0 = p[2 * e], y0 = p[2 * e + 1];
+      if (!(x0 == x0 && y0 == y0)) bad = true;
+      const int s = overlay ? startC(e) : startB(e), t = overlay ? m.endC[e] : m.endB[e];
+      for (int k = s; k < t; ++k) {
+        const int h = overlay ? m.hQ[k] : m.hP[k];
+        part += pip_step(x0, y0, m.x[h], m.y[h], rx, ry);
+        x0 = m.x[h];
+        y0 = m.y[h];
+      }
+      const int e2 = overlay ? csucc(e) : bsucc(e);
+      part += pip_step(x0, y0, p[2 * e2], p[2 * e2 + 1], rx, ry);
+    }
+    return g.sum(part) & 1;
+  };
+  int inP = 0, inQ = 0;  // of a single component
+  if (ncb == 1) inP = inside(true, b[0], b[1]);
+  if (ncc == 1) inQ = inside(false, c[0], c[1]);
+  for (int side = 0; side < 2; ++side) {
+    const int n = side ? ncc : ncb;
+    if (n == 1) continue;
+    for (int k = 0; k < n; ++k) {
+      const int v = side ? in.rootC[k] : in.rootB[k];
+      const int x = side ? inside(false, c[2 * v], c[2 * v + 1]) : inside(true, b[2 * v], b[2 * v + 1]);
+      if (lane == 0) (side ? in.inC : in.inB)[k] = x;
+    }
+  }
+  // a component: its vertices [v0, v1), its crossings [lo, hi), and whether
+  // its first vertex is inside
+  struct Comp {
+    int v0, v1, lo, hi, in;
+  };
+  auto comp = [&](int side, int k) {
+    Comp r;
+    if (side) {
+      r.v0 = ncc == 1 ? 0 : in.rootC[k];
+      r.v1 = ncc == 1 ? nc : in.rootC[k + 1];
+      r.lo = startC(r.v0);
+      r.hi = m.endC[r.v1 - 1];
+      r.in = ncc == 1 ? inQ : in.inC[k];
+    } else {
+      r.v0 = ncb == 1 ? 0 : in.rootB[k];
+      r.v1 = ncb == 1 ? nb : in.rootB[k + 1];
+      r.lo = startB(r.v0);
+      r.hi = m.endB[r.v1 - 1];
+      r.in = ncb == 1 ? inP : in.inB[k];
+    }
+    return r;
+  };
+  auto comp_of = [&](int side, int e) {  // of the edge (or vertex) e
+    int lo = 0, hi = (side ? ncc : ncb) - 1;
+    const int* root = side ? in.rootC : in.rootB;
+    while (lo < hi) {
+      const int x = (lo + hi + 1) >> 1;
+      if (root[x] <= e) lo = x;
+      else hi = x - 1;
+    }
+    return comp(side, lo);
+  };
+  if (g.any(bad)) return false;  // also: the flags are visible
+  for (int side = 0; side < 2; ++side)
+    for (int k = lane; k < (side ? ncc : ncb); k += N) {
+      const Comp r = comp(side, k);
+      if ((r.hi - r.lo) & 1) bad = true;
+    }
+  if (g.any(bad)) return false;
+  // ---- rings: first the components without crossings that lie inside (or
+  // outside, for the union), whole and in order
+  int rings = 0, verts = 0;
+  for (int side = 0; side < 2; ++side)
+    for (int k = 0; k < (side ? ncc : ncb); ++k) {
+      const Comp r = comp(side, k);
+      if (r.hi != r.lo || !(r.in ^ in.unite)) continue;
+      if (rings >= in.rcap) return false;
+      const double* p = side ? c : b;
+      for (int v = r.v0 + lane; v < r.v1; v += N) {
+        const int at = verts + v - r.v0;
+        in.rxy[2 * at] = p[2 * v];
+        in.rxy[2 * at + 1] = p[2 * v + 1];
+        in.tape[at] = make_int4(side, v, 0, rings);
+      }
+      if (lane == 0) in.roff[rings] = verts;
+      ++rings;
+      verts += r.v1 - r.v0;
+    }
+  // ---- then the traced ones.  The legs from crossing k (rank along the
+  // base): along the base to crossing kp, then along the overlay, from its
+  // rank m1 to m2, which is crossing kn
+  struct Leg {
+    int e, cnt, v0, v1, to;  // cnt vertices from edge e on, to the crossing of rank `to`
+    bool fwd;
+  };
+  auto leg = [&](int side, int k) {
+    const int* ek = side ? m.eQ : m.eP;
+    Leg l;
+    l.e = ek[k];
+    const Comp r = (side ? ncc : ncb) == 1 ? comp(side, 0) : comp_of(side, l.e);
+    const int entry = (r.in ^ 1) ^ ((k - r.lo) & 1);
+    l.fwd = entry != in.unite;
+    l.to = l.fwd ? (k + 1 == r.hi ? r.lo : k + 1) : (k == r.lo ? r.hi - 1 : k - 1);
+    l.v0 = r.v0;
+    l.v1 = r.v1;
+    l.cnt = l.fwd ? ek[l.to] - l.e : l.e - ek[l.to];
+    if (l.cnt < 0 || (l.cnt == 0 && (l.fwd ? l.to < k : l.to > k))) l.cnt += r.v1 - r.v0;
+    return l;
+  };
+  int4* A = m.A;
+  int4* B = m.B;
+  for (int k = lane; k < K; k += N) {
+    const Leg p = leg(0, k), q = leg(1, m.rQ[m.hP[p.to]]);
+    A[k] = make_int4(m.rP[m.hQ[q.to]], k, 0, p.cnt + q.cnt + 2);
+  }
+  g.sync();
+  // orbits of k -> kn (see pw_label_trace_block): the least crossing, and the
+  // vertices to it
+  while (K > 0) {
+    bool changed = false;
+    for (int k = lane; k < K; k += N) {
+      int4 x = A[k];
+      const int4 y = A[x.x];
+      if (y.y < x.y) {
+        x.y = y.y;
+        x.z = (int)((unsigned)x.w + (unsigned)y.z);
+        changed = true;
+      }
+      x.x = y.x;
+      x.w = (int)((unsigned)x.w + (unsigned)y.w);
+      B[k] = x;
+    }
+    int4* t = A;
+    A = B;
+    B = t;
+    if (!g.any(changed)) break;
+  }
+  // B: {offset, length, number} of the ring, at its first crossing
+  for (int i0 = 0; i0 < K; i0 += N) {
+    const int k = i0 + lane;
+    int len = 0;
+    if (k < K && A[k].y == k) {
+      const Leg p = leg(0, k);
+      if (k < A[p.to].y) {
+        const Leg q = leg(1, m.rQ[m.hP[p.to]]);
+        len = p.cnt + q.cnt + 2 + A[m.rP[m.hQ[q.to]]].z;
+      }
+    }
+    int tr, tv;
+    const int r = rings + g.before(len > 0, &tr);
+    const int o = verts + g.excl(len, &tv);
+    if (len > 0) {
+      B[k] = make_int4(o, len, r, 0);
+      if (r < in.rcap) in.roff[r] = o;
+    }
+    rings += tr;
+    verts += tv;
+  }
+  if (rings > in.rcap) return false;
+  if (lane == 0) in.roff[rings] = verts;
+  g.sync();
+  // the legs to their places: a lane writes a short one, the warp a long one
+  constexpr int kShort = 8;
+  for (int i0 = 0; i0 < K; i0 += N) {
+    const int k = i0 + lane;
+    bool act = false;
+    Leg p{}, q{};
+    int at = 0, ring = 0;
+    if (k < K) {
+      p = leg(0, k);
+      const int s = A[k].y;
+      act = s < A[p.to].y;  // this sense of the cycle
+      if (act) {
+        q = leg(1, m.rQ[m.hP[p.to]]);
+        const int4 o = B[s];
+        at = o.x + (s == k ? 0 : o.y - A[k].z);
+        ring = o.z;
+      }
+    }
+    for (int side = 0; side < 2; ++side) {
+      const Leg& l = side ? q : p;
+      const double* poly = side ? c : b;
+      auto put = [&](int e, int fwd, int v0, int v1, int to, int r, int t) {
+        int u = fwd ? e + 1 + t : e - t;
+        if (u >= v1) u -= v1 - v0;
+        if (u < v0) u += v1 - v0;
+        in.rxy[2 * to] = poly[2 * u];
+        in.rxy[2 * to + 1] = poly[2 * u + 1];
+        in.tape[to] = make_int4(side, u, 0, r);
+      };
+      if (act) {
+        if (l.cnt <= kShort)
+          for (int t = 0; t < l.cnt; ++t) put(l.e, l.fwd, l.v0, l.v1, at + t, ring, t);
+        const int h = side ? m.hQ[l.to] : m.hP[l.to], to = at + l.cnt;
+        in.rxy[2 * to] = m.x[h];
+        in.rxy[2 * to + 1] = m.y[h];
+        in.tape[to] = make_int4(2, in.hb[h] >> 1, in.hc[h] >> 1, ring);
+      }
+      __syncwarp();
+      for (unsigned w = __ballot_sync(0xffffffffu, act && l.cnt > kShort); w; w &= w - 1) {
+        const int src = __ffs(w) - 1;
+        const int e = __shfl_sync(0xffffffffu, l.e, src), cnt = __shfl_sync(0xffffffffu, l.cnt, src);
+        const int fwd = __shfl_sync(0xffffffffu, (int)l.fwd, src);
+        const int v0 = __shfl_sync(0xffffffffu, l.v0, src), v1 = __shfl_sync(0xffffffffu, l.v1, src);
+        const int to = __shfl_sync(0xffffffffu, at, src), r = __shfl_sync(0xffffffffu, ring, src);
+        for (int t = threadIdx.x & 31; t < cnt; t += 32) put(e, fwd, v0, v1, to + t, r, t);
+      }
+      at += l.cnt + 1;
+    }
+  }
+  g.sync();
+  // ---- clean-up removes nothing (cleanUpResult2, foster/polyclip.h:767-787,
+  // a vertex with |area3| < eps goes), and the area: the shoelace terms in an
+  // order that the rings and the group size fix
+  double s2 = 0.0;
+  for (int v = lane; v < verts; v += N) {
+    const int r = in.tape[v].w, s = in.roff[r], e = in.roff[r + 1];
+    const int vp = v + 1 == e ? s : v + 1, vm = v == s ? e - 1 : v - 1;
+    const double x = in.rxy[2 * v], y = in.rxy[2 * v + 1];
+    const double xp = in.rxy[2 * vp], yp = in.rxy[2 * vp + 1];
+    if (fabs(area3(in.rxy[2 * vm], in.rxy[2 * vm + 1], x, y, xp, yp)) < kEps) bad = true;
+    s2 = dadd(s2, dsub(dmul(x, yp), dmul(xp, y)));
+  }
+  if (g.any(bad)) return false;
+  for (int o = 16; o > 0; o >>= 1) s2 = dadd(s2, __shfl_xor_sync(0xffffffffu, s2, o));
+  if constexpr (G::kBlock) {
+    if ((lane & 31) == 0) s_sum[g.warp()] = s2;
+    g.sync();
+    s2 = s_sum[0];
+    for (int k = 1; k < G::kWarps; ++k) s2 = dadd(s2, s_sum[k]);
+  }
+  *nrings_out = rings;
+  *nverts_out = verts;
+  *area_out = dmul(0.5, s2);
+  return true;
+}
+
+}  // namespace
+}  // namespace sbc

@@ -160,3 +160,48 @@ def test_batch_rule_on_either_side(clipper):
     assert np.abs(a_many - a_few).max() <= 1e-13
     for i in (0, 511, 1029):
         assert rings_equal(many[i], want(bases[i], ovs[i], False))
+
+
+def test_general_position_and_not(mode):
+    """Batches that mix pairs in general position with pairs that are not, by
+    one reason each: a vertex on an edge, a shared vertex, overlapping edges,
+    an x value of two vertices, a ring vertex in line with its neighbours, a
+    crossing within the classifier's epsilon of a vertex.  Every pair as the
+    oracle has it, in one batch and alone."""
+    cl, union = mode
+    sq = np.array([[0.0, 0.1], [4.0, 0.0], [4.1, 4.0], [0.2, 4.2]])
+    cases = [
+        (sq, sq + [1.7, 2.3]),
+        (sq, np.array([[2.0, 0.05], [6.0, 1.1], [5.0, 3.3]])),            # vertex on an edge
+        (sq, np.array([[4.0, 0.0], [7.0, 1.3], [5.0, 3.7]])),             # shared vertex
+        (sq, np.array([[1.0, 0.075], [3.0, 0.025], [3.3, 2.0], [1.2, 2.1]])),  # overlapping edge
+        (np.array([[0.0, 0.0], [4.0, 0.0], [4.0, 4.0], [0.0, 4.0]]), sq + [1.7, 2.3]),  # shared x
+        (np.array([[0.0, 0.1], [1.0, 0.1 + 1e-10], [2.0, 0.1], [4.1, 4.0], [0.3, 4.2]]), sq + [-1.3, 1.9]),
+        (sq, np.array([[2.0, 0.05 + 1e-10], [6.0, 1.1], [5.0, 3.3]])),
+        (gen.star(60, 5), gen.star(50, 6, centre=(0.2, 0.1))),
+        (gen.star(60, 5), gen.star(50, 6, centre=(0.2, 0.1))[::-1].copy()),
+    ]
+    rings, status = cl.clip_batch([b for b, _ in cases], [c for _, c in cases])
+    for (b, c), got, st in zip(cases, rings, status):
+        alone, st1 = cl.clip_batch([b], [c])
+        assert st1[0] == st and rings_equal(alone[0], got)
+        try:
+            ref = want(b, c, union)
+        except oracle_py.OracleError:
+            assert st != 0
+            continue
+        assert st == 0 and rings_equal(got, ref)
+
+
+@pytest.mark.parametrize("n,holes,islands", [(16, 1, 0), (40, 2, 1), (150, 3, 2), (700, 5, 5)])
+def test_components_in_general_position(mode, n, holes, islands):
+    """Polygons with holes and islands on a warp (small) and on a block (wide):
+    rings as the oracle's."""
+    cl, union = mode
+    bases = [gen.holed(n, 30 + i, holes=holes, islands=islands) for i in range(6)]
+    ovs = [gen.holed(n - (n > 16), 60 + i, centre=(0.11 * i, 0.07), holes=holes, islands=islands) for i in range(6)]
+    rings, status = cl.clip_batch_components(bases, ovs)
+    assert (status == 0).all()
+    for b, c, got in zip(bases, ovs, rings):
+        o = oracle_py.clip_components(b, c, union=union)["overlays"][0]
+        assert rings_equal(got, oracle_py.rings_of(o))
