@@ -39,9 +39,10 @@ void* BufferPool::get(const std::string& name, size_t bytes) {
 }
 
 void* BufferPool::get_zeroed(const std::string& name, size_t bytes, cudaStream_t st) {
-  void* before = bufs_[name].p;
+  const size_t before = bufs_[name].n;
   void* p = get(name, bytes);
-  if (p && p != before) cudaMemsetAsync(p, 0, bufs_[name].n, st);
+  // a buffer that grew may come back at the address it had
+  if (p && bufs_[name].n != before) cudaMemsetAsync(p, 0, bufs_[name].n, st);
   return p;
 }
 
