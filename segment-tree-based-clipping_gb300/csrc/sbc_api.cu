@@ -19,6 +19,7 @@ int Pipeline::run(const double* d_bxy, int nb_, const double* d_cxy, const int* 
   outs_.assign(k_, OverlayOut());
   join_ready_ = 0;
   cover_count_pending_ = false;
+  lazy_ = LazyRecords();
   nb = nb_;
   k = k_;
   if (nb < 3) return fail(kEInput, "base polygon needs at least 3 vertices");
@@ -110,6 +111,7 @@ int Pipeline::run_from_hits(const double* d_bxy, int nb_, const double* d_cxy, i
                             const unsigned long long* rkey, long long nhits) {
   err_.clear();
   outs_.assign(1, OverlayOut());
+  lazy_ = LazyRecords();
   nb = nb_;
   k = 1;
   if (nb < 3 || nc < 3) return fail(kEInput, "polygons need at least 3 vertices");
@@ -385,6 +387,11 @@ int sbc_phase_times(const sbc_ctx* c, float* out, int n) {
 int sbc_debug_array(sbc_ctx* c, int which, void* dst, long long cap, long long* count) {
   if (!c || !count) return set_err(c, SBC_EINPUT, "null argument");
   Pipeline& p = *c->pl;
+  if (which >= SBC_ARR_UNIQ_B && which <= SBC_ARR_LABEL_C) {
+    cudaSetDevice(c->device);
+    const int rc = p.build_records();
+    if (rc) return set_err(c, rc, p.error());
+  }
   const void* src = nullptr;
   long long n = 0;
   size_t es = sizeof(int);

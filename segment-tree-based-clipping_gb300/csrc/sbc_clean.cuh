@@ -248,6 +248,8 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     for (int e = lane; e < n; e += N) {
       double x0 = p[2 * e], y0 = p[2 * e + 1];
       if (!(x0 == x0 && y0 == y0)) bad = true;
+      const int e2 = overlay ? csucc(e) : bsucc(e);
+      if (!ray_near(y0, p[2 * e2 + 1], ry)) continue;
       const int s = overlay ? startC(e) : startB(e), t = overlay ? m.endC[e] : m.endB[e];
       for (int k = s; k < t; ++k) {
         const int h = overlay ? m.hQ[k] : m.hP[k];
@@ -255,7 +257,6 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
         x0 = m.x[h];
         y0 = m.y[h];
       }
-      const int e2 = overlay ? csucc(e) : bsucc(e);
       part += pip_step(x0, y0, p[2 * e2], p[2 * e2 + 1], rx, ry);
     }
     return g.sum(part) & 1;

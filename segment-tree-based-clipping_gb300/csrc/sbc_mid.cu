@@ -546,16 +546,37 @@ int Pipeline::stage_overlay(int cType, OverlayOut& out) {
     int rc0 = stage_candidates(cType, &rb, &rc, &rt, &rkey, &nraw, out);
     if (rc0) return rc0;
   }
+  bool done = false;
+  const int rc1 = stage_general(cType, rb, rc, rt, rkey, nraw, out, &done);
+  if (rc1 || done) return rc1;
   return stage_records(cType, rb, rc, rt, rkey, nraw, out);
+}
+
+// the reference's radix sort of the overlay ids by value mod 10^d is complete
+bool Pipeline::overlay_ids_fit() const {
+  long long m = 1;
+  for (long long v = 2LL * clSize; v > 0; v /= 10) m *= 10;
+  return 2LL * (hcS[k] - 2) < m;
+}
+
+// The arrays of rows A9-A14 (sbc_debug_array) of an overlay whose rings came
+// straight from its hits.
+int Pipeline::build_records() {
+  if (!lazy_.rb) return kOk;
+  const LazyRecords l = lazy_;
+  lazy_ = LazyRecords();
+  OverlayOut unused;
+  return stage_records(l.cType, l.rb, l.rc, l.rt, l.rkey, l.nhits, unused, false, true);
 }
 
 // A9-A18 from the candidate hits of overlay cType: base ids rb, overlay ids
 // rc (offsets into the interleaved arrays), types rt, first-emission keys.
 // With `unique_sorted` the hits are already A9's output (unique pairs in base
-// id, then key order) and A9 is skipped.
+// id, then key order) and A9 is skipped; with `arrays_only` the work ends with
+// A14's arrays.
 int Pipeline::stage_records(int cType, const int* rb, const int* rc, const int* rt,
                             const unsigned long long* rkey, long long nraw, OverlayOut& out,
-                            bool unique_sorted) {
+                            bool unique_sorted, bool arrays_only) {
   cudaStream_t st = st_;
   const int cListId = cType - 1;
   const int bSize = nb;
@@ -628,17 +649,9 @@ int Pipeline::stage_records(int cType, const int* rb, const int* rc, const int* 
     }
   }
 
-  // ---- A10 counts (radixsort of overlay ids by value mod 10^d must be complete)
-  {
-    long long m = 1;
-    long long v = 2LL * clSize;
-    while (v > 0) {
-      v /= 10;
-      m *= 10;
-    }
-    long long maxCid = 2LL * (hcS[k] - 2);
-    if (maxCid >= m) return fail(kEUndef, "overlay ids exceed the reference's radix digit count");
-  }
+  // ---- A10 counts
+  if (!overlay_ids_fit())
+    return fail(kEUndef, "overlay ids exceed the reference's radix digit count");
   int* bAll = (int*)pool_.get("bAll", sizeof(int) * (bSize + 2));
   int* bND = (int*)pool_.get("bND", sizeof(int) * (bSize + 2));
   int* cAll = (int*)pool_.get("cAll", sizeof(int) * (cSize + 2));
@@ -838,6 +851,7 @@ int Pipeline::stage_records(int cType, const int* rb, const int* rc, const int* 
   dbg_isxy = isxy; dbg_aB = aB; dbg_aC = aC;
   dbg_ixB = ixB; dbg_ixC = ixC; dbg_alB = alB; dbg_alC = alC; dbg_nbB = nbB; dbg_nbC = nbC;
   dbg_labB = labB; dbg_labC = labC; dbg_nB = nB; dbg_nQ = nQ;
+  if (arrays_only) return kOk;
   return run_backend(*this, m, out);
 }
 

@@ -244,7 +244,15 @@ class Pipeline {
   int stage_overlay(int cType, OverlayOut& out);
   int stage_records(int cType, const int* rb, const int* rc, const int* rt,
                     const unsigned long long* rkey, long long nraw, OverlayOut& out,
-                    bool unique_sorted = false);
+                    bool unique_sorted = false, bool arrays_only = false);
+  // rows A9-A18 straight from the hits of a pair in general position
+  // (sbc_general.cu); *done false: not in general position, nothing changed
+  int stage_general(int cType, const int* rb, const int* rc, const int* rt,
+                    const unsigned long long* rkey, long long nhits, OverlayOut& out, bool* done);
+  bool overlay_ids_fit() const;
+  // the diagnostic arrays of rows A9-A14 of the last overlay, if its rings
+  // came without them
+  int build_records();
   // one pair's rows A10-A18 from its unique candidate hits in A9's order
   // (base id, then first-emission key; no tree): the same rings as run() on
   // that pair when the hits are the pair's own
@@ -266,6 +274,13 @@ class Pipeline {
   cudaStream_t st_;
   cudaStream_t st2_ = nullptr;         // side stream (grid stage)
   cudaEvent_t ev_setup_ = nullptr, ev_side_ = nullptr, ev_lr_ = nullptr;
+  struct LazyRecords {
+    int cType = 0;
+    const int *rb = nullptr, *rc = nullptr, *rt = nullptr;
+    const unsigned long long* rkey = nullptr;
+    long long nhits = 0;
+  };
+  LazyRecords lazy_;                   // the hits build_records() starts from
   bool cover_count_pending_ = false;
   unsigned* h_side_rd_ = nullptr;      // 256 B pinned: the grid stage's reads ([0..9]),
                                        // the cover stage's two counts ([32..35])

@@ -119,6 +119,14 @@ __device__ __forceinline__ int pip_step(double x0, double y0, double x1, double 
   return 0;
 }
 
+// Whether an edge with end heights y0 and y1, or any piece of it between two
+// of its crossings, can cross the height ry: a crossing's height is within a
+// few units in the last place of the ends' range.
+__device__ __forceinline__ bool ray_near(double y0, double y1, double ry) {
+  const double m = 1e-13 * fmax(fabs(y0), fabs(y1));
+  return ry >= fmin(y0, y1) - m && ry <= fmax(y0, y1) + m;
+}
+
 __device__ int ppip(const Pool& p, int root, double rx, double ry) {
   int w = 0, one = root;
   do {
