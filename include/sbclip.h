@@ -96,8 +96,8 @@ int sbc_clip_pair_device(sbc_ctx* ctx, const double* d_b_xy, int nb, const doubl
 #define SBC_STAT_SLOTS_B 8
 #define SBC_STAT_SLOTS_C 9
 #define SBC_STAT_SERIAL_BACKEND 10      /* 1 if the exact serial back end ran */
-#define SBC_STAT_WORK_UNITS 11          /* overlay 1: edge-box pairs tested by the grid join */
-#define SBC_STAT_GRID_PAIRS 12          /* overlay 1: box-overlapping edge pairs the grid found */
+#define SBC_STAT_WORK_UNITS 11          /* overlay 1: edge-box pairs tested by the candidate search */
+#define SBC_STAT_GRID_PAIRS 12          /* overlay 1: box-overlapping edge pairs it found */
 #define SBC_STAT_VERTEX_SORT 13         /* the endpoint order came from: 0 the endpoint sort,
                                            1 the vertex sort on 64-bit keys, 2 the vertex sort
                                            on 32-bit keys with equal-key runs fixed up */

@@ -34,13 +34,19 @@ int Pipeline::run(const double* d_bxy, int nb_, const double* d_cxy, const int* 
   };
   mark(0);
   int rc = stage_setup(d_bxy, d_cxy, c_sizes);
-  // The grid stage and the first overlay's box join read only the setup's
-  // arrays: they run on the side stream, issued by the side worker thread,
+  // Few edges: candidates without the grid, on the main stream.  Otherwise
+  // the grid stage and the first overlay's box join, which read only the
+  // setup's arrays, run on the side stream, issued by the side worker thread,
   // while this thread issues the tree stages on the main stream.  Each
   // thread's host reads wait for its own stream only.
+  direct_ = !rc && direct_fits();
+  from_ranks_ = false;
+  const bool ranks = !force_endpoint_sort && !force_wide_vertex_sort;
   bool side_posted = false;
   int side_rc = 0;
-  if (!rc) {
+  if (direct_) {
+    rc = stage_direct_boxes();
+  } else if (!rc) {
     if (!side_stream()) {
       rc = fail(kECuda, "side stream");
     } else {
@@ -71,11 +77,11 @@ int Pipeline::run(const double* d_bxy, int nb_, const double* d_cxy, const int* 
     }
   }
   mark(1);
-  if (!rc) rc = stage_elementary();
+  if (!rc) rc = ranks ? stage_ranks(direct_) : stage_elementary();
   mark(2);
-  if (!rc) rc = stage_endlists();
+  if (!rc && !ranks) rc = stage_endlists();
   mark(3);
-  if (!rc) rc = stage_cover();
+  if (!rc && !(ranks && direct_)) rc = stage_cover();
   mark(4);
   if (side_posted) {
     side_rc = side_.wait();
@@ -84,7 +90,7 @@ int Pipeline::run(const double* d_bxy, int nb_, const double* d_cxy, const int* 
   // the candidate stage (main stream) reads the grid and the join; on an
   // error, later work on the main stream still waits for the side stream's
   // kernels (they read this context's buffers)
-  join_side();
+  if (!direct_) join_side();
   // a statistic, off the critical path (its kernel reads the leaf ranges)
   if (!rc) launch_cover_count();
   for (int t = 1; t <= k && !rc; ++t) rc = stage_overlay(t, outs_[t - 1]);
@@ -92,7 +98,13 @@ int Pipeline::run(const double* d_bxy, int nb_, const double* d_cxy, const int* 
   // the scans' error word lands with the final wait (take_tree_stats)
   unsigned* d_scan_err = scan_error_word();
   const unsigned* r_scan = d_scan_err ? rd_.get(d_scan_err, HostReads::kFlags + 1, st_) : nullptr;
+  const unsigned long long* r_tree =
+      !rc && from_ranks_ && direct_ ? rd_.get(d_treecnt, HostReads::kFront, st_, 2) : nullptr;
   take_tree_stats();
+  if (r_tree) {
+    stat_leaf = (long long)r_tree[0];
+    stat_cover = (long long)r_tree[1];
+  }
   finish_counts();
   if (cudaGetLastError() != cudaSuccess && !rc) rc = fail(kECuda, "CUDA error in the pipeline");
   const bool scan_gave_up = r_scan ? (*r_scan != 0u && scan_error_take()) : scan_error_take();
@@ -390,6 +402,11 @@ int sbc_debug_array(sbc_ctx* c, int which, void* dst, long long cap, long long* 
   if (which >= SBC_ARR_UNIQ_B && which <= SBC_ARR_LABEL_C) {
     cudaSetDevice(c->device);
     const int rc = p.build_records();
+    if (rc) return set_err(c, rc, p.error());
+  }
+  if (which == SBC_ARR_ELEMENTARY) {
+    cudaSetDevice(c->device);
+    const int rc = p.build_elementary();
     if (rc) return set_err(c, rc, p.error());
   }
   const void* src = nullptr;

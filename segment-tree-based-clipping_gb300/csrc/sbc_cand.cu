@@ -599,9 +599,287 @@ k_pair_exact(long long n, const int2* __restrict__ pairs, const int* __restrict_
   if (lane == 0 && my_raw) atomicAdd(&counters[3], my_raw);
 }
 
+// ------------------------------------------------------------------ direct
+// Candidate pairs without the grid, for polygons of up to some 100,000 edges:
+// consecutive edges lie near one another, so the box of 32 of them says much.
+// Every pair of such groups is tested by their boxes (a lane per overlay
+// group), the pairs that meet are listed, and a warp takes each one, a base
+// edge per lane, straight through the box test, LSMF and the float test to
+// the classifier.  Four launches and one host read, where the grid and its
+// join take 13 launches and five reads.
+// first edge group of each polygon (base, overlays), and their count
+struct EdgeGroups {
+  int g0[11];
+};
+
+// Float edge boxes and vertex pairs, the groups' boxes, and the bounds of the
+// base's edges and of the overlays' (bnd as in k_edge_fbox); a warp per group.
+__global__ void __launch_bounds__(256)
+k_direct_boxes(EdgeGroups eg, int nb, int k, const int* __restrict__ cS, const int* __restrict__ cc,
+               const double* __restrict__ bP, const double* __restrict__ cP,
+               float4* __restrict__ fbox, float4* __restrict__ vfB, float4* __restrict__ vfC,
+               float4* __restrict__ gbox, unsigned* __restrict__ bnd) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int q = blockIdx.x * 8 + w;
+  const bool on = q < eg.g0[k + 1];
+  const float inf = __int_as_float(0x7f800000);
+  float4 box = make_float4(inf, inf, -inf, -inf);
+  int cl = 0;
+  if (on) {
+    while (cl < k && eg.g0[cl + 1] <= q) ++cl;
+    const int j = (q - eg.g0[cl]) * 32 + lane;
+    const int n = cl == 0 ? nb : cc[cl] - cc[cl - 1];
+    if (j < n) {
+      const int at = cl == 0 ? j : cS[cl - 1] + j;
+      const double* p = (cl == 0 ? bP : cP) + 2LL * at;
+      float4* vf = (cl == 0 ? vfB : vfC) + at;
+      box = make_float4(__double2float_rd(fmin(p[0], p[2])), __double2float_rd(fmin(p[1], p[3])),
+                        __double2float_ru(fmax(p[0], p[2])), __double2float_ru(fmax(p[1], p[3])));
+      fbox[cl == 0 ? j : nb + cc[cl - 1] + j] = box;
+      auto pair = [](double x, double y) {
+        const float hx = __double2float_rn(x), hy = __double2float_rn(y);
+        return make_float4(hx, hy, __double2float_rn(dsub(x, (double)hx)),
+                           __double2float_rn(dsub(y, (double)hy)));
+      };
+      vf[0] = pair(p[0], p[1]);
+      if (j == n - 1) vf[1] = pair(p[2], p[3]);  // the closing vertex
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, o));
+    box.y = fminf(box.y, __shfl_xor_sync(0xffffffffu, box.y, o));
+    box.z = fmaxf(box.z, __shfl_xor_sync(0xffffffffu, box.z, o));
+    box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, o));
+  }
+  if (on && lane == 0) gbox[q] = box;
+  // per class one set of atomics per block
+  __shared__ float4 s_box[8];
+  __shared__ int s_cl[8];
+  if (lane == 0) {
+    s_box[w] = box;
+    s_cl[w] = on ? (cl == 0 ? 0 : 1) : 2;
+  }
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    const int c = threadIdx.x >> 2, f = threadIdx.x & 3;
+    unsigned v = f < 2 ? 0xffffffffu : 0u;
+    for (int i = 0; i < 8; ++i) {
+      if (s_cl[i] != c) continue;
+      const unsigned x = fkey(f == 0 ? s_box[i].x : f == 1 ? s_box[i].y : f == 2 ? s_box[i].z : s_box[i].w);
+      v = f < 2 ? min(v, x) : max(v, x);
+    }
+    if (f < 2) atomicMin(&bnd[threadIdx.x], v);
+    else atomicMax(&bnd[threadIdx.x], v);
+  }
+}
+
+// edges outside the common MBR (k_grid_count's filter), a statistic
+__global__ void __launch_bounds__(256) k_direct_outside(int E, const float4* __restrict__ fbox,
+                                                        const unsigned* __restrict__ bnd,
+                                                        unsigned* __restrict__ outside) {
+  auto unkey = [](unsigned u) { return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u); };
+  const float x0 = fmaxf(unkey(bnd[0]), unkey(bnd[4])), y0 = fmaxf(unkey(bnd[1]), unkey(bnd[5]));
+  const float x1 = fminf(unkey(bnd[2]), unkey(bnd[6])), y1 = fminf(unkey(bnd[3]), unkey(bnd[7]));
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  int out = 0;
+  if (e < E) {
+    const float4 f = fbox[e];
+    out = f.x > x1 || f.z < x0 || f.y > y1 || f.w < y0;
+  }
+  const int n = __syncthreads_count(out);
+  if (threadIdx.x == 0 && n) atomicAdd(outside, (unsigned)n);
+}
+
+__device__ __forceinline__ bool boxes_touch(const float4& a, const float4& b) {
+  return !(a.x > b.z || a.z < b.x || a.y > b.w || a.w < b.y);
+}
+
+// pairs of groups whose boxes meet (cap of them kept, all counted): a warp
+// takes 32 overlay groups against kDirectRows base groups
+constexpr int kDirectRows = 16;
+__global__ void __launch_bounds__(128)
+k_direct_groups(int gB, int gC0, int gC, int chunks, const float4* __restrict__ gbox,
+                unsigned long long* __restrict__ count, long long cap, int2* __restrict__ list) {
+  const int lane = threadIdx.x & 31;
+  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int b0 = (int)(item / chunks) * kDirectRows, q = (int)(item % chunks) * 32 + lane;
+  if (b0 >= gB) return;
+  const float inf = __int_as_float(0x7f800000);
+  const float4 c = q < gC ? gbox[gC0 + q] : make_float4(inf, inf, -inf, -inf);
+  unsigned met = 0;  // bit i: meets base group b0 + i
+#pragma unroll
+  for (int i = 0; i < kDirectRows; ++i)
+    if (b0 + i < gB && boxes_touch(gbox[b0 + i], c)) met |= 1u << i;
+  const int n = __popc(met);
+  int s = n;
+  for (int d = 1; d < 32; d <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, s, d);
+    if (lane >= d) s += t;
+  }
+  const int total = __shfl_sync(0xffffffffu, s, 31);
+  if (!total) return;
+  unsigned long long at = 0;
+  if (lane == 0) at = atomicAdd(count, (unsigned long long)total);
+  at = __shfl_sync(0xffffffffu, at, 0) + (s - n);
+  for (; met; met &= met - 1, ++at)
+    if ((long long)at < cap) list[at] = make_int2(b0 + __ffs(met) - 1, q);
+}
+
+// counters as in k_pair_exact, and [2] box-overlapping edge pairs, [4] edge
+// pairs tested, [5] listed group pairs
+__global__ void __launch_bounds__(128)
+k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long list_cap,
+               const float4* __restrict__ fbox, const int* __restrict__ e_id, const double* __restrict__ bP,
+               const double* __restrict__ cP, const long long* __restrict__ bK,
+               const long long* __restrict__ cK, const float4* __restrict__ vfB,
+               const float4* __restrict__ vfC, const int2* __restrict__ lr,
+               const int* __restrict__ aft, const int* __restrict__ bef, int logL,
+               unsigned long long* __restrict__ counters, long long cap, int* __restrict__ rb,
+               int* __restrict__ rc, int* __restrict__ rt, unsigned long long* __restrict__ rkey,
+               double2* __restrict__ rab) {
+  __shared__ int2 s_q[4][64];
+  __shared__ float4 s_box[4][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const float inf = __int_as_float(0x7f800000);
+  const long long items = min((long long)counters[5], list_cap);
+  int nq = 0;
+  unsigned long long raw = 0;
+  unsigned tested = 0, boxes = 0, work = 0;
+  auto classify = [&](int count) {
+    bool hit = false;
+    int2 e = make_int2(0, 0);
+    int ty = 0, cid = 0;
+    double al = 0.0, bt = 0.0;
+    unsigned long long key = 0;
+    if (lane < count) {
+      e = s_q[w][lane];
+      cid = e_id[e.y];
+      const double* pb = bP + 2LL * e.x;
+      const double* pc = cP + cid;
+      ty = seg_isect(pb[0], pb[1], pb[2], pb[3], pc[0], pc[1], pc[2], pc[3], &al, &bt);
+      if (ty) {
+        const unsigned n = emission(e.x, e.y, cid, lr, aft, bef, logL, &key);
+        hit = n > 0;
+        raw += n;
+      }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, hit);
+    if (m) {
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(&counters[0], (unsigned long long)__popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      const long long idx = (long long)at + __popc(m & lt);
+      if (hit && idx < cap) {
+        rb[idx] = 2 * e.x;
+        rc[idx] = cid;
+        rt[idx] = ty;
+        rkey[idx] = key;
+        rab[idx] = make_double2(al, bt);
+      }
+    }
+    __syncwarp();
+  };
+  for (long long i = (long long)blockIdx.x * 4 + w; i < items; i += 4LL * gridDim.x) {
+    const int2 pair = list[i];
+    const int be = pair.x * 32 + lane, j0 = pair.y * 32, n = min(32, nc - j0);
+    float4 fb = make_float4(inf, inf, -inf, -inf), p1 = fb, p2 = fb;
+    long long kb[4] = {0, 0, 0, 0};
+    __syncwarp();
+    if (lane < n) s_box[w][lane] = fbox[c0 + j0 + lane];
+    if (be < nb) {
+      fb = fbox[be];
+      p1 = vfB[be];
+      p2 = vfB[be + 1];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kb[j] = bK[2LL * be + j];
+      work += n;
+    }
+    __syncwarp();
+    for (int t = 0; t < n; ++t) {
+      bool keep = false;
+      const int ce = c0 + j0 + t;
+      if (boxes_touch(fb, s_box[w][t])) {
+        ++boxes;
+        const int v = e_id[ce] >> 1;
+        const long long* kc = cK + 2LL * v;
+        if (lsmf_keys(kb[0], kb[1], kb[2], kb[3], kc[0], kc[1], kc[2], kc[3])) {
+          ++tested;
+          keep = !certainly_disjoint(p1, p2, vfC[v], vfC[v + 1]);
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (!m) continue;
+      if (keep) s_q[w][nq + __popc(m & lt)] = make_int2(be, ce);
+      nq += __popc(m);
+      __syncwarp();
+      if (nq >= 32) {
+        classify(32);
+        const int rest = nq - 32;
+        const int2 x = lane < rest ? s_q[w][32 + lane] : make_int2(0, 0);
+        __syncwarp();
+        if (lane < rest) s_q[w][lane] = x;
+        nq = rest;
+        __syncwarp();
+      }
+    }
+  }
+  if (nq > 0) classify(nq);
+  for (int o = 16; o > 0; o >>= 1) raw += __shfl_xor_sync(0xffffffffu, raw, o);
+  tested = __reduce_add_sync(0xffffffffu, tested);
+  boxes = __reduce_add_sync(0xffffffffu, boxes);
+  work = __reduce_add_sync(0xffffffffu, work);
+  if (lane == 0) {
+    if (tested) atomicAdd(&counters[1], (unsigned long long)tested);
+    if (boxes) atomicAdd(&counters[2], (unsigned long long)boxes);
+    if (raw) atomicAdd(&counters[3], raw);
+    if (work) atomicAdd(&counters[4], (unsigned long long)work);
+  }
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------ host
+// whether every overlay of this run takes the direct search
+bool Pipeline::direct_fits() const {
+  for (int t = 0; t < k; ++t)
+    if (nb * (long long)(hcc[t + 1] - hcc[t]) > kDirectMost) return false;
+  return true;
+}
+
+int Pipeline::stage_direct_boxes() {
+  h_tstart_.assign(k + 2, 0);
+  EdgeGroups eg{};
+  for (int t = 0; t <= k; ++t) {
+    const int n = t == 0 ? nb : hcc[t] - hcc[t - 1];
+    h_tstart_[t + 1] = nb + hcc[t];
+    d_group0_[t] = eg.g0[t];
+    eg.g0[t + 1] = eg.g0[t] + (n + 31) / 32;
+  }
+  const int groups = eg.g0[k + 1];
+  fbox = (float4*)side_pool_.get("grid_fbox", sizeof(float4) * (E + 1));
+  vfB = (float4*)side_pool_.get("grid_vfB", sizeof(float4) * (nb + 1));
+  vfC = (float4*)side_pool_.get("grid_vfC", sizeof(float4) * ((long long)clSize + k));
+  gbox_ = (float4*)side_pool_.get("direct_gbox", sizeof(float4) * groups);
+  // bounds (8 words), edges outside, counters
+  auto* words = (unsigned*)side_pool_.get("direct_words", 256);
+  if (side_pool_.failed) return fail(kENoMem, "device allocation failed (edge boxes)");
+  g_bnd = words;
+  join_counters_ = (unsigned long long*)(words + 16);
+  static const unsigned init[16] = {0xffffffffu, 0xffffffffu, 0u, 0u, 0xffffffffu, 0xffffffffu};
+  cudaMemcpyAsync(words, init, sizeof(init), cudaMemcpyHostToDevice, st_);
+  {
+    ::sbc::KProbe kp_("k_direct_boxes", st_, 48.0 * E);
+    k_direct_boxes<<<grid_for(groups, 8), 256, 0, st_>>>(eg, nb, k, cS, cc, bP, cP, fbox, vfB, vfC,
+                                                        gbox_, g_bnd);
+  }
+  {
+    ::sbc::KProbe kp_("k_direct_outside", st_, 16.0 * E);
+    k_direct_outside<<<grid_for(E, 256), 256, 0, st_>>>(E, fbox, g_bnd, words + 8);
+  }
+  return kOk;
+}
+
 // The grid stage does not depend on the tree: it runs on the pipeline's
 // second stream (side_stream()), issued in three steps that run() interleaves
 // with the tree stages, so its kernels overlap the tree build and its two
@@ -805,6 +1083,7 @@ int Pipeline::stage_join(int cType, cudaStream_t st) {
 int Pipeline::stage_candidates(int cType, int** rb_out, int** rc_out, int** rt_out,
                                unsigned long long** rkey_out, long long* nhits, OverlayOut& out) {
   cudaStream_t st = st_;
+  if (direct_) return direct_candidates(cType, rb_out, rc_out, rt_out, rkey_out, nhits, out);
   if (join_ready_ != cType) {
     const int rj = stage_join(cType, st);
     if (rj) return rj;
@@ -823,14 +1102,24 @@ int Pipeline::stage_candidates(int cType, int** rb_out, int** rc_out, int** rt_o
   auto* rab = (double2*)pool_.get("raw_ab", sizeof(double2) * hcap);
   if (pool_.failed) return fail(kENoMem, "device allocation failed (hits)");
   raw_ab_ = rab;
-  if (npairs > 0) {
-    ::sbc::KProbe kp_("k_pair_exact", st, 72.0 * npairs);  // pair + both edges' coordinates
-    k_pair_exact<<<grid_for(npairs, kExChunk), kExBlock, 0, st>>>(
-        npairs, pairs, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL, counters, hcap, rb, rc,
-        rt, rkey, rab);
+  const unsigned long long* hc = nullptr;
+  for (;;) {
+    if (npairs > 0) {
+      ::sbc::KProbe kp_("k_pair_exact", st, 72.0 * npairs);  // pair + both edges' coordinates
+      k_pair_exact<<<grid_for(npairs, kExChunk), kExBlock, 0, st>>>(
+          npairs, pairs, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL, counters, hcap, rb, rc,
+          rt, rkey, rab);
+    }
+    hc = rd_.get(counters, HostReads::kCand + 8, st, 4);
+    const unsigned* r_fl = rd_.get(d_flags, HostReads::kCand + 14, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return fail(kECuda, "exact stage");
+    if (!ranks_failed(*r_fl)) break;
+    // the ranks did not do: the tree's arrays, then the pairs again
+    const int rt0 = redo_tree(*r_fl);
+    if (rt0) return rt0;
+    cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st);
+    cudaMemsetAsync(counters + 3, 0, sizeof(unsigned long long), st);
   }
-  const unsigned long long* hc = rd_.get(counters, HostReads::kCand + 8, st, 4);
-  if (cudaStreamSynchronize(st) != cudaSuccess) return fail(kECuda, "exact stage");
   if ((long long)hc[0] > hcap) return fail(kEInternal, "hit buffer overflow");
   if (hc[0] >= (1ULL << 31)) return fail(kEInput, "too many intersections");
   *rb_out = rb;
@@ -842,6 +1131,68 @@ int Pipeline::stage_candidates(int cType, int** rb_out, int** rc_out, int** rt_o
   out.tests = (long long)hc[1];
   out.raw_hits = (long long)hc[3];
   out.work = join_work_;
+  return kOk;
+}
+
+int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_out,
+                                unsigned long long** rkey_out, long long* nhits, OverlayOut& out) {
+  cudaStream_t st = st_;
+  const int nc = hcc[cType] - hcc[cType - 1], c0 = nb + hcc[cType - 1];
+  const int gB = (nb + 31) / 32, gC = (nc + 31) / 32, chunks = (gC + 31) / 32;
+  // room for group pairs and hits: what sufficed last time, or a guess that
+  // few pairs exceed
+  long long lcap = std::max(group_cap_, std::min((long long)gB * gC, 16LL * (gB + gC) + 16384));
+  long long cap = std::max(hit_cap_, std::min((long long)nb * nc, 4LL * E + 65536));
+  auto* counters = join_counters_;
+  const unsigned long long* hc = nullptr;
+  for (;;) {
+    int* rb = (int*)pool_.get("raw_b", sizeof(int) * (cap + 1));
+    int* rc = (int*)pool_.get("raw_c", sizeof(int) * (cap + 1));
+    int* rt = (int*)pool_.get("raw_t", sizeof(int) * (cap + 1));
+    auto* rkey = (unsigned long long*)pool_.get("raw_key", sizeof(unsigned long long) * (cap + 1));
+    auto* rab = (double2*)pool_.get("raw_ab", sizeof(double2) * (cap + 1));
+    auto* list = (int2*)pool_.get("direct_list", sizeof(int2) * (lcap + 1));
+    if (pool_.failed) return fail(kENoMem, "device allocation failed (hits)");
+    cudaMemsetAsync(counters, 0, 6 * sizeof(unsigned long long), st);
+    {
+      const long long rows = (gB + kDirectRows - 1) / kDirectRows;
+      ::sbc::KProbe kp_("k_direct_groups", st, 16.0 * (gB + gC));
+      k_direct_groups<<<grid_for(rows * chunks, 4), 128, 0, st>>>(gB, d_group0_[cType], gC, chunks,
+                                                                  gbox_, counters + 5, lcap, list);
+    }
+    {
+      ::sbc::KProbe kp_("k_direct_exact", st, 16.0 * (nb + nc));
+      k_direct_exact<<<(unsigned)std::min(grid_for((long long)gB * gC, 4), 1216u), 128, 0, st>>>(
+          nb, c0, nc, list, lcap, fbox, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL, counters,
+          cap, rb, rc, rt, rkey, rab);
+    }
+    hc = rd_.get(counters, HostReads::kCand + 8, st, 6);
+    const unsigned* r_fl = rd_.get(d_flags, HostReads::kCand + 14, st);
+    const unsigned* r_out = rd_.get(g_bnd + 8, HostReads::kCand + 15, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return fail(kECuda, "exact stage");
+    stat_outside_cmbr = *r_out;
+    if (ranks_failed(*r_fl)) {
+      const int rt0 = redo_tree(*r_fl);
+      if (rt0) return rt0;
+      continue;
+    }
+    raw_ab_ = rab;
+    *rb_out = rb;
+    *rc_out = rc;
+    *rt_out = rt;
+    *rkey_out = rkey;
+    if ((long long)hc[0] <= cap && (long long)hc[5] <= lcap) break;
+    if (hc[0] >= (1ULL << 31)) return fail(kEInput, "too many intersections");
+    cap = std::max(cap, (long long)hc[0] + (long long)hc[0] / 8);
+    lcap = std::max(lcap, (long long)hc[5]);
+  }
+  hit_cap_ = cap;
+  group_cap_ = lcap;
+  *nhits = (long long)hc[0];
+  out.survivors = (long long)hc[2];
+  out.tests = (long long)hc[1];
+  out.raw_hits = (long long)hc[3];
+  out.work = (long long)hc[4];
   return kOk;
 }
 

@@ -512,15 +512,26 @@ static int npow2_host(int n) {
 // (full key, vertex) order, the order of the stable sort on full keys.
 constexpr int kFixRun = 32;  // longer runs fall back to the 64-bit sort
 
+struct Narrow {
+  double scale, shift;
+  __device__ explicit Narrow(const unsigned long long* mm) {
+    const double lo = dkey_value(mm[0]), hi = dkey_value(mm[1]);
+    scale = hi > lo ? (4294967296.0 - 1048576.0) / (hi - lo) : 0.0;
+    shift = 524288.0 - lo * scale;
+  }
+  __device__ unsigned operator()(unsigned long long key) const {
+    return __double2uint_rz(__fma_rn(dkey_value(key), scale, shift));
+  }
+};
+
 __global__ void k_vertex_narrow(int E, const unsigned long long* __restrict__ vkey,
                                 const unsigned long long* __restrict__ mm,
                                 unsigned* __restrict__ g, unsigned* __restrict__ gid) {
   __shared__ double s_scale, s_shift;
   if (threadIdx.x == 0) {
-    const double lo = dkey_value(mm[0]), hi = dkey_value(mm[1]);
-    const double sc = hi > lo ? (4294967296.0 - 1048576.0) / (hi - lo) : 0.0;
-    s_scale = sc;
-    s_shift = 524288.0 - lo * sc;
+    const Narrow n(mm);
+    s_scale = n.scale;
+    s_shift = n.shift;
   }
   __syncthreads();
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -572,6 +583,324 @@ __global__ void k_vertex_full(int E, const unsigned* __restrict__ g, unsigned* _
     skey[i + t] = kk[t];
     gid[i + t] = ii[t];
   }
+}
+
+// ---- the tree's quantities from ranks, where no x value is shared
+//
+// With distinct vertex x values the elementary array is those values in order
+// without the largest, padded with the second largest, and every position in
+// it is a rank: each edge's end leaves and leaf range follow from the ranks of
+// its two vertices and the arithmetic of findBoarder's search
+// (border_by_position), without the endpoint order, the elementary array or a
+// host read in between.  A shared x value, many zero border keys, or values
+// whose keys leave the reference's range set kFlagSharedX, and the stages that
+// build the arrays run instead (redo_tree).
+//
+// The vertices' full keys in the narrow order with equal-key runs sorted, as
+// k_vertex_full does, and each vertex's rank.
+__global__ void k_vertex_rank(int E, const unsigned* __restrict__ g, const unsigned* __restrict__ gid,
+                              const unsigned long long* __restrict__ vkey,
+                              unsigned long long* __restrict__ skey, int* __restrict__ rank,
+                              unsigned* __restrict__ flags) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= E) return;
+  const unsigned gi = g[i];
+  const bool prev_eq = i > 0 && g[i - 1] == gi;
+  const bool next_eq = i + 1 < E && g[i + 1] == gi;
+  if (!prev_eq && !next_eq) {
+    const unsigned v = gid[i];
+    skey[i] = vkey[v];
+    rank[v] = i;
+    return;
+  }
+  if (prev_eq) return;
+  int m = 1;
+  while (i + m < E && g[i + m] == gi && m < kFixRun) ++m;
+  if (i + m < E && g[i + m] == gi) {
+    atomicOr(flags, (unsigned)kFlagSharedX);
+    return;
+  }
+  unsigned long long kk[kFixRun];
+  unsigned ii[kFixRun];
+  for (int t = 0; t < m; ++t) {
+    ii[t] = gid[i + t];
+    kk[t] = vkey[ii[t]];
+  }
+  for (int t = 1; t < m; ++t) {
+    const unsigned long long k0 = kk[t];
+    const unsigned i0 = ii[t];
+    int u = t - 1;
+    while (u >= 0 && kk[u] > k0) {
+      kk[u + 1] = kk[u];
+      ii[u + 1] = ii[u];
+      --u;
+    }
+    kk[u + 1] = k0;
+    ii[u + 1] = i0;
+  }
+  for (int t = 0; t < m; ++t) {
+    skey[i + t] = kk[t];
+    rank[ii[t]] = i + t;
+    if (t > 0 && kk[t] == kk[t - 1]) atomicOr(flags, (unsigned)kFlagSharedX);
+  }
+}
+
+// The position of the never-written border slot: after the leading zero ones
+// of realToInt's border keys (oacc_segment_tree.cpp:203-206); all keys lie in
+// the reference's range when the largest does.  One thread.
+__device__ void rank_zero(int E, int epc, const unsigned long long* skey,
+                          const unsigned long long* mm, int* zero, unsigned* flags) {
+  constexpr int kMaxZero = 64;
+  const double lo = dkey_value(mm[0]), absMin = fabs(lo), dv = dadd(dkey_value(mm[1]), absMin);
+  int z = 0;
+  bool bad = !(dv < 2147483647.0);
+  if (!bad) {
+    int digits = 1;
+    for (int iv = (int)trunc(dv); iv / 10 > 0; iv /= 10) ++digits;
+    double scale = 1.0;
+    for (int t = 0; t < 11 - digits; ++t) scale = dmul(scale, 10.0);
+    auto key = [&](int i) -> long long {
+      const double v = dkey_value(skey[min(i, E - 2)]);
+      return (long long)(lo < 0 ? dmul(scale, dadd(v, absMin)) : dmul(scale, v));
+    };
+    const long long top = key(E - 2);
+    bad = top < 0 || top >= 100000000000LL;
+    while (!bad && z + 1 < epc && key(z + 1) == 0)
+      if (++z > kMaxZero) bad = true;
+  }
+  *zero = z;
+  if (bad) atomicOr(flags, (unsigned)kFlagSharedX);
+}
+
+__global__ void k_rank_zero(int E, int epc, const unsigned long long* __restrict__ skey,
+                            const unsigned long long* __restrict__ mm, int* __restrict__ zero,
+                            unsigned* __restrict__ flags) {
+  rank_zero(E, epc, skey, mm, zero, flags);
+}
+
+// The same for few vertices, by one block in shared memory: a bitonic network
+// over (key, vertex).  Up to 4,096 vertices it takes 6 to 15 us, the radix
+// sort's eight launches 25 to 40.  kFlagLongRun: 32-bit keys would have had a
+// run too long to fix up (what SBC_STAT_VERTEX_SORT reports).
+constexpr int kRankSmall = 4096;
+__global__ void __launch_bounds__(1024) k_rank_small(int E, const unsigned long long* __restrict__ vkey,
+                                                     const unsigned long long* __restrict__ mm,
+                                                     unsigned long long* __restrict__ skey,
+                                                     int* __restrict__ rank, int epc,
+                                                     int* __restrict__ zero, unsigned* __restrict__ flags) {
+  __shared__ unsigned long long s_key[kRankSmall];
+  __shared__ unsigned short s_v[kRankSmall];
+  int np = 32;
+  while (np < E) np <<= 1;
+  for (int i = threadIdx.x; i < np; i += 1024) {
+    s_key[i] = i < E ? vkey[i] : ~0ull;
+    s_v[i] = (unsigned short)i;
+  }
+  __syncthreads();
+  for (int k = 2; k <= np; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int q = threadIdx.x; q < (np >> 1); q += 1024) {
+        const int m = ((q & ~(j - 1)) << 1) | (q & (j - 1)), l = m | j;
+        const unsigned long long x = s_key[m], y = s_key[l];
+        if ((x > y) == ((m & k) == 0) && x != y) {
+          s_key[m] = y;
+          s_key[l] = x;
+          const unsigned short t = s_v[m];
+          s_v[m] = s_v[l];
+          s_v[l] = t;
+        }
+      }
+      __syncthreads();
+    }
+  const Narrow narrow(mm);
+  for (int i = threadIdx.x; i < E; i += 1024) {
+    skey[i] = s_key[i];
+    if (i + kFixRun < E && narrow(s_key[i]) == narrow(s_key[i + kFixRun]))
+      atomicOr(flags, (unsigned)kFlagLongRun);
+    if (s_v[i] < E) rank[s_v[i]] = i;
+    if (i > 0 && s_key[i] == s_key[i - 1]) atomicOr(flags, (unsigned)kFlagSharedX);
+  }
+  if (threadIdx.x == 0) rank_zero(E, epc, s_key, mm, zero, flags);
+}
+
+// Per edge from its vertices' ranks: the end-list leaves
+// (insertToLeafLevelEdgeListMulticore, oacc_segment_tree.cpp:2010-2113) and
+// the leaf range of its cover lists (insertEdgeParallel, :2496-2564), as
+// k_edge_tree has them.  cnt[0] counts the end-list leaves, cnt[1] the cover
+// entries (kCover; otherwise k_cover_count does).
+template <bool kCover>
+__global__ void __launch_bounds__(256)
+k_rank_tree(int E, int nb, int k, const int* __restrict__ cc, const int* __restrict__ rank,
+            const int* __restrict__ zero, const double* __restrict__ es,
+            const double* __restrict__ ee, int epc, int logL, int* __restrict__ aft,
+            int* __restrict__ bef, int2* __restrict__ lr, unsigned long long* __restrict__ cnt) {
+  const int z = *zero;
+  // findBoarder for a value at positions [x, y): the search meets the
+  // never-written slot 0 (z = 0) only on its way to the first two positions,
+  // and finds any other single position where it is
+  auto border = [&](int2 p, double q) {
+    if (z == 0 && p.x >= 2 && p.y == p.x + 1) return p.x;
+    return border_by_position(epc, z, p.x, p.y, q);
+  };
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned n_leaf = 0, n_cover = 0;
+  if (e < E) {
+    const int L = 1 << logL, last = E - 2;
+    int v2;
+    if (e < nb) {
+      v2 = e + 1 == nb ? 0 : e + 1;
+    } else {
+      const int g = e - nb, o = overlay_of(cc, k, g);
+      v2 = g + 1 == cc[o + 1] ? nb + cc[o] : e + 1;
+    }
+    // (a flagged run leaves ranks unwritten: in range all the same)
+    const int r0 = min(max(rank[e], 0), E - 1), r1 = min(max(rank[v2], 0), E - 1);
+    const int rs = min(r0, r1), re = max(r0, r1);
+    // a rank's positions [x, y) in the padded array
+    auto range = [&](int r) {
+      return r > last ? make_int2(epc, epc) : make_int2(r, r == last ? epc : r + 1);
+    };
+    auto J = [&](int m) { return m < z ? m : (m == z ? epc - 1 : m - 1); };
+    const int2 S = range(rs), T = range(re);
+    int a = -1, b = -1;
+    const int en = border(T, ee[e]);
+    if (en >= 0) {
+      const int j = J(en);  // right[j]
+      int node = 0;
+      if (j <= epc - 2) {
+        const int i = j + 1;
+        node = L + i;
+        if (i != 1 && i + 1 < epc && i >= last) node = L + i + 1;
+      }
+      if (node >= L && node < 2 * L && node - L < last) a = node;
+    }
+    const int st = border(S, es[e]);
+    if (st >= 0) {
+      const int j = J(st);  // left[j]
+      int node = 0;
+      if (j <= epc - 2) node = L + j;
+      if (node >= L && node < 2 * L && node - L < last) b = node;
+    }
+    aft[e] = a;
+    bef[e] = b;
+    n_leaf = (a >= 0) + (b >= 0);
+    const int l = min(S.x, L);
+    int r = T.y - 1;
+    r = r < 0 ? 0 : (r > L ? L : r);
+    lr[e] = make_int2(l, max(l, r));
+    if (kCover)
+      for (int x = l + L, y = max(l, r) + L; x < y; x >>= 1, y >>= 1) {
+        if (x & 1) {
+          ++n_cover;
+          ++x;
+        }
+        if (y & 1) {
+          ++n_cover;
+          --y;
+        }
+      }
+  }
+  const unsigned long long t0 = block_sum((unsigned long long)n_leaf);
+  if (threadIdx.x == 0 && t0) atomicAdd(cnt, t0);
+  if (kCover) {
+    const unsigned long long t1 = block_sum((unsigned long long)n_cover);
+    if (threadIdx.x == 0 && t1) atomicAdd(cnt + 1, t1);
+  }
+}
+
+__global__ void k_rank_ea(int E, int epc, const unsigned long long* __restrict__ skey,
+                          double* __restrict__ ea) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < epc) ea[i] = dkey_value(skey[min(i, E - 2)]);
+}
+
+int Pipeline::stage_ranks(bool cover) {
+  auto* skey = (unsigned long long*)pool_.get("v_key2", sizeof(unsigned long long) * E);
+  int* rank = (int*)pool_.get("v_rank", sizeof(int) * E);
+  int* zero = (int*)pool_.get("zcount", 256);
+  aft = (int*)pool_.get("aft", sizeof(int) * E);
+  bef = (int*)pool_.get("bef", sizeof(int) * E);
+  lr = (int2*)pool_.get("edge_leaf_range", sizeof(int2) * (E + 1));
+  d_treecnt = (unsigned long long*)pool_.get("tree_counts", 256);
+  if (pool_.failed) return fail(kENoMem, "device allocation failed (ranks)");
+  ele_count = E - 1;
+  epc = npow2_host(ele_count) + 1;
+  numLeaves = epc - 1;
+  ts = 2 * numLeaves;
+  logL = 0;
+  while ((1 << logL) < numLeaves) ++logL;
+  cudaMemsetAsync(d_treecnt, 0, 2 * sizeof(unsigned long long), st_);
+  if (E <= kRankSmall) {
+    ::sbc::KProbe kp_("k_rank_small", st_, 20.0 * E);
+    k_rank_small<<<1, 1024, 0, st_>>>(E, v_key, d_minmax, skey, rank, epc, zero, d_flags);
+  } else {
+    auto* vid2 = (unsigned*)pool_.get("v_id2", sizeof(unsigned) * E);
+    auto* vg = (unsigned*)pool_.get("v_g", sizeof(unsigned) * E);
+    auto* vg2 = (unsigned*)pool_.get("v_g2", sizeof(unsigned) * E);
+    auto* vgid = (unsigned*)pool_.get("v_gid", sizeof(unsigned) * E);
+    void* rscr = pool_.get("radix_scr", radix_scratch_bytes(2LL * E));
+    if (pool_.failed) return fail(kENoMem, "device allocation failed (ranks)");
+    {
+      ::sbc::KProbe kp_("k_vertex_narrow", st_, 16.0 * E);
+      k_vertex_narrow<<<grid_for(E, 256), 256, 0, st_>>>(E, v_key, d_minmax, vg, vgid);
+    }
+    radix_sort_u32(vg, vgid, vg2, vid2, E, 32, rscr, st_);
+    {
+      ::sbc::KProbe kp_("k_vertex_rank", st_, 28.0 * E);
+      k_vertex_rank<<<grid_for(E, 256), 256, 0, st_>>>(E, vg, vgid, v_key, skey, rank, d_flags);
+    }
+    {
+      ::sbc::KProbe kp_("k_rank_zero", st_);
+      k_rank_zero<<<1, 1, 0, st_>>>(E, epc, skey, d_minmax, zero, d_flags);
+    }
+  }
+  {
+    ::sbc::KProbe kp_("k_rank_tree", st_, 40.0 * E);
+    if (cover)
+      k_rank_tree<true><<<grid_for(E, 256), 256, 0, st_>>>(E, nb, k, cc, rank, zero, e_s, e_e, epc, logL,
+                                                           aft, bef, lr, d_treecnt);
+    else
+      k_rank_tree<false><<<grid_for(E, 256), 256, 0, st_>>>(E, nb, k, cc, rank, zero, e_s, e_e, epc, logL,
+                                                            aft, bef, lr, d_treecnt);
+  }
+  stat_vertex_sort = 2;
+  stat_edges = E;
+  stat_epc = epc;
+  stat_ts = ts;
+  from_ranks_ = lr_ready = true;
+  return kOk;
+}
+
+// whether the stages that build the arrays have to run after all
+bool Pipeline::ranks_failed(unsigned flags) {
+  if (!from_ranks_) return false;
+  if (flags & kFlagLongRun) stat_vertex_sort = 1;
+  return (flags & ~(unsigned)kFlagLongRun) != 0;
+}
+
+int Pipeline::redo_tree(unsigned flags) {
+  from_ranks_ = false;
+  if (flags & kFlagUndef) return fail(kEInput, "non-finite vertex coordinate");
+  clear_flags();
+  // the side stream may still count cover entries of the ranges replaced here
+  if (st2_) cudaStreamSynchronize(st2_);
+  int rc = stage_elementary();
+  if (!rc) rc = stage_endlists();
+  if (!rc) rc = stage_cover();
+  if (!rc) launch_cover_count();
+  return rc;
+}
+
+// the elementary array of a run from ranks (sbc_debug_array)
+int Pipeline::build_elementary() {
+  if (ea || !from_ranks_) return kOk;
+  double* p = (double*)pool_.get("ea", sizeof(double) * (epc + 1));
+  auto* skey = (unsigned long long*)pool_.get("v_key2", sizeof(unsigned long long) * E);
+  if (pool_.failed) return fail(kENoMem, "device allocation failed (ea)");
+  ::sbc::KProbe kp_("k_rank_ea", st_, 16.0 * epc);
+  k_rank_ea<<<grid_for(epc, 256), 256, 0, st_>>>(E, epc, skey, p);
+  ea = p;
+  return kOk;
 }
 
 int Pipeline::stage_elementary() {

@@ -97,13 +97,15 @@ __global__ void k_gp_scatter(Gp g) {
 // (k_gp_order_long).  With the warp's line at 32, 10,000 x 8,000 stars (19 to
 // 24 crossings an edge, up to a hundred) left 0.17 ms to the blocks.
 constexpr int kGpLane = 4, kGpWarp = 128, kGpLongMost = 4096;
-__global__ void __launch_bounds__(256) k_gp_order(Gp g) {
+// A warp looks after `per` edges: 32, or 4 where edges have many crossings (a
+// warp's edges take turns).
+__global__ void __launch_bounds__(256) k_gp_order(Gp g, int per) {
   const int lane = threadIdx.x & 31;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int x = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per + lane;
   const int n = g.nb + g.nc;
   const bool base = x < g.nb;
   int s = 0, m = 0;
-  if (x < n) {
+  if (lane < per && x < n) {
     const int e = base ? x : x - g.nb;
     s = base ? g.startB(e) : g.startC(e);
     m = (base ? g.endB[e] : g.endC[e]) - s;
@@ -128,6 +130,26 @@ __global__ void __launch_bounds__(256) k_gp_order(Gp g) {
     const int ss = __shfl_sync(0xffffffffu, s, src), mm = __shfl_sync(0xffffffffu, m, src);
     const bool bb = __shfl_sync(0xffffffffu, (int)base, src);
     int* v = (bb ? g.hP : g.hQ) + ss;
+    if (mm <= 32) {
+      const int h = lane < mm ? v[lane] : -1;
+      const int a = lane < mm ? (bb ? g.aB[h] : g.aC[h]) : INT_MAX;
+      int rank = 0;
+      bool tie = false;
+      for (int j = 0; j < mm; ++j) {
+        const int aj = __shfl_sync(0xffffffffu, a, j);
+        rank += aj < a;
+        tie |= aj == a && j != lane;
+      }
+      if (__any_sync(0xffffffffu, tie && lane < mm)) {
+        rank = 0;
+        if (lane < mm)
+          for (int j = 0; j < mm; ++j) rank += bb ? g.lessB(v[j], h) : g.lessC(v[j], h);
+      }
+      __syncwarp();
+      if (lane < mm) v[rank] = h;
+      __syncwarp();
+      continue;
+    }
     constexpr int kPer = kGpWarp / 32;
     int h[kPer], a[kPer], rank[kPer];
     bool tie = false;
@@ -208,26 +230,43 @@ __global__ void k_gp_rank(Gp g) {
 }
 
 // pointInPoly (foster/polygon.h:427-448) of each polygon's first vertex in the
-// other, over the list's edges: blockIdx.y 0 the overlay's edges, 1 the base's
+// other, over the list's edges: blockIdx.y 0 the overlay's edges, 1 the base's.
+// Few polygon edges reach the ray's height; a warp takes each of those with
+// its crossings together (an edge may have hundreds).
 __global__ void __launch_bounds__(256) k_gp_pip(Gp g) {
   const bool base = blockIdx.y == 1;
   const int n = base ? g.nb : g.nc;
   const double2* p = (const double2*)(base ? g.b : g.c);
   const double2 r = ((const double2*)(base ? g.c : g.b))[0];
   int part = 0;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    double2 u = p[e];
-    const double2 v = p[e + 1];
-    if (!ray_near(u.y, v.y, r.y)) continue;
-    if (g.K > 0) {
-      const int s = base ? g.startB(e) : g.startC(e), t = base ? g.endB[e] : g.endC[e];
-      for (int k = s; k < t; ++k) {
-        const double2 x = g.xy[base ? g.hP[k] : g.hQ[k]];
-        part += pip_step(u.x, u.y, x.x, x.y, r.x, r.y);
-        u = x;
+  const int lane = threadIdx.x & 31;
+  for (int e0 = blockIdx.x * blockDim.x + threadIdx.x - lane; e0 < n; e0 += gridDim.x * blockDim.x) {
+    const int e = e0 + lane;
+    double2 u = make_double2(0.0, 0.0), v = u;
+    int s = 0, t = 0;
+    bool near = false;
+    if (e < n) {
+      u = p[e];
+      v = p[e + 1];
+      if (!(u.x == u.x && u.y == u.y)) *g.bad = 1u;
+      near = ray_near(u.y, v.y, r.y);
+      if (near && g.K > 0) {
+        s = base ? g.startB(e) : g.startC(e);
+        t = base ? g.endB[e] : g.endC[e];
+      }
+      if (near && t == s) part += pip_step(u.x, u.y, v.x, v.y, r.x, r.y);
+    }
+    for (unsigned w = __ballot_sync(0xffffffffu, near && t > s); w; w &= w - 1) {
+      const int src = __ffs(w) - 1, ee = e0 + src;
+      const int ss = __shfl_sync(0xffffffffu, s, src), m = __shfl_sync(0xffffffffu, t, src) - ss;
+      // pieces 0 .. m: from point i - 1 (the vertex before all) to point i
+      for (int i = lane; i <= m; i += 32) {
+        const int* hs = base ? g.hP : g.hQ;
+        const double2 a = i == 0 ? p[ee] : g.xy[hs[ss + i - 1]];
+        const double2 b = i == m ? p[ee + 1] : g.xy[hs[ss + i]];
+        part += pip_step(a.x, a.y, b.x, b.y, r.x, r.y);
       }
     }
-    part += pip_step(u.x, u.y, v.x, v.y, r.x, r.y);
   }
   part = __reduce_add_sync(0xffffffffu, part);
   if ((threadIdx.x & 31) == 0 && part) atomicAdd(&g.wind[base ? 1 : 0], part);
@@ -594,7 +633,8 @@ int Pipeline::stage_general(int cType, const int* rb, const int* rc, const int* 
     }
     {
       ::sbc::KProbe kp_("k_gp_order", st, 4.0 * (nb + nc) + 16.0 * K);
-      k_gp_order<<<grid_for(nb + (long long)nc, 256), 256, 0, st>>>(g);
+      const int per = K > 2LL * (nb + nc) ? 4 : 32;
+      k_gp_order<<<grid_for((nb + (long long)nc) * (32 / per), 256), 256, 0, st>>>(g, per);
     }
     {
       ::sbc::KProbe kp_("k_gp_order_long", st);

@@ -65,7 +65,7 @@ class HostReads {
   static constexpr int kWords = 256;
   static constexpr int kFlags = 0;       // read_flags
   static constexpr int kFront = 8;       // elementary and end-list stages
-  static constexpr int kCand = 24;       // candidate and exact stages
+  static constexpr int kCand = 24;       // candidate and exact stages (16 words)
   static constexpr int kMid = 40;        // record and merge stages
   static constexpr int kBack = 64;       // back end
   static constexpr int kCounts = 128;    // per overlay (1..9): ring and vertex counts
@@ -223,6 +223,10 @@ class Pipeline {
 
   // stage entry points (return Status)
   int stage_setup(const double* d_bxy, const double* d_cxy, const int* c_sizes);
+  int stage_ranks(bool cover);    // A4-A7 from vertex ranks (no shared x value)
+  bool ranks_failed(unsigned flags);
+  int redo_tree(unsigned flags);  // A4-A7 by the stages below where ranks do not do
+  int build_elementary();         // the elementary array of a run from ranks, for diagnostics
   int stage_elementary();
   int stage_endlists();
   int stage_cover();
@@ -239,6 +243,11 @@ class Pipeline {
   void join_side();               // later work on the main stream waits for the side stream
   void take_tree_stats();         // the cover stage's statistics, once their copy landed
   void launch_cover_count();      // the cover-entry statistic on the side stream
+  // the candidate stage without the grid: edge boxes, then (per overlay) hits
+  bool direct_fits() const;
+  int stage_direct_boxes();
+  int direct_candidates(int cType, int** rb, int** rc, int** rt, unsigned long long** rkey,
+                        long long* nhits, OverlayOut& out);
   int stage_candidates(int cType, int** rb, int** rc, int** rt, unsigned long long** rkey,
                        long long* nhits, OverlayOut& out);
   int stage_overlay(int cType, OverlayOut& out);
@@ -281,6 +290,16 @@ class Pipeline {
     long long nhits = 0;
   };
   LazyRecords lazy_;                   // the hits build_records() starts from
+  // Edge pairs (base x one overlay) up to which the direct candidate search
+  // replaces the grid.  A clip with it and with the grid: 24 x 18 vertices
+  // 0.20 and 0.34 ms, 10,000 x 8,000 0.61 and 0.73, 100,000 x 100,000 0.43 and
+  // 0.51, 200,000 x 150,000 0.55 and 0.54, 400,000 x 300,000 1.09 and 0.66.
+  static constexpr long long kDirectMost = 20000000000LL;
+  bool direct_ = false;                // this run searches without the grid
+  bool from_ranks_ = false;            // this run's tree quantities came from ranks
+  long long hit_cap_ = 0, group_cap_ = 0;  // room for hits and group pairs that sufficed
+  float4* gbox_ = nullptr;             // boxes of 32 edges each, polygon after polygon
+  int d_group0_[11] = {};              // each polygon's first one
   bool cover_count_pending_ = false;
   unsigned* h_side_rd_ = nullptr;      // 256 B pinned: the grid stage's reads ([0..9]),
                                        // the cover stage's two counts ([32..35])

@@ -85,3 +85,34 @@ def test_every_overlay_of_a_tree(clipper):
     ref = oracle_py.clip(b, ovs)["overlays"]
     for got, r in zip(clipper.clip(b, ovs), ref):
         assert rings_equal(got, oracle_py.rings_of(r))
+
+
+@pytest.mark.parametrize("n", [1, 30, 64, 65, 66, 90])
+def test_zero_border_keys(clipper, n):
+    """n vertices within a border key of the least x value: their keys are
+    zero, and the reference's never-written border slot comes after them.  Up
+    to 64 the ranks follow it, above that the stages that build the arrays."""
+    t = np.arange(n + 1)
+    left = np.stack([-1.0 + 1e-12 * t, 1.0 - 2.0 * t / (n + 1)], 1)
+    b = np.concatenate([left, [[-0.999, -1.01], [1.0, 0.0], [0.3, 1.1]]])
+    c = gen.star(40, 90 + n, centre=(-0.9, 0.02), R=0.5)
+    o = oracle_py.clip(b, [c])
+    assert rings_equal(clipper.clip_pair(b, c), oracle_py.rings_of(o["overlays"][0]))
+    assert np.array_equal(clipper.debug_array("elementary"), o["tree"]["ea"])
+    st = clipper.stats()
+    assert st["cover_entries"] == o["stats"]["cover_total"]
+    assert st["leaf_end_entries"] == o["stats"]["leaf_end_total"]
+    assert np.array_equal(clipper.debug_array("uniq_b"), o["overlays"][0]["uniq_b"])
+
+
+def test_more_hits_than_the_first_guess(clipper):
+    """Spiky stars whose edge groups and hits overflow the direct search's
+    first buffers on a new context."""
+    cl = sbclip.Clipper(0)
+    try:
+        b, c = gen.star(9000, 3, R=1000.0), gen.star(7000, 4, centre=(150.0, 90.0), R=1000.0)
+        ref = oracle_py.rings_of(oracle_py.clip(b, [c])["overlays"][0])
+        for _ in range(2):
+            assert rings_equal(cl.clip_pair(b, c), ref)
+    finally:
+        cl.close()
