@@ -1453,7 +1453,7 @@ __device__ void order_hits(G& g, PairWork& w, int nb, int K) {
         const int m = start[e + 1] - start[e];
         return m > 1 ? m : 0;
       },
-      [&](int e) {
+      [&](int e, int) {
         int* v = w.hsort + start[e];
         const int m = start[e + 1] - start[e];
         for (int i = 1; i < m; ++i) {
@@ -1467,7 +1467,7 @@ __device__ void order_hits(G& g, PairWork& w, int nb, int K) {
           v[j] = x;
         }
       },
-      [&](auto& gg, int e) {
+      [&](auto& gg, int e, int) {
         // a network over hit indices, compared by their keys
         const int s = start[e], m = start[e + 1] - s, np = npow2_dev(m);
         unsigned long long* scr = w.pw.sscr + 2 * s;
@@ -1502,10 +1502,12 @@ __device__ void order_hits(G& g, PairWork& w, int nb, int K) {
 // holes and islands, which used to walk their lists on one thread each:
 // 16.4 -> 1.1 ms.
 constexpr int kCleanSmem = 6144;
+constexpr int kSortRoom = 512;  // a block's sorts: keys per warp
 
 template <class G>
 __device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, int nc,
-                            unsigned char* smem, size_t smem_bytes, double* s_sum) {
+                            unsigned char* smem, size_t smem_bytes, unsigned long long* sort,
+                            int sort_room, double* s_sum) {
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   if (w.state[0] != PS_OK) return;
@@ -1523,10 +1525,11 @@ __device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, in
     // larger ones after it
     Carver cv{clean_bytes(nb, nc, K) <= smem_bytes ? smem : (unsigned char*)w.csorted, 0};
     const CleanMem m = clean_carve(cv, nb, nc, K);
-    const CleanIn in{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.bnx, w.cnx, K,
-                     w.hb, w.hc, w.ht, w.hkey, w.hal, w.hbt, A.unite, cp.rcap, w.rootB, w.rootC,
-                     w.vl, w.vloc, w.roff, w.rxy, w.tape};
-    done = clean_clip(g, in, m, s_sum, &nr, &nv, &area);
+    const CleanIn<SoaHits> in{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.bnx, w.cnx, K,
+                              SoaHits{w.hb, w.hc, w.ht, w.hkey, w.hal, w.hbt}, 0, A.unite, cp.rcap,
+                              cp.capR, w.rootB, w.rootC, w.vl, w.vloc, w.roff, w.rxy,
+                              sort, sort_room, w.tape};
+    done = clean_clip(g, in, m, s_sum, &nr, &nv, &area) == CLEAN_DONE;
   }
   if (g.rank() == 0) {
     A.status[p] = done ? SBC_OK : kPending;
@@ -1545,19 +1548,21 @@ __global__ void __launch_bounds__(128) k_batch_clean(ClipArgs A) {
   int nb, nc;
   if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
   WarpGroup g;
-  batch_clean(g, A, p, pass, nb, nc, s_mem[threadIdx.x >> 5], kCleanSmem, nullptr);
+  batch_clean(g, A, p, pass, nb, nc, s_mem[threadIdx.x >> 5], kCleanSmem, nullptr, 0,
+              nullptr);
 }
 
 __global__ void __launch_bounds__(kWideBlock, 3) k_batch_clean_wide(ClipArgs A) {
   using G = BlockGroup<kWideBlock>;
   __shared__ G::Shared sh;
+  __shared__ unsigned long long s_sort[G::kWarps * kSortRoom];
   __shared__ double s_sum[G::kWarps];
   const int p = A.wide[blockIdx.x];
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
   if (pass < 0 || !A.small(p, &nb, &nc)) return;
   G g(&sh);
-  batch_clean(g, A, p, pass, nb, nc, nullptr, 0, s_sum);
+  batch_clean(g, A, p, pass, nb, nc, nullptr, 0, s_sort, kSortRoom, s_sum);
 }
 
 // ---- the pairs left pending
@@ -2142,7 +2147,7 @@ k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ b
     };
     group_items(
         grp, n, w.R.nb, [&](int e) { return max(1, start[e + 1] - start[e]); },
-        [&](int e) {
+        [&](int e, int) {
           int* l = list + start[e];
           const int m = start[e + 1] - start[e];
           for (int i = 1; i < m; ++i) {
@@ -2158,7 +2163,7 @@ k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ b
           for (int i = 0; i < m; ++i) part(l[i], e, &own, &end);
           store(e, own, end);
         },
-        [&](auto& gg, int e) {
+        [&](auto& gg, int e, int) {
           // lane by lane over the ordered list, the lanes' sums in a fixed order
           // (scratch: R.x and R.y, adjacent in the arena)
           int* l = list + start[e];

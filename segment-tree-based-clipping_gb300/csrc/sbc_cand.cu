@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "sbc_disjoint.cuh"
 #include "sbc_pipeline.cuh"
 
 namespace sbc {
@@ -429,69 +430,11 @@ __device__ __forceinline__ unsigned emission(int b, int c, int cId, const int2* 
 }
 
 // ------------------------------------------------------------------ exact stage
-__device__ __forceinline__ float vdx(const float4& a, const float4& b) {
-  return __fadd_rn(__fsub_rn(a.x, b.x), __fsub_rn(a.z, b.z));
-}
-__device__ __forceinline__ float vdy(const float4& a, const float4& b) {
-  return __fadd_rn(__fsub_rn(a.y, b.y), __fsub_rn(a.w, b.w));
-}
-__device__ __forceinline__ float fcross(float ax, float ay, float bx, float by) {
-  return __fsub_rn(__fmul_rn(ax, by), __fmul_rn(ay, bx));
-}
-
-// True only when lineSegmentIntersection2 (seg_isect) certainly returns 0
-// for P = (p1, p2), Q = (q1, q2), decided in float from vertex hi/lo pairs.
-//
-// With a = q1 - p1, b = q2 - p1, w = p2 - p1 the four areas seg_isect uses
-// are AP1 = a x b, AQ1 = w x a, AQ2 = w x b and AP2 = AP1 + AQ1 - AQ2.
-//  * If AP1 and AP2 have the same strict sign, |AP1| > 2e-9 and
-//    |AP1| > 2e-9 |AP2|, then alpha = AP1 / (AP1 - AP2) is > 1 or
-//    < -EPSILON, and the collinear branch (|AP1| < EPSILON) is excluded:
-//    the type is 0.
-//  * If AQ1 and AQ2 have the same strict sign, |AQ1| > 2e-9 |AQ2| and
-//    |AP1| > 2e-9, then beta is > 1 or < -EPSILON in the general branch and
-//    the collinear branch is excluded again: the type is 0.
-// Segments that do not meet satisfy one of the two unless they are within
-// the float error of touching.  Each float area carries the bound
-// 32 u m^2 + 64 u^2 m M (u = 2^-24, m = largest difference component,
-// M = coordinate magnitude), at least 2.6 times the worst case of the
-// difference and product rounding; the FP64 areas of seg_isect differ from
-// the exact ones by about 1e-15 m^2, far inside it.
-__device__ __forceinline__ bool certainly_disjoint(const float4& p1, const float4& p2,
-                                                   const float4& q1, const float4& q2) {
-  const float ax = vdx(q1, p1), ay = vdy(q1, p1);
-  const float bx = vdx(q2, p1), by = vdy(q2, p1);
-  const float wx = vdx(p2, p1), wy = vdy(p2, p1);
-  const float AP1 = fcross(ax, ay, bx, by);
-  const float AQ1 = fcross(wx, wy, ax, ay);
-  const float AQ2 = fcross(wx, wy, bx, by);
-  const float AP2 = __fsub_rn(__fadd_rn(AP1, AQ1), AQ2);
-  const float m = fmaxf(fmaxf(fmaxf(fabsf(ax), fabsf(ay)), fmaxf(fabsf(bx), fabsf(by))),
-                        fmaxf(fabsf(wx), fabsf(wy)));
-  const float M = __fadd_rn(fmaxf(fabsf(p1.x), fabsf(p1.y)), __fmul_rn(2.f, m));
-  const float u = 5.9604645e-8f;  // 2^-24
-  const float Bx = __fadd_rn(__fmul_rn(__fmul_rn(32.f * u, m), m),
-                             __fadd_rn(__fmul_rn(__fmul_rn(64.f * u * u, m), M), 1e-30f));
-  const float B2 = __fadd_rn(__fmul_rn(3.f, Bx),
-                             __fmul_rn(4.f * u, __fadd_rn(__fadd_rn(fabsf(AP1), fabsf(AQ1)), fabsf(AQ2))));
-  const float L1 = __fsub_rn(fabsf(AP1), Bx);
-  if (!(L1 > 2e-9f)) return false;  // also keeps the collinear branch out
-  const bool sameP = (AP1 > Bx && AP2 > B2) || (AP1 < -Bx && AP2 < -B2);
-  if (sameP && L1 > __fmul_rn(2e-9f, __fadd_rn(fabsf(AP2), B2))) return true;
-  const bool sameQ = (AQ1 > Bx && AQ2 > Bx) || (AQ1 < -Bx && AQ2 < -Bx);
-  const float LQ1 = __fsub_rn(fabsf(AQ1), Bx);
-  return sameQ && LQ1 > __fmul_rn(2e-9f, __fadd_rn(fabsf(AQ2), Bx));
-}
-
-// Vertex coordinates as float pairs: hi = x rounded to float, lo = (x - hi)
-// rounded to float, so hi + lo is within 2^-48 |x| of the double.
+// every vertex as a float pair
 __global__ void k_vertex_f4(long long nv, const double* __restrict__ xy, float4* __restrict__ out) {
   long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nv) return;
-  const double x = xy[2 * v], y = xy[2 * v + 1];
-  const float hx = __double2float_rn(x), hy = __double2float_rn(y);
-  out[v] = make_float4(hx, hy, __double2float_rn(dsub(x, (double)hx)),
-                       __double2float_rn(dsub(y, (double)hy)));
+  out[v] = float_pair(xy[2 * v], xy[2 * v + 1]);
 }
 
 // Exact stage per candidate pair.  Phase 1 (one pair per thread): FP64 LSMF,
@@ -636,13 +579,8 @@ k_direct_boxes(EdgeGroups eg, int nb, int k, const int* __restrict__ cS, const i
       box = make_float4(__double2float_rd(fmin(p[0], p[2])), __double2float_rd(fmin(p[1], p[3])),
                         __double2float_ru(fmax(p[0], p[2])), __double2float_ru(fmax(p[1], p[3])));
       fbox[cl == 0 ? j : nb + cc[cl - 1] + j] = box;
-      auto pair = [](double x, double y) {
-        const float hx = __double2float_rn(x), hy = __double2float_rn(y);
-        return make_float4(hx, hy, __double2float_rn(dsub(x, (double)hx)),
-                           __double2float_rn(dsub(y, (double)hy)));
-      };
-      vf[0] = pair(p[0], p[1]);
-      if (j == n - 1) vf[1] = pair(p[2], p[3]);  // the closing vertex
+      vf[0] = float_pair(p[0], p[1]);
+      if (j == n - 1) vf[1] = float_pair(p[2], p[3]);  // the closing vertex
     }
   }
   for (int o = 16; o > 0; o >>= 1) {

@@ -26,6 +26,47 @@
 namespace sbc {
 namespace {
 
+// The hits of a pair: base and overlay edge, type, first emission, alpha and
+// beta.  kSparse: sorted by base edge, of a base so large that nothing is
+// kept per base edge.
+struct SoaHits {
+  static constexpr bool kSparse = false;
+  const int *hb, *hc, *ht;  // 2 * base edge, 2 * overlay edge, type
+  const unsigned long long* hkey;
+  const double *hal, *hbt;
+  __device__ int b(int h) const { return hb[h] >> 1; }
+  __device__ int c(int h) const { return hc[h] >> 1; }
+  __device__ int type(int h) const { return ht[h]; }
+  __device__ unsigned long long key(int h) const { return hkey[h]; }
+  __device__ double al(int h) const { return hal[h]; }
+  __device__ double bt(int h) const { return hbt[h]; }
+};
+
+// one past the last k < n that in_run(k) accepts, from x (accepted) on; the
+// run is contiguous
+template <class InRun>
+__device__ __forceinline__ int run_end(int n, int x, InRun in_run) {
+  int in = x, out = x + 1;
+  for (int d = 1; out < n && in_run(out); d *= 2) {
+    in = out;
+    out += d;
+  }
+  if (out > n) out = n;
+  while (out - in > 1) {
+    const int k = (in + out) >> 1;
+    if (in_run(k)) in = k;
+    else out = k;
+  }
+  return out;
+}
+
+__device__ __forceinline__ void swap_arrays(int*& a, int*& b) {
+  int* t = a;
+  a = b;
+  b = t;
+}
+
+template <class Hits>
 struct CleanIn {
   const double* b;
   int nb;
@@ -33,16 +74,17 @@ struct CleanIn {
   int nc;
   const int* bnx;  // successor of each vertex within its component (null: one ring)
   const int* cnx;
-  int K;  // hits: 2 * base edge, 2 * overlay edge, type, first emission, alpha, beta
-  const int *hb, *hc, *ht;
-  const unsigned long long* hkey;
-  const double *hal, *hbt;
+  int K;
+  Hits hits;
+  int base_steps;  // sparse: the base edges' winding steps about the overlay's first vertex
   int unite;
-  int rcap;            // room for rings
+  int rcap, vcap;      // room for rings and their vertices
   int *rootB, *rootC;  // scratch: first vertices of the components (n + 1)
   int *inB, *inC;      // scratch: per component, first vertex inside the other polygon
   int* roff;           // out: rings, their vertices, and where each vertex comes from
   double* rxy;
+  unsigned long long* sort;  // shared memory: room for sort_room keys per warp
+  int sort_room;
   int4* tape;  // {0, base vertex} {1, overlay vertex} {2, base edge, overlay edge}, ring in .w
 };
 
@@ -56,9 +98,10 @@ struct CleanMem {
   int4 *A, *B;
 };
 
+// nb: base edges to keep an end for (0: a sparse base)
 __host__ __device__ __forceinline__ CleanMem clean_carve(Carver& cv, int nb, int nc, int K) {
   CleanMem m;
-  m.endB = cv.take<int>(nb + 1);
+  m.endB = cv.take<int>(nb > 0 ? nb + 1 : 0);
   m.endC = cv.take<int>(nc + 1);
   m.hP = cv.take<int>(K);
   m.hQ = cv.take<int>(K);
@@ -98,12 +141,16 @@ __device__ int clean_components(G& g, int n, const int* nx, int* root) {
   return count;
 }
 
-// Done (true: rings, their count and vertices, and the area), or not in
-// general position (false, the same on every thread; the outputs' contents
-// are then unspecified).  s_sum: a shared double per warp of a block.
-template <class G>
-__device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s_sum,
-                           int* nrings_out, int* nverts_out, double* area_out) {
+// Done (rings, their count and vertices, and the area), not in general
+// position, or out of room for ring vertices; the same on every thread, and
+// where not done the outputs' contents are unspecified.  s_sum: a shared
+// double per warp of a block.
+enum { CLEAN_DONE = 0, CLEAN_NOT = 1, CLEAN_ROOM = 2 };
+template <class G, class Hits>
+__device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_sum,
+                          int* nrings_out, int* nverts_out, double* area_out) {
+  constexpr bool kSparse = Hits::kSparse;
+  const Hits hits = in.hits;
   const int lane = g.rank();
   constexpr int N = G::N;
   const int K = in.K, nb = in.nb, nc = in.nc;
@@ -111,23 +158,25 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
   auto bsucc = [&](int i) { return in.bnx ? in.bnx[i] : (i + 1 == nb ? 0 : i + 1); };
   auto csucc = [&](int i) { return in.cnx ? in.cnx[i] : (i + 1 == nc ? 0 : i + 1); };
   // ---- A10-A12: ranks along both polygons
-  for (int i = lane; i <= nb; i += N) m.endB[i] = 0;
+  if (!kSparse)
+    for (int i = lane; i <= nb; i += N) m.endB[i] = 0;
   for (int i = lane; i <= nc; i += N) m.endC[i] = 0;
   g.sync();
   bool bad = false;
   for (int h = lane; h < K; h += N) {
-    const int e = in.hb[h] >> 1, f = in.hc[h] >> 1;
-    if (in.ht[h] != 1) bad = true;
-    atomicAdd(&m.endB[e], 1);
+    const int e = hits.b(h), f = hits.c(h);
+    if (hits.type(h) != 1) bad = true;
+    if (kSparse) m.hP[h] = h;
+    else atomicAdd(&m.endB[e], 1);
     atomicAdd(&m.endC[f], 1);
     // the crossing (saveIntersectionsParallel, oacc_segment_tree.cpp:7257-7341)
-    const double al = in.hal[h], oma = dsub(1.0, al);
+    const double al = hits.al(h), oma = dsub(1.0, al);
     const int e2 = bsucc(e), f2 = csucc(f);
     const double p1x = b[2 * e], p1y = b[2 * e + 1], p2x = b[2 * e2], p2y = b[2 * e2 + 1];
     const double x = dadd(dmul(oma, p1x), dmul(al, p2x)), y = dadd(dmul(oma, p1y), dmul(al, p2y));
     m.x[h] = x;
     m.y[h] = y;
-    const int a = alpha_to_int(al), t = alpha_to_int(in.hbt[h]);
+    const int a = alpha_to_int(al), t = alpha_to_int(hits.bt(h));
     if (a < 0 || t < 0) bad = true;
     m.aB[h] = a % 1000000000;
     m.aC[h] = t % 1000000000;
@@ -138,69 +187,122 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
         meets(c[2 * f2], c[2 * f2 + 1]))
       bad = true;
   }
-  if (g.any(bad)) return false;
+  if (g.any(bad)) return CLEAN_NOT;
   if (K > 0) {
-    group_scan(g, m.endB, nb + 1);
+    if (!kSparse) group_scan(g, m.endB, nb + 1);
     group_scan(g, m.endC, nc + 1);
     g.sync();
     for (int h = lane; h < K; h += N) {  // a start moves up to its end
-      m.hP[atomicAdd(&m.endB[in.hb[h] >> 1], 1)] = h;
-      m.hQ[atomicAdd(&m.endC[in.hc[h] >> 1], 1)] = h;
+      if (!kSparse) m.hP[atomicAdd(&m.endB[hits.b(h)], 1)] = h;
+      m.hQ[atomicAdd(&m.endC[hits.c(h)], 1)] = h;
     }
     g.sync();
   }
-  auto startB = [&](int e) { return e == 0 ? 0 : m.endB[e - 1]; };
   auto startC = [&](int e) { return e == 0 ? 0 : m.endC[e - 1]; };
-  // per edge: alpha order, ties in record order (base edge, then emission)
-  auto order = [&](int n, auto start, const int* end, int* list, auto less) {
+  auto startB = [&](int e) { return e == 0 ? 0 : m.endB[e - 1]; };  // (not sparse)
+  auto countB = [&](int e) { return m.endB[e] - startB(e); };
+  auto countC = [&](int f) { return m.endC[f] - startC(f); };
+  // per edge: alpha order, ties in record order (base edge, then emission).
+  // A hit of a short run counts the run's hits before it: its loads do not
+  // wait for one another, and no thread sorts alone.  (An insertion sort per
+  // edge, each step a trip to the arena, took a third of the pairwise block
+  // kernel.)  A long run is sorted by alpha and index as one key, in the
+  // group's shared memory where it fits.  From v to out: src(k) is entry k of
+  // v, start(k) and end(k) the run's.
+  constexpr int kRankMost = 64;
+  auto order = [&](auto src, auto start, auto end, int* out, const int* alpha, auto less) {
     group_items(
-        g, n, m.eP, [&](int e) { const int k = end[e] - start(e); return k > 1 ? k : 0; },
-        [&](int e) {
-          int* v = list + start(e);
-          const int k = end[e] - start(e);
-          for (int i = 1; i < k; ++i) {
-            const int x = v[i];
-            int j = i;
-            while (j > 0 && less(x, v[j - 1])) {
-              v[j] = v[j - 1];
-              --j;
-            }
-            v[j] = x;
+        g, K, m.eP,
+        [&](int k) {
+          const int s = start(k), t = end(k);
+          if (t - s > kRankMost) return k == s ? t - s : 0;
+          const int h = src(k), a = alpha[h];
+          int r = s;
+#pragma unroll 4
+          for (int i = s; i < t; ++i) {
+            const int o = src(i), ao = alpha[o];
+            r += ao < a || (ao == a && o != h && less(o, h));
           }
+          out[r] = h;
+          return 0;
         },
-        [&](auto& gg, int e) {
-          const int s = start(e), k = end[e] - s, np = npow2_dev(k);
-          unsigned* scr = (unsigned*)m.A + 4 * s;
-          for (int i = gg.rank(); i < np; i += gg.N) scr[i] = i < k ? (unsigned)list[s + i] : ~0u;
+        [](int, int) {},
+        [&](auto& gg, int s, int k) {
+          const int np = npow2_dev(k);
+          constexpr bool whole = G::kBlock && std::remove_reference_t<decltype(gg)>::kBlock;
+          const int room = whole ? in.sort_room * G::N / 32 : in.sort_room;
+          unsigned long long* o = (unsigned long long*)m.A + 2 * s;
+          if (np <= room) o = in.sort + (whole ? 0 : in.sort_room * (int)(threadIdx.x >> 5));
+          for (int i = gg.rank(); i < np; i += gg.N) {
+            unsigned long long x = ~0ull;
+            if (i < k) {
+              const int h = src(s + i);
+              x = ((unsigned long long)(unsigned)alpha[h] << 32) | (unsigned)h;
+            }
+            o[i] = x;
+          }
           gg.sync();
           group_bitonic(gg, np, [&](int i, int j, bool up) {
-            const unsigned x = scr[i], y = scr[j];
-            const bool lt = x != ~0u && (y == ~0u || (x != y && less((int)x, (int)y)));
-            const bool gt = y != ~0u && (x == ~0u || (x != y && less((int)y, (int)x)));
-            if (up ? gt : lt) {
-              scr[i] = y;
-              scr[j] = x;
+            const unsigned long long x = o[i], y = o[j];
+            if ((x > y) == up) {
+              o[i] = y;
+              o[j] = x;
             }
           });
-          for (int i = gg.rank(); i < k; i += gg.N) list[s + i] = (int)scr[i];
+          int* v = out + s;
+          bool tie = false;
+          for (int i = gg.rank(); i < k; i += gg.N) {
+            tie |= i > 0 && (o[i] >> 32) == (o[i - 1] >> 32);
+            v[i] = (int)(unsigned)o[i];
+          }
+          if (gg.any(tie)) {
+            unsigned* scr = (unsigned*)o;
+            for (int i = gg.rank(); i < np; i += gg.N) scr[i] = i < k ? (unsigned)v[i] : ~0u;
+            gg.sync();
+            group_bitonic(gg, np, [&](int i, int j, bool up) {
+              const unsigned x = scr[i], y = scr[j];
+              const bool lt = x != ~0u && (y == ~0u || (x != y && less((int)x, (int)y)));
+              const bool gt = y != ~0u && (x == ~0u || (x != y && less((int)y, (int)x)));
+              if (up ? gt : lt) {
+                scr[i] = y;
+                scr[j] = x;
+              }
+            });
+            for (int i = gg.rank(); i < k; i += gg.N) v[i] = (int)scr[i];
+          }
           gg.sync();
         });
     g.sync();
   };
   if (K > 0) {
-    order(nb, startB, m.endB, m.hP, [&](int u, int v) {
-      return m.aB[u] != m.aB[v] ? m.aB[u] < m.aB[v] : in.hkey[u] < in.hkey[v];
-    });
-    order(nc, startC, m.endC, m.hQ, [&](int u, int v) {
-      if (m.aC[u] != m.aC[v]) return m.aC[u] < m.aC[v];
-      return in.hb[u] != in.hb[v] ? in.hb[u] < in.hb[v] : in.hkey[u] < in.hkey[v];
-    });
+    // (out is the inverses' arrays, which come after)
+    order([&](int k) { return kSparse ? k : m.hP[k]; },
+          [&](int k) {
+            if (!kSparse) return startB(hits.b(m.hP[k]));
+            const int e = hits.b(k);  // the run's first: its mirror image's end
+            return K - run_end(K, K - 1 - k, [&](int i) { return hits.b(K - 1 - i) == e; });
+          },
+          [&](int k) {
+            if (!kSparse) return m.endB[hits.b(m.hP[k])];
+            const int e = hits.b(k);
+            return run_end(K, k, [&](int i) { return hits.b(i) == e; });
+          },
+          m.rP, m.aB, [&](int u, int v) {
+            return m.aB[u] != m.aB[v] ? m.aB[u] < m.aB[v] : hits.key(u) < hits.key(v);
+          });
+    order([&](int k) { return m.hQ[k]; }, [&](int k) { return startC(hits.c(m.hQ[k])); },
+          [&](int k) { return m.endC[hits.c(m.hQ[k])]; }, m.rQ, m.aC, [&](int u, int v) {
+            if (m.aC[u] != m.aC[v]) return m.aC[u] < m.aC[v];
+            return hits.b(u) != hits.b(v) ? hits.b(u) < hits.b(v) : hits.key(u) < hits.key(v);
+          });
+    swap_arrays(m.hP, m.rP);
+    swap_arrays(m.hQ, m.rQ);
     for (int k = lane; k < K; k += N) {
       const int h = m.hP[k], q = m.hQ[k];
       m.rP[h] = k;
-      m.eP[k] = in.hb[h] >> 1;
+      m.eP[k] = hits.b(h);
       m.rQ[q] = k;
-      m.eQ[k] = in.hc[q] >> 1;
+      m.eQ[k] = hits.c(q);
     }
     g.sync();
     // ---- A14: every initial label a crossing (calculateInitLabelParallel,
@@ -209,7 +311,8 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     for (int k = lane; k < K && !bad; k += N) {
       const int h = m.hP[k], e = m.eP[k], q = m.rQ[h], f = m.eQ[q];
       const double cx = m.x[h], cy = m.y[h];
-      const int hm = k > startB(e) ? m.hP[k - 1] : -1, hp = k + 1 < m.endB[e] ? m.hP[k + 1] : -1;
+      const int hm = k > 0 && m.eP[k - 1] == e ? m.hP[k - 1] : -1;
+      const int hp = k + 1 < K && m.eP[k + 1] == e ? m.hP[k + 1] : -1;
       const int gm = q > startC(f) ? m.hQ[q - 1] : -1, gp = q + 1 < m.endC[f] ? m.hQ[q + 1] : -1;
       // a crossing next to this one on both polygons: another label
       if ((hm >= 0 && (hm == gm || hm == gp)) || (hp >= 0 && (hp == gm || hp == gp))) {
@@ -235,31 +338,39 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
       const bool rp = gp >= 0 ? right(m.x[gp], m.y[gp]) : right(c[2 * f2], c[2 * f2 + 1]);
       if (rm == rp) bad = true;
     }
-    if (g.any(bad)) return false;
+    if (g.any(bad)) return CLEAN_NOT;
   }
   // ---- components, and whether each one's first vertex lies in the other
-  // polygon (pointInPoly over the list's edges, a thread per polygon edge)
+  // polygon (pointInPoly over the list's edges): a thread per polygon edge
+  // without crossings and per piece between two list nodes, not per edge (an
+  // edge near the ray can hold most of a pair's crossings)
   const int ncb = in.bnx ? clean_components(g, nb, in.bnx, in.rootB) : 1;
   const int ncc = in.cnx ? clean_components(g, nc, in.cnx, in.rootC) : 1;
   auto inside = [&](bool overlay, double rx, double ry) {
     const double* p = overlay ? c : b;
-    const int n = overlay ? nc : nb;
+    const bool sparse = kSparse && !overlay;
+    const int* list = overlay ? m.hQ : m.hP;
+    const int* edge = overlay ? m.eQ : m.eP;
     int part = 0;
-    for (int e = lane; e < n; e += N) {
-      double x0 = p[2 * e], y0 = p[2 * e + 1];
+    for (int e = lane; e < (sparse ? 0 : overlay ? nc : nb); e += N) {
+      const double x0 = p[2 * e], y0 = p[2 * e + 1];
       if (!(x0 == x0 && y0 == y0)) bad = true;
+      if ((overlay ? countC(e) : countB(e)) > 0) continue;
       const int e2 = overlay ? csucc(e) : bsucc(e);
-      if (!ray_near(y0, p[2 * e2 + 1], ry)) continue;
-      const int s = overlay ? startC(e) : startB(e), t = overlay ? m.endC[e] : m.endB[e];
-      for (int k = s; k < t; ++k) {
-        const int h = overlay ? m.hQ[k] : m.hP[k];
-        part += pip_step(x0, y0, m.x[h], m.y[h], rx, ry);
-        x0 = m.x[h];
-        y0 = m.y[h];
-      }
       part += pip_step(x0, y0, p[2 * e2], p[2 * e2 + 1], rx, ry);
     }
-    return g.sum(part) & 1;
+    for (int k = lane; k < K; k += N) {  // the piece that ends at crossing k, and the last
+      const int h = list[k], e = edge[k];
+      const bool first = k == 0 || edge[k - 1] != e;
+      const int o = first ? 0 : list[k - 1];
+      part += pip_step(first ? p[2 * e] : m.x[o], first ? p[2 * e + 1] : m.y[o], m.x[h], m.y[h], rx,
+                       ry);
+      if (k + 1 < K && edge[k + 1] == e) continue;
+      const int e2 = overlay ? csucc(e) : bsucc(e);
+      part += pip_step(m.x[h], m.y[h], p[2 * e2], p[2 * e2 + 1], rx, ry);
+      if (sparse) part -= pip_step(p[2 * e], p[2 * e + 1], p[2 * e2], p[2 * e2 + 1], rx, ry);
+    }
+    return (g.sum(part) + (sparse ? in.base_steps : 0)) & 1;
   };
   int inP = 0, inQ = 0;  // of a single component
   if (ncb == 1) inP = inside(true, b[0], b[1]);
@@ -289,8 +400,8 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     } else {
       r.v0 = ncb == 1 ? 0 : in.rootB[k];
       r.v1 = ncb == 1 ? nb : in.rootB[k + 1];
-      r.lo = startB(r.v0);
-      r.hi = m.endB[r.v1 - 1];
+      r.lo = kSparse ? 0 : startB(r.v0);
+      r.hi = kSparse ? K : m.endB[r.v1 - 1];
       r.in = ncb == 1 ? inP : in.inB[k];
     }
     return r;
@@ -305,13 +416,13 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     }
     return comp(side, lo);
   };
-  if (g.any(bad)) return false;  // also: the flags are visible
+  if (g.any(bad)) return CLEAN_NOT;  // also: the flags are visible
   for (int side = 0; side < 2; ++side)
     for (int k = lane; k < (side ? ncc : ncb); k += N) {
       const Comp r = comp(side, k);
       if ((r.hi - r.lo) & 1) bad = true;
     }
-  if (g.any(bad)) return false;
+  if (g.any(bad)) return CLEAN_NOT;
   // ---- rings: first the components without crossings that lie inside (or
   // outside, for the union), whole and in order
   int rings = 0, verts = 0;
@@ -319,7 +430,8 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     for (int k = 0; k < (side ? ncc : ncb); ++k) {
       const Comp r = comp(side, k);
       if (r.hi != r.lo || !(r.in ^ in.unite)) continue;
-      if (rings >= in.rcap) return false;
+      if (rings >= in.rcap) return CLEAN_NOT;
+      if (verts + r.v1 - r.v0 > in.vcap) return CLEAN_ROOM;
       const double* p = side ? c : b;
       for (int v = r.v0 + lane; v < r.v1; v += N) {
         const int at = verts + v - r.v0;
@@ -401,7 +513,8 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     rings += tr;
     verts += tv;
   }
-  if (rings > in.rcap) return false;
+  if (rings > in.rcap) return CLEAN_NOT;
+  if (verts > in.vcap) return CLEAN_ROOM;
   if (lane == 0) in.roff[rings] = verts;
   g.sync();
   // the legs to their places: a lane writes a short one, the warp a long one
@@ -439,7 +552,7 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
         const int h = side ? m.hQ[l.to] : m.hP[l.to], to = at + l.cnt;
         in.rxy[2 * to] = m.x[h];
         in.rxy[2 * to + 1] = m.y[h];
-        in.tape[to] = make_int4(2, in.hb[h] >> 1, in.hc[h] >> 1, ring);
+        in.tape[to] = make_int4(2, hits.b(h), hits.c(h), ring);
       }
       __syncwarp();
       for (unsigned w = __ballot_sync(0xffffffffu, act && l.cnt > kShort); w; w &= w - 1) {
@@ -466,7 +579,7 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
     if (fabs(area3(in.rxy[2 * vm], in.rxy[2 * vm + 1], x, y, xp, yp)) < kEps) bad = true;
     s2 = dadd(s2, dsub(dmul(x, yp), dmul(xp, y)));
   }
-  if (g.any(bad)) return false;
+  if (g.any(bad)) return CLEAN_NOT;
   for (int o = 16; o > 0; o >>= 1) s2 = dadd(s2, __shfl_xor_sync(0xffffffffu, s2, o));
   if constexpr (G::kBlock) {
     if ((lane & 31) == 0) s_sum[g.warp()] = s2;
@@ -477,7 +590,7 @@ __device__ bool clean_clip(G& g, const CleanIn& in, const CleanMem& m, double* s
   *nrings_out = rings;
   *nverts_out = verts;
   *area_out = dmul(0.5, s2);
-  return true;
+  return CLEAN_DONE;
 }
 
 }  // namespace

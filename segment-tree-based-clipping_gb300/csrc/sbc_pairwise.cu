@@ -51,6 +51,8 @@
 #include "../../include/sbclip.h"
 #include "sbc_pipeline.cuh"
 #include "sbc_pairops.cuh"
+#include "sbc_clean.cuh"
+#include "sbc_disjoint.cuh"
 #include "sbc_pwpair.cuh"
 #include "sbc_serial.cuh"
 
@@ -68,9 +70,19 @@ constexpr int kPwPairBlock = 64;
 // per 10 records, a block's about a sixth of that plus its barriers, so the
 // line is where the kernel's tail stops being a warp's: a job of 237 overlays
 // took 7.6 ms with the line at 2,048 records, 5.9 at 1,024 and below; 34
-// overlays 5.2, 4.0 (1,024) and 3.4 (512); 3,466 overlays 8.2, 6.3 and 5.5.
+// overlays 5.2, 4.0 (1,024) and 3.4 (512); 3,466 overlays 8.2, 6.3 and 5.5
+// (all of them by the lists).
 constexpr int kPwWideBlock = 256;
 constexpr long long kPwWideCost = 8 * 512;
+// In general position the blocks are done soon enough that the largest pairs
+// are the tail again (10,000 overlays: 5.4 ms, the average block busy for 2.1):
+// those of 2,048 records and more take 1,024 threads: 2.3 ms (line at 4,096:
+// 2.1 but 0.3 ms more in all, at 8,192: 0.6 more; 512 threads: 3.1).
+constexpr long long kPwHugeCost = 8 * 2048;
+constexpr int kPwHugeBlock = 1024;
+constexpr int kPwListSplit = 8;      // see run()
+constexpr int kPwSortRoom = 512;     // and its sorts' keys
+constexpr int kPwCleanSmem = 8192;  // a warp's working arrays: some 80 records
 
 enum { PW_FAST = 0, PW_FALLBACK = 1, PW_INPUT = 2 };
 
@@ -173,26 +185,65 @@ __device__ void pw_edge_tree(const PwTree& T, int rs, double s, int re, double e
 }
 
 // ------------------------------------------------------------------ base preparation
-__global__ void k_pw_base_edges(int nb, const double* __restrict__ b,
-                                unsigned long long* __restrict__ keys, unsigned* __restrict__ vals,
-                                float4* __restrict__ fbox, PwBaseStats* st) {
+// keys, boxes and float pairs of the base's vertices and edges, and its
+// statistics (one set of atomics per block: from every thread they took 0.7
+// ms for 200,000 vertices)
+__global__ void __launch_bounds__(256)
+k_pw_base_edges(int nb, const double* __restrict__ b, unsigned long long* __restrict__ keys,
+                unsigned* __restrict__ vals, float4* __restrict__ fbox, float4* __restrict__ vf,
+                PwBaseStats* st) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nb) return;
-  const int w = v + 1 == nb ? 0 : v + 1;
-  const double x0 = b[2 * v], y0 = b[2 * v + 1], x1 = b[2 * w], y1 = b[2 * w + 1];
-  keys[v] = dkey(x0);
-  vals[v] = v;
-  fbox[v] = make_float4(__double2float_rd(fmin(x0, x1)), __double2float_rd(fmin(y0, y1)),
-                        __double2float_ru(fmax(x0, x1)), __double2float_ru(fmax(y0, y1)));
   unsigned f = 0;
-  if (!isfinite(x0) || !isfinite(y0)) f |= 1u;
-  if (x0 == x1) f |= 2u;
-  if (f) atomicOr(&st->flags, f);
-  atomicMin(&st->mnx, dkey(x0));
-  atomicMax(&st->mxx, dkey(x0));
-  atomicMin(&st->mny, dkey(y0));
-  atomicMax(&st->mxy, dkey(y0));
-  atomicAdd(&st->ext, fmax(fabs(x1 - x0), fabs(y1 - y0)));
+  unsigned long long mm[4] = {~0ull, 0ull, ~0ull, 0ull};
+  double ext = 0.0;
+  if (v < nb) {
+    const int w = v + 1 == nb ? 0 : v + 1;
+    const double x0 = b[2 * v], y0 = b[2 * v + 1], x1 = b[2 * w], y1 = b[2 * w + 1];
+    keys[v] = dkey(x0);
+    vals[v] = v;
+    fbox[v] = make_float4(__double2float_rd(fmin(x0, x1)), __double2float_rd(fmin(y0, y1)),
+                          __double2float_ru(fmax(x0, x1)), __double2float_ru(fmax(y0, y1)));
+    vf[v] = float_pair(x0, y0);
+    if (!isfinite(x0) || !isfinite(y0)) f |= 1u;
+    if (x0 == x1) f |= 2u;
+    mm[0] = mm[1] = dkey(x0);
+    mm[2] = mm[3] = dkey(y0);
+    ext = fmax(fabs(x1 - x0), fabs(y1 - y0));
+  }
+  f = __reduce_or_sync(kFullMask, f);
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const unsigned long long t = __shfl_xor_sync(kFullMask, mm[i], o);
+      mm[i] = (i & 1) ? max(mm[i], t) : min(mm[i], t);
+    }
+    ext += __shfl_xor_sync(kFullMask, ext, o);
+  }
+  __shared__ unsigned long long s_mm[8][4];
+  __shared__ double s_ext[8];
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    for (int i = 0; i < 4; ++i) s_mm[w][i] = mm[i];
+    s_ext[w] = ext;
+    if (f) atomicOr(&st->flags, f);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) {
+      for (int i = 0; i < 4; ++i) mm[i] = (i & 1) ? max(mm[i], s_mm[k][i]) : min(mm[i], s_mm[k][i]);
+      ext += s_ext[k];
+    }
+    atomicMin(&st->mnx, mm[0]);
+    atomicMax(&st->mxx, mm[1]);
+    atomicMin(&st->mny, mm[2]);
+    atomicMax(&st->mxy, mm[3]);
+    atomicAdd(&st->ext, ext);
+  }
+}
+
+__global__ void k_pw_vf(long long n, const double* __restrict__ xy, float4* __restrict__ vf) {
+  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < n) vf[v] = float_pair(xy[2 * v], xy[2 * v + 1]);
 }
 
 __global__ void k_pw_uflag(int n, const unsigned long long* __restrict__ keys, int* __restrict__ flag) {
@@ -421,6 +472,8 @@ struct PwCandArgs {
   const int* lng;
   const unsigned* nlong;
   const float4* fbox;
+  const float4* vfB;           // vertices as float pairs
+  const float4* vfC;
   PwPair* pp;
   const int* rankB;
   const int* rankC;
@@ -550,33 +603,64 @@ __device__ __forceinline__ unsigned long long warp_append(bool take, unsigned lo
   return base + __popc(m & ((1u << lane) - 1u));
 }
 
-__global__ void k_pw_cand_test(PwCandArgs A) {
-  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ok = c < A.ncand;
-  int ty = 0, t = 0, be = 0, i = 0, j = 0;
-  double al = 0.0, bt = 0.0;
-  bool lsmf = false;
-  if (ok) {
-    const int2 cb = A.cand[c];
-    t = cb.x;
-    be = cb.y;
-    i = A.tpair[t];
-    const long long o = A.coff[i];
-    const int n = (int)(A.coff[i + 1] - o);
-    j = (int)(t - o);
-    const int j2 = j + 1 == n ? 0 : j + 1;
-    const double* cc = A.cxy + 2 * o;
-    const double q1x = cc[2 * j], q1y = cc[2 * j + 1], q2x = cc[2 * j2], q2y = cc[2 * j2 + 1];
-    const int be2 = be + 1 == A.nb ? 0 : be + 1;
-    const double p1x = A.b[2 * be], p1y = A.b[2 * be + 1];
-    const double p2x = A.b[2 * be2], p2y = A.b[2 * be2 + 1];
-    lsmf = lsmf_d(p1x, p1y, p2x, p2y, q1x, q1y, q2x, q2y);
-    if (lsmf) ty = seg_isect(p1x, p1y, p2x, p2y, q1x, q1y, q2x, q2y, &al, &bt);
+// LSMF on order keys, then the float test (sbc_disjoint.cuh); what it cannot
+// rule out is queued per block and classified in full warps.  Straight FP64 on
+// every candidate kept the FP64 pipe 86 % busy: 3.2 ms for 27 M candidates.
+constexpr int kTestBlock = 256, kTestPer = 4;
+__global__ void __launch_bounds__(kTestBlock) k_pw_cand_test(PwCandArgs A) {
+  __shared__ int4 q[kTestBlock * kTestPer];
+  __shared__ int qn;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) qn = 0;
+  __syncthreads();
+  const long long base = (long long)blockIdx.x * (kTestBlock * kTestPer);
+  int tested = 0;
+  for (int r = 0; r < kTestPer; ++r) {
+    const long long c = base + r * kTestBlock + threadIdx.x;
+    bool keep = false;
+    int4 e = make_int4(0, 0, 0, 0);
+    if (c < A.ncand) {
+      const int2 cb = A.cand[c];
+      const int i = A.tpair[cb.x];
+      const long long o = A.coff[i];
+      const int n = (int)(A.coff[i + 1] - o), j = (int)(cb.x - o), j2 = j + 1 == n ? 0 : j + 1;
+      const int be = cb.y, be2 = be + 1 == A.nb ? 0 : be + 1;
+      const double2 p1 = ((const double2*)A.b)[be], p2 = ((const double2*)A.b)[be2];
+      const double2 q1 = ((const double2*)A.cxy)[o + j], q2 = ((const double2*)A.cxy)[o + j2];
+      if (lsmf_d(p1.x, p1.y, p2.x, p2.y, q1.x, q1.y, q2.x, q2.y)) {
+        ++tested;
+        keep = !certainly_disjoint(A.vfB[be], A.vfB[be2], A.vfC[o + j], A.vfC[o + j2]);
+        e = make_int4(i, be, j, 0);
+      }
+    }
+    const unsigned m = __ballot_sync(kFullMask, keep);
+    if (m) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&qn, __popc(m));
+      at = __shfl_sync(kFullMask, at, 0) + __popc(m & ((1u << lane) - 1u));
+      if (keep) q[at] = e;
+    }
   }
-  const unsigned tm = __ballot_sync(kFullMask, lsmf);
-  if ((threadIdx.x & 31) == 0 && tm) atomicAdd(A.tested, (unsigned long long)__popc(tm));
-  const unsigned long long h = warp_append(ty != 0, A.nraw);
-  if (ty != 0 && h < A.rawcap) A.raw[h] = PwHit{i, be, j, ty, 0ull, al, bt};
+  tested = __reduce_add_sync(kFullMask, tested);
+  if (lane == 0 && tested) atomicAdd(A.tested, (unsigned long long)tested);
+  __syncthreads();
+  const int nq = qn, nq32 = (nq + 31) & ~31;
+  for (int k = threadIdx.x; k < nq32; k += kTestBlock) {
+    int ty = 0;
+    int4 e = make_int4(0, 0, 0, 0);
+    double al = 0.0, bt = 0.0;
+    if (k < nq) {
+      e = q[k];
+      const long long o = A.coff[e.x];
+      const int n = (int)(A.coff[e.x + 1] - o), j2 = e.z + 1 == n ? 0 : e.z + 1;
+      const int be2 = e.y + 1 == A.nb ? 0 : e.y + 1;
+      const double2 p1 = ((const double2*)A.b)[e.y], p2 = ((const double2*)A.b)[be2];
+      const double2 q1 = ((const double2*)A.cxy)[o + e.z], q2 = ((const double2*)A.cxy)[o + j2];
+      ty = seg_isect(p1.x, p1.y, p2.x, p2.y, q1.x, q1.y, q2.x, q2.y, &al, &bt);
+    }
+    const unsigned long long h = warp_append(ty != 0, A.nraw);
+    if (ty != 0 && h < A.rawcap) A.raw[h] = PwHit{e.x, e.y, e.z, ty, 0ull, al, bt};
+  }
 }
 
 __global__ void k_pw_hit_tree(PwCandArgs A, long long nraw) {
@@ -616,25 +700,17 @@ __global__ void k_pw_hit_tree(PwCandArgs A, long long nraw) {
   }
 }
 
-// The hits of every pair in the reference's record order (base id, then
-// first emission; removeDuplicatesAtEdge after radixsort, src/clip.cpp:368-
-// 493): a stable sort by the emission key, then a stable sort by (pair, base
-// edge), then a gather.
+// The hits of every pair grouped and in base edge order (a sort by (pair, base
+// edge), then a gather).  The reference's record order within a base edge
+// (first emission; removeDuplicatesAtEdge after radixsort, src/clip.cpp:368-
+// 493) only matters to pairs that are not in general position, which sort
+// their edges' hits themselves (pw_order_runs).
 __global__ void k_pw_hit_keys(long long nh, const PwHit* __restrict__ hits,
                               unsigned long long* __restrict__ keys, unsigned* __restrict__ vals) {
   const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= nh) return;
-  keys[h] = hits[h].key;
+  keys[h] = ((unsigned long long)(unsigned)hits[h].pair << 32) | (unsigned)hits[h].b;
   vals[h] = (unsigned)h;
-}
-
-__global__ void k_pw_hit_keys2(long long nh, const PwHit* __restrict__ hits,
-                               const unsigned* __restrict__ vals,
-                               unsigned long long* __restrict__ keys) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nh) return;
-  const PwHit& x = hits[vals[t]];
-  keys[t] = ((unsigned long long)(unsigned)x.pair << 32) | (unsigned)x.b;
 }
 
 __global__ void k_pw_gather(long long nh, const PwHit* __restrict__ hits,
@@ -642,6 +718,66 @@ __global__ void k_pw_gather(long long nh, const PwHit* __restrict__ hits,
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nh) return;
   out[t] = hits[vals[t]];
+}
+
+// Each base edge's hits in order of their first emissions, by the group; H
+// holds one pair's K hits in base edge order.  A hit of a short run counts the
+// run's hits before it; a long run is sorted.  list: room for K ints, scr and
+// tmp: for K hits each.
+template <class G>
+__device__ void pw_order_runs(G& g, PwHit* H, int K, int* list, PwHit* scr, PwHit* tmp) {
+  constexpr int kRankMost = 64;
+  group_items(
+      g, K, list,
+      [&](int k) {
+        const int e = H[k].b;
+        const int s = K - run_end(K, K - 1 - k, [&](int i) { return H[K - 1 - i].b == e; });
+        const int t = run_end(K, k, [&](int i) { return H[i].b == e; });
+        if (t - s > kRankMost) return k == s ? t - s : 0;
+        const unsigned long long key = H[k].key;
+        int r = s;
+        for (int i = s; i < t; ++i) r += H[i].key < key || (H[i].key == key && i < k);
+        tmp[r] = H[k];
+        return 0;
+      },
+      [](int, int) {},
+      [&](auto& gg, int s, int n) {
+        const int np = npow2_dev(n);  // at most 2 n: keys, then indices
+        unsigned long long* key = (unsigned long long*)(scr + s);
+        int* idx = (int*)(key + np);
+        for (int i = gg.rank(); i < np; i += gg.N) {
+          key[i] = i < n ? H[s + i].key : ~0ull;
+          idx[i] = i < n ? s + i : K;
+        }
+        gg.sync();
+        group_bitonic(gg, np, [&](int i, int j, bool up) {
+          const unsigned long long u = key[i], v = key[j];
+          const int x = idx[i], y = idx[j];
+          const bool gt = u > v || (u == v && x > y);
+          if (gt == up) {
+            key[i] = v;
+            key[j] = u;
+            idx[i] = y;
+            idx[j] = x;
+          }
+        });
+        for (int i = gg.rank(); i < n; i += gg.N) tmp[s + i] = H[idx[i]];
+        gg.sync();
+      });
+  g.sync();
+  for (int k = g.rank(); k < K; k += G::N) H[k] = tmp[k];
+  g.sync();
+}
+
+// the same for the pairs that go to the pair pipeline, a block each
+__global__ void __launch_bounds__(1024)
+k_pw_order_big(const int* __restrict__ pairs, const int* __restrict__ hstart,
+               const int* __restrict__ pairK, PwHit* hits, PwHit* tmp, PwHit* scr, int* list) {
+  using G = BlockGroup<1024>;
+  __shared__ G::Shared sh;
+  G g(&sh);
+  const int p = pairs[blockIdx.x], h0 = hstart[p];
+  pw_order_runs(g, hits + h0, pairK[p], list + h0, scr + h0, tmp + h0);
 }
 
 // one pair's records as the pair pipeline's candidate hits
@@ -684,30 +820,49 @@ struct PwPip {
     const int v = runIds[lo - 1];
     return u + 1 <= P.rv0[v] + P.run[v];
   }
+  __device__ int step(int u, double rx, double ry) const {
+    const int u2 = u + 1 == nb ? 0 : u + 1;
+    return pip_step(b[2 * u], b[2 * u + 1], b[2 * u2], b[2 * u2 + 1], rx, ry);
+  }
+  // This thread's part of the steps of the base edges that keep(edge) accepts:
+  // the entries of the ray's row of cells, from the point's cell on (an edge
+  // to the left has no step), and the long edges.  Boxes first: few edges span
+  // the ray's height, and only those with a step need the cell the entry is in
+  // (an edge counts in its first cell there) and keep.
+  template <class G, class Keep>
+  __device__ int row_steps(G& grp, double rx, double ry, const Keep& keep) const {
+    const float fx = __double2float_rd(rx), y0 = __double2float_rd(ry), y1 = __double2float_ru(ry);
+    const int c0 = pw_cellx(g, fx), row = pw_celly(g, y0) * g.gx;
+    int part = 0;
+    const int last = gstart[row + g.gx];
+    for (int k = gstart[row + c0] + grp.rank(); k < last; k += G::N) {
+      const int u = gent[k];
+      const float4 f = fbox[u];
+      if (f.w < y0 || f.y > y1 || f.z < fx) continue;
+      const int st = step(u, rx, ry);
+      if (!st) continue;
+      int lo = c0, hi = g.gx;  // the last cell that starts at k or before
+      while (hi - lo > 1) {
+        const int m = (lo + hi) >> 1;
+        if (gstart[row + m] <= k) lo = m;
+        else hi = m;
+      }
+      if (max(pw_cellx(g, f.x), c0) == lo && keep(u)) part += st;
+    }
+    for (int k = grp.rank(); k < nlong; k += G::N) {
+      const int st = step(lng[k], rx, ry);
+      if (st && keep(lng[k])) part += st;
+    }
+    return part;
+  }
   template <class G>
   __device__ int operator()(G& grp, const Pool& P, double rx, double ry) const {
-    const int lane = grp.rank();
-    // the edges between list nodes: every pool node is on the list
-    int part = 0;
-    for (int v = lane; v < P.n; v += G::N) {
+    // the edges between list nodes (every pool node is on the list), then the
+    // base edges within runs
+    int part = row_steps(grp, rx, ry, [&](int u) { return internal(P, u); });
+    for (int v = grp.rank(); v < P.n; v += G::N) {
       const int nx = P.next[v];
       part += pip_step(last_x(P, v), last_y(P, v), P.x[nx], P.y[nx], rx, ry);
-    }
-    const int cy = pw_celly(g, __double2float_rd(ry));
-    // the step first: most edges of the row do not cross the ray, and only
-    // those that do need the cell and run-membership tests
-    for (int cx = lane; cx < g.gx; cx += G::N) {
-      const int cell = cy * g.gx + cx;
-      for (int k = gstart[cell]; k < gstart[cell + 1]; ++k) {
-        const int u = gent[k];
-        const int st = pip_step(b[2 * u], b[2 * u + 1], b[2 * u + 2], b[2 * u + 3], rx, ry);
-        if (st && pw_cellx(g, fbox[u].x) == cx && internal(P, u)) part += st;
-      }
-    }
-    for (int k = lane; k < nlong; k += G::N) {
-      const int u = lng[k];
-      const int st = pip_step(b[2 * u], b[2 * u + 1], b[2 * u + 2], b[2 * u + 3], rx, ry);
-      if (st && internal(P, u)) part += st;
     }
     return (grp.sum(part) % 2) != 0;
   }
@@ -722,7 +877,7 @@ struct PwPairArgs {
   const PwPair* pp;
   const int* hstart;
   const PwHit* hits;
-  const int* pass_of;  // null: every fast pair, pass 0
+  const int* pass_of;
   const int* order;    // pairs by decreasing expected work
   unsigned char* arena;
   const long long* aoff;
@@ -731,7 +886,30 @@ struct PwPairArgs {
   int* nrings;
   int* nverts;
   PwPip pip;
+  // general position (sbc_clean.cuh)
+  int* clean;          // per pair: clipped so (its tape is in the arena)
+  double* area;        // of those
+  const int* steps;    // the base's winding steps about the overlay's first vertex
+  // the other pairs' hits to put in record order, with scratch as large
+  PwHit* order_hits;
+  PwHit *order_tmp, *order_scr;
+  int* order_list;
 };
+
+struct PwHits {
+  static constexpr bool kSparse = true;
+  const PwHit* H;
+  __device__ int b(int h) const { return H[h].b; }
+  __device__ int c(int h) const { return H[h].j; }
+  __device__ int type(int h) const { return H[h].type; }
+  __device__ unsigned long long key(int h) const { return H[h].key; }
+  __device__ double al(int h) const { return H[h].al; }
+  __device__ double bt(int h) const { return H[h].bt; }
+};
+
+// where a pair clipped in general position leaves its provenance: over the
+// ring pool's coordinates, which only the list-walking steps use
+__device__ __forceinline__ int4* pw_tape(const PwWork& w) { return (int4*)w.R.x; }
 
 __global__ void k_pw_sizes(int nov, const long long* __restrict__ coff, int nb,
                            const PwPair* __restrict__ pp, const int* __restrict__ pairK,
@@ -747,12 +925,103 @@ __global__ void k_pw_sizes(int nov, const long long* __restrict__ coff, int nb,
   bytes[p] = run ? (long long)pw_arena_bytes(nb, (int)(coff[p + 1] - coff[p]), pairK[p], pass) : 0;
 }
 
-// entry wi of the queue by the calling group
+// The base's winding steps about the first vertex of each listed overlay, a
+// warp each: the row of cells is a few thousand entries, two dependent loads
+// each, which many light warps hide (within the clipping kernels it was their
+// longest step: 70 % of the warp kernel).
+__global__ void __launch_bounds__(256)
+k_pw_inside(PwPairArgs A, int n, int* __restrict__ steps) {
+  const int k = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (k >= n) return;
+  const int p = A.order[k];
+  const double* c = A.cxy + 2 * A.coff[p];
+  WarpGroup g;
+  const int sum = g.sum(A.pip.row_steps(g, c[0], c[1], [](int) { return true; }));
+  if (g.rank() == 0) steps[p] = sum;
+}
+
+// the pairs of a work queue (by decreasing expected work), one after another
+// by each warp
+template <class Pair>
+__device__ __forceinline__ void warp_queue(int n, int* queue, Pair pair) {
+  for (;;) {
+    int wi = 0;
+    if ((threadIdx.x & 31) == 0) wi = atomicAdd(queue, 1);
+    wi = __shfl_sync(kFullMask, wi, 0);
+    if (wi >= n) return;
+    pair(wi);
+    __syncwarp();
+  }
+}
+// and by each block
+template <class G, class Pair>
+__device__ __forceinline__ void block_queue(G& g, int n, int* queue, Pair pair) {
+  for (;;) {
+    int wi = 0;
+    if (threadIdx.x == 0) wi = atomicAdd(queue, 1);
+    wi = g.same(wi);
+    if (wi >= n) return;
+    pair(wi);
+    g.sync();
+  }
+}
+
+// ---- pairs in general position: entry wi of the queue by the calling group
+template <class G>
+__device__ void pw_clean_pair(G& g, const PwPairArgs& A, const int* pairK, int wi,
+                              unsigned char* smem, size_t smem_bytes, unsigned long long* sort,
+                              int sort_room, double* s_sum) {
+  const int p = A.order[wi];
+  const long long o = A.coff[p];
+  const int nc = (int)(A.coff[p + 1] - o), K = pairK[p];
+  const PwCaps cp = pw_caps(A.nb, nc, K, A.pass_of[p]);
+  Carver cv{A.arena + A.aoff[p], 0};
+  const PwWork w = pw_carve(cv, cp);
+  // working arrays in shared memory, or over the arena's list-walking ones
+  Carver mv{clean_bytes(0, nc, K) <= smem_bytes ? smem : (unsigned char*)w.hord, 0};
+  const CleanMem m = clean_carve(mv, 0, nc, K);
+  const CleanIn<PwHits> in{A.b, A.nb, A.cxy + 2 * o, nc, nullptr, nullptr, K,
+                           PwHits{A.hits + A.hstart[p]}, A.steps[p], A.unite, cp.rcap, cp.capR,
+                           nullptr, nullptr, nullptr, nullptr, w.roff, w.rxy, sort, sort_room,
+                           pw_tape(w)};
+  int nr = 0, nv = 0;
+  double area = 0.0;
+  const int r = clean_clip(g, in, m, s_sum, &nr, &nv, &area);
+  if (g.rank() != 0) return;
+  A.clean[p] = r != CLEAN_NOT;
+  if (r == CLEAN_NOT) return;
+  A.status[p] = r == CLEAN_DONE ? PS_OK : PS_CAP;
+  A.nrings[p] = r == CLEAN_DONE ? nr : 0;
+  A.nverts[p] = r == CLEAN_DONE ? nv : 0;
+  A.area[p] = area;
+}
+
+__global__ void __launch_bounds__(kPwPairBlock)
+k_pw_clean(PwPairArgs A, const int* __restrict__ pairK, int* __restrict__ queue) {
+  __shared__ __align__(16) unsigned char s_mem[kPwPairBlock / 32][kPwCleanSmem];
+  WarpGroup g;
+  warp_queue(A.nov, queue, [&](int wi) {
+    pw_clean_pair(g, A, pairK, wi, s_mem[threadIdx.x >> 5], kPwCleanSmem, nullptr, 0, nullptr);
+  });
+}
+
+template <int kBlock>
+__global__ void __launch_bounds__(kBlock)
+k_pw_clean_wide(PwPairArgs A, const int* __restrict__ pairK, int* __restrict__ queue) {
+  using G = BlockGroup<kBlock>;
+  __shared__ typename G::Shared sh;
+  __shared__ double s_sum[G::kWarps];
+  extern __shared__ unsigned long long s_sort[];
+  G g(&sh);
+  block_queue(g, A.nov, queue, [&](int wi) {
+    pw_clean_pair(g, A, pairK, wi, nullptr, 0, s_sort, kPwSortRoom, s_sum);
+  });
+}
+
+// ---- the other pairs
 template <class G>
 __device__ void pw_queue_pair(G& g, const PwPairArgs& A, const int* pairK, int wi) {
   const int p = A.order[wi];
-  const int pass = A.pass_of ? A.pass_of[p] : 0;
-  if (pass < 0) return;
   if (A.pp[p].mode != PW_FAST) {
     A.status[p] = A.pp[p].mode == PW_INPUT ? PS_UNDEF + 100 : PS_FALLBACK;
     A.nrings[p] = A.nverts[p] = 0;
@@ -760,12 +1029,15 @@ __device__ void pw_queue_pair(G& g, const PwPairArgs& A, const int* pairK, int w
   }
   const long long o = A.coff[p];
   const int nc = (int)(A.coff[p + 1] - o);
-  const PwCaps cp = pw_caps(A.nb, nc, pairK[p], pass);
+  const PwCaps cp = pw_caps(A.nb, nc, pairK[p], A.pass_of[p]);
   Carver cv{A.arena + A.aoff[p], 0};
   PwWork w = pw_carve(cv, cp);
+  const int h0 = A.hstart[p];
+  pw_order_runs(g, A.order_hits + h0, cp.K, A.order_list + h0,
+                A.order_scr + h0, A.order_tmp + h0);
   int nr = 0, nv = 0;
-  const int st = pw_clip_core(g, A.b, A.nb, A.cxy + 2 * o, nc, A.hits + A.hstart[p], cp, w, A.pip,
-                              A.unite, &nr, &nv);
+  const int st = pw_clip_core(g, A.b, A.nb, A.cxy + 2 * o, nc, A.hits + h0, cp, w, A.pip, A.unite,
+                              &nr, &nv);
   A.status[p] = st;
   A.nrings[p] = st == PS_OK ? nr : 0;
   A.nverts[p] = st == PS_OK ? nv : 0;
@@ -773,39 +1045,24 @@ __device__ void pw_queue_pair(G& g, const PwPairArgs& A, const int* pairK, int w
 
 // Persistent work queue, one pair per warp at a time (32 pairs sharing a warp
 // would take turns through diverging paths; one warp shares a pair's
-// data-parallel steps among its lanes instead).  The queue hands out pairs by
-// decreasing expected work; a warp takes the next one until the queue is
-// empty.
+// data-parallel steps among its lanes instead).
 __global__ void __launch_bounds__(kPwPairBlock)
 k_pw_pairs(PwPairArgs A, const int* __restrict__ pairK, int* __restrict__ queue) {
   WarpGroup g;
-  for (;;) {
-    int wi = 0;
-    if ((threadIdx.x & 31) == 0) wi = atomicAdd(queue, 1);
-    wi = __shfl_sync(kFullMask, wi, 0);
-    if (wi >= A.nov) return;
-    pw_queue_pair(g, A, pairK, wi);
-  }
+  warp_queue(A.nov, queue, [&](int wi) { pw_queue_pair(g, A, pairK, wi); });
 }
 
 // The same with a block per pair, for the head of the queue.  Bound by the
 // latency of its steps (dependent loads between barriers), not by bytes: the
 // largest pairs used to be the whole kernel's tail on one warp each (4,000
-// overlays of a 200,000-vertex base: 15.3 ms, and 40 pairs beside it on the
-// workers; here 5.2 ms with those 40 among them).
+// overlays of a 200,000-vertex base, all by the list: 15.3 ms on warps, 5.2
+// so).
 __global__ void __launch_bounds__(kPwWideBlock)
 k_pw_pairs_wide(PwPairArgs A, const int* __restrict__ pairK, int* __restrict__ queue) {
   using G = BlockGroup<kPwWideBlock>;
   __shared__ G::Shared sh;
   G g(&sh);
-  for (;;) {
-    int wi = 0;
-    if (threadIdx.x == 0) wi = atomicAdd(queue, 1);
-    wi = g.same(wi);
-    if (wi >= A.nov) return;
-    pw_queue_pair(g, A, pairK, wi);
-    g.sync();
-  }
+  block_queue(g, A.nov, queue, [&](int wi) { pw_queue_pair(g, A, pairK, wi); });
 }
 
 // where a pair's rings live: pass 0 arena, or the retry arena
@@ -823,7 +1080,8 @@ struct PwArenas {
 __global__ void k_pw_pack(int nov, const long long* __restrict__ coff, int nb,
                           const int* __restrict__ pairK, PwArenas ar, const int* __restrict__ fast,
                           const long long* __restrict__ rpre, const long long* __restrict__ vpre,
-                          long long* __restrict__ ring_off, double* __restrict__ xy) {
+                          const int* __restrict__ clean, long long* __restrict__ ring_off,
+                          double* __restrict__ xy, int4* __restrict__ tape) {
   // one warp per pair, its lanes over the ring offsets and coordinates
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int p = (int)(t >> 5), lane = threadIdx.x & 31;
@@ -837,6 +1095,14 @@ __global__ void k_pw_pack(int nov, const long long* __restrict__ coff, int nb,
   for (int r = lane; r < nr; r += 32) ring_off[r0 + r] = v0 + w.roff[r];
   const int nv = w.roff[nr];
   for (int i = lane; i < 2 * nv; i += 32) xy[2 * v0 + i] = w.rxy[i];
+  if (clean[p]) {
+    const int4* t = pw_tape(w);
+    for (int i = lane; i < nv; i += 32) {
+      int4 x = t[i];
+      x.w += (int)r0;
+      tape[v0 + i] = x;
+    }
+  }
 }
 
 }  // namespace
@@ -859,25 +1125,14 @@ struct PairwiseRunner::BigWorker {
 // persistent grid of the per-pair kernel: every block slot of every SM, less
 // `pair_reserve` slots per SM while big pairs run beside it (their pipeline
 // kernels need room on the SMs)
-unsigned PairwiseRunner::pair_grid(int nov, bool reserve) {
-  static_assert(kPwPairBlock % 32 == 0, "whole warps");
+unsigned PairwiseRunner::pair_grid(const void* kernel, int block, size_t smem, int need,
+                                   bool reserve) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pw_pairs, kPwPairBlock, 0);
-  const int slots = std::max(1, reserve ? per_sm - pair_reserve : per_sm);
-  pair_blocks_ = (unsigned)std::max(1, sms * slots);
-  const unsigned need = grid_for(32LL * nov, kPwPairBlock);
-  return need < pair_blocks_ ? need : pair_blocks_;
-}
-
-// a block per wide pair, up to every block slot of every SM
-unsigned PairwiseRunner::wide_grid(int n) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pw_pairs_wide, kPwWideBlock, 0);
-  return (unsigned)std::min(n, std::max(1, sms * per_sm));
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+  if (reserve) per_sm -= pair_reserve;
+  return (unsigned)std::min(need, std::max(1, sms * per_sm));
 }
 
 // Time the job under a few settings and keep the fastest (results depend on
@@ -996,6 +1251,8 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   auto* vals2 = (unsigned*)pool.get("pw_bvals2", sizeof(unsigned) * nb);
   void* rscr = pool.get("pw_rscr", radix_scratch_bytes(nb));
   auto* fbox = (float4*)pool.get("pw_fbox", sizeof(float4) * nb);
+  auto* vfB = (float4*)pool.get("pw_vfb", sizeof(float4) * nb);
+  auto* vfC = (float4*)pool.get("pw_vfc", sizeof(float4) * (totalC + 1));
   auto* stats = (PwBaseStats*)pool.get("pw_bstats", sizeof(PwBaseStats));
   int* flag = (int*)pool.get("pw_uflag", sizeof(int) * (nb + 1));
   void* sscr = pool.get("pw_scan", scan_scratch_bytes((long long)nb + nov + 2) * 2);
@@ -1006,7 +1263,11 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   cudaMemcpyAsync(stats, &hs0, sizeof(hs0), cudaMemcpyHostToDevice, st);
   {
     ::sbc::KProbe kp_("k_pw_base_edges", st, 16.0 * nb + 28.0 * nb);
-    k_pw_base_edges<<<grid_for(nb, 256), 256, 0, st>>>(nb, d_bxy, keys, vals, fbox, stats);
+    k_pw_base_edges<<<grid_for(nb, 256), 256, 0, st>>>(nb, d_bxy, keys, vals, fbox, vfB, stats);
+  }
+  if (totalC > 0) {
+    ::sbc::KProbe kp_("k_pw_vf", st, 32.0 * totalC);
+    k_pw_vf<<<grid_for(totalC, 256), 256, 0, st>>>(totalC, d_cxy, vfC);
   }
   radix_sort_u64(keys, vals, keys2, vals2, nb, rscr, st);
   {
@@ -1120,6 +1381,8 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   ca.lng = lng;
   ca.nlong = nlong;
   ca.fbox = fbox;
+  ca.vfB = vfB;
+  ca.vfC = vfC;
   ca.pp = pp;
   ca.rankB = rankB;
   ca.rankC = rankC;
@@ -1160,7 +1423,7 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     cudaMemsetAsync(&cnt[1], 0, 2 * sizeof(unsigned long long), st);
     if (ncand > 0) {
       ::sbc::KProbe kp_("k_pw_cand_test", st, 72.0 * ncand);
-      k_pw_cand_test<<<grid_for(ncand, 256), 256, 0, st>>>(ca);
+      k_pw_cand_test<<<grid_for(ncand, kTestBlock * kTestPer), kTestBlock, 0, st>>>(ca);
     }
     unsigned long long hc[2];
     cudaMemcpyAsync(hc, &cnt[1], sizeof(hc), cudaMemcpyDeviceToHost, st);
@@ -1203,11 +1466,6 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     }
     radix_sort_u64(hk, hv, hk2, hv2, (long long)nh, hscr, st);
     {
-      ::sbc::KProbe kp_("k_pw_hit_keys2", st, 20.0 * (double)nh);
-      k_pw_hit_keys2<<<grid_for((long long)nh, 256), 256, 0, st>>>((long long)nh, hbuf, hv, hk);
-    }
-    radix_sort_u64(hk, hv, hk2, hv2, (long long)nh, hscr, st);
-    {
       ::sbc::KProbe kp_("k_pw_gather", st, 84.0 * (double)nh);
       k_pw_gather<<<grid_for((long long)nh, 256), 256, 0, st>>>((long long)nh, hbuf, hv, grouped);
     }
@@ -1221,7 +1479,10 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   int* pass = (int*)pool.get("pw_pass", sizeof(int) * (nov + 1));
   int* nrings = (int*)pool.get("pw_nrings", sizeof(int) * (nov + 1));
   int* nverts = (int*)pool.get("pw_nverts", sizeof(int) * (nov + 1));
+  clean = (int*)pool.get("pw_clean", sizeof(int) * (nov + 1));
+  pair_area = (double*)pool.get("pw_area", sizeof(double) * (nov + 1));
   if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise)");
+  cudaMemsetAsync(clean, 0, sizeof(int) * (nov + 1), st);
   std::vector<int> hK(nov + 1);
   std::vector<PwPair> hpp(nov);
   unsigned hlong = 0;
@@ -1243,25 +1504,18 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     }
   }
   cudaMemcpyAsync(pass, hpass.data(), sizeof(int) * nov, cudaMemcpyHostToDevice, st);
-  // longest first: the warps that start first take the pairs with the most
-  // records and vertices, and the first `wide` of them get a block each
-  int wide = 0;
-  {
-    std::vector<long long> cost(nov);
-    order_h.resize(nov);
-    for (int p = 0; p < nov; ++p) {
-      order_h[p] = p;
-      cost[p] = 8LL * hK[p] + (hoff[p + 1] - hoff[p]);
-    }
-    std::stable_sort(order_h.begin(), order_h.end(),
-                     [&](int a, int b) { return cost[a] > cost[b]; });
-    while (wide < nov && cost[order_h[wide]] >= kPwWideCost) ++wide;
+  // longest first: the groups that start first take the pairs with the most
+  // records and vertices, those above kPwWideCost on a block each
+  std::vector<long long> cost(nov);
+  order_h.resize(nov);
+  for (int p = 0; p < nov; ++p) {
+    order_h[p] = p;
+    cost[p] = 8LL * hK[p] + (hoff[p + 1] - hoff[p]);
   }
+  std::stable_sort(order_h.begin(), order_h.end(), [&](int a, int b) { return cost[a] > cost[b]; });
   int* order = (int*)pool.get("pw_order", sizeof(int) * (nov + 1));
   int* queue = (int*)pool.get("pw_queue", 256);
   if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise)");
-  cudaMemcpyAsync(order, order_h.data(), sizeof(int) * nov, cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(queue, 0, 4 * sizeof(int), st);
   PwPip pip{d_bxy, nb, g, gstart, gent, lng, (int)hlong, fbox, nullptr, 0};
   {
     ::sbc::KProbe kp_("k_pw_sizes", st);
@@ -1278,28 +1532,71 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   if (!ev_[0] && (cudaEventCreateWithFlags(&ev_[0], cudaEventDisableTiming) != cudaSuccess ||
                   cudaEventCreateWithFlags(&ev_[1], cudaEventDisableTiming) != cudaSuccess))
     return pl_.fail(kECuda, "pairwise events");
+  int* steps = (int*)pool.get("pw_steps", sizeof(int) * (nov + 1));
+  if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise)");
   PwPairArgs pa{nov, d_coff, d_cxy, d_bxy, nb, pp, hstart, grouped, pass, order, arena0, aoff0,
-                status, pl_.unite ? 1 : 0, nrings, nverts, pip};
-  cudaEventRecord(ev_[0], st);
-  cudaStreamWaitEvent(st2_, ev_[0], 0);
-  // the two queues side by side
-  auto clip_pairs = [&](cudaStream_t sw, cudaStream_t sn, int* q, bool reserve) {
-    PwPairArgs part = pa;
-    part.nov = wide;
-    if (wide > 0) {
-      ::sbc::KProbe kp_("k_pw_pairs_wide", sw);
-      k_pw_pairs_wide<<<wide_grid(wide), kPwWideBlock, 0, sw>>>(part, pairK, q);
+                status, pl_.unite ? 1 : 0, nrings, nverts, pip, clean, pair_area, steps,
+                grouped, ca.raw, hbuf, (int*)hk};
+  // The pairs that `which` picks, in cost order: blocks and warps side by side
+  // (on st2_ and st), joined on st.
+  std::vector<int> hst(nov), list;
+  h_clean_.assign(nov, 0);
+  auto clip_pairs = [&](bool in_general_position, auto which, bool reserve) {
+    list.clear();
+    int huge = 0, wide = 0;
+    for (int p : order_h)
+      if (which(p)) {
+        list.push_back(p);
+        huge += cost[p] >= kPwHugeCost;
+        wide += cost[p] >= kPwWideCost;
+      }
+    if (list.empty()) return false;
+    const int n = (int)list.size();
+    cudaMemcpyAsync(order, list.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
+    cudaMemsetAsync(queue, 0, 3 * sizeof(int), st);
+    if (in_general_position) {
+      ::sbc::KProbe kp_("k_pw_inside", st);
+      k_pw_inside<<<grid_for(32LL * n, 256), 256, 0, st>>>(pa, n, steps);
     }
-    part.nov = nov - wide;
-    part.order = order + wide;
-    if (nov > wide) {
-      // coordinates and records in; rings out
-      ::sbc::KProbe kp_("k_pw_pairs", sn, 16.0 * totalC + 40.0 * (double)nh);
-      k_pw_pairs<<<pair_grid(nov - wide, reserve), kPwPairBlock, 0, sn>>>(part, pairK, q + 1);
+    cudaEventRecord(ev_[1], st);
+    cudaStreamWaitEvent(st2_, ev_[1], 0);
+    auto launch = [&](const char* name, auto kernel, int block, size_t smem, int from, int to,
+                      int per_block, bool leave, cudaStream_t s, int* q) {
+      if (to <= from) return;
+      PwPairArgs part = pa;
+      part.nov = to - from;
+      part.order = order + from;
+      const int need = (to - from + per_block - 1) / per_block;
+      ::sbc::KProbe kp_(name, s);
+      kernel<<<pair_grid((const void*)kernel, block, smem, need, leave), block, smem, s>>>(
+          part, pairK, q);
+    };
+    const int per = kPwPairBlock / 32;
+    if (in_general_position) {
+      const auto large = k_pw_clean_wide<kPwHugeBlock>;
+      const size_t room = sizeof(unsigned long long) * kPwSortRoom;
+      const size_t smem = room * (kPwHugeBlock / 32);
+      cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      launch("k_pw_clean_huge", large, kPwHugeBlock, smem, 0, huge, 1, false, st, queue);
+      launch("k_pw_clean_wide", k_pw_clean_wide<kPwWideBlock>, kPwWideBlock,
+             room * (kPwWideBlock / 32), huge, wide, 1, false, st2_, queue + 1);
+      launch("k_pw_clean", k_pw_clean, kPwPairBlock, 0, wide, n, per, reserve, st, queue + 2);
+    } else {
+      launch("k_pw_pairs_wide", k_pw_pairs_wide, kPwWideBlock, 0, 0, wide, 1, false, st2_, queue);
+      launch("k_pw_pairs", k_pw_pairs, kPwPairBlock, 0, wide, n, per, reserve, st, queue + 1);
     }
+    cudaEventRecord(ev_[1], st2_);
+    cudaStreamWaitEvent(st, ev_[1], 0);
+    return true;
   };
-  clip_pairs(st2_, st, queue, big_pairs > 0);
-  cudaEventRecord(ev_[1], st2_);
+  auto clean_of = [&](int p) {
+    return nub == nb && hpp[p].mode == PW_FAST && hpp[p].nuc == (int)(hoff[p + 1] - hoff[p]);
+  };
+  auto results = [&]() {
+    cudaMemcpyAsync(hst.data(), status, sizeof(int) * nov, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(h_clean_.data(), clean, sizeof(int) * nov, cudaMemcpyDeviceToHost, st);
+    return cudaStreamSynchronize(st) == cudaSuccess;
+  };
   struct Stash {
     std::vector<int> off;
     std::vector<double> xy;
@@ -1327,9 +1624,19 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   // take them one at a time (a pair's pipeline waits on the host between its
   // stages; several pairs in flight keep the GPU busy meanwhile)
   std::vector<int> bigs;
-  for (int p = 0; p < nov; ++p)
-    if (is_big[p]) bigs.push_back(p);
-  if (!bigs.empty()) {
+  auto order_big = [&]() -> int {  // the reference's record order for the pairs that leave
+    if (bigs.empty()) return kOk;
+    int* d_list = (int*)pool.get("pw_big_list", sizeof(int) * bigs.size());
+    if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise)");
+    cudaMemcpyAsync(d_list, bigs.data(), sizeof(int) * bigs.size(), cudaMemcpyHostToDevice, st);
+    ::sbc::KProbe kp_("k_pw_order_big", st);
+    k_pw_order_big<<<(unsigned)bigs.size(), 1024, 0, st>>>(d_list, hstart, pairK, grouped, ca.raw,
+                                                          hbuf, (int*)hk);
+    cudaEventRecord(ev_[0], st);
+    return kOk;
+  };
+  auto clip_big = [&]() -> int {
+    if (bigs.empty()) return kOk;
     const int nw = std::max(1, std::min<int>(big_workers, (int)bigs.size()));
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1425,11 +1732,37 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     for (auto& t : th) t.join();
     for (int w = 0; w < nw; ++w)
       if (workers_[w]->rc) return pl_.fail(workers_[w]->rc, workers_[w]->msg);
+    return kOk;
+  };
+  for (int p = 0; p < nov; ++p)
+    if (is_big[p]) bigs.push_back(p);
+  if (const int rc = order_big()) return rc;
+  // Pairs in general position first; big pairs run beside them (and beside
+  // the others, if there are only others).
+  const bool any_clean =
+      clip_pairs(true, [&](int p) { return !is_big[p] && clean_of(p); }, big_pairs > 0);
+  if (!any_clean) clip_pairs(false, [&](int p) { return !is_big[p]; }, big_pairs > 0);
+  if (const int rc = clip_big()) return rc;
+  if (!results()) return pl_.fail(kECuda, "pairwise clip");
+  if (any_clean) {
+    // A few large ones left: the pair pipeline's parallel steps take less time
+    // than the list walks of one block each (16,394 records: 4.3 ms on a block,
+    // under 1 ms of kernels on a worker; blocks run side by side, so they win
+    // once each worker has several).
+    bigs.clear();
+    for (int p = 0; p < nov; ++p)
+      if (!is_big[p] && !h_clean_[p] && hpp[p].mode == PW_FAST && hK[p] >= big_k / kPwListSplit)
+        bigs.push_back(p);
+    if ((int)bigs.size() > 4 * big_workers) bigs.clear();
+    for (int p : bigs) is_big[p] = 1;
+    for (int p : bigs) maxBig = std::max(maxBig, hK[p]);
+    big_pairs += (int)bigs.size();
+    if (const int rc = order_big()) return rc;
+    const bool rest =
+        clip_pairs(false, [&](int p) { return !is_big[p] && !h_clean_[p]; }, !bigs.empty());
+    if (const int rc = clip_big()) return rc;
+    if (rest && !results()) return pl_.fail(kECuda, "pairwise clip");
   }
-  cudaStreamWaitEvent(st, ev_[1], 0);
-  std::vector<int> hst(nov);
-  cudaMemcpyAsync(hst.data(), status, sizeof(int) * nov, cudaMemcpyDeviceToHost, st);
-  if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise clip");
   int retry = 0;
   for (int p = 0; p < nov; ++p) {
     hpass[p] = -1;
@@ -1452,9 +1785,11 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise arena)");
     pa.arena = arena1;
     pa.aoff = aoff1;
-    clip_pairs(st, st, queue + 2, false);
-    cudaMemcpyAsync(hst.data(), status, sizeof(int) * nov, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise clip");
+    // with room for all their rings, each as before
+    clip_pairs(true, [&](int p) { return hpass[p] == 1 && h_clean_[p]; }, false);
+    if (!results()) return pl_.fail(kECuda, "pairwise clip");
+    if (clip_pairs(false, [&](int p) { return hpass[p] == 1 && !h_clean_[p]; }, false) && !results())
+      return pl_.fail(kECuda, "pairwise clip");
   }
   for (int p = 0; p < nov; ++p) hpass[p] = hpass[p] == 1 ? 1 : 0;
   cudaMemcpyAsync(pass, hpass.data(), sizeof(int) * nov, cudaMemcpyHostToDevice, st);
@@ -1519,6 +1854,7 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
   long long* d_rpre = (long long*)pool.get("pw_rpre", sizeof(long long) * (nov + 1));
   long long* d_vpre = (long long*)pool.get("pw_vpre", sizeof(long long) * (nov + 1));
   int* d_fast = (int*)pool.get("pw_fast", sizeof(int) * (nov + 1));
+  tape_ = pool.get("pw_tape", sizeof(int4) * (total_verts + 1));
   ring_off = (long long*)pool.get("pw_ring_off", sizeof(long long) * (total_rings + 1));
   xy = (double*)pool.get("pw_xy", sizeof(double) * 2 * (total_verts + 1));
   pair_ring = d_rpre;
@@ -1530,7 +1866,7 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
     const PwArenas ar{arena0, aoff0, arena1, aoff1, pass};
     ::sbc::KProbe kp_("k_pw_pack", st);
     k_pw_pack<<<grid_for(32LL * nov, 128), 128, 0, st>>>(nov, d_coff, nb, pairK, ar, d_fast, d_rpre,
-                                                  d_vpre, ring_off, xy);
+                                                  d_vpre, clean, ring_off, xy, (int4*)tape_);
   }
   std::vector<long long> roff_h;
   for (int p = 0; p < nov; ++p) {
@@ -1548,7 +1884,12 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
                   st);
   cudaMemcpyAsync(status, h_status.data(), sizeof(int) * nov, cudaMemcpyHostToDevice, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise output");
+  // provenance and area are known where the result came from sbc_clean.cuh
+  for (int p = 0; p < nov; ++p) h_clean_[p] = h_clean_[p] && fast[p];
   // kept for the area gradient
+  base_distinct_ = nub == nb;
+  h_vpre_ = vpre;
+  h_K_ = hK;
   last_nb_ = nb;
   last_totalC_ = totalC;
   last_nh_ = (long long)nh;
@@ -1570,30 +1911,38 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
 namespace sbc {
 namespace {
 
-// one warp per pair: each ring's shoelace terms summed lane by lane, the
-// lanes' sums combined in a fixed order (the area does not depend on the
-// launch shape)
-__global__ void k_pwa_area(int nov, const long long* __restrict__ pair_ring,
-                           const long long* __restrict__ ring_off, const double* __restrict__ xy,
-                           const int* __restrict__ status, double* __restrict__ area) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  if ((t >> 5) >= nov) return;
-  const int p = (int)(t >> 5);
+// The areas of the listed pairs, a block each: shoelace terms vertex by
+// vertex, the warps' sums in a fixed order (the area does not depend on the
+// launch shape).  The others were summed where they were clipped.
+constexpr int kAreaBlock = 512;
+__global__ void __launch_bounds__(kAreaBlock)
+k_pwa_area(const int* __restrict__ pairs, const long long* __restrict__ pair_ring,
+           const long long* __restrict__ ring_off, const double* __restrict__ xy,
+           const int* __restrict__ status, double* __restrict__ area) {
+  __shared__ double s_sum[kAreaBlock / 32];
+  const int p = pairs[blockIdx.x], lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double a = 0.0;
-  if (status[p] == SBC_OK) {
-    for (long long r = pair_ring[p]; r < pair_ring[p + 1]; ++r) {
-      const long long s = ring_off[r], e = ring_off[r + 1];
-      double s2 = 0.0;
-      for (long long i = s + lane; i < e; i += 32) {
-        const long long j = (i + 1 == e) ? s : i + 1;
-        s2 = dadd(s2, dsub(dmul(xy[2 * i], xy[2 * j + 1]), dmul(xy[2 * j], xy[2 * i + 1])));
+  const long long r0 = pair_ring[p], r1 = pair_ring[p + 1];
+  if (status[p] == SBC_OK && r1 > r0) {
+    const long long v1 = ring_off[r1];
+    for (long long i = ring_off[r0] + threadIdx.x; i < v1; i += kAreaBlock) {
+      long long lo = r0, hi = r1;  // the ring of vertex i
+      while (hi - lo > 1) {
+        const long long m = (lo + hi) >> 1;
+        if (ring_off[m] <= i) lo = m;
+        else hi = m;
       }
-      for (int o = 16; o > 0; o >>= 1) s2 = dadd(s2, __shfl_xor_sync(0xffffffffu, s2, o));
-      a = dadd(a, dmul(0.5, s2));
+      const long long j = i + 1 == ring_off[lo + 1] ? ring_off[lo] : i + 1;
+      a = dadd(a, dsub(dmul(xy[2 * i], xy[2 * j + 1]), dmul(xy[2 * j], xy[2 * i + 1])));
     }
   }
-  if (lane == 0) area[p] = a;
+  for (int o = 16; o > 0; o >>= 1) a = dadd(a, __shfl_xor_sync(kFullMask, a, o));
+  if (lane == 0) s_sum[w] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < kAreaBlock / 32; ++k) a = dadd(a, s_sum[k]);
+    area[p] = dmul(0.5, a);
+  }
 }
 
 __global__ void k_pwa_base_keys(int nb, const double* __restrict__ b,
@@ -1606,14 +1955,19 @@ __global__ void k_pwa_base_keys(int nb, const double* __restrict__ b,
   val[i] = (unsigned)i;
 }
 
-// per-pair candidates: overlay vertices, then the type-1 records of the
-// batched pairs (hits), then those of pairs the pair pipeline clipped
+}  // namespace
+
+// Candidates for the provenance of the listed pairs' ring vertices: their
+// overlay vertices, then their type-1 records (hits), then those of pairs the
+// pair pipeline clipped.
 struct PwaCand {
-  int nov;
+  int npairs;               // listed pairs, ascending
+  const int* pairs;
+  const long long* voff;    // their first candidates among the vertices (npairs + 1)
+  const long long* hoff;    // and among the hits
   const long long* coff;
-  long long totalC;
   const double* cxy;
-  long long nh;
+  const int* hstart;        // a pair's first hit
   const PwHit* hits;
   int nb;
   const double* b;
@@ -1621,66 +1975,6 @@ struct PwaCand {
   const int4* fb_rec;   // pair, base edge, overlay edge, type
   const double* fb_xy;  // crossing coordinates
 };
-
-__device__ __forceinline__ void pwa_decode(const PwaCand& C, long long i, int* pair, int4* t) {
-  if (i < C.totalC) {
-    int lo = 0, hi = C.nov;
-    while (hi - lo > 1) {
-      const int m = (lo + hi) >> 1;
-      if (C.coff[m] <= i) lo = m;
-      else hi = m;
-    }
-    *pair = lo;
-    *t = make_int4(1, (int)(i - C.coff[lo]), 0, 0);
-  } else if (i < C.totalC + C.nh) {
-    const PwHit& h = C.hits[i - C.totalC];
-    *pair = h.pair;
-    *t = make_int4(2, h.b, h.j, h.type);
-  } else {
-    const int4 r = C.fb_rec[i - C.totalC - C.nh];
-    *pair = r.x;
-    *t = make_int4(2, r.y, r.z, r.w);
-  }
-}
-
-__global__ void k_pwa_cand(PwaCand C, long long n, unsigned long long* __restrict__ kx,
-                           unsigned long long* __restrict__ ky, unsigned long long* __restrict__ kp,
-                           unsigned* __restrict__ val) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int pair;
-  int4 t;
-  pwa_decode(C, i, &pair, &t);
-  double x = 0.0, y = 0.0;
-  bool use = true;
-  if (t.x == 1) {
-    x = C.cxy[2 * (C.coff[pair] + t.y)];
-    y = C.cxy[2 * (C.coff[pair] + t.y) + 1];
-  } else if (i < C.totalC + C.nh) {
-    use = t.w == 1;
-    if (use) {  // I = (1 - a) b1 + a b2, as the record stage computed it
-      const double al = C.hits[i - C.totalC].al;
-      const int i2 = t.y + 1 == C.nb ? 0 : t.y + 1;
-      const double oma = dsub(1.0, al);
-      x = dadd(dmul(oma, C.b[2 * t.y]), dmul(al, C.b[2 * i2]));
-      y = dadd(dmul(oma, C.b[2 * t.y + 1]), dmul(al, C.b[2 * i2 + 1]));
-    }
-  } else {
-    const long long r = i - C.totalC - C.nh;
-    x = C.fb_xy[2 * r];
-    y = C.fb_xy[2 * r + 1];
-  }
-  kx[i] = use ? dkey(x) : ~0ull;
-  ky[i] = use ? dkey(y) : ~0ull;
-  kp[i] = use ? (unsigned long long)pair : ~0ull;
-  val[i] = (unsigned)i;
-}
-
-__global__ void k_pwa_gather(long long n, const unsigned long long* __restrict__ src,
-                             const unsigned* __restrict__ val, unsigned long long* __restrict__ dst) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) dst[t] = src[val[t]];
-}
 
 struct PwaLook {
   int nov;
@@ -1700,31 +1994,112 @@ struct PwaLook {
   PwaCand C;
 };
 
-// the ring and pair that own output vertex v
-__device__ __forceinline__ void pwa_owner(const PwaLook& L, long long v, long long* ring, int* pair) {
+namespace {
+
+// the last k in [0, n) with off[k] <= i
+__device__ __forceinline__ int pwa_find(const long long* off, int n, long long i) {
+  int lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int m = (lo + hi) >> 1;
+    if (off[m] <= i) lo = m;
+    else hi = m;
+  }
+  return lo;
+}
+
+// candidate i: its pair and provenance; *hit: its index among the hits, or -1
+__device__ __forceinline__ void pwa_decode(const PwaCand& C, long long i, int* pair, int4* t,
+                                           long long* hit) {
+  const long long V = C.voff[C.npairs], H = C.hoff[C.npairs];
+  *hit = -1;
+  if (i < V) {
+    const int k = pwa_find(C.voff, C.npairs, i);
+    *pair = C.pairs[k];
+    *t = make_int4(1, (int)(i - C.voff[k]), 0, 0);
+  } else if (i < V + H) {
+    const int k = pwa_find(C.hoff, C.npairs, i - V);
+    *pair = C.pairs[k];
+    *hit = C.hstart[*pair] + (i - V - C.hoff[k]);
+    const PwHit& h = C.hits[*hit];
+    *t = make_int4(2, h.b, h.j, h.type);
+  } else {
+    const int4 r = C.fb_rec[i - V - H];
+    *pair = r.x;
+    *t = make_int4(2, r.y, r.z, r.w);
+  }
+}
+
+__global__ void k_pwa_cand(PwaCand C, long long n, unsigned long long* __restrict__ kx,
+                           unsigned long long* __restrict__ ky, unsigned long long* __restrict__ kp,
+                           unsigned* __restrict__ val) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int pair;
+  int4 t;
+  long long hit;
+  pwa_decode(C, i, &pair, &t, &hit);
+  double x = 0.0, y = 0.0;
+  bool use = true;
+  if (t.x == 1) {
+    x = C.cxy[2 * (C.coff[pair] + t.y)];
+    y = C.cxy[2 * (C.coff[pair] + t.y) + 1];
+  } else if (hit >= 0) {
+    use = t.w == 1;
+    if (use) {  // I = (1 - a) b1 + a b2, as the record stage computed it
+      const double al = C.hits[hit].al;
+      const int i2 = t.y + 1 == C.nb ? 0 : t.y + 1;
+      const double oma = dsub(1.0, al);
+      x = dadd(dmul(oma, C.b[2 * t.y]), dmul(al, C.b[2 * i2]));
+      y = dadd(dmul(oma, C.b[2 * t.y + 1]), dmul(al, C.b[2 * i2 + 1]));
+    }
+  } else {
+    const long long r = i - C.voff[C.npairs] - C.hoff[C.npairs];
+    x = C.fb_xy[2 * r];
+    y = C.fb_xy[2 * r + 1];
+  }
+  kx[i] = use ? dkey(x) : ~0ull;
+  ky[i] = use ? dkey(y) : ~0ull;
+  kp[i] = use ? (unsigned long long)pair : ~0ull;
+  val[i] = (unsigned)i;
+}
+
+__global__ void k_pwa_gather(long long n, const unsigned long long* __restrict__ src,
+                             const unsigned* __restrict__ val, unsigned long long* __restrict__ dst) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) dst[t] = src[val[t]];
+}
+
+// the ring that owns output vertex v, and a ring's pair
+__device__ __forceinline__ long long pwa_ring(const PwaLook& L, long long v) {
   long long lo = 0, hi = L.nrings;
   while (hi - lo > 1) {
     const long long m = (lo + hi) >> 1;
     if (L.ring_off[m] <= v) lo = m;
     else hi = m;
   }
-  *ring = lo;
+  return lo;
+}
+__device__ __forceinline__ int pwa_pair(const PwaLook& L, long long ring) {
   int a = 0, b = L.nov;  // last pair with pair_ring <= ring (and rings to own)
   while (b - a > 1) {
     const int m = (a + b) >> 1;
-    if (L.pair_ring[m] <= lo) a = m;
+    if (L.pair_ring[m] <= ring) a = m;
     else b = m;
   }
-  while (a + 1 < L.nov && L.pair_ring[a + 1] <= lo) ++a;
-  *pair = a;
+  while (a + 1 < L.nov && L.pair_ring[a + 1] <= ring) ++a;
+  return a;
 }
 
-__global__ void k_pwa_tape(PwaLook L, long long nv, int4* __restrict__ tape) {
-  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  long long ring;
-  int pair;
-  pwa_owner(L, v, &ring, &pair);
+// the listed pairs' ring vertices: nv of them, pair k's from rv[k] (its first
+// one at vpre[k] of the output)
+__global__ void k_pwa_tape(PwaLook L, long long nv, const long long* __restrict__ rv,
+                           const long long* __restrict__ vpre, int4* __restrict__ tape) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nv) return;
+  const int k = pwa_find(rv, L.C.npairs, i);
+  const int pair = L.C.pairs[k];
+  const long long v = vpre[k] + (i - rv[k]);
+  const long long ring = pwa_ring(L, v);
   const unsigned long long qx = dkey(L.xy[2 * v]), qy = dkey(L.xy[2 * v + 1]);
   int4 t = make_int4(-1, 0, 0, 0);
   {
@@ -1749,10 +2124,12 @@ __global__ void k_pwa_tape(PwaLook L, long long nv, int4* __restrict__ tape) {
     if (lo < L.nc && L.ckp[lo] == qp && L.ckx[lo] == qx && L.cky[lo] == qy) {
       int pr;
       int4 d;
-      pwa_decode(L.C, (long long)L.cval[lo], &pr, &d);
+      long long hit;
+      pwa_decode(L.C, (long long)L.cval[lo], &pr, &d, &hit);
       t = d.x == 1 ? make_int4(1, d.y, 0, 0) : make_int4(2, d.y, d.z, 0);
     }
   }
+  t.w = (int)ring;
   tape[v] = t;
 }
 
@@ -1762,15 +2139,14 @@ __global__ void k_pwa_backward(PwaLook L, long long nv, const int4* __restrict__
                                double* __restrict__ gb, double* __restrict__ gc) {
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nv) return;
-  long long ring;
-  int pair;
-  pwa_owner(L, v, &ring, &pair);
+  const int4 t = tape[v];
+  const long long ring = t.w;
+  const int pair = pwa_pair(L, ring);
   const long long s = L.ring_off[ring], e = L.ring_off[ring + 1];
   const long long ip = (v + 1 == e) ? s : v + 1, im = (v == s) ? e - 1 : v - 1;
   const double g = gA[pair];
   const double gx = 0.5 * g * (L.xy[2 * ip + 1] - L.xy[2 * im + 1]);
   const double gy = 0.5 * g * (L.xy[2 * im] - L.xy[2 * ip]);
-  const int4 t = tape[v];
   const int nb = L.nb;
   const long long c0 = coff[pair];
   const int nc = (int)(coff[pair + 1] - c0);
@@ -1808,23 +2184,29 @@ __global__ void k_pwa_backward(PwaLook L, long long nv, const int4* __restrict__
 int PairwiseRunner::area(double* d_area, cudaStream_t st) {
   if (!valid) return pl_.fail(kEInput, "no pairwise result to take the area of");
   if (np <= 0) return kOk;
-  ::sbc::KProbe kp_("k_pwa_area", st, 16.0 * (double)total_verts);
-  k_pwa_area<<<grid_for(32LL * np, 128), 128, 0, st>>>(np, pair_ring, ring_off, xy, status, d_area);
+  cudaMemcpyAsync(d_area, pair_area, sizeof(double) * np, cudaMemcpyDeviceToDevice, st);
+  std::vector<int> list;
+  for (int p = 0; p < np; ++p)
+    if (!h_clean_[p]) list.push_back(p);
+  if (list.empty()) return kOk;
+  int* d_list = (int*)pl_.pool().get("pwa_area_list", sizeof(int) * list.size());
+  if (pl_.pool().failed) return pl_.fail(kENoMem, "device allocation failed (pairwise area)");
+  cudaMemcpyAsync(d_list, list.data(), sizeof(int) * list.size(), cudaMemcpyHostToDevice, st);
+  ::sbc::KProbe kp_("k_pwa_area", st);
+  k_pwa_area<<<(unsigned)list.size(), kAreaBlock, 0, st>>>(d_list, pair_ring, ring_off, xy, status, d_area);
   return kOk;
 }
 
-int PairwiseRunner::backward(const double* d_bxy, const double* d_cxy, const long long* d_coff,
-                             const double* d_gA, double* d_gb, double* d_gc, cudaStream_t st) {
-  if (!valid) return pl_.fail(kEInput, "no pairwise result to differentiate");
+// The provenance of the listed pairs' ring vertices by exact coordinates.
+// pre: prefix sums over the list of overlay vertices, hits and ring vertices;
+// v0: each pair's first ring vertex.
+int PairwiseRunner::lookup_tape(const double* d_bxy, const double* d_cxy, const long long* d_coff,
+                                const std::vector<int>& pairs, const std::vector<long long>* pre,
+                                const std::vector<long long>& v0, PwaLook& L, int4* tape,
+                                cudaStream_t st) {
   BufferPool& pool = pl_.pool();
-  const int nb = last_nb_;
-  const long long totalC = last_totalC_, nh = last_nh_, nfb = (long long)fb_rec_.size();
-  cudaMemsetAsync(d_gb, 0, sizeof(double) * 2 * nb, st);
-  if (totalC > 0) cudaMemsetAsync(d_gc, 0, sizeof(double) * 2 * totalC, st);
-  if (np <= 0 || total_verts == 0) {
-    if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise backward");
-    return kOk;
-  }
+  const int nb = last_nb_, n = (int)pairs.size();
+  const long long nfb = (long long)fb_rec_.size();
   // base vertices sorted by (x, y): by y, then stably by x
   auto* bkx = (unsigned long long*)pool.get("pwa_bkx", sizeof(unsigned long long) * (nb + 1));
   auto* bky = (unsigned long long*)pool.get("pwa_bky", sizeof(unsigned long long) * (nb + 1));
@@ -1832,7 +2214,7 @@ int PairwiseRunner::backward(const double* d_bxy, const double* d_cxy, const lon
   auto* bk3 = (unsigned long long*)pool.get("pwa_bk3", sizeof(unsigned long long) * (nb + 1));
   auto* bval = (unsigned*)pool.get("pwa_bval", sizeof(unsigned) * (nb + 1));
   auto* bval2 = (unsigned*)pool.get("pwa_bval2", sizeof(unsigned) * (nb + 1));
-  const long long nc = totalC + nh + nfb;
+  const long long nc = pre[0].back() + pre[1].back() + nfb;
   auto* ckx = (unsigned long long*)pool.get("pwa_ckx", sizeof(unsigned long long) * (nc + 1));
   auto* cky = (unsigned long long*)pool.get("pwa_cky", sizeof(unsigned long long) * (nc + 1));
   auto* ckp = (unsigned long long*)pool.get("pwa_ckp", sizeof(unsigned long long) * (nc + 1));
@@ -1843,9 +2225,16 @@ int PairwiseRunner::backward(const double* d_bxy, const double* d_cxy, const lon
   void* rscr = pool.get("pwa_rscr", radix_scratch_bytes((nc > nb ? nc : nb) + 1));
   int4* fbr = (int4*)pool.get("pwa_fbrec", sizeof(int4) * (nfb + 1));
   double* fbxy = (double*)pool.get("pwa_fbxy", sizeof(double) * 2 * (nfb + 1));
-  int4* tape = (int4*)pool.get("pwa_tape", sizeof(int4) * (total_verts + 1));
-  const PwHit* hits = (const PwHit*)pool.get("pw_hits_grouped", sizeof(PwHit) * (nh + 1));
+  const PwHit* hits = (const PwHit*)pool.get("pw_hits_grouped", sizeof(PwHit) * (last_nh_ + 1));
+  const int* hstart = (const int*)pool.get("pw_hstart", sizeof(int) * (np + 1));
+  int* d_pairs = (int*)pool.get("pwa_pairs", sizeof(int) * n);
+  auto* d_pre = (long long*)pool.get("pwa_pre", sizeof(long long) * 4 * (n + 1));
   if (pool.failed) return pl_.fail(kENoMem, "device allocation failed (pairwise backward)");
+  cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st);
+  for (int i = 0; i < 3; ++i)
+    cudaMemcpyAsync(d_pre + i * (n + 1), pre[i].data(), sizeof(long long) * (n + 1),
+                    cudaMemcpyHostToDevice, st);
+  cudaMemcpyAsync(d_pre + 3 * (n + 1), v0.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, st);
   if (nfb) {
     std::vector<int4> h(nfb);
     for (long long r = 0; r < nfb; ++r)
@@ -1858,13 +2247,19 @@ int PairwiseRunner::backward(const double* d_bxy, const double* d_cxy, const lon
     ::sbc::KProbe kp_("k_pwa_base_keys", st, 36.0 * nb);
     k_pwa_base_keys<<<grid_for(nb, 256), 256, 0, st>>>(nb, d_bxy, bkx, bky, bval);
   }
+  if (base_distinct_) {  // the order by x of the forward pass
+    bk2 = (unsigned long long*)pool.get("pw_bkeys", sizeof(unsigned long long) * nb);
+    bval = (unsigned*)pool.get("pw_bvals", sizeof(unsigned) * nb);
+  } else {
   cudaMemcpyAsync(bk2, bky, sizeof(unsigned long long) * nb, cudaMemcpyDeviceToDevice, st);
   radix_sort_u64(bk2, bval, bk3, bval2, nb, rscr, st);
   k_pwa_gather<<<grid_for(nb, 256), 256, 0, st>>>(nb, bkx, bval, bk2);
   radix_sort_u64(bk2, bval, bk3, bval2, nb, rscr, st);
+  }
   // bk2: x keys in (x, y) order; bk3: the y keys in that order
   k_pwa_gather<<<grid_for(nb, 256), 256, 0, st>>>(nb, bky, bval, bk3);
-  PwaCand C{np, d_coff, totalC, d_cxy, nh, hits, nb, d_bxy, nfb, fbr, fbxy};
+  const PwaCand C{n, d_pairs, d_pre, d_pre + (n + 1), d_coff, d_cxy, hstart, hits, nb, d_bxy,
+                  nfb, fbr, fbxy};
   {
     ::sbc::KProbe kp_("k_pwa_cand", st, 40.0 * (double)nc);
     k_pwa_cand<<<grid_for(nc, 256), 256, 0, st>>>(C, nc, ckx, cky, ckp, cval);
@@ -1880,11 +2275,59 @@ int PairwiseRunner::backward(const double* d_bxy, const double* d_cxy, const lon
   k_pwa_gather<<<grid_for(nc, 256), 256, 0, st>>>(nc, ckx, cval, ck3);
   k_pwa_gather<<<grid_for(nc, 256), 256, 0, st>>>(nc, cky, cval, ckx);
   // (ckx reused for sorted y keys: the unsorted x keys are no longer needed)
-  const PwaLook L{np, pair_ring, total_rings, ring_off, xy, nb, bk2, bk3, bval, nc, ck2, ck3, ckx,
-                  cval, C};
+  L.bkx = bk2;
+  L.bky = bk3;
+  L.bval = bval;
+  L.nc = nc;
+  L.ckp = ck2;
+  L.ckx = ck3;
+  L.cky = ckx;
+  L.cval = cval;
+  L.C = C;
   {
-    ::sbc::KProbe kp_("k_pwa_tape", st, 48.0 * (double)total_verts);
-    k_pwa_tape<<<grid_for(total_verts, 256), 256, 0, st>>>(L, total_verts, tape);
+    ::sbc::KProbe kp_("k_pwa_tape", st, 48.0 * (double)pre[2].back());
+    k_pwa_tape<<<grid_for(pre[2].back(), 256), 256, 0, st>>>(L, pre[2].back(), d_pre + 2 * (n + 1),
+                                                             d_pre + 3 * (n + 1), tape);
+  }
+  // the host vectors stay until their copies are done
+  if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise backward");
+  return kOk;
+}
+
+int PairwiseRunner::backward(const double* d_bxy, const double* d_cxy, const long long* d_coff,
+                             const double* d_gA, double* d_gb, double* d_gc, cudaStream_t st) {
+  if (!valid) return pl_.fail(kEInput, "no pairwise result to differentiate");
+  const int nb = last_nb_;
+  const long long totalC = last_totalC_;
+  cudaMemsetAsync(d_gb, 0, sizeof(double) * 2 * nb, st);
+  if (totalC > 0) cudaMemsetAsync(d_gc, 0, sizeof(double) * 2 * totalC, st);
+  if (np <= 0 || total_verts == 0) {
+    if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "pairwise backward");
+    return kOk;
+  }
+  int4* tape = (int4*)tape_;
+  PwaLook L{};
+  L.nov = np;
+  L.pair_ring = pair_ring;
+  L.nrings = total_rings;
+  L.ring_off = ring_off;
+  L.xy = xy;
+  L.nb = nb;
+  // pairs whose provenance is not known from the clipping: looked up
+  std::vector<int> pairs;
+  std::vector<long long> pre[3] = {{0}, {0}, {0}}, v0;  // vertices, hits, ring vertices
+  for (int p = 0; p < np; ++p) {
+    const long long nv = h_vpre_[p + 1] - h_vpre_[p];
+    if (h_clean_[p] || nv == 0) continue;
+    pairs.push_back(p);
+    pre[0].push_back(pre[0].back() + h_coff_[p + 1] - h_coff_[p]);
+    pre[1].push_back(pre[1].back() + h_K_[p]);
+    pre[2].push_back(pre[2].back() + nv);
+    v0.push_back(h_vpre_[p]);
+  }
+  if (!pairs.empty()) {
+    const int rc = lookup_tape(d_bxy, d_cxy, d_coff, pairs, pre, v0, L, tape, st);
+    if (rc) return rc;
   }
   {
     ::sbc::KProbe kp_("k_pwa_backward", st, 64.0 * (double)total_verts);

@@ -478,12 +478,21 @@ class PairwiseRunner {
   cudaStream_t st2_ = nullptr;      // the per-pair kernel's stream
   cudaEvent_t ev_[2] = {nullptr, nullptr};
   std::vector<int> order_h;
-  unsigned pair_blocks_ = 0;
-  unsigned pair_grid(int nov, bool reserve);
-  unsigned wide_grid(int n);
+  unsigned pair_grid(const void* kernel, int block, size_t smem, int need, bool reserve);
   // the last run, for area and backward
   int last_nb_ = 0;
   long long last_totalC_ = 0, last_nh_ = 0;
+  // per pair, device and host: clipped in general position, so that its area
+  // (pair_area) and its ring vertices' provenance (tape_) are known
+  int* clean = nullptr;
+  double* pair_area = nullptr;
+  void* tape_ = nullptr;
+  std::vector<int> h_clean_, h_K_;
+  bool base_distinct_ = false;  // no x value twice among the base's vertices
+  std::vector<long long> h_vpre_;
+  int lookup_tape(const double* d_bxy, const double* d_cxy, const long long* d_coff,
+                  const std::vector<int>& pairs, const std::vector<long long>* pre,
+                  const std::vector<long long>& v0, struct PwaLook& L, int4* tape, cudaStream_t st);
   std::vector<long long> h_coff_;
   std::vector<std::array<int, 4>> fb_rec_;  // records of pipeline-clipped pairs: pair, b, c, type
   std::vector<double> fb_xy_;

@@ -772,7 +772,7 @@ __device__ __forceinline__ int pw_slot(const PwWork& w, int nr, int s, int* vtx,
 }
 
 constexpr int kWarpSortMin = 32;     // runs longer than this are sorted by a whole warp
-constexpr int kBlockSortMin = 1024;  // and, in a block, above this by the block
+constexpr int kBlockSortMin = 512;   // and, in a block, above this by the block
 
 // sorts scr[0..n) -- distinct 64-bit values, key(m) for m < n -- ascending,
 // by the group: a bitonic network over the next power of two (padding sorts
@@ -810,34 +810,46 @@ __device__ bool group_alpha_sort(G& g, int s, int t, const int* alpha, const int
   return true;
 }
 
-// The items i < n: small(i) by one thread each; those with a length (len(i))
-// above kWarpSortMin by large(group, i): a warp each, or in a block the whole
-// block above kBlockSortMin.  list: room for the long items of a block.
+// The items i < n of length m = len(i): small(i, m) by one thread each; those
+// longer than kWarpSortMin by large(group, i, m): a warp each, or in a block
+// the whole block above kBlockSortMin.  list: room for the long items of a
+// block and their lengths (asking len again, every thread for every item, was
+// the longest step of a pair with many long runs).
 template <class G, class Len, class Small, class Large>
 __device__ void group_items(G& g, int n, int* list, Len len, Small small, Large large) {
   if constexpr (!G::kBlock) {
     for (int i0 = 0; i0 < n; i0 += 32) {
       const int i = i0 + g.rank();
       const int m = i < n ? len(i) : 0;
-      if (m > 0 && m <= kWarpSortMin) small(i);
-      for (unsigned b = __ballot_sync(kFullMask, m > kWarpSortMin); b; b &= b - 1)
-        large(g, i0 + __ffs(b) - 1);
+      if (m > 0 && m <= kWarpSortMin) small(i, m);
+      for (unsigned b = __ballot_sync(kFullMask, m > kWarpSortMin); b; b &= b - 1) {
+        const int src = __ffs(b) - 1;
+        large(g, i0 + src, __shfl_sync(kFullMask, m, src));
+      }
     }
   } else {
     if (g.rank() == 0) g.s->count = 0;
     g.sync();
+    bool longest = false;
     for (int i = g.rank(); i < n; i += G::N) {
       const int m = len(i);
-      if (m > kWarpSortMin) list[atomicAdd(&g.s->count, 1)] = i;
-      else if (m > 0) small(i);
+      if (m > kWarpSortMin) {
+        const int k = atomicAdd(&g.s->count, 1);
+        list[2 * k] = i;
+        list[2 * k + 1] = m;
+        longest |= m > kBlockSortMin;
+      } else if (m > 0) {
+        small(i, m);
+      }
     }
     g.sync();
     const int cnt = g.s->count;
-    for (int k = 0; k < cnt; ++k)
-      if (len(list[k]) > kBlockSortMin) large(g, list[k]);
+    if (g.any(longest))
+      for (int k = 0; k < cnt; ++k)
+        if (list[2 * k + 1] > kBlockSortMin) large(g, list[2 * k], list[2 * k + 1]);
     WarpGroup wg;
     for (int k = g.warp(); k < cnt; k += G::kWarps)
-      if (len(list[k]) <= kBlockSortMin) large(wg, list[k]);
+      if (list[2 * k + 1] <= kBlockSortMin) large(wg, list[2 * k], list[2 * k + 1]);
     g.sync();
   }
 }
@@ -1005,7 +1017,7 @@ __device__ int pw_clip_head(G& g, const double* b, int nb, const double* c, int 
         const int m = w.cAll[e + 1] - w.cAll[e];
         return m > 1 ? m : 0;
       },
-      [&](int e) {
+      [&](int e, int) {
         int* v = w.csorted + w.cAll[e];
         const int m = w.cAll[e + 1] - w.cAll[e];
         for (int i = 1; i < m; ++i) {
@@ -1018,7 +1030,7 @@ __device__ int pw_clip_head(G& g, const double* b, int nb, const double* c, int 
           v[j] = x;
         }
       },
-      [&](auto& gg, int e) {
+      [&](auto& gg, int e, int) {
         const int s = w.cAll[e], m = w.cAll[e + 1] - s;
         unsigned long long* scr = w.sscr + 2 * s;  // an edge's own part
         group_sort(gg, m, scr, [&](int k) { return (unsigned long long)w.csorted[s + k]; });
@@ -1086,20 +1098,20 @@ __device__ int pw_clip_head(G& g, const double* b, int nb, const double* c, int 
   bool bad = false;
   group_items(
       g, nr, w.htmp, [&](int r) { return w.re_nd[r] > 1 ? w.re_s[r + 1] - w.re_s[r] : 0; },
-      [&](int r) {
+      [&](int r, int) {
         if (!isort(w.re_s[r], w.re_s[r + 1], w.aB, nullptr, w.sB)) bad = true;
       },
-      [&](auto& gg, int r) {
+      [&](auto& gg, int r, int) {
         const int s = w.re_s[r];
         if (!group_alpha_sort(gg, s, w.re_s[r + 1], w.aB, nullptr, w.sB, w.sscr + 2 * s)) bad = true;
       });
   group_items(
       g, nc, w.htmp,
       [&](int e) { return w.cND[e + 1] - w.cND[e] > 1 ? w.cAll[e + 1] - w.cAll[e] : 0; },
-      [&](int e) {
+      [&](int e, int) {
         if (!isort(w.cAll[e], w.cAll[e + 1], w.aC, w.csorted, w.sC)) bad = true;
       },
-      [&](auto& gg, int e) {
+      [&](auto& gg, int e, int) {
         const int s = w.cAll[e];
         if (!group_alpha_sort(gg, s, w.cAll[e + 1], w.aC, w.csorted, w.sC, w.sscr + 2 * s)) bad = true;
       });

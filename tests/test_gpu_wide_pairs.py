@@ -48,11 +48,17 @@ def test_plain_crossings(mode):
                            (301, -35.0, 95.0), (1200, 25.0, 100.0), (2400, 3.0, 100.0),
                            (700, 0.0, 30.0), (40, 0.0, 1000.0), (50, 900.0, 20.0))]
     ovs.append(ovs[5][::-1].copy())
-    rings, status = cl.clip_pairwise(base, ovs)
-    assert (status == 0).all()
-    for got, o in zip(rings, ovs):
-        assert rings_equal(got, want(base, o, union))
-    assert cl.pairwise_info()["big_pairs"] == 0
+    # with and without the rule that hands a few large pairs to the pipeline
+    few, few_status = cl.clip_pairwise(base, ovs)
+    cl.set_pairwise_split(1 << 30)
+    try:
+        rings, status = cl.clip_pairwise(base, ovs)
+        assert cl.pairwise_info()["big_pairs"] == 0
+    finally:
+        cl.set_pairwise_split(32768)
+    assert (status == 0).all() and (few_status == 0).all()
+    for got, same, o in zip(rings, few, ovs):
+        assert rings_equal(got, want(base, o, union)) and rings_equal(got, same)
 
 
 def test_overlaps_and_touches(mode):
@@ -71,6 +77,65 @@ def test_overlaps_and_touches(mode):
             assert st != 0
             continue
         assert st == 0 and rings_equal(got, ref)
+
+
+@pytest.mark.parametrize("shared", [False, True], ids=["apart", "shared_x"])
+def test_pairwise_general_position_and_not(mode, shared):
+    """Overlays in general position, and not: vertices and edges on the base,
+    a vertex of the base, an x value twice, a crossing within the classifier's
+    epsilon of a vertex, several records on one edge, the whole base in the
+    result (more ring vertices than a pair's first arena), none.  With a base
+    whose x values are apart and one that has two alike.  Rings as the
+    oracle's; areas to 1e-12 of the rings' absolute terms and gradients to
+    1e-11 of their largest entry (FP64 sums in another order)."""
+    import area_grad
+    torch = pytest.importorskip("torch")
+    cl, union = mode
+    base = gen.star(1500, 171, R=100.0)
+    if shared:
+        base[700, 0] = base[3, 0]
+    v, e = base[100], (base[200] + base[201]) / 2
+    out = np.array([170.0, 60.0])
+    ovs = [gen.star(n, 700 + n, centre=(x, 3.0), R=r)
+           for n, x, r in ((3, 1.0, 80.0), (33, 9.0, 60.0), (90, 20.0, 90.0), (400, -9.0, 100.0),
+                           (40, 0.0, 1000.0), (30, 0.0, 5.0), (20, 900.0, 20.0))]
+    ovs += [np.array([v, out, out + [3.0, 60.0]]), np.array([e, out, out + [3.0, 60.0]]),
+            np.array([base[300], base[301], out]), np.array([v + 1e-10, out, out + [3.0, 60.0]]),
+            np.array([[-150.0, -1.3], [150.0, 2.1], [150.0, 9.7], [-140.0, 5.2]]),
+            np.array([[-150.0, -1.3], [150.0, 2.1], [145.0, 9.7], [-140.0, 5.2]]),
+            ovs[2][::-1].copy()]
+    rings, status = cl.clip_pairwise(base, ovs)
+    seen = []
+    for i, (got, o, st) in enumerate(zip(rings, ovs, status)):
+        try:
+            ref = oracle_py.clip(base, [o], union=union)["overlays"][0]
+        except oracle_py.OracleError:
+            assert st != 0
+            continue
+        assert st == 0 and rings_equal(got, oracle_py.rings_of(ref)), i
+        seen.append((i, ref))
+    assert len(seen) >= 10
+    ga = np.zeros(len(ovs))
+    ga[[i for i, _ in seen]] = np.random.default_rng(3).uniform(0.5, 2.0, len(seen))
+    cxy, coff = sbclip.pack_polygons(ovs)
+    tb, tc, to, tg = (torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (base, cxy, coff, ga))
+    ta, ts = torch.zeros_like(tg), torch.zeros(len(ovs), dtype=torch.int32, device="cuda")
+    job = (tb.data_ptr(), len(base), len(ovs), tc.data_ptr(), to.data_ptr())
+    cl.pairwise_area_device(*job, ta.data_ptr(), ts.data_ptr())
+    tgb, tgc = torch.zeros_like(tb), torch.zeros_like(tc)
+    cl.pairwise_area_backward_device(*job, tg.data_ptr(), tgb.data_ptr(), tgc.data_ptr())
+    area, gb, gc = ta.cpu().numpy(), tgb.cpu().numpy(), np.split(tgc.cpu().numpy(), coff[1:-1])
+    sum_b = np.zeros_like(base)
+    for i, ref in seen:
+        rs = oracle_py.rings_of(ref)
+        scale = sum(float(np.abs(r).max() ** 2) * len(r) for r in rs) + 1e-300
+        assert abs(area[i] - area_grad.shoelace(rs)) <= 1e-12 * scale, i
+        _, rb, rc = area_grad.gradient_of_rings(base, ovs[i], rs, ref["uniq_b"], ref["uniq_c"],
+                                                ref["uniq_t"], ref["isect_xy"])
+        top = ga[i] * max(np.abs(rb).max(), np.abs(rc).max(), 1e-300)
+        assert np.abs(gc[i] - ga[i] * rc).max() <= 1e-11 * top, i
+        sum_b += ga[i] * rb
+    assert np.abs(gb - sum_b).max() <= 1e-11 * max(np.abs(sum_b).max(), 1e-300)
 
 
 # ------------------------------------------------------------------ batches
