@@ -625,9 +625,10 @@ __global__ void __launch_bounds__(kTestBlock) k_pw_cand_test(PwCandArgs A) {
       const long long o = A.coff[i];
       const int n = (int)(A.coff[i + 1] - o), j = (int)(cb.x - o), j2 = j + 1 == n ? 0 : j + 1;
       const int be = cb.y, be2 = be + 1 == A.nb ? 0 : be + 1;
-      const double2 p1 = ((const double2*)A.b)[be], p2 = ((const double2*)A.b)[be2];
-      const double2 q1 = ((const double2*)A.cxy)[o + j], q2 = ((const double2*)A.cxy)[o + j2];
-      if (lsmf_d(p1.x, p1.y, p2.x, p2.y, q1.x, q1.y, q2.x, q2.y)) {
+      // (a caller's array need not be aligned to more than a double)
+      const double *p1 = A.b + 2 * be, *p2 = A.b + 2 * be2;
+      const double *q1 = A.cxy + 2 * (o + j), *q2 = A.cxy + 2 * (o + j2);
+      if (lsmf_d(p1[0], p1[1], p2[0], p2[1], q1[0], q1[1], q2[0], q2[1])) {
         ++tested;
         keep = !certainly_disjoint(A.vfB[be], A.vfB[be2], A.vfC[o + j], A.vfC[o + j2]);
         e = make_int4(i, be, j, 0);
@@ -654,9 +655,9 @@ __global__ void __launch_bounds__(kTestBlock) k_pw_cand_test(PwCandArgs A) {
       const long long o = A.coff[e.x];
       const int n = (int)(A.coff[e.x + 1] - o), j2 = e.z + 1 == n ? 0 : e.z + 1;
       const int be2 = e.y + 1 == A.nb ? 0 : e.y + 1;
-      const double2 p1 = ((const double2*)A.b)[e.y], p2 = ((const double2*)A.b)[be2];
-      const double2 q1 = ((const double2*)A.cxy)[o + e.z], q2 = ((const double2*)A.cxy)[o + j2];
-      ty = seg_isect(p1.x, p1.y, p2.x, p2.y, q1.x, q1.y, q2.x, q2.y, &al, &bt);
+      const double *p1 = A.b + 2 * e.y, *p2 = A.b + 2 * be2;
+      const double *q1 = A.cxy + 2 * (o + e.z), *q2 = A.cxy + 2 * (o + j2);
+      ty = seg_isect(p1[0], p1[1], p2[0], p2[1], q1[0], q1[1], q2[0], q2[1], &al, &bt);
     }
     const unsigned long long h = warp_append(ty != 0, A.nraw);
     if (ty != 0 && h < A.rawcap) A.raw[h] = PwHit{e.x, e.y, e.z, ty, 0ull, al, bt};

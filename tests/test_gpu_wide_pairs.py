@@ -270,3 +270,43 @@ def test_components_in_general_position(mode, n, holes, islands):
     for b, c, got in zip(bases, ovs, rings):
         o = oracle_py.clip_components(b, c, union=union)["overlays"][0]
         assert rings_equal(got, oracle_py.rings_of(o))
+
+
+def test_device_arrays_aligned_to_a_double(clipper):
+    """Coordinates that start 8 bytes past a 16-byte boundary: the same areas
+    and gradients, from every engine that takes device arrays (the pairwise
+    gradients to 1e-13 of the largest: atomic sums of a few terms)."""
+    torch = pytest.importorskip("torch")
+
+    def on_device(x, shift):
+        x = torch.from_numpy(np.ascontiguousarray(x, dtype=np.float64)).cuda()
+        t = torch.zeros(x.numel() + 1, dtype=torch.float64, device="cuda")[shift:][:x.numel()]
+        t.copy_(x.reshape(-1))
+        assert t.data_ptr() % 16 == 8 * shift
+        return t
+
+    base = gen.star(700, 81, R=100.0)
+    ovs = [gen.star(n, 800 + n, centre=(x, 3.0), R=80.0) for n, x in ((5, 1.0), (60, 9.0), (600, -20.0))]
+    cxy, coff = sbclip.pack_polygons(ovs)
+    bxy, boff = sbclip.pack_polygons([base] * len(ovs))
+    tco, tbo = torch.from_numpy(coff).cuda(), torch.from_numpy(boff).cuda()
+    got = []
+    for shift in (0, 1):
+        tb, tc, tbb = on_device(base, shift), on_device(cxy, shift), on_device(bxy, shift)
+        tg = torch.ones(len(ovs), dtype=torch.float64, device="cuda")
+        ta, ta2 = torch.zeros_like(tg), torch.zeros_like(tg)
+        ts = torch.zeros(len(ovs), dtype=torch.int32, device="cuda")
+        gb, gc, gb2, gc2 = (on_device(np.zeros(x.numel()), shift) for x in (tb, tc, tbb, tc))
+        job = (tb.data_ptr(), len(base), len(ovs), tc.data_ptr(), tco.data_ptr())
+        clipper.pairwise_area_device(*job, ta.data_ptr(), ts.data_ptr())
+        clipper.pairwise_area_backward_device(*job, tg.data_ptr(), gb.data_ptr(), gc.data_ptr())
+        job = (len(ovs), tbb.data_ptr(), tbo.data_ptr(), tc.data_ptr(), tco.data_ptr())
+        clipper.area_forward_device(*job, ta2.data_ptr(), ts.data_ptr())
+        clipper.area_backward_device(*job, tg.data_ptr(), gb2.data_ptr(), gc2.data_ptr())
+        counts = clipper.clip_pair_device(tb.data_ptr(), len(base), tc.data_ptr(), len(ovs[0]))
+        got.append([x.cpu().numpy() for x in (ta, ta2, gb, gc, gb2, gc2)] + [np.array(counts[:2])])
+    for i, (x, y) in enumerate(zip(*got)):
+        if i in (2, 3):
+            assert np.abs(x - y).max() <= 1e-13 * np.abs(x).max()
+        else:
+            assert np.array_equal(x, y), i
