@@ -26,6 +26,7 @@
 #include "../../include/sbclip.h"
 #include "sbc_pipeline.cuh"
 #include "sbc_clean.cuh"
+#include "sbc_disjoint.cuh"
 #include "sbc_pairops.cuh"
 #include "sbc_pwpair.cuh"
 #include "sbc_serial.cuh"
@@ -88,6 +89,7 @@ struct PairWork {
   double *es, *ee;
   long long *kes, *kee;
   float4* fbox;
+  float4* vf;  // vertices as float pairs (over kes and kee, once those are done with)
   // elementary intervals
   int *sidx, *stmp, *vl, *vloc;
   double* ea;
@@ -168,6 +170,7 @@ __host__ __device__ __forceinline__ PairWork carve(Carver& cv, const Caps& c) {
   w.ee = cv.take<double>(E);
   w.kes = cv.take<long long>(E);
   w.kee = cv.take<long long>(E);
+  w.vf = (float4*)w.kes;
   w.fbox = cv.take<float4>(E);
   w.sidx = cv.take<int>(n2);
   w.stmp = cv.take<int>(n2);
@@ -339,6 +342,172 @@ struct FrontRange {
   }
 };
 
+// the least and greatest keys of a group's threads, on all of them
+template <class G>
+__device__ void range_join(G& g, FrontRange& fr, FrontRange* s_range) {
+  for (int o = 16; o > 0; o >>= 1)
+    fr.join(__shfl_xor_sync(kFullMask, fr.kmin, o), __shfl_xor_sync(kFullMask, fr.kmax, o),
+            __shfl_xor_sync(kFullMask, fr.imin, o), __shfl_xor_sync(kFullMask, fr.imax, o));
+  if constexpr (G::kBlock) {
+    if ((threadIdx.x & 31) == 0) s_range[g.warp()] = fr;
+    g.sync();
+    for (int k = 0; k < G::kWarps; ++k)
+      fr.join(s_range[k].kmin, s_range[k].kmax, s_range[k].imin, s_range[k].imax);
+  }
+}
+
+// decimal scale of realToInt's keys (oacc_segment_tree.cpp:203-206) for a
+// largest shifted value dv
+__device__ __forceinline__ double border_scale(double dv) {
+  int digits = 1;
+  for (int iv = (int)trunc(dv); iv / 10 > 0; iv /= 10) ++digits;
+  double scale = 1.0;
+  for (int t = 0; t < 11 - digits; ++t) scale = dmul(scale, 10.0);
+  return scale;
+}
+
+// Rows A1-A7 where no two vertices share an x value, from the vertices' ranks
+// by x (as the pair pipeline's stage_ranks): the elementary array is the
+// values in order without the largest, padded with the second largest, so an
+// edge's end leaves and leaf range follow from the ranks of its two vertices.
+// Sorts E vertices instead of 2 E endpoints, and replaces the array, its
+// border keys and the searches (12,000 pairs of 3 to 2,048 vertices, forward
+// and backward: 8.1 ms of blocks, 2.6 so; 512 pairs of 4 to 64 on warps: 46 us
+// and 25).  A warp counts each vertex's lesser ones, a block sorts
+// (np = npow2_dev(E) entries of key and val).  False: something was shared,
+// has a zero border key or is out of range; nothing but fbox is written.
+template <class G>
+__device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, int nc,
+                                PairWork& w, long long* key, int* val, int* rank,
+                                FrontRange* s_range) {
+  const int lane = g.rank();
+  constexpr int N = G::N;
+  const int E = nb + nc, last = E - 2;
+  // (a caller's array need not be aligned to more than a double)
+  auto vertex = [&](int v) { return v < nb ? b + 2 * v : c + 2 * (v - nb); };
+  auto vx = [&](int v) { return vertex(v)[0]; };
+  auto succ = [&](int e) {
+    return e < nb ? vsucc(w.bnx, nb, e) : nb + vsucc(w.cnx, nc, e - nb);
+  };
+  FrontRange fr{LLONG_MAX, LLONG_MIN, INT_MAX, INT_MAX};
+  for (int e = lane; e < E; e += N) {
+    const int t = succ(e);
+    const double *pv = vertex(e), *qv = vertex(t);
+    const double2 p = make_double2(pv[0], pv[1]), q = make_double2(qv[0], qv[1]);
+    const long long k = okey(p.x);
+    key[e] = k;
+    fr.join(k, k, e, e);
+    const bool xs = k < okey(q.x), ys = okey(p.y) < okey(q.y);
+    w.fbox[e] = make_float4(__double2float_rd(xs ? p.x : q.x), __double2float_rd(ys ? p.y : q.y),
+                            __double2float_ru(xs ? q.x : p.x), __double2float_ru(ys ? q.y : p.y));
+  }
+  range_join(g, fr, s_range);
+  const double lo = vx(fr.imin), absMin = fabs(lo), dv = dadd(vx(fr.imax), absMin);
+  if (!(dv < 2147483647.0)) return false;
+  const double scale = border_scale(dv);
+  bool bad = false;
+  // vertex v has rank r: the second value's border key is not zero, and the
+  // last one's is in the reference's range
+  auto place = [&](int v, int r) {
+    rank[v] = r;
+    if (r != 1 && r != last) return;
+    const double x = vx(v);
+    const long long k = (long long)(lo < 0 ? dmul(scale, dadd(x, absMin)) : dmul(scale, x));
+    if (k <= 0 || k >= 100000000000LL) bad = true;
+  };
+  if constexpr (!G::kBlock) {
+    g.sync();
+    constexpr int kPer = 4;  // vertices per lane and sweep over the keys
+    for (int v0 = lane; v0 - lane < E; v0 += kPer * N) {
+      long long k[kPer];
+      int r[kPer], same[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        k[i] = v0 + i * N < E ? key[v0 + i * N] : LLONG_MAX;
+        r[i] = same[i] = 0;
+      }
+      for (int u = 0; u < E; ++u) {
+        const long long x = key[u];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          r[i] += x < k[i];
+          same[i] += x == k[i];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kPer; ++i)
+        if (v0 + i * N < E) {
+          place(v0 + i * N, r[i]);
+          if (same[i] != 1) bad = true;
+        }
+    }
+  } else {
+    const int np = npow2_dev(E);
+    for (int i = lane; i < np; i += N) {
+      if (i >= E) key[i] = LLONG_MAX;
+      val[i] = i;
+    }
+    g.sync();
+    group_bitonic(g, np, [&](int m, int l, bool up) {
+      const long long x = key[m], y = key[l];
+      if ((x > y) == up && x != y) {
+        key[m] = y;
+        key[l] = x;
+        const int t = val[m];
+        val[m] = val[l];
+        val[l] = t;
+      }
+    });
+    for (int i = lane; i < E; i += N) {
+      if (val[i] < E) place(val[i], i);
+      if (val[i] >= E || (i > 0 && key[i] == key[i - 1])) bad = true;
+    }
+  }
+  if (g.any(bad)) return false;
+  const int epc = npow2_dev(E - 1) + 1, L = epc - 1;
+  int logL = 0;
+  while ((1 << logL) < L) ++logL;
+  // a rank's positions [x, y) in the padded array; findBoarder's search meets
+  // the never-written slot 0 only on its way to the first two positions
+  auto range = [&](int r) {
+    return r > last ? make_int2(epc, epc) : make_int2(r, r == last ? epc : r + 1);
+  };
+  auto border = [&](int2 at, int v) {
+    if (at.x >= 2 && at.y == at.x + 1) return at.x;
+    return border_by_position(epc, 0, at.x, at.y, vx(v));
+  };
+  for (int e = lane; e < E; e += N) {
+    const int t = succ(e), r0 = rank[e], r1 = rank[t];
+    const int2 S = range(min(r0, r1)), T = range(max(r0, r1));
+    int a = -1, z = -1;
+    const int en = border(T, r0 < r1 ? t : e), st = border(S, r0 < r1 ? e : t);
+    if (en >= 0) {
+      const int j = en == 0 ? epc - 1 : en - 1;  // right[j]
+      int node = 0;
+      if (j <= epc - 2) {
+        const int i = j + 1;
+        node = L + i;
+        if (i != 1 && i + 1 < epc && i >= last) node = L + i + 1;
+      }
+      if (node >= L && node < 2 * L && node - L < last) a = node;
+    }
+    if (st >= 0) {
+      const int j = st == 0 ? epc - 1 : st - 1;  // left[j]
+      const int node = j <= epc - 2 ? L + j : 0;
+      if (node >= L && node < 2 * L && node - L < last) z = node;
+    }
+    w.aft[e] = a;
+    w.bef[e] = z;
+    const int l = min(S.x, L), r = max(0, min(T.y - 1, L));
+    w.lr[e] = make_int2(l, max(l, r));
+  }
+  if (lane == 0) {
+    w.state[1] = logL;
+    w.state[2] = w.state[3] = w.state[4] = 0;
+  }
+  return true;
+}
+
 template <class G>
 __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, int nc,
                                const Caps& cp, PairWork& w, long long* skey, int* sval, int n_sort,
@@ -380,15 +549,7 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
     w.fbox[e] = make_float4(__double2float_rd(xs ? a0 : a1), __double2float_rd(ys ? y0 : y1),
                             __double2float_ru(xs ? a1 : a0), __double2float_ru(ys ? y1 : y0));
   }
-  for (int o = 16; o > 0; o >>= 1)
-    fr.join(__shfl_xor_sync(kFullMask, fr.kmin, o), __shfl_xor_sync(kFullMask, fr.kmax, o),
-            __shfl_xor_sync(kFullMask, fr.imin, o), __shfl_xor_sync(kFullMask, fr.imax, o));
-  if constexpr (G::kBlock) {
-    if ((threadIdx.x & 31) == 0) s_range[g.warp()] = fr;
-    g.sync();
-    for (int k = 0; k < G::kWarps; ++k)
-      fr.join(s_range[k].kmin, s_range[k].kmax, s_range[k].imin, s_range[k].imax);
-  }
+  range_join(g, fr, s_range);
   // the vertex values behind the extreme keys (edge e's first vertex)
   auto vx0 = [&](int e) { return e < nb ? bvx(b, nb, e) : bvx(c, nc, e - nb); };
   const double minI = vx0(fr.imin), maxI = vx0(fr.imax);
@@ -489,10 +650,7 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
   const double absMin = fabs(minI);
   const double dv = dadd(maxI, absMin);
   if (!(dv < 2147483647.0)) return PS_UNDEF;
-  int digits = 1;
-  for (int iv = (int)trunc(dv); iv / 10 > 0; iv /= 10) ++digits;
-  double scale = 1.0;
-  for (int t = 0; t < 11 - digits; ++t) scale = dmul(scale, 10.0);
+  const double scale = border_scale(dv);
   const bool shift = minI < 0;
   g.sync();
   int zl = 0;
@@ -551,11 +709,21 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
     }
     w.lr[e] = make_int2(l, lo > l ? lo : l);
   }
-  g.sync();
   if (lane == 0) {
     w.state[1] = logL;
     w.state[2] = w.state[3] = 0;
     w.state[4] = shared_x;
+  }
+  return PS_OK;
+}
+
+// what the candidate kernels read beside the boxes
+template <class G>
+__device__ void front_floats(G& g, const double* b, int nb, const double* c, int nc, PairWork& w) {
+  g.sync();
+  for (int v = g.rank(); v < nb + nc; v += G::N) {
+    const double* p = v < nb ? b + 2 * v : c + 2 * (v - nb);
+    w.vf[v] = float_pair(p[0], p[1]);
   }
   if constexpr (G::kBlock) {
     // the box of each group of overlay edges, a lane per edge
@@ -572,15 +740,15 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
       if ((threadIdx.x & 31) == 0) w.gbox[q] = x;
     }
   }
-  g.sync();
-  return PS_OK;
 }
 
-// A8 for one pair: the edge pairs whose float boxes meet and that pass LSMF
-// are queued per warp (kCandQ entries of shared memory) and classified 32 at
-// a time, so that lineSegmentIntersection's FP64 work runs in full warps: only
-// a few pairs in a hundred pass the filters, and FP64 run by a few lanes costs
-// the issue slots of all 32.
+// A8 for one pair: the edge pairs whose float boxes meet and that the float
+// test does not rule out are queued per warp (kCandQ entries of shared memory)
+// and classified 32 at a time, LSMF and lineSegmentIntersection, so that their
+// FP64 work runs in full warps: only a few pairs in a hundred pass the filters,
+// and FP64 run by a few lanes costs the issue slots of all 32.  With LSMF as
+// the second filter in place of the float test the 12,000 pairs above took 9.3
+// ms of blocks here, 5.4 so.
 constexpr int kCandQ = 64;
 
 __device__ __forceinline__ bool boxes_meet(const float4& fb, const float4& fc) {
@@ -602,6 +770,10 @@ struct CandQueue {
 
   __device__ int bsucc(int i) const { return vsucc(kComp ? w.bnx : nullptr, nb, i); }
   __device__ int csucc(int i) const { return vsucc(kComp ? w.cnx : nullptr, nc, i); }
+  // false where the two edges certainly do not meet
+  __device__ bool may_meet(const float4& b0, const float4& b1, int j) const {
+    return !certainly_disjoint(b0, b1, w.vf[nb + j], w.vf[nb + csucc(j)]);
+  }
   __device__ bool lsmf(int be, int j) const {
     const int bt2 = bsucc(be), ct2 = csucc(j);
     return lsmf_d(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
@@ -617,8 +789,9 @@ struct CandQueue {
       be = e.x;
       j = e.y;
       const int bt2 = bsucc(be), ct2 = csucc(j);
-      ty = seg_isect(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
-                     bvx(c, nc, j), bvy(c, nc, j), bvx(c, nc, ct2), bvy(c, nc, ct2), &al, &bt);
+      if (lsmf(be, j))
+        ty = seg_isect(bvx(b, nb, be), bvy(b, nb, be), bvx(b, nb, bt2), bvy(b, nb, bt2),
+                       bvx(c, nc, j), bvy(c, nc, j), bvx(c, nc, ct2), bvy(c, nc, ct2), &al, &bt);
       hit = ty && emission_s(be, nb + j, 2 * j, w, w.state[1], &key) > 0;
     }
     // one counter step per warp; out of room: only counted, for the retry's
@@ -668,7 +841,8 @@ __device__ void clip_pair_cand(CandQueue<kComp>& cq) {
     ++be;
   }
   while (__any_sync(kFullMask, be < nb)) {
-    const bool pass = be < nb && boxes_meet(w.fbox[be], w.fbox[nb + j]) && cq.lsmf(be, j);
+    const bool pass = be < nb && boxes_meet(w.fbox[be], w.fbox[nb + j]) &&
+                      cq.may_meet(w.vf[be], w.vf[cq.bsucc(be)], j);
     cq.add(pass, be, j);
     j += 32;
     while (j >= nc && be < nb) {
@@ -692,6 +866,7 @@ __device__ void clip_pair_cand_group(CandQueue<kComp>& cq, int be0, float4* box)
   const int be = be0 + lane;
   const float inf = __int_as_float(0x7f800000);
   const float4 fb = be < nb ? w.fbox[be] : make_float4(inf, inf, -inf, -inf);
+  const float4 v0 = w.vf[min(be, nb - 1)], v1 = w.vf[cq.bsucc(min(be, nb - 1))];
   float4 all = fb;
   for (int o = 16; o > 0; o >>= 1) {
     all.x = fminf(all.x, __shfl_xor_sync(kFullMask, all.x, o));
@@ -707,7 +882,7 @@ __device__ void clip_pair_cand_group(CandQueue<kComp>& cq, int be0, float4* box)
       if (lane < n) box[lane] = w.fbox[nb + j0 + lane];
       __syncwarp();
       for (int t = 0; t < n; ++t) {
-        const bool pass = boxes_meet(fb, box[t]) && cq.lsmf(be, j0 + t);
+        const bool pass = boxes_meet(fb, box[t]) && cq.may_meet(v0, v1, j0 + t);
         cq.add(pass, be, j0 + t);
       }
     }
@@ -1219,6 +1394,8 @@ __device__ __forceinline__ void front_done(const ClipArgs& A, int p, PairWork& w
 }
 
 __global__ void __launch_bounds__(128) k_batch_front(ClipArgs A) {
+  __shared__ long long s_key[4][kWideEdges];
+  __shared__ int s_rank[4][kWideEdges];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   if ((t >> 5) >= A.np) return;
@@ -1238,13 +1415,17 @@ __global__ void __launch_bounds__(128) k_batch_front(ClipArgs A) {
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   WarpGroup g;
-  const int st = clip_pair_front(g, A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp, w,
-                                 nullptr, nullptr, 0, nullptr);
+  const double *b = A.bxy + 2 * A.boff[p], *c = A.cxy + 2 * A.coff[p];
+  int st = PS_OK;
+  if (!clip_pair_ranks(g, b, nb, c, nc, w, s_key[threadIdx.x >> 5], nullptr,
+                       s_rank[threadIdx.x >> 5], nullptr))
+    st = clip_pair_front(g, b, nb, c, nc, cp, w, nullptr, nullptr, 0, nullptr);
+  front_floats(g, b, nb, c, nc, w);
   if (lane == 0) front_done(A, p, w, st);
 }
 
-// the front of the wide pairs, a block each; pairs of up to 1,024 edges (the
-// endpoints padded to a power of two) sort in shared memory
+// the front of the wide pairs, a block each; pairs of up to 2,048 vertices (or
+// endpoints) sort in shared memory
 constexpr int kFrontSort = 2048;
 __global__ void __launch_bounds__(kWideBlock) k_batch_front_wide(ClipArgs A) {
   using G = BlockGroup<kWideBlock>;
@@ -1259,8 +1440,13 @@ __global__ void __launch_bounds__(kWideBlock) k_batch_front_wide(ClipArgs A) {
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
   G g(&sh);
-  const int st = clip_pair_front(g, A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp, w,
-                                 s_key, s_val, kFrontSort, s_range);
+  const double *b = A.bxy + 2 * A.boff[p], *c = A.cxy + 2 * A.coff[p];
+  const bool fits = npow2_dev(nb + nc) <= kFrontSort;
+  int st = PS_OK;
+  if (!clip_pair_ranks(g, b, nb, c, nc, w, fits ? s_key : w.fkey, fits ? s_val : w.fval, w.vl,
+                       s_range))
+    st = clip_pair_front(g, b, nb, c, nc, cp, w, s_key, s_val, kFrontSort, s_range);
+  front_floats(g, b, nb, c, nc, w);
   if (threadIdx.x == 0) front_done(A, p, w, st);
 }
 
