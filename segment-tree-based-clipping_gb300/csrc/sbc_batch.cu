@@ -1713,7 +1713,7 @@ __device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, in
     const CleanMem m = clean_carve(cv, nb, nc, K);
     const CleanIn<SoaHits> in{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.bnx, w.cnx, K,
                               SoaHits{w.hb, w.hc, w.ht, w.hkey, w.hal, w.hbt}, 0, A.unite, cp.rcap,
-                              cp.capR, w.rootB, w.rootC, w.vl, w.vloc, w.roff, w.rxy,
+                              cp.capR, w.rootB, w.rootC, w.vl, w.vloc, w.R.next, w.R.prev, w.roff, w.rxy,
                               sort, sort_room, w.tape};
     done = clean_clip(g, in, m, s_sum, &nr, &nv, &area) == CLEAN_DONE;
   }

@@ -1,7 +1,6 @@
 // sbc_clean.cuh -- rows A9-A18 of one pair in general position: every hit a
-// proper crossing inside both edges, labelled a crossing, and no ring vertex
-// in line with its neighbours.  That is nearly every pair of real-valued
-// polygons, with any number of components.
+// proper crossing inside both edges, labelled a crossing.  That is nearly
+// every pair of real-valued polygons, with any number of components.
 //
 // In general position the reference's linked lists (copyToLinkedList,
 // src/clip.cpp:606-695; labelIntersections2 and createResult2,
@@ -81,6 +80,7 @@ struct CleanIn {
   int rcap, vcap;      // room for rings and their vertices
   int *rootB, *rootC;  // scratch: first vertices of the components (n + 1)
   int *inB, *inC;      // scratch: per component, first vertex inside the other polygon
+  int *nxt, *prv;      // scratch: vcap each
   int* roff;           // out: rings, their vertices, and where each vertex comes from
   double* rxy;
   unsigned long long* sort;  // shared memory: room for sort_room keys per warp
@@ -567,19 +567,116 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     }
   }
   g.sync();
-  // ---- clean-up removes nothing (cleanUpResult2, foster/polyclip.h:767-787,
-  // a vertex with |area3| < eps goes), and the area: the shoelace terms in an
-  // order that the rings and the group size fix
+  // ---- cleanUpResult2 (foster/polyclip.h:767-787): a vertex with |area3| <
+  // eps goes.  And the area: the shoelace terms in an order that the rings and
+  // the group size fix.
+  auto area_at = [&](int u, int v, int x) {
+    return fabs(area3(in.rxy[2 * u], in.rxy[2 * u + 1], in.rxy[2 * v], in.rxy[2 * v + 1],
+                      in.rxy[2 * x], in.rxy[2 * x + 1]));
+  };
+  auto term = [&](int v, int vp) {
+    return dsub(dmul(in.rxy[2 * v], in.rxy[2 * vp + 1]), dmul(in.rxy[2 * vp], in.rxy[2 * v + 1]));
+  };
   double s2 = 0.0;
+  bool flat = false;
   for (int v = lane; v < verts; v += N) {
     const int r = in.tape[v].w, s = in.roff[r], e = in.roff[r + 1];
-    const int vp = v + 1 == e ? s : v + 1, vm = v == s ? e - 1 : v - 1;
-    const double x = in.rxy[2 * v], y = in.rxy[2 * v + 1];
-    const double xp = in.rxy[2 * vp], yp = in.rxy[2 * vp + 1];
-    if (fabs(area3(in.rxy[2 * vm], in.rxy[2 * vm + 1], x, y, xp, yp)) < kEps) bad = true;
-    s2 = dadd(s2, dsub(dmul(x, yp), dmul(xp, y)));
+    const int vp = v + 1 == e ? s : v + 1;
+    if (area_at(v == s ? e - 1 : v - 1, v, vp) < kEps) {
+      flat = true;
+      in.tape[v].w = ~r;
+    }
+    s2 = dadd(s2, term(v, vp));
   }
-  if (g.any(bad)) return CLEAN_NOT;
+  if (g.any(flat)) {  // (rare: one pair in thousands of random ones)
+    // The reference's walk, a thread per ring, over links that start as the
+    // ring's order; a vertex with its first neighbours that was not flat then
+    // is passed over.  tape[].w < 0 ends as "removed".
+    for (int v = lane; v < verts; v += N) {
+      const int w = in.tape[v].w, r = w < 0 ? ~w : w, s = in.roff[r], e = in.roff[r + 1];
+      in.nxt[v] = v + 1 == e ? s : v + 1;
+      in.prv[v] = v == s ? e - 1 : v - 1;
+    }
+    g.sync();
+    for (int r = lane; r < rings; r += N) {
+      const int s = in.roff[r], e = in.roff[r + 1];
+      int root = s;
+      auto is_flat = [&](int v) { return area_at(in.prv[v], v, in.nxt[v]) < kEps; };
+      auto remove = [&](int v) {
+        if (root == v) {
+          root = in.nxt[v];
+          if (in.nxt[root] == root) root = -1;
+        }
+        in.nxt[in.prv[v]] = in.nxt[v];
+        in.prv[in.nxt[v]] = in.prv[v];
+        in.tape[v].w = ~r;
+      };
+      while (root >= 0 && is_flat(root)) remove(root);
+      if (root < 0) {
+        for (int v = s; v < e; ++v) in.tape[v].w = ~r;
+      } else {
+        for (int v = root; v < e; ++v) {
+          if (in.tape[v].w >= 0 && in.prv[v] == v - 1 && in.nxt[v] == v + 1) continue;
+          if (is_flat(v)) remove(v);
+          else in.tape[v].w = r;
+        }
+      }
+      in.nxt[s] = root;  // (the ring's links are done with)
+    }
+    g.sync();
+    // the rings left get new numbers; each vertex: its ring's, and whether it
+    // is the first
+    int left = 0;
+    for (int r0 = 0; r0 < rings; r0 += N) {
+      const int r = r0 + lane;
+      const bool keep = r < rings && in.nxt[in.roff[r]] >= 0;
+      int n;
+      const int id = left + g.before(keep, &n);
+      if (r < rings) in.prv[in.roff[r]] = id;
+      left += n;
+    }
+    g.sync();
+    for (int v = lane; v < verts; v += N) {
+      const int r = in.tape[v].w;
+      if (r < 0) continue;
+      const int s = in.roff[r];
+      in.tape[v].w = 2 * in.prv[s] + (in.nxt[s] == v);
+    }
+    g.sync();
+    int kept = 0;
+    for (int v0 = 0; v0 < verts; v0 += N) {  // to lower places, chunk by chunk
+      const int v = v0 + lane;
+      int4 t = make_int4(0, 0, 0, -1);
+      double x = 0.0, y = 0.0;
+      if (v < verts) {
+        t = in.tape[v];
+        x = in.rxy[2 * v];
+        y = in.rxy[2 * v + 1];
+      }
+      g.sync();
+      const bool first = t.w & 1;
+      int n;
+      const int to = kept + g.before(t.w >= 0, &n);
+      kept += n;
+      if (t.w >= 0) {
+        t.w >>= 1;
+        in.tape[to] = t;
+        in.rxy[2 * to] = x;
+        in.rxy[2 * to + 1] = y;
+        if (first) in.roff[t.w] = to;
+      }
+      g.sync();
+    }
+    verts = kept;
+    rings = left;
+    if (lane == 0) in.roff[rings] = verts;
+    g.sync();
+    s2 = 0.0;
+    for (int v = lane; v < verts; v += N) {
+      const int r = in.tape[v].w, e = in.roff[r + 1];
+      s2 = dadd(s2, term(v, v + 1 == e ? in.roff[r] : v + 1));
+    }
+  }
   for (int o = 16; o > 0; o >>= 1) s2 = dadd(s2, __shfl_xor_sync(0xffffffffu, s2, o));
   if constexpr (G::kBlock) {
     if ((lane & 31) == 0) s_sum[g.warp()] = s2;

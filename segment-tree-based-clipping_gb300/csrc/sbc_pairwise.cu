@@ -983,8 +983,8 @@ __device__ void pw_clean_pair(G& g, const PwPairArgs& A, const int* pairK, int w
   const CleanMem m = clean_carve(mv, 0, nc, K);
   const CleanIn<PwHits> in{A.b, A.nb, A.cxy + 2 * o, nc, nullptr, nullptr, K,
                            PwHits{A.hits + A.hstart[p]}, A.steps[p], A.unite, cp.rcap, cp.capR,
-                           nullptr, nullptr, nullptr, nullptr, w.roff, w.rxy, sort, sort_room,
-                           pw_tape(w)};
+                           nullptr, nullptr, nullptr, nullptr, w.R.next, w.R.prev, w.roff, w.rxy,
+                           sort, sort_room, pw_tape(w)};
   int nr = 0, nv = 0;
   double area = 0.0;
   const int r = clean_clip(g, in, m, s_sum, &nr, &nv, &area);

@@ -272,6 +272,71 @@ def test_components_in_general_position(mode, n, holes, islands):
         assert rings_equal(got, oracle_py.rings_of(o))
 
 
+def with_points(poly, edges, where):
+    """poly with a point on each listed edge, `where` of the way (in line up to
+    rounding)."""
+    out = []
+    for i, v in enumerate(poly):
+        out.append(v)
+        if i in edges:
+            w = poly[(i + 1) % len(poly)]
+            out += [v + t * (w - v) for t in where]
+    return np.array(out)
+
+
+@pytest.mark.parametrize("n", [12, 45, 300, 700])
+def test_ring_vertices_in_line(mode, n):
+    """Vertices in line with their neighbours, which the reference removes: one
+    on an edge, on many, two and three in a row, the ring's first vertex, on
+    edges with crossings, whole rings; on warps and on blocks, one component and several,
+    one base against many overlays.  Rings as the oracle's."""
+    cl, union = mode
+    b = gen.star(n, 210 + n, R=50.0)
+    cases = []
+    for k, (edges, where) in enumerate((((1,), (0.4,)), (range(0, n, 3), (0.37,)), ((2, 7), (0.3, 0.8)),
+                                        ((0, n - 1), (0.55,)), (range(n), (0.5,)),
+                                        ((4, 5), (0.2, 0.5, 0.9)))):
+        c = gen.star(n - k, 300 + n + k, centre=(4.1 + k, -2.3), R=45.0)
+        cases.append((with_points(b, edges, where), c))
+        cases.append((np.roll(with_points(b, edges, where), 2, axis=0), with_points(c, edges, where)))
+    for k, deep in enumerate((1e-6, 4e-6, 3e-5)):  # a corner just across an edge: a sliver of a ring
+        v, w = b[3 + k], b[4 + k]
+        t = (w - v) / np.hypot(*(w - v))
+        inward = np.array([-t[1], t[0]])
+        tip = (v + w) / 2 + deep * inward
+        cases.append((b, np.array([tip, tip - inward * 30.0 + 0.1 * t, tip - inward * 29.0 - 0.2 * t])))
+        cases.append((b, np.array([tip - inward * 29.0 - 0.2 * t, tip + deep * t, tip - deep * t,
+                                   tip - inward * 30.0 + 0.1 * t])))
+
+    def expected(x, c, st):
+        try:
+            return want(x, c, union)
+        except oracle_py.OracleError:
+            assert st != 0
+            return None
+
+    rings, status = cl.clip_batch([x for x, _ in cases], [x for _, x in cases])
+    for (x, c), got, st in zip(cases, rings, status):
+        ref = expected(x, c, st)
+        assert ref is None or (st == 0 and rings_equal(got, ref))
+    for x in (cases[0][0], cases[3][1], cases[4][0]):
+        ovs = [c for _, c in cases]
+        rings, status = cl.clip_pairwise(x, ovs)
+        for c, got, st in zip(ovs, rings, status):
+            ref = expected(x, c, st)
+            assert ref is None or (st == 0 and rings_equal(got, ref))
+        comps = [[x, x * 0.5 + [300.3, 0.7]]] * 3
+        others = [[ovs[0]], [ovs[3], ovs[0] + [299.1, 1.3]], [ovs[5]]]
+        rings, status = cl.clip_batch_components(comps, others)
+        for c, got, st in zip(others, rings, status):
+            try:
+                o = oracle_py.clip_components(comps[0], c, union=union)["overlays"][0]
+            except oracle_py.OracleError:
+                assert st != 0
+                continue
+            assert st == 0 and rings_equal(got, oracle_py.rings_of(o))
+
+
 def test_device_arrays_aligned_to_a_double(clipper):
     """Coordinates that start 8 bytes past a 16-byte boundary: the same areas
     and gradients, from every engine that takes device arrays (the pairwise
