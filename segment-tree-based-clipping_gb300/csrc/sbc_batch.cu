@@ -1470,12 +1470,13 @@ __global__ void __launch_bounds__(128) k_batch_cand(ClipArgs A) {
 }
 
 // the wide pairs, a warp per group of base edges
+constexpr int kCandWarps = 4, kCandBlocks = 5;
 template <bool kComp>
-__global__ void __launch_bounds__(128) k_batch_cand_wide(ClipArgs A) {
-  __shared__ int2 s_q[4][kCandQ];
-  __shared__ float4 s_box[4][kEdgeGroup];
+__global__ void __launch_bounds__(32 * kCandWarps, kCandBlocks) k_batch_cand_wide(ClipArgs A) {
+  __shared__ int2 s_q[kCandWarps][kCandQ];
+  __shared__ float4 s_box[kCandWarps][kEdgeGroup];
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-  const int item = blockIdx.x * 4 + wi;
+  const int item = blockIdx.x * kCandWarps + wi;
   if (item >= A.nitems) return;
   int lo = 0, hi = A.nwide - 1;  // the pair holding the item
   while (lo < hi) {
@@ -1741,8 +1742,8 @@ __global__ void __launch_bounds__(128) k_batch_clean(ClipArgs A) {
 __global__ void __launch_bounds__(kWideBlock, 3) k_batch_clean_wide(ClipArgs A) {
   using G = BlockGroup<kWideBlock>;
   __shared__ G::Shared sh;
-  __shared__ unsigned long long s_sort[G::kWarps * kSortRoom];
   __shared__ double s_sum[G::kWarps];
+  __shared__ unsigned long long s_sort[G::kWarps * kSortRoom];
   const int p = A.wide[blockIdx.x];
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
@@ -2022,8 +2023,8 @@ void launch_clip(const ClipArgs& A, const BatchShape& sh, double in_bytes, cudaS
   }
   if (A.nwide > 0) {
     ::sbc::KProbe kp_("k_batch_cand_wide", st);
-    if (comps) k_batch_cand_wide<true><<<grid_for(A.nitems, 4), 128, 0, st>>>(A);
-    else k_batch_cand_wide<false><<<grid_for(A.nitems, 4), 128, 0, st>>>(A);
+    if (comps) k_batch_cand_wide<true><<<grid_for(A.nitems, kCandWarps), 32 * kCandWarps, 0, st>>>(A);
+    else k_batch_cand_wide<false><<<grid_for(A.nitems, kCandWarps), 32 * kCandWarps, 0, st>>>(A);
   }
   {
     ::sbc::KProbe kp_("k_batch_clean", st, in_bytes + 20.0 * A.np);
@@ -2120,38 +2121,42 @@ __global__ void k_batch_pack(int np, const long long* __restrict__ boff,
 // edges b1b2 and c1c2: I = (1 - alpha) b1 + alpha b2, alpha = A1 / (A1 - A2),
 // A1 = A(b1, c1, c2), A2 = A(b2, c1, c2); A(P, Q, R) partials: dP = (Qy - Ry,
 // Rx - Qx), dQ = (Ry - Py, Px - Rx), dR = (Py - Qy, Qx - Px)
+// One reciprocal and explicit fused multiply-adds: the FP64 rate bounds the
+// backward pass, and three divisions without fma took about twice as many
+// operations.
 struct CrossGrad {
-  double gx, gy, b1x, b1y, b2x, b2y, c1x, c1y, c2x, c2y, al, k1, k2;
+  double gx, gy, al, k1, k2;
+  double2 b1c1, b1c2, b2c1, b2c2, c12;  // c1 - b1, c2 - b1, c1 - b2, c2 - b2, c1 - c2
   __device__ __forceinline__ CrossGrad(const double* b, int i1, int i2, const double* c, int j1,
                                        int j2, double gx_, double gy_)
       : gx(gx_), gy(gy_) {
-    b1x = b[2 * i1];
-    b1y = b[2 * i1 + 1];
-    b2x = b[2 * i2];
-    b2y = b[2 * i2 + 1];
-    c1x = c[2 * j1];
-    c1y = c[2 * j1 + 1];
-    c2x = c[2 * j2];
-    c2y = c[2 * j2 + 1];
-    const double A1 = (c1x - b1x) * (c2y - b1y) - (c1y - b1y) * (c2x - b1x);
-    const double A2 = (c1x - b2x) * (c2y - b2y) - (c1y - b2y) * (c2x - b2x);
-    const double d = A1 - A2;
-    al = A1 / d;
-    const double ga = gx * (b2x - b1x) + gy * (b2y - b1y);  // dA/dalpha
-    k1 = -A2 / (d * d) * ga;  // dalpha/dA1
-    k2 = A1 / (d * d) * ga;   // dalpha/dA2
+    const double b1x = b[2 * i1], b1y = b[2 * i1 + 1], b2x = b[2 * i2], b2y = b[2 * i2 + 1];
+    const double c1x = c[2 * j1], c1y = c[2 * j1 + 1], c2x = c[2 * j2], c2y = c[2 * j2 + 1];
+    b1c1 = make_double2(c1x - b1x, c1y - b1y);
+    b1c2 = make_double2(c2x - b1x, c2y - b1y);
+    b2c1 = make_double2(c1x - b2x, c1y - b2y);
+    b2c2 = make_double2(c2x - b2x, c2y - b2y);
+    c12 = make_double2(c1x - c2x, c1y - c2y);
+    const double A1 = fma(b1c1.x, b1c2.y, -(b1c1.y * b1c2.x));
+    const double A2 = fma(b2c1.x, b2c2.y, -(b2c1.y * b2c2.x));
+    const double d = A1 - A2, r = 1.0 / d, q = A1 * r;
+    al = fma(fma(-q, d, A1), r, q);  // A1 / d, corrected once
+    const double ga = fma(gx, b2x - b1x, gy * (b2y - b1y)) * r * r;  // dA/dalpha / d^2
+    k1 = -A2 * ga;  // dalpha/dA1
+    k2 = A1 * ga;   // dalpha/dA2
   }
   __device__ __forceinline__ double2 b1() const {
-    return make_double2((1.0 - al) * gx + k1 * (c1y - c2y), (1.0 - al) * gy + k1 * (c2x - c1x));
+    const double u = 1.0 - al;
+    return make_double2(fma(k1, c12.y, u * gx), fma(-k1, c12.x, u * gy));
   }
   __device__ __forceinline__ double2 b2() const {
-    return make_double2(al * gx + k2 * (c1y - c2y), al * gy + k2 * (c2x - c1x));
+    return make_double2(fma(k2, c12.y, al * gx), fma(-k2, c12.x, al * gy));
   }
   __device__ __forceinline__ double2 c1() const {
-    return make_double2(k1 * (c2y - b1y) + k2 * (c2y - b2y), k1 * (b1x - c2x) + k2 * (b2x - c2x));
+    return make_double2(fma(k1, b1c2.y, k2 * b2c2.y), -fma(k1, b1c2.x, k2 * b2c2.x));
   }
   __device__ __forceinline__ double2 c2() const {
-    return make_double2(k1 * (b1y - c1y) + k2 * (b2y - c1y), k1 * (c1x - b1x) + k2 * (c1x - b2x));
+    return make_double2(-fma(k1, b1c1.y, k2 * b2c1.y), fma(k1, b1c1.x, k2 * b2c1.x));
   }
 };
 
@@ -2243,13 +2248,18 @@ k_batch_backward(int np, const double* __restrict__ bxy, const long long* __rest
 }
 
 // The wide pairs' gradients, a block each, gathered: a ring vertex that is
-// vertex e, and a crossing on edge e, go on edge e's list (a counting sort by
-// edge); a thread per edge adds up its list in ring order, the part of the
-// edge's far end kept aside and added to that vertex last.  A crossing is
-// computed for each of its two edges, and every sum has an order fixed by the
-// rings.  (One warp per pair added its groups to global memory 32 ring
-// vertices at a time: 14.1 ms for 12,000 pairs of 3 to 2,048 vertices.)
-__global__ void __launch_bounds__(kWideBlock)
+// vertex e, and a crossing on edge e, are items of edge e (a counting sort by
+// edge, then each item's rank in ring order within its edge).  Every ring
+// vertex is computed once and its parts left at its items' places; a thread
+// per edge adds them up, the part of the edge's far end kept aside and added
+// to that vertex last, so every sum has an order fixed by the rings.  Bound by
+// FP64: 12,000 pairs of 3 to 2,048 vertices took 4.4 ms with every crossing
+// computed for each of its two edges, 1.05 so (14.1 ms with a warp per pair that
+// added its groups to global memory 32 ring vertices at a time).
+struct __align__(16) GradPart {
+  double2 own, end;
+};
+__global__ void __launch_bounds__(kWideBlock, 3)
 k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ bxy,
                       const long long* __restrict__ boff, const double* __restrict__ cxy,
                       const long long* __restrict__ coff, Arenas ar,
@@ -2285,88 +2295,100 @@ k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ b
   int* next = w.R.next;
   int* prev = w.R.prev;
   ring_links(grp, w.roff, nr, nv, next, prev);
+  // per side: first item of each edge, the items' ring vertices as they came,
+  // and their parts, {own vertex, far end}, over arrays of the clipping that
+  // hold 32 bytes per ring vertex and more
+  auto starts = [&](int side) { return side ? w.cAll : w.bAll; };
+  auto lists = [&](int side) { return side ? w.R.label : w.R.enex; };
+  auto parts = [&](int side) { return (GradPart*)(side ? (void*)w.pw.hord : (void*)w.P.x); };
+  auto edge_of = [&](int side, int4 tp) {
+    return tp.x == 2 ? (side ? tp.z : tp.y) : (tp.x == side ? tp.y : -1);
+  };
+  for (int i = lane; i <= nb; i += N) w.bAll[i] = w.bND[i] = 0;
+  for (int i = lane; i <= nc; i += N) w.cAll[i] = w.cND[i] = 0;
+  grp.sync();
+  for (int v = lane; v < nv; v += N) {
+    const int4 tp = w.tape[v];
+    for (int side = 0; side < 2; ++side) {
+      const int e = edge_of(side, tp);
+      if (e >= 0) atomicAdd(&starts(side)[e], 1);
+    }
+  }
+  grp.sync();
+  group_scan(grp, w.bAll, nb + 1);
+  grp.sync();
+  group_scan(grp, w.cAll, nc + 1);
+  grp.sync();
+  for (int v = lane; v < nv; v += N) {
+    const int4 tp = w.tape[v];
+    for (int side = 0; side < 2; ++side) {
+      const int e = edge_of(side, tp);
+      if (e >= 0) lists(side)[starts(side)[e] + atomicAdd(&(side ? w.cND : w.bND)[e], 1)] = v;
+    }
+  }
+  grp.sync();
+  for (int v = lane; v < nv; v += N) {
+    const int ip = next[v], im = prev[v];
+    // shoelace: dA/dx_i = (y_{i+1} - y_{i-1}) / 2, dA/dy_i = (x_{i-1} - x_{i+1}) / 2
+    const double gx = 0.5 * g * (w.rxy[2 * ip + 1] - w.rxy[2 * im + 1]);
+    const double gy = 0.5 * g * (w.rxy[2 * im] - w.rxy[2 * ip]);
+    const int4 tp = w.tape[v];
+    auto place = [&](int side) {
+      const int e = edge_of(side, tp), s = starts(side)[e], t = starts(side)[e + 1];
+      const int* l = lists(side);
+      int r = s;
+      for (int i = s; i < t; ++i) r += l[i] < v;
+      return parts(side) + r;
+    };
+    if (tp.x == 2) {
+      const CrossGrad k(b, tp.y, vsucc(bn, nb, tp.y), c, tp.z, vsucc(cn, nc, tp.z), gx, gy);
+      double2 d = k.b1(), f = k.b2();
+      *place(0) = GradPart{d, f};
+      d = k.c1();
+      f = k.c2();
+      *place(1) = GradPart{d, f};
+    } else if (tp.x >= 0) {
+      *place(tp.x) = GradPart{make_double2(gx, gy), make_double2(0.0, 0.0)};
+    }
+  }
+  grp.sync();
   for (int side = 0; side < 2; ++side) {
     const int n = side ? nc : nb;
-    int* start = side ? w.cAll : w.bAll;
-    int* fill = side ? w.cND : w.bND;
-    int* list = side ? w.R.label : w.R.enex;
+    const int* start = starts(side);
+    const GradPart* part = parts(side);
     double2* far = (double2*)(side ? w.ixC : w.ixB);  // the far ends' part
     double* out = side ? gcp : gbp;
-    auto edge_of = [&](int4 tp) { return tp.x == 2 ? (side ? tp.z : tp.y) : (tp.x == side ? tp.y : -1); };
-    for (int i = lane; i <= n; i += N) start[i] = fill[i] = 0;
-    grp.sync();
-    for (int v = lane; v < nv; v += N) {
-      const int e = edge_of(w.tape[v]);
-      if (e >= 0) atomicAdd(&start[e], 1);
-    }
-    grp.sync();
-    group_scan(grp, start, n + 1);
-    grp.sync();
-    for (int v = lane; v < nv; v += N) {
-      const int e = edge_of(w.tape[v]);
-      if (e >= 0) list[start[e] + atomicAdd(&fill[e], 1)] = v;
-    }
-    grp.sync();
-    // ring vertex v's part for this side's edge e: its own vertex, its far end
-    auto part = [&](int v, int e, double2* own, double2* end) {
-      const int ip = next[v], im = prev[v];
-      // shoelace: dA/dx_i = (y_{i+1} - y_{i-1}) / 2, dA/dy_i = (x_{i-1} - x_{i+1}) / 2
-      const double gx = 0.5 * g * (w.rxy[2 * ip + 1] - w.rxy[2 * im + 1]);
-      const double gy = 0.5 * g * (w.rxy[2 * im] - w.rxy[2 * ip]);
-      const int4 tp = w.tape[v];
-      if (tp.x != 2) {
-        own->x += gx;
-        own->y += gy;
-        return;
+    auto sum = [&](int e, int from, int step) {
+      GradPart a{make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+      for (int i = start[e] + from; i < start[e + 1]; i += step) {
+        const GradPart x = part[i];
+        a.own.x += x.own.x;
+        a.own.y += x.own.y;
+        a.end.x += x.end.x;
+        a.end.y += x.end.y;
       }
-      const CrossGrad k(b, tp.y, vsucc(bn, nb, tp.y), c, tp.z, vsucc(cn, nc, tp.z), gx, gy);
-      const double2 d = side ? k.c1() : k.b1(), f = side ? k.c2() : k.b2();
-      own->x += d.x;
-      own->y += d.y;
-      end->x += f.x;
-      end->y += f.y;
+      return a;
     };
-    auto store = [&](int e, double2 own, double2 end) {
-      out[2 * e] = own.x;
-      out[2 * e + 1] = own.y;
-      far[e] = end;
+    auto store = [&](int e, const GradPart& a) {
+      out[2 * e] = a.own.x;
+      out[2 * e + 1] = a.own.y;
+      far[e] = a.end;
     };
     group_items(
         grp, n, w.R.nb, [&](int e) { return max(1, start[e + 1] - start[e]); },
-        [&](int e, int) {
-          int* l = list + start[e];
-          const int m = start[e + 1] - start[e];
-          for (int i = 1; i < m; ++i) {
-            const int x = l[i];
-            int j = i;
-            while (j > 0 && l[j - 1] > x) {
-              l[j] = l[j - 1];
-              --j;
-            }
-            l[j] = x;
-          }
-          double2 own = make_double2(0.0, 0.0), end = own;
-          for (int i = 0; i < m; ++i) part(l[i], e, &own, &end);
-          store(e, own, end);
-        },
+        [&](int e, int) { store(e, sum(e, 0, 1)); },
         [&](auto& gg, int e, int) {
-          // lane by lane over the ordered list, the lanes' sums in a fixed order
-          // (scratch: R.x and R.y, adjacent in the arena)
-          int* l = list + start[e];
-          const int m = start[e + 1] - start[e];
-          unsigned long long* scr = (unsigned long long*)w.R.x + 2 * start[e];
-          group_sort(gg, m, scr, [&](int k) { return (unsigned long long)l[k]; });
-          const int lane32 = threadIdx.x & 31;
+          // lane by lane, the lanes' sums in a fixed order
           if (gg.warp() == 0) {
-            double2 own = make_double2(0.0, 0.0), end = own;
-            for (int i = lane32; i < m; i += 32) part((int)scr[i], e, &own, &end);
+            const int lane32 = threadIdx.x & 31;
+            GradPart a = sum(e, lane32, 32);
             for (int o = 16; o > 0; o >>= 1) {
-              own.x += __shfl_xor_sync(kFullMask, own.x, o);
-              own.y += __shfl_xor_sync(kFullMask, own.y, o);
-              end.x += __shfl_xor_sync(kFullMask, end.x, o);
-              end.y += __shfl_xor_sync(kFullMask, end.y, o);
+              a.own.x += __shfl_xor_sync(kFullMask, a.own.x, o);
+              a.own.y += __shfl_xor_sync(kFullMask, a.own.y, o);
+              a.end.x += __shfl_xor_sync(kFullMask, a.end.x, o);
+              a.end.y += __shfl_xor_sync(kFullMask, a.end.y, o);
             }
-            if (lane32 == 0) store(e, own, end);
+            if (lane32 == 0) store(e, a);
           }
           gg.sync();
         });
