@@ -1470,7 +1470,11 @@ __global__ void __launch_bounds__(128) k_batch_cand(ClipArgs A) {
 }
 
 // the wide pairs, a warp per group of base edges
-constexpr int kCandWarps = 4, kCandBlocks = 5;
+// (A warp per block, 64 registers: the groups' work varies, and warps that
+// were done held their block's registers until its longest one was.  12,000
+// pairs of 3 to 2,048 vertices: 5.4 ms with blocks of four warps of 96
+// registers, 5.0 with 64, 4.3 so.)
+constexpr int kCandWarps = 1, kCandBlocks = 32;
 template <bool kComp>
 __global__ void __launch_bounds__(32 * kCandWarps, kCandBlocks) k_batch_cand_wide(ClipArgs A) {
   __shared__ int2 s_q[kCandWarps][kCandQ];
