@@ -372,10 +372,14 @@ __device__ __forceinline__ double border_scale(double dv) {
 // edge's end leaves and leaf range follow from the ranks of its two vertices.
 // Sorts E vertices instead of 2 E endpoints, and replaces the array, its
 // border keys and the searches (12,000 pairs of 3 to 2,048 vertices, forward
-// and backward: 8.1 ms of blocks, 2.6 so; 512 pairs of 4 to 64 on warps: 46 us
-// and 25).  A warp counts each vertex's lesser ones, a block sorts
-// (np = npow2_dev(E) entries of key and val).  False: something was shared,
-// has a zero border key or is out of range; nothing but fbox is written.
+// and backward: 8.1 ms of blocks, 2.4 so; 512 pairs of 4 to 64 on warps: 46 us
+// and 21).  A warp counts each vertex's lesser ones by the values rounded to
+// float (65,536 pairs of 4 to 64 vertices: 0.31 ms with 64-bit keys, 0.27 so),
+// a block sorts (np = npow2_dev(E) entries of key and val).  False: something was shared,
+// has a zero border key or is out of range; nothing but vf is written.
+template <int V>
+using Const = std::integral_constant<int, V>;
+
 template <class G>
 __device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, int nc,
                                 PairWork& w, long long* key, int* val, int* rank,
@@ -390,16 +394,12 @@ __device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, 
     return e < nb ? vsucc(w.bnx, nb, e) : nb + vsucc(w.cnx, nc, e - nb);
   };
   FrontRange fr{LLONG_MAX, LLONG_MIN, INT_MAX, INT_MAX};
-  for (int e = lane; e < E; e += N) {
-    const int t = succ(e);
-    const double *pv = vertex(e), *qv = vertex(t);
-    const double2 p = make_double2(pv[0], pv[1]), q = make_double2(qv[0], qv[1]);
-    const long long k = okey(p.x);
-    key[e] = k;
-    fr.join(k, k, e, e);
-    const bool xs = k < okey(q.x), ys = okey(p.y) < okey(q.y);
-    w.fbox[e] = make_float4(__double2float_rd(xs ? p.x : q.x), __double2float_rd(ys ? p.y : q.y),
-                            __double2float_ru(xs ? q.x : p.x), __double2float_ru(ys ? q.y : p.y));
+  for (int v = lane; v < E; v += N) {
+    const double x = vertex(v)[0];
+    const long long k = okey(x);
+    if constexpr (G::kBlock) key[v] = k;
+    fr.join(k, k, v, v);
+    w.vf[v] = float_pair(x, vertex(v)[1]);
   }
   range_join(g, fr, s_range);
   const double lo = vx(fr.imin), absMin = fabs(lo), dv = dadd(vx(fr.imax), absMin);
@@ -416,30 +416,54 @@ __device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, 
     if (k <= 0 || k >= 100000000000LL) bad = true;
   };
   if constexpr (!G::kBlock) {
-    g.sync();
-    constexpr int kPer = 4;  // vertices per lane and sweep over the keys
-    for (int v0 = lane; v0 - lane < E; v0 += kPer * N) {
-      long long k[kPer];
-      int r[kPer], same[kPer];
+    // Ranks by the values rounded to float; where two of those are equal, by
+    // the values.  A shared rank leaves another vertex in its place.
+    float* fx = (float*)key;
+    int* at = (int*)(fx + E);  // vertex of each rank
+    auto count = [&](auto per, auto less) {
+      constexpr int kPer = decltype(per)::value;
+      int r[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) r[i] = 0;
+      for (int u = 0; u < E; ++u)
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) r[i] += less(u, i);
+      g.sync();
 #pragma unroll
       for (int i = 0; i < kPer; ++i) {
-        k[i] = v0 + i * N < E ? key[v0 + i * N] : LLONG_MAX;
-        r[i] = same[i] = 0;
-      }
-      for (int u = 0; u < E; ++u) {
-        const long long x = key[u];
-#pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-          r[i] += x < k[i];
-          same[i] += x == k[i];
+        const int v = lane + i * N;
+        if (v < E) {
+          place(v, r[i]);
+          at[r[i]] = v;
         }
       }
+      g.sync();
+      bool same = false;
 #pragma unroll
       for (int i = 0; i < kPer; ++i)
-        if (v0 + i * N < E) {
-          place(v0 + i * N, r[i]);
-          if (same[i] != 1) bad = true;
-        }
+        if (lane + i * N < E && at[r[i]] != lane + i * N) same = true;
+      return g.any(same);
+    };
+    auto by_float = [&](auto per) {
+      constexpr int kPer = decltype(per)::value;
+      float x[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) x[i] = lane + i * N < E ? fx[lane + i * N] : 0.f;
+      return count(per, [&](int u, int i) { return fx[u] < x[i]; });
+    };
+    for (int v = lane; v < E; v += N) fx[v] = w.vf[v].x;
+    g.sync();
+    bool same;
+    if (E <= 32) same = by_float(Const<1>{});
+    else if (E <= 64) same = by_float(Const<2>{});
+    else if (E <= 96) same = by_float(Const<3>{});
+    else if (E <= 128) same = by_float(Const<4>{});
+    else same = by_float(Const<8>{});
+    if (same) {
+      bad = false;
+      long long k[8];
+      for (int i = 0; i < 8; ++i) k[i] = lane + i * N < E ? okey(vx(lane + i * N)) : 0;
+      if (count(Const<8>{}, [&](int u, int i) { return okey(vx(u)) < k[i]; })) bad = true;
     }
   } else {
     const int np = npow2_dev(E);
@@ -478,6 +502,7 @@ __device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, 
   };
   for (int e = lane; e < E; e += N) {
     const int t = succ(e), r0 = rank[e], r1 = rank[t];
+    w.fbox[e] = float_box(w.vf[e], w.vf[t]);
     const int2 S = range(min(r0, r1)), T = range(max(r0, r1));
     int a = -1, z = -1;
     const int en = border(T, r0 < r1 ? t : e), st = border(S, r0 < r1 ? e : t);
@@ -719,9 +744,10 @@ __device__ int clip_pair_front(G& g, const double* b, int nb, const double* c, i
 
 // what the candidate kernels read beside the boxes
 template <class G>
-__device__ void front_floats(G& g, const double* b, int nb, const double* c, int nc, PairWork& w) {
+__device__ void front_floats(G& g, const double* b, int nb, const double* c, int nc, PairWork& w,
+                             bool have) {
   g.sync();
-  for (int v = g.rank(); v < nb + nc; v += G::N) {
+  for (int v = have ? nb + nc : g.rank(); v < nb + nc; v += G::N) {
     const double* p = v < nb ? b + 2 * v : c + 2 * (v - nb);
     w.vf[v] = float_pair(p[0], p[1]);
   }
@@ -1393,7 +1419,7 @@ __device__ __forceinline__ void front_done(const ClipArgs& A, int p, PairWork& w
   }
 }
 
-__global__ void __launch_bounds__(128) k_batch_front(ClipArgs A) {
+__global__ void __launch_bounds__(128, 8) k_batch_front(ClipArgs A) {
   __shared__ long long s_key[4][kWideEdges];
   __shared__ int s_rank[4][kWideEdges];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1417,10 +1443,11 @@ __global__ void __launch_bounds__(128) k_batch_front(ClipArgs A) {
   WarpGroup g;
   const double *b = A.bxy + 2 * A.boff[p], *c = A.cxy + 2 * A.coff[p];
   int st = PS_OK;
-  if (!clip_pair_ranks(g, b, nb, c, nc, w, s_key[threadIdx.x >> 5], nullptr,
-                       s_rank[threadIdx.x >> 5], nullptr))
+  const bool ranked = clip_pair_ranks(g, b, nb, c, nc, w, s_key[threadIdx.x >> 5], nullptr,
+                                      s_rank[threadIdx.x >> 5], nullptr);
+  if (!ranked)
     st = clip_pair_front(g, b, nb, c, nc, cp, w, nullptr, nullptr, 0, nullptr);
-  front_floats(g, b, nb, c, nc, w);
+  front_floats(g, b, nb, c, nc, w, ranked);
   if (lane == 0) front_done(A, p, w, st);
 }
 
@@ -1443,16 +1470,19 @@ __global__ void __launch_bounds__(kWideBlock) k_batch_front_wide(ClipArgs A) {
   const double *b = A.bxy + 2 * A.boff[p], *c = A.cxy + 2 * A.coff[p];
   const bool fits = npow2_dev(nb + nc) <= kFrontSort;
   int st = PS_OK;
-  if (!clip_pair_ranks(g, b, nb, c, nc, w, fits ? s_key : w.fkey, fits ? s_val : w.fval, w.vl,
-                       s_range))
+  const bool ranked = clip_pair_ranks(g, b, nb, c, nc, w, fits ? s_key : w.fkey,
+                                      fits ? s_val : w.fval, w.vl, s_range);
+  if (!ranked)
     st = clip_pair_front(g, b, nb, c, nc, cp, w, s_key, s_val, kFrontSort, s_range);
-  front_floats(g, b, nb, c, nc, w);
+  front_floats(g, b, nb, c, nc, w, ranked);
   if (threadIdx.x == 0) front_done(A, p, w, st);
 }
 
 // the all-pairs test of the small pairs, with or without component successors
+// (bound by the latency of its loads: 65,536 pairs of 4 to 64 vertices take
+// 0.50 ms with 86 registers, 0.34 with 64, 0.28 with 40 and some spilled)
 template <bool kComp>
-__global__ void __launch_bounds__(128) k_batch_cand(ClipArgs A) {
+__global__ void __launch_bounds__(128, 12) k_batch_cand(ClipArgs A) {
   __shared__ int2 s_q[4][kCandQ];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -1730,7 +1760,10 @@ __device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, in
   }
 }
 
-__global__ void __launch_bounds__(128) k_batch_clean(ClipArgs A) {
+// (The kernel's code is larger than the instruction cache: with the warps of a
+// block entering its steps together 65,536 pairs of 4 to 64 vertices take 0.75
+// ms, 0.81 without.)
+__global__ void __launch_bounds__(128, 5) k_batch_clean(ClipArgs A) {
   __shared__ __align__(16) unsigned char s_mem[4][kCleanSmem];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if ((t >> 5) >= A.np) return;
@@ -1738,7 +1771,7 @@ __global__ void __launch_bounds__(128) k_batch_clean(ClipArgs A) {
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
   if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
-  WarpGroup g;
+  PhasedWarp g;
   batch_clean(g, A, p, pass, nb, nc, s_mem[threadIdx.x >> 5], kCleanSmem, nullptr, 0,
               nullptr);
 }
@@ -2164,90 +2197,132 @@ struct CrossGrad {
   }
 };
 
+struct BackArgs {
+  int np;
+  const int* wide;
+  int wide_min;
+  const double* bxy;
+  const long long* boff;
+  const double* cxy;
+  const long long* coff;
+  Arenas ar;
+  const int* status;
+  const int* nrings;
+  const double* gA;
+  const int* bnx;
+  const int* cnx;
+  double* gb;
+  double* gc;
+};
+// a pair's gradients zeroed, where it has no rings
+template <class G>
+__device__ bool backward_none(G& g, const BackArgs& A, int p, int nb, int nc) {
+  if (A.status[p] == SBC_OK && A.nrings[p] != 0 && A.ar.pass[p] >= 0) return false;
+  for (int i = g.rank(); i < 2 * nb; i += G::N) A.gb[2 * A.boff[p] + i] = 0.0;
+  for (int i = g.rank(); i < 2 * nc; i += G::N) A.gc[2 * A.coff[p] + i] = 0.0;
+  return true;
+}
+
 // d(area)/d(vertices), one warp per pair, from the forward pass's tape.  The
-// lanes take 32 ring vertices at a time and compute their contributions
-// (the crossings' FP64 chain rule in parallel, up to four target vertices
-// each, in four rounds).  In each round the lanes naming the same vertex
-// form a group (match_any) whose lowest lane sums their values in lane order
-// and adds the sum: every gradient entry is summed in an order fixed by the
-// rings alone, whatever the launch shape.
-__global__ void __launch_bounds__(128)
-k_batch_backward(int np, const double* __restrict__ bxy, const long long* __restrict__ boff,
-                 const double* __restrict__ cxy, const long long* __restrict__ coff, Arenas ar,
-                 const int* __restrict__ status, const int* __restrict__ nrings,
-                 const double* __restrict__ gA, const int* __restrict__ bnx,
-                 const int* __restrict__ cnx, int wide_min, double* __restrict__ gb,
-                 double* __restrict__ gc) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// lanes take 32 ring vertices at a time, over all rings, first the crossings
+// (the FP64 chain rule, four target vertices each, in four rounds), then the
+// polygons' own vertices.  In each round the lanes naming the same
+// vertex form a group (match_any) whose lowest lane sums their values in lane
+// order and adds the sum: every gradient entry is summed in an order fixed by
+// the rings alone, whatever the launch shape.  Bound by FP64, which costs a
+// warp the same for one lane as for 32: 65,536 pairs of 4 to 64 vertices took
+// 0.40 ms ring by ring, few of which fill a warp, 0.36 over all rings with
+// crossings and vertices mixed, 0.32 so (0.44 by the wide pairs' gather).
+__global__ void __launch_bounds__(128, 8) k_batch_backward(BackArgs A) {
   const int lane = threadIdx.x & 31;
-  if ((t >> 5) >= np) return;
-  const int p = (int)(t >> 5);
-  const int nb = (int)(boff[p + 1] - boff[p]), nc = (int)(coff[p + 1] - coff[p]);
-  if (ar.pass[p] >= 0 && wide_pair(nb, nc, wide_min)) return;  // k_batch_backward_wide
-  double* gbp = gb + 2 * boff[p];
-  double* gcp = gc + 2 * coff[p];
+  const int p = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (p >= A.np) return;
+  const int nb = (int)(A.boff[p + 1] - A.boff[p]), nc = (int)(A.coff[p + 1] - A.coff[p]);
+  if (A.ar.pass[p] >= 0 && wide_pair(nb, nc, A.wide_min)) return;  // k_batch_backward_wide
+  WarpGroup grp;
+  if (backward_none(grp, A, p, nb, nc)) return;
+  double* gbp = A.gb + 2 * A.boff[p];
+  double* gcp = A.gc + 2 * A.coff[p];
   for (int i = lane; i < 2 * nb; i += 32) gbp[i] = 0.0;
   for (int i = lane; i < 2 * nc; i += 32) gcp[i] = 0.0;
-  if (status[p] != SBC_OK || nrings[p] == 0 || ar.pass[p] < 0) return;
-  __syncwarp();
-  const double* b = bxy + 2 * boff[p];
-  const double* c = cxy + 2 * coff[p];
-  const int* bn = bnx ? bnx + boff[p] : nullptr;
-  const int* cn = cnx ? cnx + coff[p] : nullptr;
-  const Caps cp = caps_of(nb, nc, hit_cap(nb, nc, ar.pass[p], ar.need[p]));
-  Carver cv{const_cast<unsigned char*>(ar.at(p)), 0};
+  const double* b = A.bxy + 2 * A.boff[p];
+  const double* c = A.cxy + 2 * A.coff[p];
+  const int* bn = A.bnx ? A.bnx + A.boff[p] : nullptr;
+  const int* cn = A.cnx ? A.cnx + A.coff[p] : nullptr;
+  const Caps cp = caps_of(nb, nc, hit_cap(nb, nc, A.ar.pass[p], A.ar.need[p]));
+  Carver cv{const_cast<unsigned char*>(A.ar.at(p)), 0};
   const PairWork w = carve(cv, cp);
-  const double g = gA[p];
-  const int nr = nrings[p];
-  for (int r = 0; r < nr; ++r) {
-    const int s = w.roff[r], e = w.roff[r + 1];
-    for (int i0 = s; i0 < e; i0 += 32) {
-      const int i = i0 + lane;
-      int tg[4] = {-1, -1, -1, -1};
-      double2 vv[4];
-      if (i < e) {
-        const int ip = (i + 1 == e) ? s : i + 1, im = (i == s) ? e - 1 : i - 1;
-        // shoelace: dA/dx_i = (y_{i+1} - y_{i-1}) / 2, dA/dy_i = (x_{i-1} - x_{i+1}) / 2
-        const double gx = 0.5 * g * (w.rxy[2 * ip + 1] - w.rxy[2 * im + 1]);
-        const double gy = 0.5 * g * (w.rxy[2 * im] - w.rxy[2 * ip]);
-        const int4 tp = w.tape[i];
-        if (tp.x == 0 || tp.x == 1) {
-          tg[0] = (tp.x << 30) | tp.y;
-          vv[0] = make_double2(gx, gy);
-        } else if (tp.x == 2) {
-          const int i1 = tp.y, i2 = vsucc(bn, nb, tp.y), j1 = tp.z, j2 = vsucc(cn, nc, tp.z);
-          const CrossGrad k(b, i1, i2, c, j1, j2, gx, gy);
-          tg[0] = i1;
-          vv[0] = k.b1();
-          tg[1] = i2;
-          vv[1] = k.b2();
-          tg[2] = (1 << 30) | j1;
-          vv[2] = k.c1();
-          tg[3] = (1 << 30) | j2;
-          vv[3] = k.c2();
-        }
+  const double g = A.gA[p];
+  const int nr = A.nrings[p], nv = w.roff[nr];
+  ring_links(grp, w.roff, nr, nv, w.R.next, w.R.prev);
+  int ncross = 0, nown = 0;  // the ring vertices that are crossings, and vertices
+  for (int i0 = 0; i0 < nv; i0 += 32) {
+    const int i = i0 + lane, kind = i < nv ? w.tape[i].x : -1;
+    int n, k = ncross + grp.before(kind == 2, &n);
+    if (kind == 2) w.R.label[k] = i;
+    ncross += n;
+    k = nown + grp.before(kind == 0 || kind == 1, &n);
+    if (kind == 0 || kind == 1) w.R.enex[k] = i;
+    nown += n;
+  }
+  __syncwarp();
+  // shoelace: dA/dx_i = (y_{i+1} - y_{i-1}) / 2, dA/dy_i = (x_{i-1} - x_{i+1}) / 2
+  auto grad = [&](int i) {
+    const int ip = w.R.next[i], im = w.R.prev[i];
+    return make_double2(0.5 * g * (w.rxy[2 * ip + 1] - w.rxy[2 * im + 1]),
+                        0.5 * g * (w.rxy[2 * im] - w.rxy[2 * ip]));
+  };
+  // the lanes' values v added to vertices t (side in bit 30; -1: none)
+  auto add = [&](int t, const double2& v) {
+    const unsigned act = __ballot_sync(kFullMask, t >= 0);
+    if (t >= 0) {
+      const unsigned same = __match_any_sync(act, t);
+      const int first = __ffs(same) - 1;
+      double sx = __shfl_sync(same, v.x, first), sy = __shfl_sync(same, v.y, first);
+      for (unsigned m = same & (same - 1); m; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        sx += __shfl_sync(same, v.x, l);
+        sy += __shfl_sync(same, v.y, l);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const unsigned act = __ballot_sync(0xffffffffu, tg[j] >= 0);
-        if (tg[j] >= 0) {
-          const unsigned grp = __match_any_sync(act, tg[j]);
-          double sx = 0.0, sy = 0.0;
-          for (unsigned m = grp; m; m &= m - 1) {
-            const int l = __ffs(m) - 1;
-            sx += __shfl_sync(grp, vv[j].x, l);
-            sy += __shfl_sync(grp, vv[j].y, l);
-          }
-          if (lane == __ffs(grp) - 1) {
-            double* gp = (tg[j] >> 30) ? gcp : gbp;
-            const int v = tg[j] & 0x3fffffff;
-            gp[2 * v] += sx;
-            gp[2 * v + 1] += sy;
-          }
-        }
-        __syncwarp();
+      if (lane == first) {
+        double* gp = (t >> 30) ? gcp : gbp;
+        gp[2 * (t & 0x3fffffff)] += sx;
+        gp[2 * (t & 0x3fffffff) + 1] += sy;
       }
     }
+    __syncwarp();
+  };
+  for (int k0 = 0; k0 < ncross; k0 += 32) {
+    const int k = k0 + lane;
+    int tg[4] = {-1, -1, -1, -1};
+    double2 vv[4];
+    if (k < ncross) {
+      const int i = w.R.label[k];
+      const int4 tp = w.tape[i];
+      const double2 d = grad(i);
+      tg[0] = tp.y;
+      tg[1] = vsucc(bn, nb, tp.y);
+      tg[2] = (1 << 30) | tp.z;
+      tg[3] = (1 << 30) | vsucc(cn, nc, tp.z);
+      const CrossGrad x(b, tg[0], tg[1], c, tp.z, tg[3] & 0x3fffffff, d.x, d.y);
+      vv[0] = x.b1();
+      vv[1] = x.b2();
+      vv[2] = x.c1();
+      vv[3] = x.c2();
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) add(tg[j], vv[j]);
+  }
+  for (int k0 = 0; k0 < nown; k0 += 32) {
+    const int k = k0 + lane;
+    int t = -1;
+    double2 v = make_double2(0.0, 0.0);
+    if (k < nown) {
+      const int4 tp = w.tape[w.R.enex[k]];
+      t = (tp.x << 30) | tp.y;
+      v = grad(w.R.enex[k]);
+    }
+    add(t, v);
   }
 }
 
@@ -2258,44 +2333,32 @@ k_batch_backward(int np, const double* __restrict__ bxy, const long long* __rest
 // per edge adds them up, the part of the edge's far end kept aside and added
 // to that vertex last, so every sum has an order fixed by the rings.  Bound by
 // FP64: 12,000 pairs of 3 to 2,048 vertices took 4.4 ms with every crossing
-// computed for each of its two edges, 1.05 so (14.1 ms with a warp per pair that
-// added its groups to global memory 32 ring vertices at a time).
+// computed for each of its two edges, 1.05 so (14.1 ms with a warp per pair
+// that added groups to global memory).
 struct __align__(16) GradPart {
   double2 own, end;
 };
-__global__ void __launch_bounds__(kWideBlock, 3)
-k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ bxy,
-                      const long long* __restrict__ boff, const double* __restrict__ cxy,
-                      const long long* __restrict__ coff, Arenas ar,
-                      const int* __restrict__ status, const int* __restrict__ nrings,
-                      const double* __restrict__ gA, const int* __restrict__ bnx,
-                      const int* __restrict__ cnx, double* __restrict__ gb,
-                      double* __restrict__ gc) {
+__global__ void __launch_bounds__(kWideBlock, 3) k_batch_backward_wide(BackArgs A) {
   using G = BlockGroup<kWideBlock>;
   __shared__ G::Shared sh;
   constexpr int N = G::N;
-  const int p = wide[blockIdx.x];
-  if (ar.pass[p] < 0) return;
-  const int nb = (int)(boff[p + 1] - boff[p]), nc = (int)(coff[p + 1] - coff[p]);
-  double* gbp = gb + 2 * boff[p];
-  double* gcp = gc + 2 * coff[p];
-  const int nr = nrings[p];
-  if (status[p] != SBC_OK || nr == 0) {
-    for (int i = threadIdx.x; i < 2 * nb; i += N) gbp[i] = 0.0;
-    for (int i = threadIdx.x; i < 2 * nc; i += N) gcp[i] = 0.0;
-    return;
-  }
   G grp(&sh);
   const int lane = grp.rank();
-  const double* b = bxy + 2 * boff[p];
-  const double* c = cxy + 2 * coff[p];
-  const int* bn = bnx ? bnx + boff[p] : nullptr;
-  const int* cn = cnx ? cnx + coff[p] : nullptr;
-  const Caps cp = caps_of(nb, nc, hit_cap(nb, nc, ar.pass[p], ar.need[p]));
-  Carver cv{const_cast<unsigned char*>(ar.at(p)), 0};
+  const int p = A.wide[blockIdx.x];
+  if (A.ar.pass[p] < 0) return;
+  const int nb = (int)(A.boff[p + 1] - A.boff[p]), nc = (int)(A.coff[p + 1] - A.coff[p]);
+  if (backward_none(grp, A, p, nb, nc)) return;
+  double* gbp = A.gb + 2 * A.boff[p];
+  double* gcp = A.gc + 2 * A.coff[p];
+  const double* b = A.bxy + 2 * A.boff[p];
+  const double* c = A.cxy + 2 * A.coff[p];
+  const int* bn = A.bnx ? A.bnx + A.boff[p] : nullptr;
+  const int* cn = A.cnx ? A.cnx + A.coff[p] : nullptr;
+  const Caps cp = caps_of(nb, nc, hit_cap(nb, nc, A.ar.pass[p], A.ar.need[p]));
+  Carver cv{const_cast<unsigned char*>(A.ar.at(p)), 0};
   const PairWork w = carve(cv, cp);
-  const double g = gA[p];
-  const int nv = w.roff[nr];
+  const double g = A.gA[p];
+  const int nr = A.nrings[p], nv = w.roff[nr];
   int* next = w.R.next;
   int* prev = w.R.prev;
   ring_links(grp, w.roff, nr, nv, next, prev);
@@ -2404,6 +2467,17 @@ k_batch_backward_wide(const int* __restrict__ wide, const double* __restrict__ b
       out[2 * t + 1] += far[e].y;
     }
     grp.sync();
+  }
+}
+
+void launch_backward(const BackArgs& A, int nwide, int block, double bytes, cudaStream_t st) {
+  {
+    ::sbc::KProbe kp_("k_batch_backward", st, bytes);
+    k_batch_backward<<<grid_for(32LL * A.np, block), block, 0, st>>>(A);
+  }
+  if (nwide > 0) {
+    ::sbc::KProbe kp_("k_batch_backward_wide", st);
+    k_batch_backward_wide<<<nwide, kWideBlock, 0, st>>>(A);
   }
 }
 
@@ -2976,19 +3050,12 @@ int BatchRunner::backward(const double* d_bxy, const long long* d_boff, const do
     const Arenas ar{arena[0], aoff[0] + p0, abase_[0], arena[1], aoff[1] + p0, abase_[1], pass + p0,
                     need_ + p0};
     // coordinates in, one gradient per coordinate out
-    ::sbc::KProbe kp_("k_batch_backward", st,
-                      32.0 * (double)(h_boff_[p1] - h_boff_[p0] + h_coff_[p1] - h_coff_[p0]) +
-                          8.0 * n);
-    k_batch_backward<<<grid_for(32LL * n, shape.bwd), shape.bwd, 0, st>>>(
-        n, d_bxy, d_boff + p0, d_cxy, d_coff + p0, ar, status + p0, nrings + p0, d_gA + p0, bnx,
-        cnx, wide_min_, d_gb, d_gc);
-    if (nwide_ > 0) {
-      ::sbc::KProbe kw_("k_batch_backward_wide", st);
-      k_batch_backward_wide<<<nwide_, kWideBlock, 0, st>>>(wide_, d_bxy, d_boff + p0, d_cxy,
-                                                           d_coff + p0, ar, status + p0,
-                                                           nrings + p0, d_gA + p0, bnx, cnx, d_gb,
-                                                           d_gc);
-    }
+    const double bytes =
+        32.0 * (double)(h_boff_[p1] - h_boff_[p0] + h_coff_[p1] - h_coff_[p0]) +
+                          8.0 * n;
+    launch_backward(BackArgs{n, wide_, wide_min_, d_bxy, d_boff + p0, d_cxy, d_coff + p0, ar,
+                             status + p0, nrings + p0, d_gA + p0, bnx, cnx, d_gb, d_gc},
+                    nwide_, shape.bwd, bytes, st);
   }
   for (const BigOut& bo : big_) {
     if (!bo.ok || bo.nverts == 0) continue;
@@ -3132,17 +3199,9 @@ int BatchRunner::graph_record(int np_, const double* d_bxy, const long long* d_b
                                        area, unite ? 1 : 0, split_now()},
                               bnx, cnx, wide_, wide_item_, nwide_, nitems_, wide_min_));
     const Arenas ar{arena[0], aoff[0], abase_[0], arena[1], aoff[1], 0, pass, need_rec};
-    {
-      ::sbc::KProbe kp_("k_batch_backward", st);
-      k_batch_backward<<<grid_for(32LL * np, shape.bwd), shape.bwd, 0, st>>>(
-          np, d_bxy, d_boff, d_cxy, d_coff, ar, status, nrings, d_gA, bnx, cnx, wide_min_, d_gb,
-          d_gc);
-    }
-    if (nwide_ > 0) {
-      ::sbc::KProbe kp_("k_batch_backward_wide", st);
-      k_batch_backward_wide<<<nwide_, kWideBlock, 0, st>>>(
-          wide_, d_bxy, d_boff, d_cxy, d_coff, ar, status, nrings, d_gA, bnx, cnx, d_gb, d_gc);
-    }
+    launch_backward(BackArgs{np, wide_, wide_min_, d_bxy, d_boff, d_cxy, d_coff, ar, status,
+                             nrings, d_gA, bnx, cnx, d_gb, d_gc},
+                    nwide_, shape.bwd, 0.0, st);
     if (out_area) cudaMemcpyAsync(out_area, area, sizeof(double) * np, cudaMemcpyDeviceToDevice, st);
     if (out_status)
       cudaMemcpyAsync(out_status, status, sizeof(int) * np, cudaMemcpyDeviceToDevice, st);

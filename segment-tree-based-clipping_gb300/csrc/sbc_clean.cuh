@@ -182,7 +182,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     m.aC[h] = t % 1000000000;
     // apart from the four ends (an equal slot stops the list walk early, and
     // provenance goes by coordinates)
-    auto meets = [&](double px, double py) { return px == x && py == y; };
+    auto meets = [&](double px, double py) { return same_value(px, x) && same_value(py, y); };
     if (meets(p1x, p1y) || meets(p2x, p2y) || meets(c[2 * f], c[2 * f + 1]) ||
         meets(c[2 * f2], c[2 * f2 + 1]))
       bad = true;
@@ -305,6 +305,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
       m.eQ[k] = hits.c(q);
     }
     g.sync();
+    g.phase();
     // ---- A14: every initial label a crossing (calculateInitLabelParallel,
     // oacc_segment_tree.cpp:7925-7988): the overlay's neighbours of the
     // crossing lie on different sides of the base there
@@ -320,7 +321,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
         break;
       }
       // nor two crossings of an edge at one point (provenance by coordinates)
-      auto at = [&](int o) { return o >= 0 && m.x[o] == cx && m.y[o] == cy; };
+      auto at = [&](int o) { return o >= 0 && same_value(m.x[o], cx) && same_value(m.y[o], cy); };
       if (at(hm) || at(hp) || at(gm) || at(gp)) {
         bad = true;
         break;
@@ -331,8 +332,8 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
       const double s3 = area3(pmx, pmy, cx, cy, ppx, ppy);
       auto right = [&](double qx, double qy) {
         const double s1 = area3(qx, qy, pmx, pmy, cx, cy), s2 = area3(qx, qy, cx, cy, ppx, ppy);
-        if (s3 > 0) return !(s1 > 0 && s2 > 0);
-        return s1 < 0 && s2 < 0;
+        if (is_pos(s3)) return !(is_pos(s1) && is_pos(s2));
+        return is_neg(s1) && is_neg(s2);
       };
       const bool rm = gm >= 0 ? right(m.x[gm], m.y[gm]) : right(c[2 * f], c[2 * f + 1]);
       const bool rp = gp >= 0 ? right(m.x[gp], m.y[gp]) : right(c[2 * f2], c[2 * f2 + 1]);
@@ -340,35 +341,100 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     }
     if (g.any(bad)) return CLEAN_NOT;
   }
+  g.phase();
   // ---- components, and whether each one's first vertex lies in the other
   // polygon (pointInPoly over the list's edges): a thread per polygon edge
   // without crossings and per piece between two list nodes, not per edge (an
   // edge near the ray can hold most of a pair's crossings)
   const int ncb = in.bnx ? clean_components(g, nb, in.bnx, in.rootB) : 1;
   const int ncc = in.cnx ? clean_components(g, nc, in.cnx, in.rootC) : 1;
+  // The few pieces whose orientation decides go on a list (over A and B), so
+  // that their FP64 runs once, in full warps.
   auto inside = [&](bool overlay, double rx, double ry) {
     const double* p = overlay ? c : b;
     const bool sparse = kSparse && !overlay;
     const int* list = overlay ? m.hQ : m.hP;
     const int* edge = overlay ? m.eQ : m.eP;
-    int part = 0;
-    for (int e = lane; e < (sparse ? 0 : overlay ? nc : nb); e += N) {
-      const double x0 = p[2 * e], y0 = p[2 * e + 1];
-      if (!(x0 == x0 && y0 == y0)) bad = true;
-      if ((overlay ? countC(e) : countB(e)) > 0) continue;
-      const int e2 = overlay ? csucc(e) : bsucc(e);
-      part += pip_step(x0, y0, p[2 * e2], p[2 * e2 + 1], rx, ry);
+    double2 *from = (double2*)m.A, *to = (double2*)m.B;
+    int part = 0, listed = 0;  // (listed: a warp's; a block's is shared)
+    if constexpr (G::kBlock) {
+      if (lane == 0) g.s->count = 0;
+      g.sync();
     }
-    for (int k = lane; k < K; k += N) {  // the piece that ends at crossing k, and the last
-      const int h = list[k], e = edge[k];
-      const bool first = k == 0 || edge[k - 1] != e;
-      const int o = first ? 0 : list[k - 1];
-      part += pip_step(first ? p[2 * e] : m.x[o], first ? p[2 * e + 1] : m.y[o], m.x[h], m.y[h], rx,
-                       ry);
-      if (k + 1 < K && edge[k + 1] == e) continue;
-      const int e2 = overlay ? csucc(e) : bsucc(e);
-      part += pip_step(m.x[h], m.y[h], p[2 * e2], p[2 * e2 + 1], rx, ry);
-      if (sparse) part -= pip_step(p[2 * e], p[2 * e + 1], p[2 * e2], p[2 * e2 + 1], rx, ry);
+    auto piece = [&](bool act, double x0, double y0, double x1, double y1) {
+      bool area = false;
+      const int d = act ? pip_quick(x0, y0, x1, y1, rx, ry, &area) : 0;
+      if (!area) part += d;
+      const unsigned w = __ballot_sync(0xffffffffu, area);
+      if (w == 0u) return;
+      int at = listed;
+      if constexpr (G::kBlock) {
+        if ((lane & 31) == 0) at = atomicAdd(&g.s->count, __popc(w));
+        at = __shfl_sync(0xffffffffu, at, 0);
+      } else {
+        listed += __popc(w);
+      }
+      at += __popc(w & ((1u << (lane & 31)) - 1u));
+      if (area && at < K + 4) {
+        from[at] = make_double2(x0, y0);
+        to[at] = make_double2(x1, y1);
+      } else if (area) {
+        part += pip_decide(x0, y0, x1, y1, rx, ry);
+      }
+    };
+    const int n = sparse ? 0 : overlay ? nc : nb;
+    for (int e0 = 0; e0 < n; e0 += N) {
+      const int e = e0 + lane;
+      double x0 = 0.0, y0 = 0.0, x1 = 0.0, y1 = 0.0;
+      bool act = e < n;
+      if (act) {
+        x0 = p[2 * e];
+        y0 = p[2 * e + 1];
+        if (abs_bits(x0) > kInfBits || abs_bits(y0) > kInfBits) bad = true;
+        act = (overlay ? countC(e) : countB(e)) == 0;
+      }
+      if (act) {
+        const int e2 = overlay ? csucc(e) : bsucc(e);
+        x1 = p[2 * e2];
+        y1 = p[2 * e2 + 1];
+      }
+      piece(act, x0, y0, x1, y1);
+    }
+    for (int k0 = 0; k0 < K; k0 += N) {  // the piece that ends at crossing k, and the last
+      const int k = k0 + lane;
+      const bool act = k < K;
+      int e = 0;
+      bool last = false;
+      double x0 = 0.0, y0 = 0.0, x1 = 0.0, y1 = 0.0, x2 = 0.0, y2 = 0.0;
+      if (act) {
+        const int h = list[k];
+        e = edge[k];
+        if (k == 0 || edge[k - 1] != e) {
+          x0 = p[2 * e];
+          y0 = p[2 * e + 1];
+        } else {
+          x0 = m.x[list[k - 1]];
+          y0 = m.y[list[k - 1]];
+        }
+        x1 = m.x[h];
+        y1 = m.y[h];
+        last = k + 1 == K || edge[k + 1] != e;
+        if (last) {
+          const int e2 = overlay ? csucc(e) : bsucc(e);
+          x2 = p[2 * e2];
+          y2 = p[2 * e2 + 1];
+        }
+      }
+      piece(act, x0, y0, x1, y1);
+      piece(last, x1, y1, x2, y2);
+      if (sparse && last) part -= pip_step(p[2 * e], p[2 * e + 1], x2, y2, rx, ry);
+    }
+    g.sync();
+    if constexpr (G::kBlock) listed = g.s->count;
+    if (listed > K + 4) listed = K + 4;
+    for (int i = lane; i < listed; i += N) {
+      const double2 u = from[i], v = to[i];
+      part += pip_decide(u.x, u.y, v.x, v.y, rx, ry);
     }
     return (g.sum(part) + (sparse ? in.base_steps : 0)) & 1;
   };
@@ -423,6 +489,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
       if ((r.hi - r.lo) & 1) bad = true;
     }
   if (g.any(bad)) return CLEAN_NOT;
+  g.phase();
   // ---- rings: first the components without crossings that lie inside (or
   // outside, for the union), whole and in order
   int rings = 0, verts = 0;
@@ -517,6 +584,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
   if (verts > in.vcap) return CLEAN_ROOM;
   if (lane == 0) in.roff[rings] = verts;
   g.sync();
+  g.phase();
   // the legs to their places: a lane writes a short one, the warp a long one
   constexpr int kShort = 8;
   for (int i0 = 0; i0 < K; i0 += N) {
@@ -567,26 +635,28 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     }
   }
   g.sync();
+  g.phase();
   // ---- cleanUpResult2 (foster/polyclip.h:767-787): a vertex with |area3| <
   // eps goes.  And the area: the shoelace terms in an order that the rings and
   // the group size fix.
   auto area_at = [&](int u, int v, int x) {
-    return fabs(area3(in.rxy[2 * u], in.rxy[2 * u + 1], in.rxy[2 * v], in.rxy[2 * v + 1],
-                      in.rxy[2 * x], in.rxy[2 * x + 1]));
+    return area3(in.rxy[2 * u], in.rxy[2 * u + 1], in.rxy[2 * v], in.rxy[2 * v + 1],
+                 in.rxy[2 * x], in.rxy[2 * x + 1]);
   };
-  auto term = [&](int v, int vp) {
-    return dsub(dmul(in.rxy[2 * v], in.rxy[2 * vp + 1]), dmul(in.rxy[2 * vp], in.rxy[2 * v + 1]));
+  auto term = [&](double s, int v, int vp) {
+    return dadd(s, dsub(dmul(in.rxy[2 * v], in.rxy[2 * vp + 1]),
+                        dmul(in.rxy[2 * vp], in.rxy[2 * v + 1])));
   };
   double s2 = 0.0;
   bool flat = false;
   for (int v = lane; v < verts; v += N) {
     const int r = in.tape[v].w, s = in.roff[r], e = in.roff[r + 1];
     const int vp = v + 1 == e ? s : v + 1;
-    if (area_at(v == s ? e - 1 : v - 1, v, vp) < kEps) {
+    if (abs_lt(area_at(v == s ? e - 1 : v - 1, v, vp), kEps)) {
       flat = true;
       in.tape[v].w = ~r;
     }
-    s2 = dadd(s2, term(v, vp));
+    s2 = term(s2, v, vp);
   }
   if (g.any(flat)) {  // (rare: one pair in thousands of random ones)
     // The reference's walk, a thread per ring, over links that start as the
@@ -601,7 +671,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     for (int r = lane; r < rings; r += N) {
       const int s = in.roff[r], e = in.roff[r + 1];
       int root = s;
-      auto is_flat = [&](int v) { return area_at(in.prv[v], v, in.nxt[v]) < kEps; };
+      auto is_flat = [&](int v) { return abs_lt(area_at(in.prv[v], v, in.nxt[v]), kEps); };
       auto remove = [&](int v) {
         if (root == v) {
           root = in.nxt[v];
@@ -674,7 +744,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     s2 = 0.0;
     for (int v = lane; v < verts; v += N) {
       const int r = in.tape[v].w, e = in.roff[r + 1];
-      s2 = dadd(s2, term(v, v + 1 == e ? in.roff[r] : v + 1));
+      s2 = term(s2, v, v + 1 == e ? in.roff[r] : v + 1);
     }
   }
   for (int o = 16; o > 0; o >>= 1) s2 = dadd(s2, __shfl_xor_sync(0xffffffffu, s2, o));

@@ -8,11 +8,45 @@ namespace sbc {
 namespace {
 
 // A vertex as float pairs: hi = x rounded to float, lo = (x - hi) rounded to
-// float, so hi + lo is within 2^-48 |x| of the double.
+// float, so hi + lo is within 2^-48 |x| of the double, and lo has x - hi's
+// sign.  By integer operations (GB300 converts doubles at its FP64 rate)
+// except near the ends of float's range.
+__device__ __forceinline__ float2 float_parts(double x) {
+  const long long u = __double_as_longlong(x);
+  const int e = (int)(u >> 52) & 0x7ff;
+  const unsigned sign = (unsigned)(u >> 32) & 0x80000000u;
+  if (e >= 960 && e < 1150) {
+    const long long m = (u & 0xfffffffffffffll) | 0x10000000000000ll;
+    const int h = (int)((m + (1ll << 28)) >> 29);  // 24 bits, halves up
+    const int rest = (int)(m - ((long long)h << 29));
+    const float lo = __fmul_rn(__int2float_rn(rest), __int_as_float((e - 948) << 23));
+    return make_float2(__uint_as_float(sign | (unsigned)(((e - 896) << 23) + (h - 0x800000))),
+                       __uint_as_float(__float_as_uint(lo) ^ sign));
+  }
+  const float hi = __double2float_rn(x);
+  const double rest = dsub(x, (double)hi);
+  float lo = __double2float_rn(rest);
+  if (lo == 0.f && rest != 0.0) lo = rest > 0.0 ? 1.4e-45f : -1.4e-45f;
+  return make_float2(hi, lo);
+}
 __device__ __forceinline__ float4 float_pair(double x, double y) {
-  const float hx = __double2float_rn(x), hy = __double2float_rn(y);
-  return make_float4(hx, hy, __double2float_rn(dsub(x, (double)hx)),
-                     __double2float_rn(dsub(y, (double)hy)));
+  const float2 a = float_parts(x), b = float_parts(y);
+  return make_float4(a.x, b.x, a.y, b.y);
+}
+
+// hi + lo rounded to a float below (above) it
+__device__ __forceinline__ float parts_below(float hi, float lo) {
+  if (!(lo < 0.f)) return hi;
+  const int u = __float_as_int(hi);
+  return hi == 0.f ? __int_as_float(0x80000001) : __int_as_float(u > 0 ? u - 1 : u + 1);
+}
+__device__ __forceinline__ float parts_above(float hi, float lo) { return -parts_below(-hi, -lo); }
+// the box of the edge between two vertices: low x and y, high x and y
+__device__ __forceinline__ float4 float_box(const float4& a, const float4& b) {
+  return make_float4(fminf(parts_below(a.x, a.z), parts_below(b.x, b.z)),
+                     fminf(parts_below(a.y, a.w), parts_below(b.y, b.w)),
+                     fmaxf(parts_above(a.x, a.z), parts_above(b.x, b.z)),
+                     fmaxf(parts_above(a.y, a.w), parts_above(b.y, b.w)));
 }
 
 __device__ __forceinline__ float vdx(const float4& a, const float4& b) {

@@ -15,6 +15,8 @@ namespace sbc {
 namespace {
 
 struct WarpGroup {
+  // where the warps of a kernel may wait for one another (PhasedWarp)
+  __device__ __forceinline__ void phase() const {}
   static constexpr int N = 32;
   static constexpr int kWarps = 1;
   static constexpr bool kBlock = false;
@@ -59,12 +61,20 @@ struct WarpGroup {
   __device__ __forceinline__ int same(int x) const { return x; }
 };
 
+// A warp whose block's other warps do the same steps on other data: they enter
+// each step together, so that its instructions are fetched once.  (A warp that
+// is done leaves the kernel.)
+struct PhasedWarp : WarpGroup {
+  __device__ __forceinline__ void phase() const { __syncthreads(); }
+};
+
 // A block of T threads (a multiple of 32, at most 1,024).  The collectives
 // alternate between two halves of the scratch words, so one barrier each is
 // enough: a half is written again only after the next collective's barrier,
 // which every reader of it has passed.
 template <int T>
 struct BlockGroup {
+  __device__ __forceinline__ void phase() const {}
   static constexpr int N = T;
   static constexpr int kWarps = T / 32;
   static constexpr bool kBlock = true;

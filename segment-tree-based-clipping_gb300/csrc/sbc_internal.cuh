@@ -60,32 +60,60 @@ __device__ __forceinline__ double area3(double px, double py, double qx, double 
   return dsub(dmul(dsub(qx, px), dsub(ry, py)), dmul(dsub(qy, py), dsub(rx, px)));
 }
 
+// Comparisons of a double by its bits, the same decisions as on the values (a
+// NaN compares false): on GB300 an FP64 compare takes an issue of the FP64
+// pipe, an eighth of the integer rate or less.
+constexpr long long kAbsBits = 0x7fffffffffffffffll, kInfBits = 0x7ff0000000000000ll;
+__device__ __forceinline__ long long abs_bits(double x) { return __double_as_longlong(x) & kAbsBits; }
+__device__ __forceinline__ bool is_pos(double x) {
+  const long long u = __double_as_longlong(x);
+  return u > 0 && u <= kInfBits;
+}
+__device__ __forceinline__ bool is_neg(double x) { return is_pos(-x); }
+// |x| against c > 0
+__device__ __forceinline__ bool abs_lt(double x, double c) { return abs_bits(x) < __double_as_longlong(c); }
+__device__ __forceinline__ bool abs_le(double x, double c) { return abs_bits(x) <= __double_as_longlong(c); }
+__device__ __forceinline__ bool abs_gt(double x, double c) {
+  return abs_bits(x) > __double_as_longlong(c) && abs_bits(x) <= kInfBits;
+}
+// x in (lo, hi), both positive
+__device__ __forceinline__ bool between(double x, double lo, double hi) {
+  const long long u = __double_as_longlong(x);
+  return u > __double_as_longlong(lo) && u < __double_as_longlong(hi);
+}
+// x == y
+__device__ __forceinline__ bool same_value(double x, double y) {
+  const long long u = __double_as_longlong(x), v = __double_as_longlong(y);
+  return (u == v && abs_bits(x) <= kInfBits) || ((u | v) & kAbsBits) == 0;
+}
+
 // Edge-pair classification, lineSegmentIntersection(2)
 // (p_seg_tree/oacc_segment_tree.cpp:5426-5611).  Returns the type 0..8 and
 // the parameters alpha (on P) and beta (on Q).
 __device__ __forceinline__ int seg_isect(double p1x, double p1y, double p2x, double p2y,
                                          double q1x, double q1y, double q2x, double q2y,
                                          double* alpha, double* beta) {
-  double AP1 = area3(p1x, p1y, q1x, q1y, q2x, q2y);
-  double AP2 = area3(p2x, p2y, q1x, q1y, q2x, q2y);
-  double d = dsub(AP1, AP2);
-  if (fabs(d) > kEps) {
-    double AQ1 = area3(q1x, q1y, p1x, p1y, p2x, p2y);
-    double AQ2 = area3(q2x, q2y, p1x, p1y, p2x, p2y);
-    double a = ddiv(AP1, d);
-    double b = ddiv(AQ1, dsub(AQ1, AQ2));
+  // area3's differences, each taken once: those of AQ1 and AQ2 are the same
+  // negated, which changes no product
+  const double x11 = dsub(q1x, p1x), y11 = dsub(q1y, p1y), x21 = dsub(q2x, p1x), y21 = dsub(q2y, p1y);
+  const double x12 = dsub(q1x, p2x), y12 = dsub(q1y, p2y), x22 = dsub(q2x, p2x), y22 = dsub(q2y, p2y);
+  const double AP1 = dsub(dmul(x11, y21), dmul(y11, x21));
+  const double AP2 = dsub(dmul(x12, y22), dmul(y12, x22));
+  const double d = dsub(AP1, AP2);
+  if (abs_gt(d, kEps)) {
+    const double AQ1 = dsub(dmul(x11, y12), dmul(y11, x12));
+    const double AQ2 = dsub(dmul(x21, y22), dmul(y21, x22));
+    const double a = ddiv(AP1, d);
+    const double b = ddiv(AQ1, dsub(AQ1, AQ2));
     *alpha = a;
     *beta = b;
-    bool a01 = false, a0 = false, b01 = false, b0 = false;
-    if (a > kEps && a < 1.0 - kEps) a01 = true;
-    else if (fabs(a) <= kEps) a0 = true;
-    if (b > kEps && b < 1.0 - kEps) b01 = true;
-    else if (fabs(b) <= kEps) b0 = true;
+    const bool a01 = between(a, kEps, 1.0 - kEps), a0 = abs_le(a, kEps);
+    const bool b01 = between(b, kEps, 1.0 - kEps), b0 = abs_le(b, kEps);
     if (a01 && b01) return 1;
     if (a0 && b01) return 2;
     if (b0 && a01) return 3;
     if (a0 && b0) return 4;
-  } else if (fabs(AP1) < kEps) {
+  } else if (abs_lt(AP1, kEps)) {
     double dPx = dsub(p2x, p1x), dPy = dsub(p2y, p1y);
     double dQx = dsub(q2x, q1x), dQy = dsub(q2y, q1y);
     double PQx = dsub(q1x, p1x), PQy = dsub(q1y, p1y);
@@ -112,9 +140,11 @@ __device__ __forceinline__ int seg_isect(double p1x, double p1y, double p2x, dou
 // alphaToInt (oacc_segment_tree.cpp:7247-7252) with the x86-64 truncating
 // conversion: values outside int range become INT_MIN.
 __device__ __forceinline__ int alpha_to_int(double a) {
-  if (a < kEps) return 0;
-  double v = dmul(1000000000.0, a);
-  if (!(v > -2147483649.0 && v < 2147483648.0)) return (int)0x80000000;
+  const long long u = __double_as_longlong(a);
+  if (u < __double_as_longlong(kEps) && (u >= 0 || abs_bits(a) <= kInfBits)) return 0;
+  const double v = dmul(1000000000.0, a);
+  if (!(is_pos(v) && __double_as_longlong(v) < __double_as_longlong(2147483648.0)))
+    return (int)0x80000000;
   return __double2int_rz(v);
 }
 

@@ -111,12 +111,31 @@ __device__ __forceinline__ int pip_step(double x0, double y0, double x1, double 
     const int d = 2 * (ky1 > ky0) - 1;
     if (kx0 >= krx) {
       if (kx1 > krx) return d;
-      if ((area3(x0, y0, x1, y1, rx, ry) > 0) == (ky1 > ky0)) return d;
+      if (is_pos(area3(x0, y0, x1, y1, rx, ry)) == (ky1 > ky0)) return d;
     } else if (kx1 > krx) {
-      if ((area3(x0, y0, x1, y1, rx, ry) > 0) == (ky1 > ky0)) return d;
+      if (is_pos(area3(x0, y0, x1, y1, rx, ry)) == (ky1 > ky0)) return d;
     }
   }
   return 0;
+}
+
+// pip_step without its FP64: the step, or *area set where the orientation
+// decides between this step and none (pip_decide)
+__device__ __forceinline__ int pip_quick(double x0, double y0, double x1, double y1, double rx,
+                                         double ry, bool* area) {
+  const long long ky0 = okey(y0), ky1 = okey(y1), kry = okey(ry);
+  *area = false;
+  if ((ky0 < kry) == (ky1 < kry)) return 0;
+  const long long kx0 = okey(x0), kx1 = okey(x1), krx = okey(rx);
+  const int d = 2 * (ky1 > ky0) - 1;
+  if (kx0 >= krx && kx1 > krx) return d;
+  *area = kx0 >= krx || kx1 > krx;
+  return 0;
+}
+__device__ __forceinline__ int pip_decide(double x0, double y0, double x1, double y1, double rx,
+                                          double ry) {
+  const bool up = okey(y1) > okey(y0);
+  return is_pos(area3(x0, y0, x1, y1, rx, ry)) == up ? 2 * up - 1 : 0;
 }
 
 // Whether an edge with end heights y0 and y1, or any piece of it between two

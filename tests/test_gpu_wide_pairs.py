@@ -375,3 +375,24 @@ def test_device_arrays_aligned_to_a_double(clipper):
             assert np.abs(x - y).max() <= 1e-13 * np.abs(x).max()
         else:
             assert np.array_equal(x, y), i
+
+
+@pytest.mark.parametrize("sy", [1e-25, 1e-3, 1e12, 1e37, 1e39, 1e42])
+def test_heights_near_and_beyond_float(mode, sy):
+    """Heights at the ends of float's range and past it, where the float tests
+    must keep every candidate: rings as the oracle's."""
+    cl, union = mode
+    scale = np.array([1.0, sy])
+    pairs = [(gen.star(n, 20 + n, R=100.0) * scale, gen.star(m, 30 + m, centre=(7.0, 3.0), R=90.0) * scale)
+             for n, m in ((9, 7), (40, 33), (200, 150), (700, 300))]
+    pairs += [(b, c * np.array([1.0, -1e-6])) for b, c in pairs]
+    for clip in (lambda: cl.clip_batch([b for b, _ in pairs], [c for _, c in pairs]),
+                 lambda: [sum(x, []) for x in zip(*[tuple(map(list, cl.clip_pairwise(b, [c]))) for b, c in pairs])]):
+        rings, status = clip()
+        for (b, c), got, st in zip(pairs, rings, status):
+            try:
+                ref = want(b, c, union)
+            except oracle_py.OracleError:
+                assert st != 0
+                continue
+            assert st == 0 and rings_equal(got, ref)
