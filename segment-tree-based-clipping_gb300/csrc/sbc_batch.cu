@@ -2154,49 +2154,6 @@ __global__ void k_batch_pack(int np, const long long* __restrict__ boff,
   for (int i = lane; i < 2 * nv; i += 32) xy[2 * v0 + i] = w.rxy[i];
 }
 
-// The gradient (gx, gy) of a crossing's coordinates chained to the ends of its
-// edges b1b2 and c1c2: I = (1 - alpha) b1 + alpha b2, alpha = A1 / (A1 - A2),
-// A1 = A(b1, c1, c2), A2 = A(b2, c1, c2); A(P, Q, R) partials: dP = (Qy - Ry,
-// Rx - Qx), dQ = (Ry - Py, Px - Rx), dR = (Py - Qy, Qx - Px)
-// One reciprocal and explicit fused multiply-adds: the FP64 rate bounds the
-// backward pass, and three divisions without fma took about twice as many
-// operations.
-struct CrossGrad {
-  double gx, gy, al, k1, k2;
-  double2 b1c1, b1c2, b2c1, b2c2, c12;  // c1 - b1, c2 - b1, c1 - b2, c2 - b2, c1 - c2
-  __device__ __forceinline__ CrossGrad(const double* b, int i1, int i2, const double* c, int j1,
-                                       int j2, double gx_, double gy_)
-      : gx(gx_), gy(gy_) {
-    const double b1x = b[2 * i1], b1y = b[2 * i1 + 1], b2x = b[2 * i2], b2y = b[2 * i2 + 1];
-    const double c1x = c[2 * j1], c1y = c[2 * j1 + 1], c2x = c[2 * j2], c2y = c[2 * j2 + 1];
-    b1c1 = make_double2(c1x - b1x, c1y - b1y);
-    b1c2 = make_double2(c2x - b1x, c2y - b1y);
-    b2c1 = make_double2(c1x - b2x, c1y - b2y);
-    b2c2 = make_double2(c2x - b2x, c2y - b2y);
-    c12 = make_double2(c1x - c2x, c1y - c2y);
-    const double A1 = fma(b1c1.x, b1c2.y, -(b1c1.y * b1c2.x));
-    const double A2 = fma(b2c1.x, b2c2.y, -(b2c1.y * b2c2.x));
-    const double d = A1 - A2, r = 1.0 / d, q = A1 * r;
-    al = fma(fma(-q, d, A1), r, q);  // A1 / d, corrected once
-    const double ga = fma(gx, b2x - b1x, gy * (b2y - b1y)) * r * r;  // dA/dalpha / d^2
-    k1 = -A2 * ga;  // dalpha/dA1
-    k2 = A1 * ga;   // dalpha/dA2
-  }
-  __device__ __forceinline__ double2 b1() const {
-    const double u = 1.0 - al;
-    return make_double2(fma(k1, c12.y, u * gx), fma(-k1, c12.x, u * gy));
-  }
-  __device__ __forceinline__ double2 b2() const {
-    return make_double2(fma(k2, c12.y, al * gx), fma(-k2, c12.x, al * gy));
-  }
-  __device__ __forceinline__ double2 c1() const {
-    return make_double2(fma(k1, b1c2.y, k2 * b2c2.y), -fma(k1, b1c2.x, k2 * b2c2.x));
-  }
-  __device__ __forceinline__ double2 c2() const {
-    return make_double2(-fma(k1, b1c1.y, k2 * b2c1.y), fma(k1, b1c1.x, k2 * b2c1.x));
-  }
-};
-
 struct BackArgs {
   int np;
   const int* wide;
