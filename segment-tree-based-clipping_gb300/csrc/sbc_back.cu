@@ -946,6 +946,77 @@ static int serial_backend(Pipeline& pl, const Merged& m, OverlayOut& out, int ta
   return kOk;
 }
 
+// cleanUpResult2 (foster/polyclip.h:767-787) on the rings of `out`, and
+// compaction into the overlay's output buffers (which `out` must not be in).
+// The counts land with the caller's next wait on the stream.
+int clean_up_rings(Pipeline& pl, OverlayOut& out) {
+  BufferPool& bp = pl.pool();
+  HostReads& rd = pl.reads();
+  cudaStream_t st = pl.stream();
+  const int ovTag = (int)(&out - &pl.outputs()[0]);
+  const std::string tg = std::to_string(ovTag);
+  const int nR = out.nrings;
+  const long long nv = out.nverts;
+  int* ringOf = (int*)bp.get("cl_ringOf", sizeof(int) * (nv + 1));
+  int* ringFlag = (int*)bp.get("cl_flag", sizeof(int) * (nR + 1));
+  int* nxt = (int*)bp.get("cl_next", sizeof(int) * (nv + 1));
+  int* prv = (int*)bp.get("cl_prev", sizeof(int) * (nv + 1));
+  int* keep = (int*)bp.get("cl_keep", sizeof(int) * (nv + 1));
+  int* flagV = (int*)bp.get("cl_flagV", sizeof(int) * (nv + 1));
+  int* flist = (int*)bp.get("cl_flist", sizeof(int) * (nv + 1));
+  int* rpre = (int*)bp.get("cl_rpre", sizeof(int) * (nR + 2));
+  int* ooff = (int*)bp.get("ring_off_" + tg, sizeof(int) * (nR + 2));
+  double* oxy = (double*)bp.get("ring_xy_" + tg, sizeof(double) * 2 * (nv + 1));
+  void* sscr = bp.get_zeroed("cl_scan", scan_scratch_bytes(nv + nR + 4), st);
+  if (bp.failed) return pl.fail(kENoMem, "device allocation failed (clean-up)");
+  cudaMemsetAsync(ringFlag, 0, sizeof(int) * (nR + 1), st);
+  if (nv > 0) {
+    ::sbc::KProbe kp_("k_ring_of", st);
+    k_ring_of<<<grid_for(nv, 256), 256, 0, st>>>(nv, nR, out.d_off, ringOf);
+  }
+  {
+    ::sbc::KProbe kp_("k_collinear", st);
+    k_collinear<<<grid_for(nv + 1, 256), 256, 0, st>>>(nv, out.d_off, ringOf, out.d_xy, ringFlag,
+                                                      keep, flagV, nxt, prv);
+  }
+  exclusive_scan_i32(flagV, nv + 1, sscr, st, true);
+  // the flagged-vertex count stays on the device (flagV[nv]); rings
+  // without a flagged vertex leave k_cleanup_ring at once
+  if (nv > 0) {
+    {
+      ::sbc::KProbe kp_("k_flag_list", st);
+      k_flag_list<<<grid_for(nv, 256), 256, 0, st>>>(nv, flagV, flist);
+    }
+    ::sbc::KProbe kp_("k_cleanup_ring", st);
+    k_cleanup_ring<<<grid_for(nR, 128), 128, 0, st>>>(nR, out.d_off, ringFlag, flist,
+                                                    flagV + nv, out.d_xy, nxt, prv, keep);
+  }
+  int* kpv = keep;  // exclusive prefix of the keep flags (nv+1 entries)
+  exclusive_scan_i32(kpv, nv + 1, sscr, st, true);
+  {
+    ::sbc::KProbe kp_("k_ring_nonempty", st);
+    k_ring_nonempty<<<grid_for(nR + 1, 128), 128, 0, st>>>(nR, out.d_off, kpv, rpre);
+  }
+  exclusive_scan_i32(rpre, nR + 1, sscr, st, true);
+  if (nv > 0) {
+    ::sbc::KProbe kp_("k_compact_xy", st);
+    k_compact_xy<<<grid_for(nv, 256), 256, 0, st>>>(nv, kpv, out.d_xy, oxy);
+  }
+  {
+    ::sbc::KProbe kp_("k_compact_off", st);
+    k_compact_off<<<grid_for(nR + 1, 128), 128, 0, st>>>(nR, nv, out.d_off, kpv, rpre, ooff);
+  }
+  // the two counts land with the caller's next wait on the stream
+  // (Pipeline::finish_counts); both sit in one host word of this overlay
+  int* hh = (int*)rd.word(HostReads::kCounts + ovTag);
+  cudaMemcpyAsync(hh, rpre + nR, sizeof(int), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(hh + 1, kpv + nv, sizeof(int), cudaMemcpyDeviceToHost, st);
+  out.counts = hh;
+  out.d_off = ooff;
+  out.d_xy = oxy;
+  return kOk;
+}
+
 int run_backend(Pipeline& pl, const Merged& m, OverlayOut& out) {
   cudaStream_t st = pl.stream();
   BufferPool& bp = pl.pool();
@@ -1200,69 +1271,7 @@ int run_backend(Pipeline& pl, const Merged& m, OverlayOut& out) {
     out.nverts = nv;
   }
 
-  // ---- clean-up and compaction
-  {
-    const int nR = out.nrings;
-    const long long nv = out.nverts;
-    int* ringOf = (int*)bp.get("cl_ringOf", sizeof(int) * (nv + 1));
-    int* ringFlag = (int*)bp.get("cl_flag", sizeof(int) * (nR + 1));
-    int* nxt = (int*)bp.get("cl_next", sizeof(int) * (nv + 1));
-    int* prv = (int*)bp.get("cl_prev", sizeof(int) * (nv + 1));
-    int* keep = (int*)bp.get("cl_keep", sizeof(int) * (nv + 1));
-    int* flagV = (int*)bp.get("cl_flagV", sizeof(int) * (nv + 1));
-    int* flist = (int*)bp.get("cl_flist", sizeof(int) * (nv + 1));
-    int* rpre = (int*)bp.get("cl_rpre", sizeof(int) * (nR + 2));
-    int* ooff = (int*)bp.get("ring_off_" + tg, sizeof(int) * (nR + 2));
-    double* oxy = (double*)bp.get("ring_xy_" + tg, sizeof(double) * 2 * (nv + 1));
-    void* sscr = bp.get_zeroed("cl_scan", scan_scratch_bytes(nv + nR + 4), st);
-    if (bp.failed) return pl.fail(kENoMem, "device allocation failed (clean-up)");
-    cudaMemsetAsync(ringFlag, 0, sizeof(int) * (nR + 1), st);
-    if (nv > 0) {
-      ::sbc::KProbe kp_("k_ring_of", st);
-      k_ring_of<<<grid_for(nv, 256), 256, 0, st>>>(nv, nR, out.d_off, ringOf);
-    }
-    {
-      ::sbc::KProbe kp_("k_collinear", st);
-      k_collinear<<<grid_for(nv + 1, 256), 256, 0, st>>>(nv, out.d_off, ringOf, out.d_xy, ringFlag,
-                                                        keep, flagV, nxt, prv);
-    }
-    exclusive_scan_i32(flagV, nv + 1, sscr, st, true);
-    // the flagged-vertex count stays on the device (flagV[nv]); rings
-    // without a flagged vertex leave k_cleanup_ring at once
-    if (nv > 0) {
-      {
-        ::sbc::KProbe kp_("k_flag_list", st);
-        k_flag_list<<<grid_for(nv, 256), 256, 0, st>>>(nv, flagV, flist);
-      }
-      ::sbc::KProbe kp_("k_cleanup_ring", st);
-      k_cleanup_ring<<<grid_for(nR, 128), 128, 0, st>>>(nR, out.d_off, ringFlag, flist,
-                                                      flagV + nv, out.d_xy, nxt, prv, keep);
-    }
-    int* kpv = keep;  // exclusive prefix of the keep flags (nv+1 entries)
-    exclusive_scan_i32(kpv, nv + 1, sscr, st, true);
-    {
-      ::sbc::KProbe kp_("k_ring_nonempty", st);
-      k_ring_nonempty<<<grid_for(nR + 1, 128), 128, 0, st>>>(nR, out.d_off, kpv, rpre);
-    }
-    exclusive_scan_i32(rpre, nR + 1, sscr, st, true);
-    if (nv > 0) {
-      ::sbc::KProbe kp_("k_compact_xy", st);
-      k_compact_xy<<<grid_for(nv, 256), 256, 0, st>>>(nv, kpv, out.d_xy, oxy);
-    }
-    {
-      ::sbc::KProbe kp_("k_compact_off", st);
-      k_compact_off<<<grid_for(nR + 1, 128), 128, 0, st>>>(nR, nv, out.d_off, kpv, rpre, ooff);
-    }
-    // the two counts land with the caller's next wait on the stream
-    // (Pipeline::finish_counts); both sit in one host word of this overlay
-    int* hh = (int*)rd.word(HostReads::kCounts + ovTag);
-    cudaMemcpyAsync(hh, rpre + nR, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(hh + 1, kpv + nv, sizeof(int), cudaMemcpyDeviceToHost, st);
-    out.counts = hh;
-    out.d_off = ooff;
-    out.d_xy = oxy;
-  }
-  return kOk;
+  return clean_up_rings(pl, out);
 }
 
 }  // namespace sbc

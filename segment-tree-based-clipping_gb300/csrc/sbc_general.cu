@@ -2,8 +2,7 @@
 // over the whole GPU, straight from the exact stage's hits to rings.
 //
 // The same observation as sbc_clean.cuh, for the pair pipeline: where every
-// hit is a proper crossing labelled a crossing, and no result vertex lies in
-// line with its neighbours, the merged arrays, labels and linked lists
+// hit is a proper crossing labelled a crossing, the merged arrays, labels and linked lists
 // (src/clip.cpp:368-695, foster/polyclip.h:337-787) say no more than the order
 // of the crossings along each polygon.  Crossings are ranked along both
 // polygons (counting sort by edge, alpha order per edge); entry and exit
@@ -13,6 +12,8 @@
 // read, where the stages that build the arrays take 65 launches, 25 memsets
 // and four host reads.  A pair that fails a test takes those stages, from the
 // same hits; so does a request for their arrays (Pipeline::build_records).
+// Where a result vertex may lie in line with its neighbours the clean-up
+// kernels of the list-ranking back end follow (clean_up_rings).
 //
 // Bound by dependent gathers over the crossings (a few hundred bytes each,
 // L2-resident) and, below some 10,000 vertices, by the launches.  A clip
@@ -47,7 +48,7 @@ struct Gp {
   double2* xy;
   int4 *A, *B;
   int* wind;      // winding number of the base's first vertex in the overlay, and the reverse
-  unsigned* bad;  // not in general position
+  unsigned* bad;  // 1: not in general position, 2: a vertex in line with its neighbours
   int* longs;     // edges with many crossings (base edges, then nb + overlay edges)
   unsigned* nlong;
   __device__ int cedge(int h) const { return (rc[h] >> 1) - cStart; }
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(256) k_gp_legs(Gp g) {
     if (right(qm) == right(qp)) bad = true;
     const GpLeg p = gp_leg(g, 0, inP, k), own = gp_leg(g, 1, inQ, m);
     // its neighbours in the result: along each polygon in the leg's direction
-    if (gp_flat(p.fwd ? pp : pm, v, own.fwd ? qp : qm)) bad = true;
+    if (gp_flat(p.fwd ? pp : pm, v, own.fwd ? qp : qm)) atomicOr(g.bad, 2u);
     if (bad) *g.bad = 1u;
     const GpLeg q = gp_leg(g, 1, inQ, g.rQ[g.hP[p.to]]);
     g.A[k] = make_int4(g.rP[g.hQ[q.to]], k, 0, p.cnt + q.cnt + 2);
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(256) k_gp_legs(Gp g) {
   const int pe = u == 0 ? n - 1 : u - 1, ps = pe == 0 ? 0 : end[pe - 1], pt = end[pe];
   const double2 prev = pt > ps ? g.xy[hs[pt - 1]] : p[pe];
   const double2 next = end[u] > s ? g.xy[hs[s]] : p[u + 1];
-  if (gp_flat(prev, p[u], next)) *g.bad = 1u;
+  if (gp_flat(prev, p[u], next)) atomicOr(g.bad, 2u);
 }
 
 // One doubling round over this thread's crossings: x = (next, least crossing
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(256) k_gp_whole(Gp g, int* __restrict__ cnt, i
     const int u = base ? x : x - n0, n = base ? g.nb : g.nc;
     const double2* p = (const double2*)(base ? g.b : g.c);
     out[x] = p[u];
-    if (gp_flat(p[u == 0 ? n - 1 : u - 1], p[u], p[u + 1])) *g.bad = 1u;
+    if (gp_flat(p[u == 0 ? n - 1 : u - 1], p[u], p[u + 1])) atomicOr(g.bad, 2u);
   }
 }
 
@@ -684,7 +685,7 @@ int Pipeline::stage_general(int cType, const int* rb, const int* rc, const int* 
   }
   const unsigned* r_bad = rd_.get(g.bad, HostReads::kBack, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) return fail(kECuda, "general position");
-  if (*r_bad) return kOk;
+  if (*r_bad & 1u) return kOk;
   out.unique = K;
   out.slots_b = nb + (long long)K;
   out.slots_c = nc + (long long)K;
@@ -703,7 +704,16 @@ int Pipeline::stage_general(int cType, const int* rb, const int* rc, const int* 
   dbg_isxy = (double*)g.xy;
   lazy_ = {cType, rb, rc, rt, rkey, nhits};
   *done = true;
-  return kOk;
+  if (*r_bad == 0u || out.nverts == 0) return kOk;
+  // some ring may lose vertices: from a copy into the same buffers
+  int* roff = (int*)pool_.get("gp_roff", sizeof(int) * ((size_t)out.nrings + 1));
+  auto* rxy = (double2*)pool_.get("gp_rxy", sizeof(double2) * (size_t)out.nverts);
+  if (pool_.failed) return fail(kENoMem, "device allocation failed (general position)");
+  cudaMemcpyAsync(roff, ooff, sizeof(int) * ((size_t)out.nrings + 1), cudaMemcpyDeviceToDevice, st);
+  cudaMemcpyAsync(rxy, oxy, sizeof(double2) * (size_t)out.nverts, cudaMemcpyDeviceToDevice, st);
+  out.d_off = roff;
+  out.d_xy = (double*)rxy;
+  return clean_up_rings(*this, out);
 }
 
 }  // namespace sbc

@@ -333,6 +333,7 @@ struct Merged {
   const double* cP;    // overlays with closing vertices
 };
 int run_backend(Pipeline& pl, const Merged& m, OverlayOut& out);
+int clean_up_rings(Pipeline& pl, OverlayOut& out);
 
 // Many independent pairs (sbc_batch.cu): pairs whose polygons have at most
 // SBC_BATCH_MAX_VERTICES vertices one device thread each, in chunks whose

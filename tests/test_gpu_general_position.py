@@ -116,3 +116,42 @@ def test_more_hits_than_the_first_guess(clipper):
             assert rings_equal(cl.clip_pair(b, c), ref)
     finally:
         cl.close()
+
+
+@pytest.mark.parametrize("union", [False, True], ids=["intersection", "union"])
+@pytest.mark.parametrize("n", [12, 300, 3000])
+def test_result_vertices_in_line(n, union):
+    """Vertices in line with their neighbours, which the clean-up removes: one
+    on an edge, on every edge, two and three in a row, the first vertex, a ring
+    that is a sliver; with crossings, without any, one tree over several
+    overlays.  Rings as the oracle's."""
+    from test_gpu_wide_pairs import with_points
+    cl = sbclip.Clipper(0, union=union)
+    try:
+        b = gen.star(n, 1210 + n, R=50.0)
+        pairs = []
+        for k, (edges, where) in enumerate((((1,), (0.4,)), (range(n), (0.5,)), ((2, 7), (0.3, 0.8)),
+                                            ((0, n - 1), (0.2, 0.5, 0.9)))):
+            c = gen.star(n + 3 - k, 1300 + n + k, centre=(4.1 + k, -2.3), R=45.0)
+            pairs += [(with_points(b, edges, where), c), (b, with_points(c, edges, where)),
+                      (np.roll(with_points(b, edges, where), 2, axis=0), with_points(c, edges, where)),
+                      (with_points(b, edges, where), c + [400.0, 0.0]),
+                      (with_points(b, edges, where), (c - [4.1 + k, -2.3]) * 0.01 + [0.3, 0.2])]
+        v, w = b[3], b[4]
+        t = (w - v) / np.hypot(*(w - v))
+        inward = np.array([-t[1], t[0]])
+        tip = (v + w) / 2 + 2e-6 * inward
+        pairs.append((b, np.array([tip, tip - inward * 30.0 + 0.1 * t, tip - inward * 29.0 - 0.2 * t])))
+        for x, c in pairs:
+            try:
+                ref = oracle_py.rings_of(oracle_py.clip(x, [c], union=union)["overlays"][0])
+            except oracle_py.OracleError:
+                continue
+            assert rings_equal(cl.clip_pair(x, c), ref)
+        if not union:
+            ovs = [c for _, c in pairs[:4]]
+            got = cl.clip(pairs[0][0], ovs)
+            for g, o in zip(got, oracle_py.clip(pairs[0][0], ovs)["overlays"]):
+                assert rings_equal(g, oracle_py.rings_of(o))
+    finally:
+        cl.close()
