@@ -182,7 +182,11 @@ KERNEL_BOUND = {
     "k_lr_jump_coop": "latency", "k_tr_jump_coop": "latency",
     "k_grid_scatter": "hbm", "k_edge_fbox": "hbm", "k_copy_runs": "hbm",
     "k_pair_exact": "fp64", "k_pw_cand_test": "fp64", "k_batch_cand": "fp64",
-    "k_batch_cand_sweep": "fp64", "k_labels": "fp64", "k_batch_backward": "fp64",
+    "k_batch_cand_wide": "fp64", "k_labels": "fp64", "k_batch_backward": "fp64",
+    "k_batch_backward_wide": "fp64", "k_batch_clean": "fp64", "k_batch_clean_wide": "fp64",
+    "k_pw_clean": "fp64", "k_pw_clean_wide": "fp64", "k_pw_clean_huge": "latency",
+    "k_pw_overlay_prep": "latency", "k_pw_hit_tree": "latency", "k_batch_front_wide": "latency",
+    "k_gp_legs": "fp64", "k_gp_jump_coop": "latency", "k_direct_exact": "latency",
     "k_grid_warp": "latency", "k_grid_small": "latency", "k_lr_jump": "latency",
     "k_tr_jump": "latency", "k_alpha_sort": "latency", "k_batch_back": "latency",
     "k_batch_front": "latency", "k_pw_pairs": "latency", "k_pw_pairs_lists": "latency",
@@ -196,19 +200,21 @@ KERNEL_BOUND = {
 # kernel applies), keyed (kernel, workload).
 _BATCH_NCU = "profiles/k_batch_small_pairs_8192.md (8,192 pairs, the same kernel)"
 PIPES = {
-    ("k_batch_pw2", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 11.0, "warps_active_pct": 27.1, "issue_active_pct": 28.3,
-        "stall_cycles_per_issue": {"long_scoreboard": 7.0, "no_instruction": 3.3, "wait": 2.9},
+    ("k_batch_clean", "small_pairs_65536"): {
+        "fp64_pipe_pct_active": 54.8, "warps_active_pct": 27.9, "issue_active_pct": 27.6,
+        "stall_cycles_per_issue": {"long_scoreboard": 2.8, "no_instruction": 0.7, "wait": 3.4},
         "source": _BATCH_NCU},
-    ("k_batch_pw", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 27.4, "warps_active_pct": 29.0, "issue_active_pct": 29.2,
-        "stall_cycles_per_issue": {"long_scoreboard": 5.8, "no_instruction": 3.9, "wait": 3.5},
+    ("k_batch_cand", "small_pairs_65536"): {
+        "fp64_pipe_pct_active": 23.7, "warps_active_pct": 39.3, "issue_active_pct": 29.3,
+        "stall_cycles_per_issue": {"long_scoreboard": 6.2, "no_instruction": 0.3, "wait": 3.5},
         "source": _BATCH_NCU},
     ("k_batch_front", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 18.4, "warps_active_pct": 32.4, "issue_active_pct": 44.4,
+        "fp64_pipe_pct_active": 29.5, "warps_active_pct": 36.1, "issue_active_pct": 50.9,
+        "stall_cycles_per_issue": {"long_scoreboard": 1.8, "no_instruction": 0.9, "wait": 2.7},
         "source": _BATCH_NCU},
     ("k_batch_backward", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 75.2, "warps_active_pct": 22.7, "issue_active_pct": 14.6,
+        "fp64_pipe_pct_active": 68.6, "warps_active_pct": 39.8, "issue_active_pct": 18.8,
+        "stall_cycles_per_issue": {"long_scoreboard": 5.7, "no_instruction": 0.3, "wait": 4.0},
         "source": _BATCH_NCU},
 }
 

@@ -150,10 +150,11 @@ int sbc_classify_pairs(sbc_ctx* ctx, const double* pairs, int n, int* types, dou
  * per pair; the reference itself has no batched call).  Polygons are
  * concatenated: pair p's base is vertices [b_off[p], b_off[p+1]) of b_xy, its
  * overlay vertices [c_off[p], c_off[p+1]) of c_xy.  A pair whose polygons
- * have at most SBC_BATCH_MAX_VERTICES vertices is clipped by one device
- * thread, all such pairs in one launch per chunk (consecutive pairs whose
- * scratch arenas fit the budget, sbc_batch_set_arena_budget); a pair with a
- * larger polygon is clipped by the single-pair pipeline.  A polygon needs at
+ * have at most SBC_BATCH_MAX_VERTICES vertices is clipped by one warp or, if
+ * it is large, one thread block, all such pairs in the same launches per chunk
+ * (consecutive pairs whose scratch arenas fit the budget,
+ * sbc_batch_set_arena_budget); a pair with a larger polygon is clipped by the
+ * single-pair pipeline.  A polygon needs at
  * least 3 vertices; a pair with a smaller one gets status SBC_EINPUT and no
  * rings.  Per-pair failures (SBC_EUNDEF where the reference's behaviour is
  * undefined) are reported in the per-pair status; the call itself fails only
@@ -305,12 +306,13 @@ int sbc_pairwise_info(const sbc_ctx* ctx, long long* out, int n);
  * 1.  A tuning knob: results do not depend on it. */
 int sbc_pairwise_set_cell_factor(sbc_ctx* ctx, double factor);
 /* Overlays with at least `records` intersecting edge pairs leave the
- * one-warp-per-pair back end for the data-parallel one (several such overlays
- * at a time, each on its own stream); default 8192.  A tuning knob: results
- * do not depend on it. */
+ * warp- or block-per-pair back end for the data-parallel one (several such
+ * overlays at a time, each on its own stream), and a few of those that are not
+ * in general position from an eighth of that on; default 32768.  A tuning
+ * knob: results do not depend on it. */
 int sbc_pairwise_set_split(sbc_ctx* ctx, int records);
 /* Host worker threads (each with its own stream) that clip the big overlays
- * concurrently with the one-warp-per-pair kernel; default 8, 1 to 64.  A
+ * concurrently with the per-pair kernels; default 8, 1 to 64.  A
  * tuning knob: results do not depend on it (1 serialises the big overlays,
  * which per-kernel profiling needs).  sbc_pairwise_get_workers reads it. */
 int sbc_pairwise_set_workers(sbc_ctx* ctx, int workers);

@@ -1,15 +1,18 @@
 // sbc_batch.cu -- many small independent base/overlay pairs in one launch,
 // and the area of their intersections with its gradient.
 //
-// One device thread clips one pair with the same rules as the pair pipeline
-// (rows A1-A18 of the reference, multicore_clipping src/clip.cpp:1415-2115),
-// in order, over a private scratch arena: the elementary intervals and their
-// quirks, the border search, each edge's leaf range and end leaves, the
-// candidate pairs with their first-emission keys (all base x overlay edge
-// pairs are tested: small pairs need no grid), the unique records, per-edge
-// counts, alpha order, merged arrays, initial labels, and the exact
-// linked-list back end (sbc_serial.cuh).  Results are those of
-// sbc_clip_pair for every pair.
+// A warp (small pairs) or a block (wide ones) clips one pair with the same
+// rules as the pair pipeline (rows A1-A18 of the reference,
+// multicore_clipping src/clip.cpp:1415-2115), in order, over a private scratch
+// arena: each edge's leaf range and end leaves, from vertex ranks or from the
+// elementary intervals with their quirks and the border search; the candidate
+// pairs with their first-emission keys (all base x overlay edge pairs are
+// tested: no grid); then the rings straight from the hits (sbc_clean.cuh) or,
+// for a pair that is not in general position, the unique records, per-edge
+// counts, alpha order, merged arrays, initial labels and linked lists
+// (sbc_pwpair.cuh, and the exact back end of sbc_serial.cuh, one thread per
+// pair, for what that does not follow).  Results are those of sbc_clip_pair
+// for every pair.
 //
 // Area and gradient.  The area of a pair is the sum of the shoelace areas of
 // its rings.  Every ring vertex is a copy of a merged slot (base slots are

@@ -31,8 +31,10 @@
 // covers; a base edge is tested in the cell holding the low corner of the two
 // boxes' overlap only, so every box-overlapping pair is tested once.
 //
-// Back end: one warp per pair runs rows A9-A18 (src/clip.cpp:368-695,
-// foster/polyclip.h:337-787), its lanes sharing the per-record, per-run and
+// Back end: a pair in general position goes from its hits to rings without
+// lists (sbc_clean.cuh), on a warp or a block.  For the others a warp or a
+// block runs rows A9-A18 (src/clip.cpp:368-695, foster/polyclip.h:337-787),
+// its lanes sharing the per-record, per-run and
 // per-slot steps, with the overlay's merged arrays in full and the
 // base's only where intersections are: the base's merged list holds ~n_b
 // plain vertices per pair, so its linked list is built with run nodes (a
