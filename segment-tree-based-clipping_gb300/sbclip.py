@@ -126,9 +126,11 @@ class _PairwiseJob(ctypes.Structure):
 
 def pack_polygons(polys):
     """Concatenate polygons: (xy (n,2) float64, offsets (len+1,) int64)."""
-    arrs = [np.ascontiguousarray(p, dtype=np.float64).reshape(-1, 2) for p in polys]
+    f64 = np.dtype(np.float64)
+    arrs = [p if type(p) is np.ndarray and p.dtype is f64 and p.ndim == 2 and p.shape[1] == 2 else
+            np.ascontiguousarray(p, dtype=np.float64).reshape(-1, 2) for p in polys]
     off = np.zeros(len(arrs) + 1, dtype=np.int64)
-    off[1:] = np.cumsum([a.shape[0] for a in arrs])
+    off[1:] = np.cumsum([len(a) for a in arrs])
     xy = np.ascontiguousarray(np.concatenate(arrs, axis=0)) if arrs else np.zeros((0, 2))
     return xy, off
 
@@ -256,11 +258,11 @@ def _rings_from(r: _Rings):
     n = r.nrings
     if n <= 0:
         return []
-    off = np.ctypeslib.as_array(ctypes.cast(r.offsets, ctypes.POINTER(ctypes.c_int)), (n + 1,)).copy()
+    off = np.ctypeslib.as_array(ctypes.cast(r.offsets, ctypes.POINTER(ctypes.c_int)), (n + 1,)).tolist()
     nv = int(r.nverts)
     xy = np.ctypeslib.as_array(ctypes.cast(r.xy, ctypes.POINTER(ctypes.c_double)), (2 * nv,)).copy()
     xy = xy.reshape(-1, 2)
-    return [xy[off[j]:off[j + 1]] for j in range(n)]
+    return [xy[i:j] for i, j in zip(off, off[1:])]
 
 
 class Clipper:
@@ -358,20 +360,7 @@ class Clipper:
         b, keep = self._batch(bases, overlays)
         r = _BatchRings()
         self._check(self._L.sbc_clip_batch(self._h, ctypes.byref(b), ctypes.byref(r), stream))
-        np_ = len(bases)
-        pr = np.ctypeslib.as_array(ctypes.cast(r.pair_ring, ctypes.POINTER(ctypes.c_longlong)),
-                                   (np_ + 1,)).copy()
-        ro = np.ctypeslib.as_array(ctypes.cast(r.ring_off, ctypes.POINTER(ctypes.c_longlong)),
-                                   (int(r.nrings) + 1,)).copy()
-        xy = (np.ctypeslib.as_array(ctypes.cast(r.xy, ctypes.POINTER(ctypes.c_double)),
-                                    (2 * int(r.nverts),)).copy().reshape(-1, 2)
-              if r.nverts > 0 else np.zeros((0, 2)))
-        st = np.ctypeslib.as_array(ctypes.cast(r.status, ctypes.POINTER(ctypes.c_int)),
-                                   (np_,)).copy() if np_ else np.zeros(0, np.int32)
-        out = []
-        for p in range(np_):
-            out.append([xy[ro[q]:ro[q + 1]] for q in range(pr[p], pr[p + 1])])
-        return out, st
+        return self._unpack_rings(r, len(bases))
 
     def clip_components(self, base, overlay, stream: int | None = None):
         """Rings of one pair of multi-component polygons (lists of component
@@ -419,15 +408,18 @@ class Clipper:
     @staticmethod
     def _unpack_rings(r, np_):
         pr = np.ctypeslib.as_array(ctypes.cast(r.pair_ring, ctypes.POINTER(ctypes.c_longlong)),
-                                   (np_ + 1,)).copy()
+                                   (np_ + 1,))
         ro = np.ctypeslib.as_array(ctypes.cast(r.ring_off, ctypes.POINTER(ctypes.c_longlong)),
-                                   (int(r.nrings) + 1,)).copy()
+                                   (int(r.nrings) + 1,))
         xy = (np.ctypeslib.as_array(ctypes.cast(r.xy, ctypes.POINTER(ctypes.c_double)),
                                     (2 * int(r.nverts),)).copy().reshape(-1, 2)
               if r.nverts > 0 else np.zeros((0, 2)))
         st = np.ctypeslib.as_array(ctypes.cast(r.status, ctypes.POINTER(ctypes.c_int)),
                                    (np_,)).copy() if np_ else np.zeros(0, np.int32)
-        return [[xy[ro[q]:ro[q + 1]] for q in range(pr[p], pr[p + 1])] for p in range(np_)], st
+        # (slices by Python ints over lists: half the time of numpy scalars)
+        ro, pr = ro.tolist(), pr.tolist()
+        rings = [xy[i:j] for i, j in zip(ro, ro[1:])]
+        return [rings[i:j] for i, j in zip(pr, pr[1:])], st
 
     def clip_pairwise(self, base, overlays, stream: int | None = None):
         """`seg base overlay_i` for every overlay: (list of ring lists, status array)."""
