@@ -156,11 +156,17 @@ __device__ void pw_edge_tree(const PwTree& T, int rs, double s, int re, double e
   const int L = T.L, epc = T.epc;
   auto J = [&](int m) { return m < T.z ? m : (m == T.z ? epc - 1 : m - 1); };
   auto eqnext = [&](int i) { return i >= T.count - 1; };  // ea[i] == ea[i+1]
+  // findBoarder's search meets the never-written slot 0 only on its way to the
+  // first two positions, and finds any other single position where it is
+  // (k_pw_hit_tree, 5 M hits: 1.05 ms with the four searches of each, 0.43 so)
+  auto border = [&](int x, int y, double q) {
+    return T.z == 0 && x >= 2 && y == x + 1 ? x : border_by_position(T.epc, T.z, x, y, q);
+  };
   int lo, hi;
   pw_lohi(T, re, &lo, &hi);
   const int hiE = hi;
   int a = -1, b = -1;
-  const int en = border_by_position(T.epc, T.z, lo, hi, e);
+  const int en = border(lo, hi, e);
   if (en >= 0) {
     const int j = J(en);
     int node = 0;
@@ -172,7 +178,7 @@ __device__ void pw_edge_tree(const PwTree& T, int rs, double s, int re, double e
     if (node >= L && node < 2 * L && !eqnext(node - L)) a = node;
   }
   pw_lohi(T, rs, &lo, &hi);
-  const int st = border_by_position(T.epc, T.z, lo, hi, s);
+  const int st = border(lo, hi, s);
   if (st >= 0) {
     const int j = J(st);
     int node = 0;
