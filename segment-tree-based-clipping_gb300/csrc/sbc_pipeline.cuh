@@ -346,9 +346,17 @@ struct BatchShape {
   int front = 128, cand = 128, back = 128, bwd = 128;
 };
 
+// the stream of a batch's wide pairs
+struct BatchSide {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t go = nullptr, done = nullptr;
+};
+
 class BatchRunner {
  public:
   explicit BatchRunner(Pipeline& pl) : pl_(pl) {}
+  ~BatchRunner();
+  BatchRunner(const BatchRunner&) = delete;
   BatchShape shape;
   int split = SBC_BATCH_MAX_VERTICES;  // polygons above it go to the pair pipeline (<= the max)
   // components of the current call (device, pair-relative successor of each
@@ -417,6 +425,7 @@ class BatchRunner {
   int* wide_ = nullptr;
   int* wide_item_ = nullptr;
   int nwide_ = 0, nitems_ = 0, wide_min_ = 0;
+  BatchSide side_;
   unsigned char* arena[2] = {nullptr, nullptr};
   long long* aoff[2] = {nullptr, nullptr};
   long long abase_[2] = {0, 0};

@@ -396,3 +396,47 @@ def test_heights_near_and_beyond_float(mode, sy):
                 assert st != 0
                 continue
             assert st == 0 and rings_equal(got, ref)
+
+
+def test_mixed_batch_on_two_streams_and_recorded(clipper):
+    """A batch of small and wide pairs, whose kernels run side by side: the
+    recorded step gives the bits of the separate calls, and again on new
+    coordinates, on the context's stream and on a caller's."""
+    torch = pytest.importorskip("torch")
+    pairs = [p for p in batch_pairs() if len(p[0]) + len(p[1]) < 2500] + gen.small_pairs(60, seed=77, lo=4, hi=40)
+    (bxy, boff), (cxy, coff) = (sbclip.pack_polygons([p[k] for p in pairs]) for k in (0, 1))
+    n = len(pairs)
+    tb, tbo, tc, tco = (torch.from_numpy(x).cuda() for x in (bxy, boff, cxy, coff))
+    ga = torch.linspace(0.5, 2.0, n, dtype=torch.float64, device="cuda")
+    args = (n, tb.data_ptr(), tbo.data_ptr(), tc.data_ptr(), tco.data_ptr())
+
+    def separate(stream=None):
+        area, st = torch.zeros_like(ga), torch.zeros(n, dtype=torch.int32, device="cuda")
+        gb, gc = torch.zeros_like(tb), torch.zeros_like(tc)
+        torch.cuda.synchronize()
+        clipper.area_forward_device(*args, area.data_ptr(), st.data_ptr(), stream)
+        clipper.area_backward_device(*args, ga.data_ptr(), gb.data_ptr(), gc.data_ptr(), stream)
+        torch.cuda.synchronize()
+        return [x.cpu().numpy() for x in (area, st, gb, gc)]
+
+    def same(x, y):
+        return all(np.array_equal(a, b) for a, b in zip(x, y))
+
+    first = separate()
+    own = torch.cuda.Stream()
+    assert same(first, separate(own.cuda_stream))
+    out = [torch.zeros_like(x) for x in (ga, ga.to(torch.int32), tb, tc)]
+    g = clipper.area_graph(*args, ga.data_ptr(), out[2].data_ptr(), out[3].data_ptr(), out[0].data_ptr(),
+                           out[1].data_ptr())
+    torch.cuda.synchronize()
+    for scale in (1.0, 1.25):
+        tb.copy_(torch.from_numpy(bxy * scale))
+        tc.copy_(torch.from_numpy(cxy * scale))
+        torch.cuda.synchronize()
+        g.launch()
+        torch.cuda.synchronize()
+        got = [x.cpu().numpy() for x in out]
+        if scale == 1.0:
+            assert same(first, got)
+    g.close()
+    assert same(separate(), got)
