@@ -292,10 +292,18 @@ __device__ __forceinline__ GpLeg gp_leg(const Gp& g, int side, int inside, int k
 }
 
 // In line with its neighbours as cleanUpResult2 (foster/polyclip.h:767-787)
-// sees it, with room for the rounding of either order of the three points.
+// sees it, in either order of the ring: each order's area3 rounds the products
+// about its own first point.  With m the largest difference from p, either
+// area is within 1.3e-15 m^2 of the exact one (2^-53 times 16.4 m^2 about q,
+// whose differences reach 2 m, and 8.2 m^2 about p), so most vertices are
+// settled by one area.
 __device__ __forceinline__ bool gp_flat(double2 p, double2 v, double2 q) {
-  const double a = dmul(v.x - p.x, q.y - p.y), b = dmul(v.y - p.y, q.x - p.x);
-  return !(fabs(a - b) > kEps + 1e-14 * (fabs(a) + fabs(b)));
+  const double a = area3(p.x, p.y, v.x, v.y, q.x, q.y);
+  const long long u = max(max(abs_bits(dsub(v.x, p.x)), abs_bits(dsub(v.y, p.y))),
+                          max(abs_bits(dsub(q.x, p.x)), abs_bits(dsub(q.y, p.y))));
+  const double m = __longlong_as_double(u);
+  if (abs_gt(a, __fma_rn(4e-15 * m, m, kEps))) return false;
+  return abs_lt(a, kEps) || abs_lt(area3(q.x, q.y, v.x, v.y, p.x, p.y), kEps);
 }
 
 // Per crossing: its label (calculateInitLabelParallel, oacc_segment_tree.cpp:
