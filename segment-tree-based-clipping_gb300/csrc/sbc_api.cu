@@ -16,16 +16,17 @@ namespace sbc {
 
 int Pipeline::run(const double* d_bxy, int nb_, const double* d_cxy, const int* c_sizes, int k_) {
   err_.clear();
+  // a refused call leaves the last one's arrays as they are
+  if (nb_ < 3) return fail(kEInput, "base polygon needs at least 3 vertices");
+  if (k_ < 1 || k_ > 9) return fail(kEInput, "1 to 9 overlays are supported");
+  for (int i = 0; i < k_; ++i)
+    if (c_sizes[i] < 3) return fail(kEInput, "overlay polygon needs at least 3 vertices");
+  drop_records();
   outs_.assign(k_, OverlayOut());
   join_ready_ = 0;
   cover_count_pending_ = false;
-  lazy_ = LazyRecords();
   nb = nb_;
   k = k_;
-  if (nb < 3) return fail(kEInput, "base polygon needs at least 3 vertices");
-  if (k < 1 || k > 9) return fail(kEInput, "1 to 9 overlays are supported");
-  for (int i = 0; i < k; ++i)
-    if (c_sizes[i] < 3) return fail(kEInput, "overlay polygon needs at least 3 vertices");
   cudaEvent_t ev[8];
   if (timing)
     for (int i = 0; i < 8; ++i) cudaEventCreate(&ev[i]);
@@ -122,11 +123,11 @@ int Pipeline::run_from_hits(const double* d_bxy, int nb_, const double* d_cxy, i
                             const int* rb, const int* rc, const int* rt,
                             const unsigned long long* rkey, long long nhits) {
   err_.clear();
+  if (nb_ < 3 || nc < 3) return fail(kEInput, "polygons need at least 3 vertices");
+  drop_records();
   outs_.assign(1, OverlayOut());
-  lazy_ = LazyRecords();
   nb = nb_;
   k = 1;
-  if (nb < 3 || nc < 3) return fail(kEInput, "polygons need at least 3 vertices");
   const int sizes[1] = {nc};
   int rc0 = stage_setup(d_bxy, d_cxy, sizes);
   // the setup's non-finite check (run() reads it with the elementary counts)

@@ -538,6 +538,7 @@ __global__ void k_labels_c(int nQ, const int* __restrict__ cWin, const int* __re
 
 // ============================================================== stage_overlay
 int Pipeline::stage_overlay(int cType, OverlayOut& out) {
+  drop_records();  // the overlay before this one: its buffers are written here
   // ---- A8 candidate pairs: unique hits with the key of their first emission
   int *rb = nullptr, *rc = nullptr, *rt = nullptr;
   unsigned long long* rkey = nullptr;
@@ -559,12 +560,21 @@ bool Pipeline::overlay_ids_fit() const {
   return 2LL * (hcS[k] - 2) < m;
 }
 
+// No diagnostic arrays of rows A9-A14 until an overlay has them again.
+void Pipeline::drop_records() {
+  lazy_ = LazyRecords();
+  dbg_ub = dbg_uc = dbg_ut = dbg_aB = dbg_aC = nullptr;
+  dbg_alB = dbg_alC = dbg_nbB = dbg_nbC = dbg_labB = dbg_labC = nullptr;
+  dbg_isxy = dbg_ixB = dbg_ixC = nullptr;
+  dbg_K = dbg_nB = dbg_nQ = 0;
+}
+
 // The arrays of rows A9-A14 (sbc_debug_array) of an overlay whose rings came
 // straight from its hits.
 int Pipeline::build_records() {
   if (!lazy_.rb) return kOk;
   const LazyRecords l = lazy_;
-  lazy_ = LazyRecords();
+  drop_records();
   OverlayOut unused;
   return stage_records(l.cType, l.rb, l.rc, l.rt, l.rkey, l.nhits, unused, false, true);
 }

@@ -262,6 +262,7 @@ class Pipeline {
   // the diagnostic arrays of rows A9-A14 of the last overlay, if its rings
   // came without them
   int build_records();
+  void drop_records();  // forgets them
   // one pair's rows A10-A18 from its unique candidate hits in A9's order
   // (base id, then first-emission key; no tree): the same rings as run() on
   // that pair when the hits are the pair's own
