@@ -323,6 +323,10 @@ __global__ void __launch_bounds__(256) k_gp_legs(Gp g) {
     const double2 qm = gm >= 0 ? g.xy[gm] : c[f], qp = gp >= 0 ? g.xy[gp] : c[f + 1];
     bool bad = (hm >= 0 && (hm == gm || hm == gp || g.rc[hm] == g.rc[h])) ||
                (hp >= 0 && (hp == gm || hp == gp));
+    // nor two crossings of an edge at one point: the provenance of such a ring
+    // vertex is its first record's, and the hits here are in no order
+    auto at = [&](double2 q) { return same_value(q.x, v.x) && same_value(q.y, v.y); };
+    if (at(pm) || at(pp) || at(qm) || at(qp)) bad = true;
     const double s3 = area3(pm.x, pm.y, v.x, v.y, pp.x, pp.y);
     auto right = [&](double2 q) {
       const double s1 = area3(q.x, q.y, pm.x, pm.y, v.x, v.y);
