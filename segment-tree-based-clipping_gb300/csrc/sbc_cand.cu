@@ -444,7 +444,12 @@ __global__ void k_vertex_f4(long long nv, const double* __restrict__ xy, float4*
 // emission count and first key (a pair the reference never emits is
 // dropped there).
 // counters: [0] unique hits, [1] pairs passing LSMF, [3] emissions with a
-// non-zero type (the reference's raw hit count).
+// non-zero type (the reference's raw hit count), [6] non-zero where a hit is
+// no proper crossing.  ranks: the flags of a tree from vertex ranks (null:
+// another tree); where those do not do, the leaf ranges mean nothing.
+__device__ __forceinline__ bool no_tree(const unsigned* ranks) {
+  return ranks && (*ranks & ~(unsigned)kFlagLongRun) != 0u;
+}
 constexpr int kExBlock = 256;
 constexpr int kExPer = 4;
 constexpr int kExChunk = kExBlock * kExPer;
@@ -455,9 +460,10 @@ k_pair_exact(long long n, const int2* __restrict__ pairs, const int* __restrict_
              const long long* __restrict__ bK, const long long* __restrict__ cK,
              const float4* __restrict__ vfB, const float4* __restrict__ vfC,
              const int2* __restrict__ lr, const int* __restrict__ aft, const int* __restrict__ bef,
-             int logL, unsigned long long* __restrict__ counters, long long cap,
-             int* __restrict__ rb, int* __restrict__ rc, int* __restrict__ rt,
+             int logL, const unsigned* __restrict__ ranks, unsigned long long* __restrict__ counters,
+             long long cap, int* __restrict__ rb, int* __restrict__ rc, int* __restrict__ rt,
              unsigned long long* __restrict__ rkey, double2* __restrict__ rab) {
+  if (no_tree(ranks)) return;
   __shared__ int4 q[kExChunk];
   __shared__ int qn;
   __shared__ unsigned long long ntested;
@@ -526,6 +532,7 @@ k_pair_exact(long long n, const int2* __restrict__ pairs, const int* __restrict_
       unsigned long long hb = 0;
       if (lane == leader) hb = atomicAdd(&counters[0], (unsigned long long)__popc(m));
       hb = __shfl_sync(0xffffffffu, hb, leader);
+      if (hit && ty != 1) counters[6] = 1;
       if (hit) {
         const long long idx = (long long)hb + __popc(m & lt);
         if (idx < cap) {
@@ -663,8 +670,8 @@ k_direct_groups(int gB, int gC0, int gC, int chunks, const float4* __restrict__ 
     if ((long long)at < cap) list[at] = make_int2(b0 + __ffs(met) - 1, q);
 }
 
-// counters as in k_pair_exact, and [2] box-overlapping edge pairs, [4] edge
-// pairs tested, [5] listed group pairs
+// counters and ranks as in k_pair_exact, and [2] box-overlapping edge pairs,
+// [4] edge pairs tested, [5] listed group pairs
 __global__ void __launch_bounds__(128)
 k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long list_cap,
                const float4* __restrict__ fbox, const int* __restrict__ e_id, const double* __restrict__ bP,
@@ -672,9 +679,10 @@ k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long 
                const long long* __restrict__ cK, const float4* __restrict__ vfB,
                const float4* __restrict__ vfC, const int2* __restrict__ lr,
                const int* __restrict__ aft, const int* __restrict__ bef, int logL,
-               unsigned long long* __restrict__ counters, long long cap, int* __restrict__ rb,
-               int* __restrict__ rc, int* __restrict__ rt, unsigned long long* __restrict__ rkey,
-               double2* __restrict__ rab) {
+               const unsigned* __restrict__ ranks, unsigned long long* __restrict__ counters,
+               long long cap, int* __restrict__ rb, int* __restrict__ rc, int* __restrict__ rt,
+               unsigned long long* __restrict__ rkey, double2* __restrict__ rab) {
+  if (no_tree(ranks)) return;
   __shared__ int2 s_q[4][64];
   __shared__ float4 s_box[4][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -708,6 +716,7 @@ k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long 
       if (lane == 0) at = atomicAdd(&counters[0], (unsigned long long)__popc(m));
       at = __shfl_sync(0xffffffffu, at, 0);
       const long long idx = (long long)at + __popc(m & lt);
+      if (hit && ty != 1) counters[6] = 1;
       if (hit && idx < cap) {
         rb[idx] = 2 * e.x;
         rc[idx] = cid;
@@ -1045,19 +1054,19 @@ int Pipeline::stage_candidates(int cType, int** rb_out, int** rc_out, int** rt_o
     if (npairs > 0) {
       ::sbc::KProbe kp_("k_pair_exact", st, 72.0 * npairs);  // pair + both edges' coordinates
       k_pair_exact<<<grid_for(npairs, kExChunk), kExBlock, 0, st>>>(
-          npairs, pairs, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL, counters, hcap, rb, rc,
-          rt, rkey, rab);
+          npairs, pairs, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL,
+          tree_flags(), counters, hcap, rb, rc, rt, rkey, rab);
     }
-    hc = rd_.get(counters, HostReads::kCand + 8, st, 4);
+    hc = rd_.get(counters, HostReads::kCand + 4, st, 7);
     const unsigned* r_fl = rd_.get(d_flags, HostReads::kCand + 14, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return fail(kECuda, "exact stage");
     if (!ranks_failed(*r_fl)) break;
-    // the ranks did not do: the tree's arrays, then the pairs again
+    // the ranks did not do (and nothing was counted): the tree's arrays, then
+    // the pairs
     const int rt0 = redo_tree(*r_fl);
     if (rt0) return rt0;
-    cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st);
-    cudaMemsetAsync(counters + 3, 0, sizeof(unsigned long long), st);
   }
+  improper_ = hc[6] != 0;
   if ((long long)hc[0] > hcap) return fail(kEInternal, "hit buffer overflow");
   if (hc[0] >= (1ULL << 31)) return fail(kEInput, "too many intersections");
   *rb_out = rb;
@@ -1083,7 +1092,7 @@ int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_
   long long cap = std::max(hit_cap_, std::min((long long)nb * nc, 4LL * E + 65536));
   auto* counters = join_counters_;
   const unsigned long long* hc = nullptr;
-  for (;;) {
+  for (bool listed = false;;) {
     int* rb = (int*)pool_.get("raw_b", sizeof(int) * (cap + 1));
     int* rc = (int*)pool_.get("raw_c", sizeof(int) * (cap + 1));
     int* rt = (int*)pool_.get("raw_t", sizeof(int) * (cap + 1));
@@ -1091,8 +1100,8 @@ int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_
     auto* rab = (double2*)pool_.get("raw_ab", sizeof(double2) * (cap + 1));
     auto* list = (int2*)pool_.get("direct_list", sizeof(int2) * (lcap + 1));
     if (pool_.failed) return fail(kENoMem, "device allocation failed (hits)");
-    cudaMemsetAsync(counters, 0, 6 * sizeof(unsigned long long), st);
-    {
+    if (!listed) {
+      cudaMemsetAsync(counters, 0, 7 * sizeof(unsigned long long), st);
       const long long rows = (gB + kDirectRows - 1) / kDirectRows;
       ::sbc::KProbe kp_("k_direct_groups", st, 16.0 * (gB + gC));
       k_direct_groups<<<grid_for(rows * chunks, 4), 128, 0, st>>>(gB, d_group0_[cType], gC, chunks,
@@ -1101,10 +1110,10 @@ int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_
     {
       ::sbc::KProbe kp_("k_direct_exact", st, 16.0 * (nb + nc));
       k_direct_exact<<<(unsigned)std::min(grid_for((long long)gB * gC, 4), 1216u), 128, 0, st>>>(
-          nb, c0, nc, list, lcap, fbox, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL, counters,
-          cap, rb, rc, rt, rkey, rab);
+          nb, c0, nc, list, lcap, fbox, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL,
+          tree_flags(), counters, cap, rb, rc, rt, rkey, rab);
     }
-    hc = rd_.get(counters, HostReads::kCand + 8, st, 6);
+    hc = rd_.get(counters, HostReads::kCand + 4, st, 7);
     const unsigned* r_fl = rd_.get(d_flags, HostReads::kCand + 14, st);
     const unsigned* r_out = rd_.get(g_bnd + 8, HostReads::kCand + 15, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return fail(kECuda, "exact stage");
@@ -1112,8 +1121,10 @@ int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_
     if (ranks_failed(*r_fl)) {
       const int rt0 = redo_tree(*r_fl);
       if (rt0) return rt0;
+      listed = true;  // and nothing else was counted
       continue;
     }
+    listed = false;
     raw_ab_ = rab;
     *rb_out = rb;
     *rc_out = rc;
@@ -1126,6 +1137,7 @@ int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_
   }
   hit_cap_ = cap;
   group_cap_ = lcap;
+  improper_ = hc[6] != 0;
   *nhits = (long long)hc[0];
   out.survivors = (long long)hc[2];
   out.tests = (long long)hc[1];

@@ -592,9 +592,10 @@ __global__ void k_vertex_full(int E, const unsigned* __restrict__ g, unsigned* _
 // it is a rank: each edge's end leaves and leaf range follow from the ranks of
 // its two vertices and the arithmetic of findBoarder's search
 // (border_by_position), without the endpoint order, the elementary array or a
-// host read in between.  A shared x value, many zero border keys, or values
-// whose keys leave the reference's range set kFlagSharedX, and the stages that
-// build the arrays run instead (redo_tree).
+// host read in between.  A shared x value sets kFlagSharedX; many zero border
+// keys, or values whose keys leave the reference's range, set kFlagNoRanks; the
+// candidate kernels then leave at once and the stages that build the arrays run
+// (redo_tree).
 //
 // The vertices' full keys in the narrow order with equal-key runs sorted, as
 // k_vertex_full does, and each vertex's rank.
@@ -617,7 +618,7 @@ __global__ void k_vertex_rank(int E, const unsigned* __restrict__ g, const unsig
   int m = 1;
   while (i + m < E && g[i + m] == gi && m < kFixRun) ++m;
   if (i + m < E && g[i + m] == gi) {
-    atomicOr(flags, (unsigned)kFlagSharedX);
+    atomicOr(flags, (unsigned)kFlagNoRanks);
     return;
   }
   unsigned long long kk[kFixRun];
@@ -669,7 +670,7 @@ __device__ void rank_zero(int E, int epc, const unsigned long long* skey,
       if (++z > kMaxZero) bad = true;
   }
   *zero = z;
-  if (bad) atomicOr(flags, (unsigned)kFlagSharedX);
+  if (bad) atomicOr(flags, (unsigned)kFlagNoRanks);
 }
 
 __global__ void k_rank_zero(int E, int epc, const unsigned long long* __restrict__ skey,
@@ -868,14 +869,17 @@ int Pipeline::stage_ranks(bool cover) {
   stat_epc = epc;
   stat_ts = ts;
   from_ranks_ = lr_ready = true;
+  ranks_did_ = false;
   return kOk;
 }
 
 // whether the stages that build the arrays have to run after all
 bool Pipeline::ranks_failed(unsigned flags) {
-  if (!from_ranks_) return false;
+  if (!tree_flags()) return false;
   if (flags & kFlagLongRun) stat_vertex_sort = 1;
-  return (flags & ~(unsigned)kFlagLongRun) != 0;
+  if (flags & ~(unsigned)kFlagLongRun) return true;
+  ranks_did_ = true;
+  return false;
 }
 
 int Pipeline::redo_tree(unsigned flags) {
@@ -884,7 +888,7 @@ int Pipeline::redo_tree(unsigned flags) {
   clear_flags();
   // the side stream may still count cover entries of the ranges replaced here
   if (st2_) cudaStreamSynchronize(st2_);
-  int rc = stage_elementary();
+  int rc = stage_elementary((flags & kFlagSharedX) != 0);
   if (!rc) rc = stage_endlists();
   if (!rc) rc = stage_cover();
   if (!rc) launch_cover_count();
@@ -903,7 +907,8 @@ int Pipeline::build_elementary() {
   return kOk;
 }
 
-int Pipeline::stage_elementary() {
+// shared_x: two vertices are known to share an x value
+int Pipeline::stage_elementary(bool shared_x) {
   long long n2 = 2LL * E;
   auto* keys = (unsigned long long*)pool_.get("ele_keys", sizeof(unsigned long long) * n2);
   auto* keys2 = (unsigned long long*)pool_.get("ele_keys2", sizeof(unsigned long long) * n2);
@@ -922,7 +927,7 @@ int Pipeline::stage_elementary() {
   auto* vgid = (unsigned*)pool_.get("v_gid", sizeof(unsigned) * E);
   if (pool_.failed) return fail(kENoMem, "device allocation failed (elementary)");
   // every endpoint is a vertex x value: its key lies in the setup's [min, max]
-  bool by_vertex = !force_endpoint_sort;
+  bool by_vertex = !force_endpoint_sort && !shared_x;
   bool narrow = by_vertex && !force_wide_vertex_sort;
   int count = 0, before_last = 0;
   for (;;) {

@@ -43,6 +43,7 @@ enum DevFlag : unsigned {
   kFlagUnsorted = 16u,      // the elementary array is not in order
   kFlagSharedX = 32u,       // two vertices share an x value (endpoint order needs the full sort)
   kFlagLongRun = 64u,       // a run of equal 32-bit vertex keys too long to fix up in place
+  kFlagNoRanks = 128u,      // the tree does not follow from vertex ranks (x values apart all the same)
 };
 
 // ---------------------------------------------------------------- FP64 geometry

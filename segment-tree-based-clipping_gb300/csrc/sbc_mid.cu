@@ -548,8 +548,10 @@ int Pipeline::stage_overlay(int cType, OverlayOut& out) {
     if (rc0) return rc0;
   }
   bool done = false;
-  const int rc1 = stage_general(cType, rb, rc, rt, rkey, nraw, out, &done);
-  if (rc1 || done) return rc1;
+  if (!improper_) {
+    const int rc1 = stage_general(cType, rb, rc, rt, rkey, nraw, out, &done);
+    if (rc1 || done) return rc1;
+  }
   return stage_records(cType, rb, rc, rt, rkey, nraw, out);
 }
 

@@ -210,6 +210,7 @@ class Pipeline {
   const int2* join_pairs_ = nullptr;
   unsigned long long* join_counters_ = nullptr;
   const double2* raw_ab_ = nullptr;    // (alpha, beta) of each candidate hit (stage_candidates)
+  bool improper_ = false;              // one of them is no proper crossing
   long long join_npairs_ = 0, join_work_ = 0;
   // intermediate arrays of the last overlay processed (device, diagnostics)
   int *dbg_ub = nullptr, *dbg_uc = nullptr, *dbg_ut = nullptr;
@@ -225,9 +226,12 @@ class Pipeline {
   int stage_setup(const double* d_bxy, const double* d_cxy, const int* c_sizes);
   int stage_ranks(bool cover);    // A4-A7 from vertex ranks (no shared x value)
   bool ranks_failed(unsigned flags);
+  // the flags that say whether the ranks did, until the first overlay's
+  // candidates have been found by them (later stages use the word again)
+  const unsigned* tree_flags() const { return from_ranks_ && !ranks_did_ ? d_flags : nullptr; }
   int redo_tree(unsigned flags);  // A4-A7 by the stages below where ranks do not do
   int build_elementary();         // the elementary array of a run from ranks, for diagnostics
-  int stage_elementary();
+  int stage_elementary(bool shared_x = false);
   int stage_endlists();
   int stage_cover();
   // the grid in three steps on the side stream: boxes and bounds; cell
@@ -298,6 +302,7 @@ class Pipeline {
   static constexpr long long kDirectMost = 20000000000LL;
   bool direct_ = false;                // this run searches without the grid
   bool from_ranks_ = false;            // this run's tree quantities came from ranks
+  bool ranks_did_ = false;             // and stand
   long long hit_cap_ = 0, group_cap_ = 0;  // room for hits and group pairs that sufficed
   float4* gbox_ = nullptr;             // boxes of 32 edges each, polygon after polygon
   int d_group0_[11] = {};              // each polygon's first one
