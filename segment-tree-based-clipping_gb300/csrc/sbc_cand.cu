@@ -554,9 +554,9 @@ k_pair_exact(long long n, const int2* __restrict__ pairs, const int* __restrict_
 // consecutive edges lie near one another, so the box of 32 of them says much.
 // Every pair of such groups is tested by their boxes (a lane per overlay
 // group), the pairs that meet are listed, and a warp takes each one, a base
-// edge per lane, straight through the box test, LSMF and the float test to
-// the classifier.  Four launches and one host read, where the grid and its
-// join take 13 launches and five reads.
+// edge per lane: box test, LSMF, the float test and the classifier.  Four
+// launches and one host read, where the grid and its join take 13 launches and
+// five reads.
 // first edge group of each polygon (base, overlays), and their count
 struct EdgeGroups {
   int g0[11];
@@ -671,10 +671,17 @@ k_direct_groups(int gB, int gC0, int gC, int chunks, const float4* __restrict__ 
 }
 
 // counters and ranks as in k_pair_exact, and [2] box-overlapping edge pairs,
-// [4] edge pairs tested, [5] listed group pairs
+// [4] edge pairs tested, [5] listed group pairs.  Overlay edge j is edge c0 + j
+// from vertex v0 + j.  Of either group only the edges that reach the other's
+// box are tested; the pairs that pass each filter are queued, and the next one
+// runs when there are 32: a few lanes in LSMF and the float test cost the issue
+// slots of all (100,000 x 80,000 jagged vertices, 321,000 group pairs, 235,000
+// hits: 823 us with every edge against every other and no first queue, 500
+// with the edges that reach the box, 380 so).
 __global__ void __launch_bounds__(128)
-k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long list_cap,
-               const float4* __restrict__ fbox, const int* __restrict__ e_id, const double* __restrict__ bP,
+k_direct_exact(int nb, int c0, int v0, int nc, const int2* __restrict__ list, long long list_cap,
+               const float4* __restrict__ fbox, const float4* __restrict__ gboxB,
+               const float4* __restrict__ gboxC, const double* __restrict__ bP,
                const double* __restrict__ cP, const long long* __restrict__ bK,
                const long long* __restrict__ cK, const float4* __restrict__ vfB,
                const float4* __restrict__ vfC, const int2* __restrict__ lr,
@@ -682,16 +689,32 @@ k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long 
                const unsigned* __restrict__ ranks, unsigned long long* __restrict__ counters,
                long long cap, int* __restrict__ rb, int* __restrict__ rc, int* __restrict__ rt,
                unsigned long long* __restrict__ rkey, double2* __restrict__ rab) {
-  if (no_tree(ranks)) return;
-  __shared__ int2 s_q[4][64];
+  __shared__ int2 s_near[4][64], s_q[4][64];  // past the boxes, past the float test
   __shared__ float4 s_box[4][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
   const float inf = __int_as_float(0x7f800000);
   const long long items = min((long long)counters[5], list_cap);
-  int nq = 0;
+  if (no_tree(ranks)) return;
+  int nnear = 0, nq = 0;
   unsigned long long raw = 0;
   unsigned tested = 0, boxes = 0, work = 0;
+  // appends; true: 32 or more are waiting
+  auto push = [&](int2* q, int& n, bool put, int2 e) {
+    const unsigned m = __ballot_sync(0xffffffffu, put);
+    if (put) q[n + __popc(m & lt)] = e;
+    n += __popc(m);
+    __syncwarp();
+    return n >= 32;
+  };
+  // drops the first 32
+  auto shift = [&](int2* q, int& n) {
+    n -= 32;
+    const int2 x = lane < n ? q[32 + lane] : make_int2(0, 0);
+    __syncwarp();
+    if (lane < n) q[lane] = x;
+    __syncwarp();
+  };
   auto classify = [&](int count) {
     bool hit = false;
     int2 e = make_int2(0, 0);
@@ -700,12 +723,12 @@ k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long 
     unsigned long long key = 0;
     if (lane < count) {
       e = s_q[w][lane];
-      cid = e_id[e.y];
+      cid = 2 * (v0 + e.y);
       const double* pb = bP + 2LL * e.x;
       const double* pc = cP + cid;
       ty = seg_isect(pb[0], pb[1], pb[2], pb[3], pc[0], pc[1], pc[2], pc[3], &al, &bt);
       if (ty) {
-        const unsigned n = emission(e.x, e.y, cid, lr, aft, bef, logL, &key);
+        const unsigned n = emission(e.x, c0 + e.y, cid, lr, aft, bef, logL, &key);
         hit = n > 0;
         raw += n;
       }
@@ -727,50 +750,51 @@ k_direct_exact(int nb, int c0, int nc, const int2* __restrict__ list, long long 
     }
     __syncwarp();
   };
+  auto test = [&](int count) {
+    bool keep = false;
+    int2 e = make_int2(0, 0);
+    if (lane < count) {
+      e = s_near[w][lane];
+      const longlong2* kb = (const longlong2*)bK + e.x;
+      const longlong2* kc = (const longlong2*)cK + v0 + e.y;
+      const longlong2 b1 = kb[0], b2 = kb[1], c1 = kc[0], c2 = kc[1];
+      const float4 p1 = vfB[e.x], p2 = vfB[e.x + 1], q1 = vfC[v0 + e.y], q2 = vfC[v0 + e.y + 1];
+      if (lsmf_keys(b1.x, b1.y, b2.x, b2.y, c1.x, c1.y, c2.x, c2.y)) {
+        ++tested;
+        keep = !certainly_disjoint(p1, p2, q1, q2);
+      }
+    }
+    if (push(s_q[w], nq, keep, e)) {
+      classify(32);
+      shift(s_q[w], nq);
+    }
+  };
   for (long long i = (long long)blockIdx.x * 4 + w; i < items; i += 4LL * gridDim.x) {
     const int2 pair = list[i];
     const int be = pair.x * 32 + lane, j0 = pair.y * 32, n = min(32, nc - j0);
-    float4 fb = make_float4(inf, inf, -inf, -inf), p1 = fb, p2 = fb;
-    long long kb[4] = {0, 0, 0, 0};
+    const float4 gb = gboxB[pair.x], gc = gboxC[pair.y];
+    float4 fb = make_float4(inf, inf, -inf, -inf), fc = fb;
+    if (be < nb) fb = fbox[be];
+    if (lane < n) fc = fbox[c0 + j0 + lane];
+    const bool on = be < nb && boxes_touch(fb, gc);
+    unsigned left = __ballot_sync(0xffffffffu, lane < n && boxes_touch(fc, gb));
+    if (!__any_sync(0xffffffffu, on)) continue;
+    if (on) work += __popc(left);
+    s_box[w][lane] = fc;
     __syncwarp();
-    if (lane < n) s_box[w][lane] = fbox[c0 + j0 + lane];
-    if (be < nb) {
-      fb = fbox[be];
-      p1 = vfB[be];
-      p2 = vfB[be + 1];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) kb[j] = bK[2LL * be + j];
-      work += n;
-    }
-    __syncwarp();
-    for (int t = 0; t < n; ++t) {
-      bool keep = false;
-      const int ce = c0 + j0 + t;
-      if (boxes_touch(fb, s_box[w][t])) {
-        ++boxes;
-        const int v = e_id[ce] >> 1;
-        const long long* kc = cK + 2LL * v;
-        if (lsmf_keys(kb[0], kb[1], kb[2], kb[3], kc[0], kc[1], kc[2], kc[3])) {
-          ++tested;
-          keep = !certainly_disjoint(p1, p2, vfC[v], vfC[v + 1]);
-        }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      if (!m) continue;
-      if (keep) s_q[w][nq + __popc(m & lt)] = make_int2(be, ce);
-      nq += __popc(m);
-      __syncwarp();
-      if (nq >= 32) {
-        classify(32);
-        const int rest = nq - 32;
-        const int2 x = lane < rest ? s_q[w][32 + lane] : make_int2(0, 0);
-        __syncwarp();
-        if (lane < rest) s_q[w][lane] = x;
-        nq = rest;
-        __syncwarp();
+    for (; left; left &= left - 1) {
+      const int t = __ffs(left) - 1;
+      const bool near = on && boxes_touch(fb, s_box[w][t]);
+      if (!__any_sync(0xffffffffu, near)) continue;
+      boxes += near;
+      if (push(s_near[w], nnear, near, make_int2(be, j0 + t))) {
+        test(32);
+        shift(s_near[w], nnear);
       }
     }
+    __syncwarp();
   }
+  if (nnear > 0) test(nnear);
   if (nq > 0) classify(nq);
   for (int o = 16; o > 0; o >>= 1) raw += __shfl_xor_sync(0xffffffffu, raw, o);
   tested = __reduce_add_sync(0xffffffffu, tested);
@@ -1110,8 +1134,8 @@ int Pipeline::direct_candidates(int cType, int** rb_out, int** rc_out, int** rt_
     {
       ::sbc::KProbe kp_("k_direct_exact", st, 16.0 * (nb + nc));
       k_direct_exact<<<(unsigned)std::min(grid_for((long long)gB * gC, 4), 1216u), 128, 0, st>>>(
-          nb, c0, nc, list, lcap, fbox, e_id, bP, cP, bK, cK, vfB, vfC, lr, aft, bef, logL,
-          tree_flags(), counters, cap, rb, rc, rt, rkey, rab);
+          nb, c0, hcS[cType - 1], nc, list, lcap, fbox, gbox_, gbox_ + d_group0_[cType], bP, cP, bK,
+          cK, vfB, vfC, lr, aft, bef, logL, tree_flags(), counters, cap, rb, rc, rt, rkey, rab);
     }
     hc = rd_.get(counters, HostReads::kCand + 4, st, 7);
     const unsigned* r_fl = rd_.get(d_flags, HostReads::kCand + 14, st);
