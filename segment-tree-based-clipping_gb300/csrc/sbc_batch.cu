@@ -379,7 +379,8 @@ __device__ __forceinline__ double border_scale(double dv) {
 // and 21).  A warp counts each vertex's lesser ones by the values rounded to
 // float (65,536 pairs of 4 to 64 vertices: 0.31 ms with 64-bit keys, 0.27 so),
 // a block sorts (np = npow2_dev(E) entries of key and val).  False: something was shared,
-// has a zero border key or is out of range; nothing but vf is written.
+// has a zero border key or is out of range; nothing but vf is written.  (Where
+// two floats are equal and so are their values, a warp leaves at once.)
 template <int V>
 using Const = std::integral_constant<int, V>;
 
@@ -445,7 +446,13 @@ __device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, 
 #pragma unroll
       for (int i = 0; i < kPer; ++i)
         if (lane + i * N < E && at[r[i]] != lane + i * N) same = true;
-      return g.any(same);
+      if (!g.any(same)) return 0;
+      bool equal = false;
+#pragma unroll
+      for (int i = 0; i < kPer; ++i)
+        if (lane + i * N < E && okey(vx(at[r[i]])) == okey(vx(lane + i * N)) && at[r[i]] != lane + i * N)
+          equal = true;
+      return g.any(equal) ? 2 : 1;  // two vertices of one value, or of one rank only
     };
     auto by_float = [&](auto per) {
       constexpr int kPer = decltype(per)::value;
@@ -456,12 +463,13 @@ __device__ bool clip_pair_ranks(G& g, const double* b, int nb, const double* c, 
     };
     for (int v = lane; v < E; v += N) fx[v] = w.vf[v].x;
     g.sync();
-    bool same;
+    int same;
     if (E <= 32) same = by_float(Const<1>{});
     else if (E <= 64) same = by_float(Const<2>{});
     else if (E <= 96) same = by_float(Const<3>{});
     else if (E <= 128) same = by_float(Const<4>{});
     else same = by_float(Const<8>{});
+    if (same == 2) return false;
     if (same) {
       bad = false;
       long long k[8];
@@ -1413,8 +1421,13 @@ struct ClipArgs {
   }
 };
 
+// what A.status holds of a pair before it has its own: left to the kernels that
+// follow the lists, or its front to the one by the arrays
+constexpr int kPending = -1, kFrontLeft = -2;
+
 __device__ __forceinline__ void front_done(const ClipArgs& A, int p, PairWork& w, int st) {
   w.state[0] = st;
+  A.status[p] = kPending;
   if (st != PS_OK) {
     A.status[p] = st == PS_UNDEF ? SBC_EUNDEF : SBC_ENOMEM;
     A.nrings[p] = A.nverts[p] = 0;
@@ -1422,7 +1435,33 @@ __device__ __forceinline__ void front_done(const ClipArgs& A, int p, PairWork& w
   }
 }
 
-__global__ void __launch_bounds__(128, 8) k_batch_front(ClipArgs A) {
+// a small pair's front by the arrays (key, val: shared memory for kWideEdges
+// endpoints)
+__device__ __forceinline__ void front_by_arrays(const ClipArgs& A, int p, int nb, int nc, int pass,
+                                                long long* key, int* val) {
+  Caps cp;
+  PairWork w = A.work(p, nb, nc, pass, &cp);
+  WarpGroup g;
+  const double *b = A.bxy + 2 * A.boff[p], *c = A.cxy + 2 * A.coff[p];
+  const int st = clip_pair_front(g, b, nb, c, nc, cp, w, key, val, kWideEdges, nullptr);
+  front_floats(g, b, nb, c, nc, w, false);
+  if (g.rank() == 0) front_done(A, p, w, st);
+}
+__device__ __noinline__ void front_by_arrays_call(const ClipArgs& A, int p, int nb, int nc, int pass,
+                                                  long long* key, int* val) {
+  front_by_arrays(A, p, nb, nc, pass, key, val);
+}
+
+// The fronts of the small pairs by the ranks.  A pair that they do not do goes
+// on by the arrays, here (kAll) or in k_batch_front_arrays: 65,536 pairs of 4 to
+// 64 vertices with a shared x value each take 1.8 ms in one kernel, whose 64
+// registers the arrays are short of, and 1.2 in two, but a launch more costs a
+// batch of 512 pairs 4 us.  (Inlined, the arrays' code cost the pairs without a
+// shared x value 50 us of 330, and those with one took 2.4 ms with the endpoint
+// sort in global memory.)
+constexpr int kFrontAll = 4096;  // pairs up to which one kernel does both
+template <bool kAll>
+__global__ void __launch_bounds__(128, 8) k_batch_front(const __grid_constant__ ClipArgs A) {
   __shared__ long long s_key[4][kWideEdges];
   __shared__ int s_rank[4][kWideEdges];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1445,13 +1484,27 @@ __global__ void __launch_bounds__(128, 8) k_batch_front(ClipArgs A) {
   PairWork w = A.work(p, nb, nc, pass, &cp);
   WarpGroup g;
   const double *b = A.bxy + 2 * A.boff[p], *c = A.cxy + 2 * A.coff[p];
-  int st = PS_OK;
-  const bool ranked = clip_pair_ranks(g, b, nb, c, nc, w, s_key[threadIdx.x >> 5], nullptr,
-                                      s_rank[threadIdx.x >> 5], nullptr);
-  if (!ranked)
-    st = clip_pair_front(g, b, nb, c, nc, cp, w, nullptr, nullptr, 0, nullptr);
-  front_floats(g, b, nb, c, nc, w, ranked);
-  if (lane == 0) front_done(A, p, w, st);
+  long long* key = s_key[threadIdx.x >> 5];
+  int* rank = s_rank[threadIdx.x >> 5];
+  if (clip_pair_ranks(g, b, nb, c, nc, w, key, nullptr, rank, nullptr)) {
+    if (lane == 0) front_done(A, p, w, PS_OK);
+  } else if (kAll) {
+    front_by_arrays_call(A, p, nb, nc, pass, key, rank);
+  } else if (lane == 0) {
+    A.status[p] = kFrontLeft;
+  }
+}
+
+__global__ void __launch_bounds__(128) k_batch_front_arrays(ClipArgs A) {
+  __shared__ long long s_key[4][kWideEdges];
+  __shared__ int s_val[4][kWideEdges];
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = (int)(t >> 5);
+  if ((t >> 5) >= A.np || A.status[p] != kFrontLeft) return;
+  const int pass = A.pass_of ? A.pass_of[p] : 0;
+  int nb, nc;
+  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
+  front_by_arrays(A, p, nb, nc, pass, s_key[threadIdx.x >> 5], s_val[threadIdx.x >> 5]);
 }
 
 // the front of the wide pairs, a block each; pairs of up to 2,048 vertices (or
@@ -1531,9 +1584,6 @@ __global__ void __launch_bounds__(32 * kCandWarps, kCandBlocks) k_batch_cand_wid
   CandQueue<kComp> cq{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, cp.K, w, lane, s_q[wi]};
   clip_pair_cand_group(cq, (item - A.wide_item[lo]) * kEdgeGroup, s_box[wi]);
 }
-
-// status of a pair that the general-position kernels left to the others
-constexpr int kPending = -1;
 
 // The back end in three kernels: A9-A13 on one thread per pair, the labels
 // on one warp per pair, A15-A18 on one thread per pair.  w.state[0] carries
@@ -2085,7 +2135,13 @@ void launch_clip(const ClipArgs& A, const BatchShape& sh, double in_bytes, const
   auto small = [&](cudaStream_t s) {
     {
       ::sbc::KProbe kp_("k_batch_front", s, in_bytes);
-      k_batch_front<<<grid_for(32LL * A.np, sh.front), sh.front, 0, s>>>(A);
+      const unsigned blocks = grid_for(32LL * A.np, sh.front);
+      if (A.np <= kFrontAll) k_batch_front<true><<<blocks, sh.front, 0, s>>>(A);
+      else k_batch_front<false><<<blocks, sh.front, 0, s>>>(A);
+    }
+    if (A.np > kFrontAll) {
+      ::sbc::KProbe kp_("k_batch_front_arrays", s);
+      k_batch_front_arrays<<<grid_for(32LL * A.np, 128), 128, 0, s>>>(A);
     }
     {
       ::sbc::KProbe kp_("k_batch_cand", s, in_bytes);
@@ -2657,6 +2713,7 @@ int BatchRunner::plan(int np_, const long long* d_boff, const long long* d_coff,
   big_.clear();
   // the wide line: the lower one while the blocks are few
   int over = 0;
+  any_wide_ = false;
   for (int p = 0; p < np; ++p) {
     const long long nb = h_boff_[p + 1] - h_boff_[p], nc = h_coff_[p + 1] - h_coff_[p];
     if (nb >= 3 && nc >= 3 && (nb > split_now() || nc > split_now())) {
@@ -2665,6 +2722,7 @@ int BatchRunner::plan(int np_, const long long* d_boff, const long long* d_coff,
       big_.push_back(b);
     } else {
       over += nb * nc > kWideMin[0];
+      any_wide_ |= wide_pair((int)nb, (int)nc, kWideMin[0]);
     }
   }
   wide_min_ = over <= kWideFew ? kWideMin[0] : kWideMin[1];
@@ -2705,6 +2763,7 @@ BatchRunner::~BatchRunner() {
 // is the kernel's tail), and the base edge groups before each one.
 int BatchRunner::plan_wide(int p0, int n, cudaStream_t st) {
   nwide_ = nitems_ = 0;
+  if (!any_wide_) return kOk;
   std::vector<std::vector<int>> by(48);
   for (int i = 0; i < n; ++i) {
     const long long nb = h_boff_[p0 + i + 1] - h_boff_[p0 + i];

@@ -431,6 +431,7 @@ class BatchRunner {
   int* wide_ = nullptr;
   int* wide_item_ = nullptr;
   int nwide_ = 0, nitems_ = 0, wide_min_ = 0;
+  bool any_wide_ = false;        // some pair of the batch is above the lower line
   BatchSide side_;
   unsigned char* arena[2] = {nullptr, nullptr};
   long long* aoff[2] = {nullptr, nullptr};
