@@ -330,6 +330,7 @@ k_pw_overlay_prep(int nov, const long long* __restrict__ coff, const double* __r
   int* sidx = (int*)(sk + P2);
   __shared__ int s_bad, s_cnt[kPwPrepThreads / 32];
   if (tid == 0) s_bad = 0;
+  __syncthreads();  // before any thread sets it
   const double* c = cxy + 2 * o;
   for (int t = tid; t < P2; t += blockDim.x) {
     if (t < n) {
@@ -339,8 +340,8 @@ k_pw_overlay_prep(int nov, const long long* __restrict__ coff, const double* __r
       const double xn = c[2 * (t + 1 == n ? 0 : t + 1)];
       if (!isfinite(x) || !isfinite(c[2 * t + 1]) || x == xn) atomicOr(&s_bad, 1);
     } else {
-      sk[t] = ~0ull;
-      sidx[t] = -1;
+      sk[t] = ~0ull;  // (a NaN may have this key too: an index in range all the same)
+      sidx[t] = 0;
     }
   }
   __syncthreads();
