@@ -1784,27 +1784,26 @@ __device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, in
                             int sort_room, double* s_sum) {
   Caps cp;
   PairWork w = A.work(p, nb, nc, pass, &cp);
-  if (w.state[0] != PS_OK) return;
+  if (w.state[0] != PS_OK) return g.template leave<5>();
   const int K = w.state[2];
   if (K > cp.K) {
     g.sync();
     if (g.rank() == 0) batch_fail(A, p, w, PS_CAP, K);
-    return;
+    return g.template leave<5>();
   }
+  if (w.state[4]) return g.template leave<5>();  // (the status is kPending)
   bool done = false;
   int nr = 0, nv = 0;
   double area = 0.0;
-  if (!w.state[4]) {
-    // in the arena, over the thread back end's arrays: csorted and the many
-    // larger ones after it
-    Carver cv{clean_bytes(nb, nc, K) <= smem_bytes ? smem : (unsigned char*)w.csorted, 0};
-    const CleanMem m = clean_carve(cv, nb, nc, K);
-    const CleanIn<SoaHits> in{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.bnx, w.cnx, K,
-                              SoaHits{w.hb, w.hc, w.ht, w.hkey, w.hal, w.hbt}, 0, A.unite, cp.rcap,
-                              cp.capR, w.rootB, w.rootC, w.vl, w.vloc, w.R.next, w.R.prev, w.roff, w.rxy,
-                              sort, sort_room, w.tape};
-    done = clean_clip(g, in, m, s_sum, &nr, &nv, &area) == CLEAN_DONE;
-  }
+  // in the arena, over the thread back end's arrays: csorted and the many
+  // larger ones after it
+  Carver cv{clean_bytes(nb, nc, K) <= smem_bytes ? smem : (unsigned char*)w.csorted, 0};
+  const CleanMem m = clean_carve(cv, nb, nc, K);
+  const CleanIn<SoaHits> in{A.bxy + 2 * A.boff[p], nb, A.cxy + 2 * A.coff[p], nc, w.bnx, w.cnx, K,
+                            SoaHits{w.hb, w.hc, w.ht, w.hkey, w.hal, w.hbt}, 0, A.unite, cp.rcap,
+                            cp.capR, w.rootB, w.rootC, w.vl, w.vloc, w.R.next, w.R.prev, w.roff, w.rxy,
+                            sort, sort_room, w.tape};
+  done = clean_clip(g, in, m, s_sum, &nr, &nv, &area) == CLEAN_DONE;
   if (g.rank() == 0) {
     A.status[p] = done ? SBC_OK : kPending;
     A.nrings[p] = nr;
@@ -1813,18 +1812,16 @@ __device__ void batch_clean(G& g, const ClipArgs& A, int p, int pass, int nb, in
   }
 }
 
-// (The kernel's code is larger than the instruction cache: with the warps of a
-// block entering its steps together 65,536 pairs of 4 to 64 vertices take 0.75
-// ms, 0.81 without.)
+// (The kernel's code is larger than the instruction cache: PhasedWarp.)
 __global__ void __launch_bounds__(128, 5) k_batch_clean(ClipArgs A) {
   __shared__ __align__(16) unsigned char s_mem[4][kCleanSmem];
+  PhasedWarp<128> g;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if ((t >> 5) >= A.np) return;
+  if ((t >> 5) >= A.np) return g.leave<5>();
   const int p = (int)(t >> 5);
   const int pass = A.pass_of ? A.pass_of[p] : 0;
   int nb, nc;
-  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return;
-  PhasedWarp g;
+  if (pass < 0 || !A.small(p, &nb, &nc) || wide_pair(nb, nc, A.wide_min)) return g.leave<5>();
   batch_clean(g, A, p, pass, nb, nc, s_mem[threadIdx.x >> 5], kCleanSmem, nullptr, 0,
               nullptr);
 }

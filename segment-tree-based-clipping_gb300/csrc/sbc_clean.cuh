@@ -146,6 +146,8 @@ __device__ int clean_components(G& g, int n, const int* nx, int* root) {
 // where not done the outputs' contents are unspecified.  s_sum: a shared
 // double per warp of a block.
 enum { CLEAN_DONE = 0, CLEAN_NOT = 1, CLEAN_ROOM = 2 };
+template <int n>
+using Left = std::integral_constant<int, n>;
 template <class G, class Hits>
 __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_sum,
                           int* nrings_out, int* nverts_out, double* area_out) {
@@ -187,7 +189,11 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
         meets(c[2 * f2], c[2 * f2 + 1]))
       bad = true;
   }
-  if (g.any(bad)) return CLEAN_NOT;
+  auto out = [&](auto left, int r) {  // with `left` phases not entered
+    g.template leave<decltype(left)::value>();
+    return r;
+  };
+  if (g.any(bad)) return out(Left<5>{}, CLEAN_NOT);
   if (K > 0) {
     if (!kSparse) group_scan(g, m.endB, nb + 1);
     group_scan(g, m.endC, nc + 1);
@@ -305,7 +311,9 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
       m.eQ[k] = hits.c(q);
     }
     g.sync();
-    g.phase();
+  }
+  g.phase();
+  if (K > 0) {
     // ---- A14: every initial label a crossing (calculateInitLabelParallel,
     // oacc_segment_tree.cpp:7925-7988): the overlay's neighbours of the
     // crossing lie on different sides of the base there
@@ -339,7 +347,7 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
       const bool rp = gp >= 0 ? right(m.x[gp], m.y[gp]) : right(c[2 * f2], c[2 * f2 + 1]);
       if (rm == rp) bad = true;
     }
-    if (g.any(bad)) return CLEAN_NOT;
+    if (g.any(bad)) return out(Left<4>{}, CLEAN_NOT);
   }
   g.phase();
   // ---- components, and whether each one's first vertex lies in the other
@@ -482,13 +490,13 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     }
     return comp(side, lo);
   };
-  if (g.any(bad)) return CLEAN_NOT;  // also: the flags are visible
+  if (g.any(bad)) return out(Left<3>{}, CLEAN_NOT);  // also: the flags are visible
   for (int side = 0; side < 2; ++side)
     for (int k = lane; k < (side ? ncc : ncb); k += N) {
       const Comp r = comp(side, k);
       if ((r.hi - r.lo) & 1) bad = true;
     }
-  if (g.any(bad)) return CLEAN_NOT;
+  if (g.any(bad)) return out(Left<3>{}, CLEAN_NOT);
   g.phase();
   // ---- rings: first the components without crossings that lie inside (or
   // outside, for the union), whole and in order
@@ -497,8 +505,8 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     for (int k = 0; k < (side ? ncc : ncb); ++k) {
       const Comp r = comp(side, k);
       if (r.hi != r.lo || !(r.in ^ in.unite)) continue;
-      if (rings >= in.rcap) return CLEAN_NOT;
-      if (verts + r.v1 - r.v0 > in.vcap) return CLEAN_ROOM;
+      if (rings >= in.rcap) return out(Left<2>{}, CLEAN_NOT);
+      if (verts + r.v1 - r.v0 > in.vcap) return out(Left<2>{}, CLEAN_ROOM);
       const double* p = side ? c : b;
       for (int v = r.v0 + lane; v < r.v1; v += N) {
         const int at = verts + v - r.v0;
@@ -580,8 +588,8 @@ __device__ int clean_clip(G& g, const CleanIn<Hits>& in, CleanMem m, double* s_s
     rings += tr;
     verts += tv;
   }
-  if (rings > in.rcap) return CLEAN_NOT;
-  if (verts > in.vcap) return CLEAN_ROOM;
+  if (rings > in.rcap) return out(Left<2>{}, CLEAN_NOT);
+  if (verts > in.vcap) return out(Left<2>{}, CLEAN_ROOM);
   if (lane == 0) in.roff[rings] = verts;
   g.sync();
   g.phase();
