@@ -2096,11 +2096,12 @@ ClipArgs with_extras(ClipArgs a, const int* bnx, const int* cnx, const int* wide
 // The wide pairs' kernels run beside the small pairs', which share nothing with
 // them: neither fills the GPU for long in a mixed batch (1,500 pairs of polygons
 // with holes, 64 to 640 vertices, forward and backward: 786 us one after the
-// other, 605 so; 400 pairs of 8 to 700 vertices: 2.43 and 2.26 ms).
+// other, 605 so; 400 pairs of 8 to 700 vertices: 2.43 and 2.26 ms).  While
+// profiling one after the other, so that each launch's events time it alone.
 template <class Wide, class Small>
 void side_by_side(const BatchSide& side, bool wide, bool small, cudaStream_t st, Wide launch_wide,
                   Small launch_small) {
-  const bool both = wide && small && side.done;
+  const bool both = wide && small && side.done && !profiling_on();
   const cudaStream_t sw = both ? side.stream : st;
   if (both) {
     cudaEventRecord(side.go, st);

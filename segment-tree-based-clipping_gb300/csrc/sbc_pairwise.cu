@@ -1552,7 +1552,8 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
                 status, pl_.unite ? 1 : 0, nrings, nverts, pip, clean, pair_area, steps,
                 grouped, ca.raw, hbuf, (int*)hk};
   // The pairs that `which` picks, in cost order: blocks and warps side by side
-  // (on st2_ and st), joined on st.
+  // (on st2_ and st), joined on st.  While profiling one after the other, and
+  // done before the big pairs start, so that each launch's events time it alone.
   std::vector<int> hst(nov), list;
   h_clean_.assign(nov, 0);
   auto clip_pairs = [&](bool in_general_position, auto which, bool reserve) {
@@ -1572,8 +1573,9 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
       ::sbc::KProbe kp_("k_pw_inside", st);
       k_pw_inside<<<grid_for(32LL * n, 256), 256, 0, st>>>(pa, n, steps);
     }
+    const cudaStream_t s2 = profiling_on() ? st : st2_;
     cudaEventRecord(ev_[1], st);
-    cudaStreamWaitEvent(st2_, ev_[1], 0);
+    cudaStreamWaitEvent(s2, ev_[1], 0);
     auto launch = [&](const char* name, auto kernel, int block, size_t smem, int from, int to,
                       int per_block, bool leave, cudaStream_t s, int* q) {
       if (to <= from) return;
@@ -1593,14 +1595,15 @@ int PairwiseRunner::run(const double* d_bxy, int nb, int nov, const double* d_cx
       cudaFuncSetAttribute(large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       launch("k_pw_clean_huge", large, kPwHugeBlock, smem, 0, huge, 1, false, st, queue);
       launch("k_pw_clean_wide", k_pw_clean_wide<kPwWideBlock>, kPwWideBlock,
-             room * (kPwWideBlock / 32), huge, wide, 1, false, st2_, queue + 1);
+             room * (kPwWideBlock / 32), huge, wide, 1, false, s2, queue + 1);
       launch("k_pw_clean", k_pw_clean, kPwPairBlock, 0, wide, n, per, reserve, st, queue + 2);
     } else {
-      launch("k_pw_pairs_wide", k_pw_pairs_wide, kPwWideBlock, 0, 0, wide, 1, false, st2_, queue);
+      launch("k_pw_pairs_wide", k_pw_pairs_wide, kPwWideBlock, 0, 0, wide, 1, false, s2, queue);
       launch("k_pw_pairs", k_pw_pairs, kPwPairBlock, 0, wide, n, per, reserve, st, queue + 1);
     }
-    cudaEventRecord(ev_[1], st2_);
+    cudaEventRecord(ev_[1], s2);
     cudaStreamWaitEvent(st, ev_[1], 0);
+    if (profiling_on()) cudaStreamSynchronize(st);
     return true;
   };
   auto clean_of = [&](int p) {
