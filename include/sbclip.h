@@ -355,7 +355,9 @@ int sbc_batch_set_arena_budget(sbc_ctx* ctx, long long bytes);
 int sbc_batch_info(const sbc_ctx* ctx, long long* out, int n);
 /* Tuning knobs of the batch engine, shape[5]: block sizes (threads: 32, 64,
  * 96 or 128) of the per-pair front kernel, the warp-per-pair candidate
- * kernel, the per-pair back end and the backward kernel, then the small/large
+ * kernel, the thread-per-pair back end (which takes the pairs that neither the
+ * general-position kernels nor the warp back end do; tuned only where a batch
+ * has some left over) and the backward kernel, then the small/large
  * split (a pair with a polygon above it is clipped by the single-pair
  * pipeline; 3 to SBC_BATCH_MAX_VERTICES, default SBC_BATCH_MAX_VERTICES).
  * Results do not depend on them.  A graph (sbc_area_graph_create) needs a

@@ -2830,6 +2830,7 @@ int BatchRunner::run_chunk(int c, const double* d_bxy, const long long* d_boff,
       cudaMemcpyAsync(hs.data(), status + p0, sizeof(int) * n, cudaMemcpyDeviceToHost, st);
       if (cudaStreamSynchronize(st) != cudaSuccess) return pl_.fail(kECuda, "batch clip");
       if (round || std::find(hs.begin(), hs.end(), kPending) == hs.end()) return kOk;
+      lists_ran_ = true;
       launch_general(A, shape, in_bytes, st);
     }
   };
@@ -3016,7 +3017,7 @@ int BatchRunner::set_components(int np_, const long long* d_boff, const long lon
 
 int BatchRunner::forward(int np_, const double* d_bxy, const long long* d_boff,
                          const double* d_cxy, const long long* d_coff, cudaStream_t st) {
-  valid = false;
+  valid = lists_ran_ = false;
   ++generation;
   key_b = d_bxy;
   key_c = d_cxy;
@@ -3133,9 +3134,10 @@ int BatchRunner::backward(const double* d_bxy, const long long* d_boff, const do
 
 namespace sbc {
 
-// The batch autotuner: the block size of each of the four kernels, then the
-// small/large split, one knob at a time, each setting timed as forward +
-// backward (CUDA events on st, the better of two runs); a change is kept only
+// The batch autotuner: the block sizes of the kernels that have a choice (of
+// the thread back end's only where pairs of this batch were left to the lists),
+// then the small/large split, one knob at a time, each setting timed as forward
+// + backward (CUDA events on st, the better of two runs); a change is kept only
 // if it is faster.  A split below the batch's largest polygons is tried only
 // when it moves at most 64 pairs to the pair pipeline (each costs about a
 // millisecond there).  Results do not depend on any knob.
@@ -3168,6 +3170,7 @@ int BatchRunner::autotune(int np_, const double* d_bxy, const long long* d_boff,
   int rc = timed(&cur);
   int* knobs[4] = {&shape.front, &shape.cand, &shape.back, &shape.bwd};
   for (int i = 0; i < 4 && !rc; ++i) {
+    if (knobs[i] == &shape.back && !lists_ran_) continue;
     for (int b : {32, 64, 128}) {
       if (b == *knobs[i]) continue;
       const int keep = *knobs[i];

@@ -432,6 +432,7 @@ class BatchRunner {
   int* wide_item_ = nullptr;
   int nwide_ = 0, nitems_ = 0, wide_min_ = 0;
   bool any_wide_ = false;        // some pair of the batch is above the lower line
+  bool lists_ran_ = false;       // the last forward pass left pairs to the list-walking kernels
   BatchSide side_;
   unsigned char* arena[2] = {nullptr, nullptr};
   long long* aoff[2] = {nullptr, nullptr};
