@@ -181,7 +181,7 @@ KERNEL_BOUND = {
     "k_alpha_classify": "hbm", "k_cover_count": "latency", "k_alpha_sort_long": "latency",
     "k_lr_jump_coop": "latency", "k_tr_jump_coop": "latency",
     "k_grid_scatter": "hbm", "k_edge_fbox": "hbm", "k_copy_runs": "hbm",
-    "k_pair_exact": "fp64", "k_pw_cand_test": "fp64", "k_batch_cand": "fp64",
+    "k_pair_exact": "fp64", "k_pw_cand_test": "fp64", "k_batch_cand": "latency",
     "k_batch_cand_wide": "fp64", "k_labels": "fp64", "k_batch_backward": "fp64",
     "k_batch_backward_wide": "fp64", "k_batch_clean": "fp64", "k_batch_clean_wide": "fp64",
     "k_pw_clean": "fp64", "k_pw_clean_wide": "fp64", "k_pw_clean_huge": "latency",

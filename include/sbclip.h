@@ -186,7 +186,14 @@ int sbc_clip_batch_device(sbc_ctx* ctx, const sbc_batch* batch, sbc_batch_rings*
 
 /* Intersection area of every pair: the sum of the shoelace areas of its rings
  * (0 for pairs whose status is not SBC_OK).  area[npairs], status[npairs]
- * (status may be NULL).  Host arrays, or device arrays for _device. */
+ * (status may be NULL).  Host arrays, or device arrays for _device.
+ * The same batch gives the same bits every time (but for the gradients of
+ * pairs that the single-pair pipeline clips, whose terms are added as they
+ * come).  The order in which a pair's terms are added depends on what clips it,
+ * a warp or a block, and with more than 1,024 pairs above 4,096 edge pairs a
+ * batch clips those up to 16,384 on warps, otherwise on blocks: such a pair's
+ * area and gradient may differ in the last bits from one batch to another.  Its
+ * rings never do. */
 int sbc_area_forward(sbc_ctx* ctx, const sbc_batch* batch, double* area, int* status,
                      void* stream);
 int sbc_area_forward_device(sbc_ctx* ctx, const sbc_batch* batch, double* area, int* status,

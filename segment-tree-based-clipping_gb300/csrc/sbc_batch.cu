@@ -49,7 +49,9 @@ constexpr int kBatchBlock = 128;
 // of the batch are above that, else kWideMin[1]): a batch of many pairs of one
 // size fills the GPU with warps and does the least work so (pairs of 64 to
 // 127 vertices, forward and backward: 4,000 take 1.32 ms on warps and 2.1 on
-// blocks, 1,000 take 0.79 and 0.67, 128 take 0.64 and 0.34).  At 1,024 edge
+// blocks, 1,000 take 0.79 and 0.67, 128 take 0.64 and 0.34).  So the last bits
+// of such a pair's area and gradient, sums that a warp and a block take in
+// different orders, depend on the batch that it is in.  At 1,024 edge
 // pairs blocks gained nothing (512 pairs of 4 to 64 vertices: 0.37 ms on
 // warps, 0.47 on blocks).  Blocks of 64 and 128 threads were slower
 // on the largest pairs (the 12,000 pairs: 69.6 and 50.8 ms).
@@ -1337,7 +1339,7 @@ __device__ PairResult clip_pair_back2(const double* b, int nb, const double* c, 
 // The pair's area: the sum over its rings of the shoelace, one warp per pair
 // (FP64 products at the full warp rather than on one thread of each warp);
 // the lanes' partial sums combine in a fixed order, so the area does not
-// depend on how the batch was cut into chunks.
+// depend on how the batch was cut into chunks.  (A block sums in another order.)
 __device__ double pair_area_warp(const int* roff, const double* rxy, int nr, int lane) {
   double area = 0.0;
   for (int r = 0; r < nr; ++r) {
@@ -2077,8 +2079,6 @@ __global__ void k_graph_passes(int n, const int* __restrict__ pass, const int* _
   pass1[p] = pass[p] == 1 ? 1 : -1;
 }
 
-// block sizes (threads) of the three kernels: tuning knobs, each at most
-// kBatchBlock (128) and a multiple of 32
 // the batch's component successors (null: one ring per polygon) and the
 // chunk's wide pairs
 ClipArgs with_extras(ClipArgs a, const int* bnx, const int* cnx, const int* wide,
@@ -2265,10 +2265,12 @@ __device__ bool backward_none(G& g, const BackArgs& A, int p, int nb, int nc) {
 // polygons' own vertices.  In each round the lanes naming the same
 // vertex form a group (match_any) whose lowest lane sums their values in lane
 // order and adds the sum: every gradient entry is summed in an order fixed by
-// the rings alone, whatever the launch shape.  Bound by FP64, which costs a
-// warp the same for one lane as for 32: 65,536 pairs of 4 to 64 vertices took
-// 0.40 ms ring by ring, few of which fill a warp, 0.36 over all rings with
-// crossings and vertices mixed, 0.32 so (0.44 by the wide pairs' gather).
+// the rings, whatever the launch shape (k_batch_backward_wide has another one,
+// and whether a pair is wide depends on how many of its batch are).  Bound by
+// FP64, which costs a warp the same for one lane as for 32: 65,536 pairs of 4 to
+// 64 vertices took 0.40 ms ring by ring, few of which fill a warp, 0.36 over all
+// rings with crossings and vertices mixed, 0.32 so (0.44 by the wide pairs'
+// gather).
 __global__ void __launch_bounds__(128, 8) k_batch_backward(BackArgs A) {
   const int lane = threadIdx.x & 31;
   const int p = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);

@@ -1,6 +1,6 @@
-// sbc_pairops.cuh -- per-pair device helpers shared by the engines that clip
-// one pair per device thread: the batched small-pair engine (sbc_batch.cu)
-// and the one-base-many-overlays engine (sbc_pairwise.cu).
+// sbc_pairops.cuh -- per-pair device helpers shared by the batched pair engine
+// (sbc_batch.cu), the one-base-many-overlays engine (sbc_pairwise.cu) and the
+// pair pipeline's general-position stage (sbc_general.cu).
 #pragma once
 
 #include "sbc_internal.cuh"

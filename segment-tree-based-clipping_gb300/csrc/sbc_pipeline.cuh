@@ -342,8 +342,8 @@ int run_backend(Pipeline& pl, const Merged& m, OverlayOut& out);
 int clean_up_rings(Pipeline& pl, OverlayOut& out);
 
 // Many independent pairs (sbc_batch.cu): pairs whose polygons have at most
-// SBC_BATCH_MAX_VERTICES vertices one device thread each, in chunks whose
-// arenas fit a memory budget; larger pairs through the Pipeline with a
+// SBC_BATCH_MAX_VERTICES vertices on a warp or, if wide, a block each, in chunks
+// whose arenas fit a memory budget; larger pairs through the Pipeline with a
 // provenance tape.  The forward pass keeps the last chunk's rings and tapes
 // resident for rings() and backward(); other chunks are recomputed there.
 // block sizes of the batch engine's kernels (tuning knobs: results do not
