@@ -673,11 +673,14 @@ k_direct_groups(int gB, int gC0, int gC, int chunks, const float4* __restrict__ 
 // counters and ranks as in k_pair_exact, and [2] box-overlapping edge pairs,
 // [4] edge pairs tested, [5] listed group pairs.  Overlay edge j is edge c0 + j
 // from vertex v0 + j.  Of either group only the edges that reach the other's
-// box are tested; the pairs that pass each filter are queued, and the next one
-// runs when there are 32: a few lanes in LSMF and the float test cost the issue
-// slots of all (100,000 x 80,000 jagged vertices, 321,000 group pairs, 235,000
-// hits: 823 us with every edge against every other and no first queue, 500
-// with the edges that reach the box, 380 so).
+// box are tested; the pairs whose boxes meet are listed, and LSMF and the float
+// test take them 32 at a time from the groups' vertices in shared memory: a few
+// lanes in them cost the issue slots of all.  Bound by issue and the latency of
+// a group pair's loads.  100,000 x 80,000 jagged vertices (321,000 group pairs,
+// 235,000 hits): 860 us with every edge against every other and the tests as
+// they come, 500 with the edges that reach the box, 370 so; spokes of 20,000 x
+// 20,000, most of whose groups meet, 670, and 730 so (850 with the pairs of
+// several groups queued and their vertices gathered).
 __global__ void __launch_bounds__(128)
 k_direct_exact(int nb, int c0, int v0, int nc, const int2* __restrict__ list, long long list_cap,
                const float4* __restrict__ fbox, const float4* __restrict__ gboxB,
@@ -689,32 +692,19 @@ k_direct_exact(int nb, int c0, int v0, int nc, const int2* __restrict__ list, lo
                const unsigned* __restrict__ ranks, unsigned long long* __restrict__ counters,
                long long cap, int* __restrict__ rb, int* __restrict__ rc, int* __restrict__ rt,
                unsigned long long* __restrict__ rkey, double2* __restrict__ rab) {
-  __shared__ int2 s_near[4][64], s_q[4][64];  // past the boxes, past the float test
+  __shared__ unsigned short s_near[4][1024];  // lane | overlay edge << 5, past the boxes
+  __shared__ int2 s_q[4][64];                 // past the float test
   __shared__ float4 s_box[4][32];
+  __shared__ float4 s_vf[4][2][33];  // the groups' vertices: base, overlay
+  __shared__ longlong2 s_key[4][2][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
   const float inf = __int_as_float(0x7f800000);
   const long long items = min((long long)counters[5], list_cap);
   if (no_tree(ranks)) return;
-  int nnear = 0, nq = 0;
+  int nq = 0;
   unsigned long long raw = 0;
   unsigned tested = 0, boxes = 0, work = 0;
-  // appends; true: 32 or more are waiting
-  auto push = [&](int2* q, int& n, bool put, int2 e) {
-    const unsigned m = __ballot_sync(0xffffffffu, put);
-    if (put) q[n + __popc(m & lt)] = e;
-    n += __popc(m);
-    __syncwarp();
-    return n >= 32;
-  };
-  // drops the first 32
-  auto shift = [&](int2* q, int& n) {
-    n -= 32;
-    const int2 x = lane < n ? q[32 + lane] : make_int2(0, 0);
-    __syncwarp();
-    if (lane < n) q[lane] = x;
-    __syncwarp();
-  };
   auto classify = [&](int count) {
     bool hit = false;
     int2 e = make_int2(0, 0);
@@ -750,51 +740,69 @@ k_direct_exact(int nb, int c0, int v0, int nc, const int2* __restrict__ list, lo
     }
     __syncwarp();
   };
-  auto test = [&](int count) {
-    bool keep = false;
-    int2 e = make_int2(0, 0);
-    if (lane < count) {
-      e = s_near[w][lane];
-      const longlong2* kb = (const longlong2*)bK + e.x;
-      const longlong2* kc = (const longlong2*)cK + v0 + e.y;
-      const longlong2 b1 = kb[0], b2 = kb[1], c1 = kc[0], c2 = kc[1];
-      const float4 p1 = vfB[e.x], p2 = vfB[e.x + 1], q1 = vfC[v0 + e.y], q2 = vfC[v0 + e.y + 1];
-      if (lsmf_keys(b1.x, b1.y, b2.x, b2.y, c1.x, c1.y, c2.x, c2.y)) {
-        ++tested;
-        keep = !certainly_disjoint(p1, p2, q1, q2);
-      }
-    }
-    if (push(s_q[w], nq, keep, e)) {
-      classify(32);
-      shift(s_q[w], nq);
+  // vertices [v, v + n] of a polygon into shared memory, lane by lane
+  auto stage = [&](int side, const float4* vf, const long long* key, int v, int n) {
+    for (int k = lane; k <= n; k += 32) {
+      s_vf[w][side][k] = vf[v + k];
+      s_key[w][side][k] = ((const longlong2*)key)[v + k];
     }
   };
   for (long long i = (long long)blockIdx.x * 4 + w; i < items; i += 4LL * gridDim.x) {
     const int2 pair = list[i];
-    const int be = pair.x * 32 + lane, j0 = pair.y * 32, n = min(32, nc - j0);
+    const int b0 = pair.x * 32, j0 = pair.y * 32, nbe = min(32, nb - b0), n = min(32, nc - j0);
     const float4 gb = gboxB[pair.x], gc = gboxC[pair.y];
     float4 fb = make_float4(inf, inf, -inf, -inf), fc = fb;
-    if (be < nb) fb = fbox[be];
+    if (lane < nbe) fb = fbox[b0 + lane];
     if (lane < n) fc = fbox[c0 + j0 + lane];
-    const bool on = be < nb && boxes_touch(fb, gc);
+    const bool on = lane < nbe && boxes_touch(fb, gc);
     unsigned left = __ballot_sync(0xffffffffu, lane < n && boxes_touch(fc, gb));
     if (!__any_sync(0xffffffffu, on)) continue;
     if (on) work += __popc(left);
     s_box[w][lane] = fc;
     __syncwarp();
+    int near = 0;
     for (; left; left &= left - 1) {
       const int t = __ffs(left) - 1;
-      const bool near = on && boxes_touch(fb, s_box[w][t]);
-      if (!__any_sync(0xffffffffu, near)) continue;
-      boxes += near;
-      if (push(s_near[w], nnear, near, make_int2(be, j0 + t))) {
-        test(32);
-        shift(s_near[w], nnear);
+      const bool meet = on && boxes_touch(fb, s_box[w][t]);
+      const unsigned m = __ballot_sync(0xffffffffu, meet);
+      if (meet) s_near[w][near + __popc(m & lt)] = (unsigned short)(lane | t << 5);
+      near += __popc(m);
+    }
+    if (near == 0) continue;
+    if (lane == 0) boxes += near;
+    stage(0, vfB, bK, b0, nbe);
+    stage(1, vfC, cK, v0 + j0, n);
+    __syncwarp();
+    for (int k0 = 0; k0 < near; k0 += 32) {
+      bool keep = false;
+      int2 e = make_int2(0, 0);
+      if (k0 + lane < near) {
+        const int x = s_near[w][k0 + lane], l = x & 31, t = x >> 5;
+        e = make_int2(b0 + l, j0 + t);
+        const longlong2 b1 = s_key[w][0][l], b2 = s_key[w][0][l + 1];
+        const longlong2 c1 = s_key[w][1][t], c2 = s_key[w][1][t + 1];
+        if (lsmf_keys(b1.x, b1.y, b2.x, b2.y, c1.x, c1.y, c2.x, c2.y)) {
+          ++tested;
+          keep = !certainly_disjoint(s_vf[w][0][l], s_vf[w][0][l + 1], s_vf[w][1][t],
+                                     s_vf[w][1][t + 1]);
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (!m) continue;
+      if (keep) s_q[w][nq + __popc(m & lt)] = e;
+      nq += __popc(m);
+      __syncwarp();
+      if (nq >= 32) {
+        classify(32);
+        nq -= 32;
+        const int2 x = lane < nq ? s_q[w][32 + lane] : make_int2(0, 0);
+        __syncwarp();
+        if (lane < nq) s_q[w][lane] = x;
+        __syncwarp();
       }
     }
     __syncwarp();
   }
-  if (nnear > 0) test(nnear);
   if (nq > 0) classify(nq);
   for (int o = 16; o > 0; o >>= 1) raw += __shfl_xor_sync(0xffffffffu, raw, o);
   tested = __reduce_add_sync(0xffffffffu, tested);
