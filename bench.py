@@ -201,19 +201,19 @@ KERNEL_BOUND = {
 _BATCH_NCU = "profiles/k_batch_small_pairs_8192.md (8,192 pairs, the same kernel)"
 PIPES = {
     ("k_batch_clean", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 54.8, "warps_active_pct": 27.9, "issue_active_pct": 27.6,
-        "stall_cycles_per_issue": {"long_scoreboard": 2.8, "no_instruction": 0.7, "wait": 3.4},
+        "fp64_pipe_pct_active": 54.3, "warps_active_pct": 27.8, "issue_active_pct": 26.2,
+        "stall_cycles_per_issue": {"long_scoreboard": 2.7, "no_instruction": 0.8, "wait": 3.4},
         "source": _BATCH_NCU},
     ("k_batch_cand", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 23.7, "warps_active_pct": 39.3, "issue_active_pct": 29.3,
+        "fp64_pipe_pct_active": 23.6, "warps_active_pct": 39.4, "issue_active_pct": 28.7,
         "stall_cycles_per_issue": {"long_scoreboard": 6.2, "no_instruction": 0.3, "wait": 3.5},
         "source": _BATCH_NCU},
     ("k_batch_front", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 29.5, "warps_active_pct": 36.1, "issue_active_pct": 50.9,
-        "stall_cycles_per_issue": {"long_scoreboard": 1.8, "no_instruction": 0.9, "wait": 2.7},
+        "fp64_pipe_pct_active": 34.2, "warps_active_pct": 35.4, "issue_active_pct": 49.1,
+        "stall_cycles_per_issue": {"long_scoreboard": 1.9, "no_instruction": 0.4, "wait": 3.0},
         "source": _BATCH_NCU},
     ("k_batch_backward", "small_pairs_65536"): {
-        "fp64_pipe_pct_active": 68.6, "warps_active_pct": 39.8, "issue_active_pct": 18.8,
+        "fp64_pipe_pct_active": 68.3, "warps_active_pct": 39.7, "issue_active_pct": 18.5,
         "stall_cycles_per_issue": {"long_scoreboard": 5.7, "no_instruction": 0.3, "wait": 4.0},
         "source": _BATCH_NCU},
 }
